@@ -246,8 +246,30 @@ retention_chunk_out_kernel(const float* __restrict__ qk, const T* __restrict__ v
         s < n ? load4(v + (t0 + s) * v_ld + (long long)h * V + cc) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
-  // keys behind a row's own group of 16 do not count
-  tile_product<4, 8>(acc, pt + r, LP, 0, bt + c, V, V / 2, min((n + 15) / 16 * 16, (r / 16 + 1) * 16));
+  // keys behind a row's own group of 16 do not count; of that group each row takes its own tokens alone: a weight of zero would
+  // let a value that is not finite into the tokens before it
+  const int own = r / 16 * 16;
+  tile_product<4, 8>(acc, pt + r, LP, 0, bt + c, V, V / 2, min((n + 15) / 16 * 16, own));
+  if (own < n) {
+    float part[4][8] = {};
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      float x[4], y[8];
+      *reinterpret_cast<float4*>(x) = load4(pt + (own + k) * LP + r);
+      *reinterpret_cast<float4*>(y) = load4(bt + (own + k) * V + c);
+      *reinterpret_cast<float4*>(y + 4) = load4(bt + (own + k) * V + c + V / 2);
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (own + k <= r + i) {
+#pragma unroll
+          for (int j = 0; j < 8; j++) part[i][j] = fmaf(x[i], y[j], part[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 8; j++) acc[i][j] += part[i][j];
+  }
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int t = r + i;

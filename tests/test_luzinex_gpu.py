@@ -617,3 +617,38 @@ def test_retention_over_chunks_and_of_one_token_each(lens, heads, dim, vdim, dty
             err = np.linalg.norm(got_o[t] - np.einsum("hdv,hd->hv", S, q[t]), axis=1)
             assert np.all(err < 2e-6 * size), (i, t)
         assert np.linalg.norm(got_s[slot] - S.ravel()) < 2e-6 * np.linalg.norm(S)
+
+
+@pytest.mark.parametrize("t,what", [(0, "v"), (17, "v"), (63, "v"), (64, "k"), (200, "v"), (299, "k"), (130, "q")])
+@pytest.mark.parametrize("dim,vdim,dtype", [(128, 64, "float32"), (64, 128, "bfloat16")])
+def test_retention_chunks_keep_what_is_not_finite_from_earlier_tokens(t, what, dim, vdim, dtype):
+    """A value, key or query that is NaN or infinite reaches its own token and later ones: earlier tokens of its group of 16, of its
+    chunk and of the portion keep their bits, and so does the other head."""
+    import torch
+    from types import SimpleNamespace
+    from mlxforge_b200.csrc import ops
+    rng = np.random.default_rng(t)
+    T, heads = 300, 2
+    qk = rng.standard_normal((T, 2 * heads * dim)).astype(np.float32) * np.float32(dim ** -0.25)
+    v = rng.standard_normal((T, heads * vdim)).astype(np.float32)
+    state = rng.standard_normal((1, heads * dim * vdim)).astype(np.float32)
+    i32 = lambda a: dev(np.asarray(a, np.int32))
+    batch = SimpleNamespace(q_len=[T], n_seqs=1, seq_q_start=i32([0]), seq_q_len=i32([T]), slots=i32([0]))
+    res = []
+    for bad in (None, np.nan, np.inf):
+        q2, v2 = qk.copy(), v.copy()
+        if bad is not None:
+            if what == "v":
+                v2[t, 3] = bad
+            else:
+                q2[t, 5 + (heads * dim if what == "k" else 0)] = bad
+        st, o, vd = dev(state), torch.full((1, T, heads * vdim), float("nan"), device="cuda"), dev(v2, tdt(dtype))
+        chunks = ops.retention_chunks(batch, heads, dim, vdim, vd, heads * vdim, st)
+        assert chunks == 5
+        ops.retention_chunked(dev(q2), vd, heads * vdim, dev(np.array([0.97, 0.5], np.float32)), st, batch, o, heads, dim, vdim,
+                              chunks, torch.empty(chunks * heads * dim * vdim, device="cuda"))
+        res.append(o[0])
+    for o in res[1:]:
+        assert torch.equal(o[:t], res[0][:t])
+        assert not torch.isfinite(o[t]).all()
+        assert torch.equal(o[:, vdim:], res[0][:, vdim:])
