@@ -191,7 +191,7 @@ delta_runs_kernel(const float* __restrict__ qkv, const float* __restrict__ beta,
 #pragma unroll
     for (int i = 0; i < R; i++) Tm[i][c] = x[i];
   } else {
-    // meanwhile the rest writes what is done: B (zero where s > t), G_R and Kt
+    // meanwhile the rest writes what is done: B (what stands at s > t is not read)
     for (int i = c - R; i < R * R; i += D - R) out_b[i] = AB[1][i / R][i % R];
   }
   float kh[R], w[R], qh[R];
@@ -404,7 +404,8 @@ delta_state_kernel(const float* __restrict__ runs, float* __restrict__ state, lo
         const float* u_s = U_s + (run & 1) * R * NC;
         bar_wait(bar0 + 8 * (run % STAGES), (run / STAGES) & 1, status);
         product(op + D * R, S_s + (run % 3) * D * NC);
-        // B U while the partial sums are on their way
+        // B U while the partial sums are on their way, each row over its own tokens and the ones before: a zero of B would let
+        // what is not finite of a later token into it
         float x[PER];
 #pragma unroll
         for (int j = 0; j < PER; j++) x[j] = 0.f;
@@ -417,7 +418,8 @@ delta_state_kernel(const float* __restrict__ runs, float* __restrict__ state, lo
           for (int k = 0; k < 4; k++) {
             get(u, u_s + (s + k) * NC + pc);
 #pragma unroll
-            for (int j = 0; j < PER; j++) x[j] = fmaf(b[k], u[j], x[j]);
+            for (int j = 0; j < PER; j++)
+              if (s + k <= pr) x[j] = fmaf(b[k], u[j], x[j]);
           }
         }
         asm volatile("bar.sync 2, 128;\n" ::: "memory");

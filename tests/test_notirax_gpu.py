@@ -812,3 +812,38 @@ def test_delta_step_against_the_rule(n, heads, n_kv, dim, vdim):
         assert np.linalg.norm(got - want) < 1e-6 * np.linalg.norm(S) / np.sqrt(dim)
         assert np.linalg.norm(host(st[slots[t], :heads * dim * vdim]).reshape(S.shape) - S) < 1e-6 * np.linalg.norm(S)
     assert np.array_equal(st[:, heads * dim * vdim:].cpu().numpy(), state[:, heads * dim * vdim:])
+
+
+@pytest.mark.parametrize("t,what", [(0, "v"), (5, "v"), (15, "k"), (16, "v"), (40, "g"), (62, "k"), (30, "q"), (33, "b")])
+@pytest.mark.parametrize("dim,vdim,heads", [(128, 32, 2), (64, 64, 80)])
+def test_delta_runs_keep_what_is_not_finite_from_earlier_tokens(t, what, dim, vdim, heads):
+    """As for the retention's chunks: what is not finite at a token (of any operand) reaches neither the tokens before it, those of its
+    own run of 16 among them, nor the other heads; blocks of 8 and of 16 columns."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    rng = np.random.default_rng(t)
+    T, f = 63, lambda *s: rng.standard_normal(s).astype(np.float32)
+    C = 2 * heads * dim + heads * vdim
+    qkv, beta, ag, state = f(T, C), rng.random((T, heads)).astype(np.float32), rng.random((T, heads * dim)).astype(np.float32), f(1, heads * dim * vdim)
+    qkv[:, :2 * heads * dim] *= dim ** -0.5
+    i32 = lambda a: dev(np.asarray(a, np.int32))
+    batch = SimpleNamespace(q_len=[T], n_seqs=1, seq_q_start=i32([0]), seq_q_len=i32([T]), slots=i32([0]))
+    runs, floats = ops.delta_runs(batch, heads, dim, vdim)
+    res = []
+    for bad in (None, np.nan, np.inf):
+        x, g, b = qkv.copy(), ag.copy(), beta.copy()
+        if bad is not None:
+            if what == "g":
+                g[t, 7] = bad
+            elif what == "b":
+                b[t, 0] = bad
+            else:
+                x[t, {"q": 0, "k": heads * dim, "v": 2 * heads * dim}[what] + 3] = bad
+        st, o = dev(state), torch.full((T, heads * vdim), float("nan"), device="cuda")
+        ops.delta_recurrence_runs(dev(x), dev(b), dev(g), st, batch, o, heads, heads, dim, vdim, runs, torch.empty(floats, device="cuda"))
+        res.append(o)
+    ops.check_kernel_status()
+    for o in res[1:]:
+        assert torch.equal(o[:t], res[0][:t])
+        assert not torch.isfinite(o[t]).all()
+        assert torch.equal(o[:, vdim:], res[0][:, vdim:])
