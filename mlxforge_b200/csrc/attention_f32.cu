@@ -31,6 +31,11 @@ struct F32Args {
 
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
+// whether the query at `pos` (-1: none) sees `key`
+__device__ __forceinline__ bool sees(const F32Args& a, int pos, int key) {
+  return key <= pos && (a.window <= 0 || pos - key < a.window || key < a.keep_first);
+}
+
 // N floats in pieces of up to four from p on, pieces `step` apart
 template <int N>
 __device__ __forceinline__ void get(float (&x)[N], const float* p, int step) {
@@ -117,14 +122,16 @@ attention_f32_kernel(const F32Args a) {
       float* dst = kt + d * KT + (key ^ quad * 8);
       dst[0] = x.x; dst[KT] = x.y; dst[2 * KT] = x.z; dst[3 * KT] = x.w;
     }
+    bool odd = false;                              // a value that is not finite
     for (int i = tid; i < KT * VW / 4; i += 128) {
       const int key = i / (VW / 4), c = i % (VW / 4) * 4, j = k0 + key;
       float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < a.vd && j <= last && (j >= lo || j < keep))
         x = load4(a.v_pool + paged_offset(a.pv, seq, j, kvh) / hd * a.v_ld + c);
       *reinterpret_cast<float4*>(vs + key * VW + c) = x;
+      odd |= !(fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + fabsf(x.w) < INFINITY);
     }
-    __syncthreads();
+    odd = __syncthreads_or(odd);
     float s[RPT][CPT];
 #pragma unroll
     for (int i = 0; i < RPT; i++)
@@ -165,8 +172,7 @@ attention_f32_kernel(const F32Args a) {
         const int key = k0 + c0 + (j & 3) + (j >> 2) * CSTEP;
         float x = s[i][j] * a.scale;
         if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
-        const bool seen = key <= pos[i] && (a.window <= 0 || pos[i] - key < a.window || key < a.keep_first);
-        s[i][j] = seen ? x : -INFINITY;
+        s[i][j] = sees(a, pos[i], key) ? x : -INFINITY;
         top = fmaxf(top, s[i][j]);
       }
 #pragma unroll
@@ -201,15 +207,35 @@ attention_f32_kernel(const F32Args a) {
     for (int v = 0; v < VC; v++) {
       for (int j0 = 0; j0 < keys; j0 += 16) {
         float part[RPT][CPT];
-#pragma unroll
-        for (int key = 0; key < 16; key++) {
-          float x[RPT], y[CPT];
-          get(x, pt + (j0 + key) * RP + r0, 0);
-          get(y, vs + (j0 + key) * VW + v * 64 + c0, CSTEP);
+        if (odd) {
+          // each row takes the keys that it sees alone: a weight of zero would let such a value into the others
 #pragma unroll
           for (int i = 0; i < RPT; i++)
 #pragma unroll
-            for (int j = 0; j < CPT; j++) part[i][j] = key == 0 ? x[i] * y[j] : fmaf(x[i], y[j], part[i][j]);
+            for (int j = 0; j < CPT; j++) part[i][j] = 0.f;
+#pragma unroll 1
+          for (int key = 0; key < 16; key++) {
+            float x[RPT], y[CPT];
+            get(x, pt + (j0 + key) * RP + r0, 0);
+            get(y, vs + (j0 + key) * VW + v * 64 + c0, CSTEP);
+#pragma unroll
+            for (int i = 0; i < RPT; i++)
+              if (sees(a, pos[i], k0 + j0 + key)) {
+#pragma unroll
+                for (int j = 0; j < CPT; j++) part[i][j] = fmaf(x[i], y[j], part[i][j]);
+              }
+          }
+        } else {
+#pragma unroll
+          for (int key = 0; key < 16; key++) {
+            float x[RPT], y[CPT];
+            get(x, pt + (j0 + key) * RP + r0, 0);
+            get(y, vs + (j0 + key) * VW + v * 64 + c0, CSTEP);
+#pragma unroll
+            for (int i = 0; i < RPT; i++)
+#pragma unroll
+              for (int j = 0; j < CPT; j++) part[i][j] = key == 0 ? x[i] * y[j] : fmaf(x[i], y[j], part[i][j]);
+          }
         }
 #pragma unroll
         for (int i = 0; i < RPT; i++)

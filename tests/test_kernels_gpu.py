@@ -1010,3 +1010,35 @@ def test_prefill_options_on_tcgen05(form):
                              v_ld, keep, sink, gate, gate_ld)
     assert torch.isfinite(want).all()
     assert (got.float() - want.float()).abs().max() < 2.0 ** -7 * want.float().abs().max()
+
+
+@pytest.mark.parametrize("hd,vd,rep,window,keep,n,t", [(64, 64, 2, 0, 0, 70, 20), (64, 64, 2, 0, 0, 70, 69), (32, 128, 1, 16, 0, 90, 40), (128, 192, 3, 20, 5, 100, 3),
+                                                  (128, 192, 3, 20, 5, 100, 6), (40, 256, 8, 0, 0, 2, 1)])
+def test_attention_f32_keeps_unseen_values_out(hd, vd, rep, window, keep, n, t):
+    """Keys and values that are NaN or infinite stay out of the rows that do not see them (later ones, outside the window, not kept),
+    whose bits do not change, and reach all others; both heights of a tile."""
+    import torch
+    from types import SimpleNamespace
+    from mlxforge_b200.csrc import ops
+    rng = np.random.default_rng(hd)
+    kv, page, i32 = 2, 16, lambda a: dev(np.asarray(a, np.int32))
+    heads, blocks = kv * rep, -(-n // 16)
+    q = dev(rng.standard_normal((n, heads * hd)).astype(np.float32))
+    k, v = (rng.standard_normal((blocks, kv, page, d)).astype(np.float32) for d in (hd, vd))
+    batch = SimpleNamespace(seq_q_start=i32([0]), seq_q_len=i32([n]), seq_ctx_len=i32([n]), q_len=[n], n_seqs=1)
+    table = i32([np.arange(blocks)])
+    res = []
+    for bad in (None, np.nan, np.inf):
+        k2, v2 = k.copy(), v.copy()
+        if bad is not None:
+            v2[t // page, :, t % page] = bad
+            k2[t // page, :, t % page, 0] = bad
+        o = torch.full((n, heads * vd), float("nan"), device="cuda")
+        ops.attention_f32(q, dev(k2), dev(v2), o, batch, table, page, heads, kv, hd, hd ** -0.5, window, vd, vd, keep)
+        res.append(o)
+    pos = np.arange(n)
+    sees = (pos >= t) & ((window == 0) | (pos - t < window) | (t < keep))
+    for o in res[1:]:
+        blind = torch.from_numpy(~sees).cuda()
+        assert torch.equal(o[blind], res[0][blind])
+        assert not torch.isfinite(o[~blind]).all(dim=1).any()
