@@ -179,14 +179,17 @@ attention_f32_kernel(const F32Args a) {
       for (int w = 1; w < CG; w <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, w));
       top = fmaxf(top, m[i]);
       const float fade = m[i] == -INFINITY ? 0.f : expf(m[i] - top);
-      float sum = 0.f;
+      // the row's sum in one order for either height of a tile, so that it does not depend on what else is in the step: four
+      // neighbouring keys, then the two groups 32 keys apart (a lane's own, or eight lanes apart), then the lanes
+      float four[CPT / 4];
 #pragma unroll
       for (int j = 0; j < CPT; j++) {
         s[i][j] = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - top);
-        sum += s[i][j];
+        four[j / 4] = j % 4 == 0 ? s[i][j] : four[j / 4] + s[i][j];
       }
+      float sum = CPT > 4 ? four[0] + four[CPT / 4 - 1] : four[0] + __shfl_xor_sync(0xffffffffu, four[0], 8);
 #pragma unroll
-      for (int w = 1; w < CG; w <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+      for (int w = 1; w < 8; w <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
       l[i] = l[i] * fade + sum;
       m[i] = top;
 #pragma unroll

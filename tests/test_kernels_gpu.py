@@ -1042,3 +1042,28 @@ def test_attention_f32_keeps_unseen_values_out(hd, vd, rep, window, keep, n, t):
         blind = torch.from_numpy(~sees).cuda()
         assert torch.equal(o[blind], res[0][blind])
         assert not torch.isfinite(o[~blind]).all(dim=1).any()
+
+
+def test_attention_f32_a_token_alone_and_beside_a_portion():
+    """Single tokens of several sequences have the same bits in a step of their own (tiles of 16 rows) and beside a portion of 100
+    tokens (tiles of 64)."""
+    import torch
+    from types import SimpleNamespace
+    from mlxforge_b200.csrc import ops
+    rng = np.random.default_rng(1)
+    kv, rep, hd, page, i32 = 2, 4, 64, 16, lambda a: dev(np.asarray(a, np.int32))
+    heads, ctx = kv * rep, [700, 1, 333, 100]
+    blocks = [-(-c // page) for c in ctx]
+    k, v = (dev(rng.standard_normal((sum(blocks), kv, page, hd)).astype(np.float32)) for _ in range(2))
+    table, at = np.full((len(ctx), max(blocks)), -1, np.int32), 0
+    for i, b in enumerate(blocks):
+        table[i, :b], at = np.arange(at, at + b), at + b
+    q = dev(rng.standard_normal((3 + 100, heads * hd)).astype(np.float32))
+    out = []
+    for lens in ([1, 1, 1], [1, 1, 1, 100]):
+        n = len(lens)
+        batch = SimpleNamespace(seq_q_start=i32([0, 1, 2, 3][:n]), seq_q_len=i32(lens), seq_ctx_len=i32(ctx[:n]), q_len=lens, n_seqs=n)
+        o = torch.full((sum(lens), heads * hd), float("nan"), device="cuda")
+        ops.attention_f32(q, k, v, o, batch, dev(table), page, heads, kv, hd, hd ** -0.5, 0, hd, hd)
+        out.append(o[:3])
+    assert torch.equal(out[0], out[1])
