@@ -67,6 +67,7 @@ _SIGNATURES = {
                          c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],
     "mf_delta_gates": [_P, _P, _P, c_int, c_int, c_int, c_int, _P],
     "mf_delta_recurrence": [_P, _P, _P, c_int, _P, c_longlong, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P],
+    "mf_delta_step_ok": [c_int, c_int],
     "mf_delta_runs_ok": [c_int, c_int],
     "mf_delta_runs_scratch": [c_longlong, c_int, c_int, c_int],
     "mf_delta_recurrence_runs": [_P, _P, _P, c_int, _P, c_longlong, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int,

@@ -615,6 +615,9 @@ MF_API int mf_delta_gates(float* ag, const float* a_log, const float* dt_bias, i
                            n_heads * dim, dim, width);
 }
 
+// Whether a step of one token a sequence has a kernel of its own for these sizes.
+MF_API int mf_delta_step_ok(int dim, int vdim) { return (dim == 64 || dim == 128) && vdim > 0 && vdim % 32 == 0; }
+
 // `one_each`: every sequence brings exactly one token.
 MF_API int mf_delta_recurrence(const float* qkv, const float* beta, const float* ag, int ag_ld, float* state,
                                long long state_stride, const int* seq_q_start, const int* seq_q_len, const int* slots,
@@ -624,7 +627,7 @@ MF_API int mf_delta_recurrence(const float* qkv, const float* beta, const float*
   if (dim <= 0 || dim > 32 * DR_LANES || n_kv <= 0 || n_heads % n_kv || n_heads > 65535) return MF_ERR_BAD_ARG;
   dim3 grid(n_seqs, n_heads, (vdim + DR_COLS - 1) / DR_COLS);
   mf_count(MF_K_DELTA_RECURRENCE);
-  if (one_each && (dim == 64 || dim == 128) && vdim % 32 == 0) {
+  if (one_each && mf_delta_step_ok(dim, vdim)) {
     const dim3 step_grid(n_seqs, n_heads, vdim / 32);
     return (int)launch_dep(dim == 64 ? delta_step_kernel<64> : delta_step_kernel<128>, step_grid, dim3(128), 0, stream, qkv, beta,
                            ag, ag_ld, state, state_stride, seq_q_start, slots, o_out, n_heads, n_kv, vdim);

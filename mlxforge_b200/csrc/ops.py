@@ -7,6 +7,7 @@ from __future__ import annotations
 
 from ctypes import c_void_p
 from functools import lru_cache
+from types import SimpleNamespace
 from typing import NamedTuple, Optional
 
 import torch
@@ -358,6 +359,28 @@ def set_retention_rows(rows: int) -> None:
     """Rows of the state per block of the staged recurrence kernel (16, 32 or 64; for tests and measurements).
     Results do not depend on it beyond the order in which the row groups' partial read-outs are added."""
     check(library().mf_set_retention_rows(rows), "set_retention_rows", launches=0)
+
+
+def sequence_groups(batch, kind, cost=None, limit: int = 0):
+    """The step's sequences in groups of neighbours that ``kind(tokens)`` names alike, as ``(kind, batch, first token, end)``
+    with a batch of the group's own sequences.  Kernels that are chosen by the length of a portion are given a group each, so that
+    a sequence's numbers are a matter of its own tokens and not of what else is in the step.  Sequences without a token are left
+    out.  ``cost(tokens)``: a group ends where its costs would add up to more than ``limit``."""
+    groups, t = [], 0                 # [kind, first sequence, end, first token, end, cost]
+    for i, n in enumerate(batch.q_len):
+        if n:
+            k, c = kind(n), cost(n) if cost else 0
+            g = groups[-1] if groups else None
+            if g is None or g[0] != k or g[2] != i or g[5] + c > limit:
+                groups.append([k, i, i + 1, t, t + n, c])
+            else:
+                g[2], g[4], g[5] = i + 1, t + n, g[5] + c
+            t += n
+    if len(groups) == 1 and groups[0][2] - groups[0][1] == batch.n_seqs:
+        return [(groups[0][0], batch, 0, t)]
+    return [(k, SimpleNamespace(q_len=batch.q_len[a:b], n_seqs=b - a, seq_q_start=batch.seq_q_start[a:b],
+                                seq_q_len=batch.seq_q_len[a:b], slots=batch.slots[a:b]), t0, t1)
+            for k, a, b, t0, t1, _ in groups]
 
 
 def _retention_step(batch, dim: int, vdim: int) -> bool:
@@ -855,14 +878,38 @@ DELTA_RUNS_MIN_TOKENS = 48
 DELTA_RUNS_MAX_FLOATS = 1 << 28
 
 
+@lru_cache(maxsize=None)
+def _delta_sizes(n_heads: int, dim: int, vdim: int):
+    """(whether one token has a kernel of its own, floats of scratch per run of tokens or 0 where runs do not take these sizes)"""
+    lib = library()
+    return (bool(lib.mf_delta_step_ok(dim, vdim)),
+            int(lib.mf_delta_runs_scratch(1, n_heads, dim, vdim)) if lib.mf_delta_runs_ok(dim, vdim) else 0)
+
+
+def delta_groups(batch, n_heads: int, dim: int, vdim: int):
+    """``sequence_groups`` of the delta rule: ``"one"`` token (the step kernel, where it takes the sizes) and ``"serial"`` for
+    ``delta_recurrence``, ``"runs"`` for ``delta_recurrence_runs``."""
+    step, per_run = _delta_sizes(n_heads, dim, vdim)
+
+    def kind(n):
+        if n == 1 and step:
+            return "one"
+        return "runs" if n >= DELTA_RUNS_MIN_TOKENS and 0 < cost(n) <= DELTA_RUNS_MAX_FLOATS else "serial"
+
+    def cost(n):
+        return -(-n // DELTA_RUN) * per_run if n >= DELTA_RUNS_MIN_TOKENS else 0
+
+    return sequence_groups(batch, kind, cost, DELTA_RUNS_MAX_FLOATS)
+
+
 def delta_runs(batch, n_heads: int, dim: int, vdim: int):
     """(runs, floats of scratch) with which ``delta_recurrence_runs`` takes the step, or (0, 0) where
     ``delta_recurrence`` is the way: short portions, other head sizes, too much scratch."""
-    if max(batch.q_len) < DELTA_RUNS_MIN_TOKENS or not library().mf_delta_runs_ok(dim, vdim):
+    per_run = _delta_sizes(n_heads, dim, vdim)[1]
+    if max(batch.q_len) < DELTA_RUNS_MIN_TOKENS or not per_run:
         return 0, 0
     runs = sum(-(-n // DELTA_RUN) for n in batch.q_len)
-    floats = int(library().mf_delta_runs_scratch(runs, n_heads, dim, vdim))
-    return (runs, floats) if floats <= DELTA_RUNS_MAX_FLOATS else (0, 0)
+    return (runs, runs * per_run) if runs * per_run <= DELTA_RUNS_MAX_FLOATS else (0, 0)
 
 
 def delta_recurrence_runs(qkv: torch.Tensor, beta: torch.Tensor, ag: torch.Tensor, state: torch.Tensor, batch,

@@ -167,12 +167,13 @@ class ChannelDeltaMixer(Mixer):
             ops.delta_gates_ex(decay_in, decay_ld, self.decay_per_head, 0, 0.0, self.a_log, self.dt_bias, gate_in, gate_ld,
                                self.gate_act, ag, nh, d, nh * dv)
         o = rt.buffer("delta.o", (T, nh * dv), f32)
-        runs, floats = ops.delta_runs(batch, nh, d, dv)
-        if runs:
-            ops.delta_recurrence_runs(qkv, beta, ag, state, batch, o, nh, nkv, d, dv, runs,
-                                      rt.buffer("delta.runs", (floats,), f32))
-        else:
-            ops.delta_recurrence(qkv, beta, ag, state, batch, o, nh, nkv, d, dv)
+        for kind, part, _, _ in ops.delta_groups(batch, nh, d, dv):
+            if kind == "runs":
+                runs, floats = ops.delta_runs(part, nh, d, dv)
+                ops.delta_recurrence_runs(qkv, beta, ag, state, part, o, nh, nkv, d, dv, runs,
+                                          rt.buffer("delta.runs", (floats,), f32))
+            else:
+                ops.delta_recurrence(qkv, beta, ag, state, part, o, nh, nkv, d, dv)
         og = rt.buffer("delta.og", (T, nh * dv))
         ops.delta_output(o, ag[:, nh * d:], ag.shape[1], self.norm_w, self.eps, og, nh, dv)
         return rt.linear(og, self.w_o, rt.buffer("delta.delta", (T, self.hidden), f32 if self.out_f32 else None))

@@ -847,3 +847,57 @@ def test_delta_runs_keep_what_is_not_finite_from_earlier_tokens(t, what, dim, vd
         assert torch.equal(o[:t], res[0][:t])
         assert not torch.isfinite(o[t]).all()
         assert torch.equal(o[:, vdim:], res[0][:, vdim:])
+
+
+RECURRENT = {
+    "channel_delta": {"n_kv_heads": 2, "conv": 4, "decay_rank": 16, "gate_rank": 16},
+}
+
+
+def recurrent_part(kind, rt, rng, hidden=64):
+    """A mixer with a state, two heads of 128 channels."""
+    from mlxforge_b200.parts.base import MIXERS, PartSpec, build_part
+    part = build_part(MIXERS, PartSpec(kind, dict(RECURRENT[kind], hidden_size=hidden, n_heads=2, head_dim=128, eps=1e-6), "m."), rt)
+    part.bind({n: dev(rand(rng, *s.shape, std=s.shape[-1] ** -0.5)) for n, s in part.tensor_specs().items()})
+    return part
+
+
+def recurrent_runner(part, n):
+    """A runner over ``n`` open sequences with states drawn from one seed."""
+    from mlxforge_b200.cache.manager import CacheLayout, CacheManager, GroupLayout
+    from mlxforge_b200.engine.step import ModelRunner
+    layout = CacheLayout(paged=(), state=(GroupLayout(part.cache_need(), 1),), item_lane=(("state", 0, 0),))
+    cache = CacheManager(layout, page_size=16, max_tokens=64, max_seqs=n, dtype=part.rt.dtype, device="cuda")
+    seqs, states = [cache.open_sequence() for _ in range(n)], cache.lane(0).tensor
+    rng = np.random.default_rng(n)
+    for s in seqs:
+        states[s.slot] = dev(rng.standard_normal(states.shape[1]).astype(np.float32))
+    stub = SimpleNamespace(graph_safe=False, spec=SimpleNamespace(vocab_size=1 << 20))
+    return ModelRunner(stub, cache, part.rt), seqs, states
+
+
+@pytest.mark.parametrize("kind", list(RECURRENT))
+def test_a_sequence_has_the_same_bits_alone_and_beside_others(kind):
+    """Single tokens, portions that go token after token and portions that go over runs or chunks, in one step and each in a step of
+    its own: outputs and states to the bit (float32)."""
+    import torch
+    from mlxforge_b200.engine.runtime import Runtime
+    from mlxforge_b200.engine.step import StepEntry
+    lens = [1, 300, 40, 1, 20, 700, 90, 64, 48, 130, 257]          # enough behind one another for blocks of 16 columns
+    rng = np.random.default_rng(0)
+    part = recurrent_part(kind, Runtime(torch.float32), rng)
+    xs, results = [rand(rng, n, 64) for n in lens], []
+    for steps in ([range(len(lens))], [[i] for i in range(len(lens))]):
+        runner, seqs, states = recurrent_runner(part, len(lens))
+        got = [None] * len(lens)
+        for step in steps:
+            entries = [StepEntry(seqs[i], [0] * lens[i], []) for i in step]
+            runner.cache.reserve([(e.seq, len(e.tokens)) for e in entries])
+            order = sorted(step, key=lambda i: (lens[i] != 1, i))
+            out, at = part.forward(dev(np.concatenate([xs[i] for i in order])), runner._build(entries), runner.cache.lane(0)), 0
+            for i in order:
+                got[i], at = out[at:at + lens[i]].clone(), at + lens[i]
+        results.append((got, [states[s.slot].clone() for s in seqs]))
+    (together, s_together), (alone, s_alone) = results
+    differ = [lens[i] for i in range(len(lens)) if not (torch.equal(together[i], alone[i]) and torch.equal(s_together[i], s_alone[i]))]
+    assert not differ, differ
