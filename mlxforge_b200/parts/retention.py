@@ -112,12 +112,15 @@ class Retention(Mixer):
             ops.retention_prepare(proj, nh, d, self.rot, self.k_scale, batch.positions, self.inv_f, self.inv_d, qk)
             v, v_ld = proj[:, 2 * nh * d:], ld
         chunks = ops.retention_chunks(batch, nh, d, dv, v, v_ld, cache.tensor)
+        # the read-outs token by token in the buffer's name (its rows are reserved), partial ones behind one another in its use
+        parts = ops.retention_parts(d, dv, v, v_ld)
+        o = rt.buffer("ret.o", (T, parts * nh * dv), f32).view(parts, T, nh * dv)
         if chunks:
-            o = rt.buffer("ret.o", (1, T, nh * dv), f32)
+            o = o[:1]
             ops.retention_chunked(qk, v, v_ld, self.decay, cache.tensor, batch, o, nh, d, dv, chunks,
                                   rt.buffer("ret.states", (chunks * nh * d * dv,), f32))
         else:
-            o = rt.buffer("ret.o", (ops.retention_parts(d, dv, v, v_ld, batch), T, nh * dv), f32)
+            o = o[:ops.retention_parts(d, dv, v, v_ld, batch)]
             ops.retention_recurrence(qk, v, v_ld, self.decay, cache.tensor, batch, o, nh, d, dv)
         og = rt.buffer("ret.og", (T, nh * dv))
         ops.retention_output(o, proj[:, 2 * nh * d + nh * dv:], ld, self.eps, og, nh, dv, self.norm_w,

@@ -652,3 +652,30 @@ def test_retention_chunks_keep_what_is_not_finite_from_earlier_tokens(t, what, d
         assert torch.equal(o[:t], res[0][:t])
         assert not torch.isfinite(o[t]).all()
         assert torch.equal(o[:, vdim:], res[0][:, vdim:])
+
+
+def retention_128(rt, rng, hidden=64):
+    """Two heads of 128 x 128."""
+    return build("MIXERS", "retention", {"hidden_size": hidden, "n_heads": 2, "head_dim": 128, "v_head_dim": 128, "rotary_dim": 128,
+                                         "rope_base": 1e4, "decay": [0.97, 0.999], "eps": 1e-6}, rt,
+                 {"m." + n: rand(rng, *s, std=s[1] ** -0.5) for n, s in (("q", (256, hidden)), ("k", (256, hidden)), ("v", (256, hidden)),
+                                                                        ("g", (256, hidden)), ("o", (hidden, 256)))})
+
+
+@pytest.mark.parametrize("lens", [[1], [40], [300]])
+def test_the_read_outs_of_a_step_reserve_rows_of_the_token_budget(lens):
+    """The engine reserves every per-token buffer for its token budget: a step's partial read-outs are floats of so many tokens, not
+    so many copies of the step."""
+    import torch
+    from mlxforge_b200.engine.runtime import Runtime
+    from mlxforge_b200.engine.step import StepEntry
+    from test_notirax_gpu import recurrent_runner
+    rt = Runtime(torch.bfloat16)
+    rt.reserve_rows = 2048
+    rng = np.random.default_rng(0)
+    part = retention_128(rt, rng)
+    runner, seqs, _ = recurrent_runner(part, len(lens))
+    entries = [StepEntry(s, [0] * n, []) for s, n in zip(seqs, lens)]
+    runner.cache.reserve([(e.seq, len(e.tokens)) for e in entries])
+    part.forward(dev(rand(rng, sum(lens), 64), torch.bfloat16), runner._build(entries), runner.cache.lane(0))
+    assert max(b.numel() for n, b in rt._buffers.items() if n.startswith("ret.o:")) <= 2048 * 4 * 256
