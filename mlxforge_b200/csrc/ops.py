@@ -383,8 +383,15 @@ def sequence_groups(batch, kind, cost=None, limit: int = 0):
             for k, a, b, t0, t1, _ in groups]
 
 
+@lru_cache(maxsize=None)
+def _retention_sizes(dim: int, vdim: int, v_ld: int):
+    """(whether one token has a kernel of its own, whether chunks take these sizes)"""
+    lib = library()
+    return bool(lib.mf_retention_step_ok(dim, vdim)), bool(lib.mf_retention_chunked_ok(dim, vdim, v_ld))
+
+
 def _retention_step(batch, dim: int, vdim: int) -> bool:
-    return min(batch.q_len) == 1 == max(batch.q_len) and bool(library().mf_retention_step_ok(dim, vdim))
+    return min(batch.q_len) == 1 == max(batch.q_len) and _retention_sizes(dim, vdim, 0)[0]
 
 
 def retention_parts(dim: int, vdim: int, v: torch.Tensor, v_ld: int, batch=None) -> int:
@@ -419,11 +426,32 @@ RETENTION_CHUNKED_MIN_TOKENS = 256
 RETENTION_CHUNKED_MAX_FLOATS = 1 << 28
 
 
+def _retention_chunked_ok(dim: int, vdim: int, v: torch.Tensor, v_ld: int, state: torch.Tensor) -> bool:
+    return (_retention_sizes(dim, vdim, v_ld)[1] and not v.data_ptr() % (4 * v.element_size())
+            and not state.stride(0) % 4 and not state.data_ptr() % 16)
+
+
+def retention_groups(batch, n_heads: int, dim: int, vdim: int, v: torch.Tensor, v_ld: int, state: torch.Tensor):
+    """``sequence_groups`` of the retention: ``"one"`` token (the step kernel, where it takes the sizes) and ``"serial"`` for
+    ``retention_recurrence``, ``"chunks"`` for ``retention_chunked``."""
+    step = _retention_sizes(dim, vdim, v_ld)[0]
+    size = n_heads * dim * vdim if _retention_chunked_ok(dim, vdim, v, v_ld, state) else 0
+
+    def kind(n):
+        if n == 1 and step:
+            return "one"
+        return "chunks" if n >= RETENTION_CHUNKED_MIN_TOKENS and 0 < cost(n) <= RETENTION_CHUNKED_MAX_FLOATS else "serial"
+
+    def cost(n):
+        return -(-n // RETENTION_CHUNK) * size if n >= RETENTION_CHUNKED_MIN_TOKENS else 0
+
+    return sequence_groups(batch, kind, cost, RETENTION_CHUNKED_MAX_FLOATS)
+
+
 def retention_chunks(batch, n_heads: int, dim: int, vdim: int, v: torch.Tensor, v_ld: int, state: torch.Tensor) -> int:
     """Chunks with which ``retention_chunked`` takes the step, or 0 where ``retention_recurrence`` is the way: short
     portions, other head sizes, operands that are not whole 16-byte pieces, too much scratch."""
-    if (max(batch.q_len) < RETENTION_CHUNKED_MIN_TOKENS or not library().mf_retention_chunked_ok(dim, vdim, v_ld)
-            or v.data_ptr() % (4 * v.element_size()) or state.stride(0) % 4 or state.data_ptr() % 16):
+    if max(batch.q_len) < RETENTION_CHUNKED_MIN_TOKENS or not _retention_chunked_ok(dim, vdim, v, v_ld, state):
         return 0
     chunks = sum(-(-n // RETENTION_CHUNK) for n in batch.q_len)
     return chunks if chunks * n_heads * dim * vdim <= RETENTION_CHUNKED_MAX_FLOATS else 0
@@ -446,9 +474,9 @@ def retention_chunked(qk: torch.Tensor, v: torch.Tensor, v_ld: int, decay: torch
 def retention_output(o: torch.Tensor, gate: torch.Tensor, gate_ld: int, eps: float, out: torch.Tensor, n_heads: int,
                      vdim: int, weight: Optional[torch.Tensor] = None, whole: bool = False,
                      gate_act: str = "silu") -> None:
-    """``o`` [parts, T, n_heads * vdim]: the partial read-outs, summed here.  ``gate`` points at the first gate of
+    """``o`` [parts, T, n_heads * vdim]: the partial read-outs (any distance apart), summed here.  ``gate`` points at the first gate of
     the first token; rows are ``gate_ld`` elements apart."""
-    _need_cuda(o, out)
+    _need_cuda(o[0], out)
     check(library().mf_retention_output(o.data_ptr(), o.shape[0], o.stride(0), gate.data_ptr(), dtype_code(out), gate_ld,
                                         eps, out.data_ptr(), o.shape[1], n_heads, vdim, _ptr(weight), int(whole),
                                         {"silu": 0, "sigmoid": 1}[gate_act], _stream()), "retention_output")

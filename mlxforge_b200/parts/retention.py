@@ -111,18 +111,20 @@ class Retention(Mixer):
         else:
             ops.retention_prepare(proj, nh, d, self.rot, self.k_scale, batch.positions, self.inv_f, self.inv_d, qk)
             v, v_ld = proj[:, 2 * nh * d:], ld
-        chunks = ops.retention_chunks(batch, nh, d, dv, v, v_ld, cache.tensor)
         # the read-outs token by token in the buffer's name (its rows are reserved), partial ones behind one another in its use
         parts = ops.retention_parts(d, dv, v, v_ld)
         o = rt.buffer("ret.o", (T, parts * nh * dv), f32).view(parts, T, nh * dv)
-        if chunks:
-            o = o[:1]
-            ops.retention_chunked(qk, v, v_ld, self.decay, cache.tensor, batch, o, nh, d, dv, chunks,
-                                  rt.buffer("ret.states", (chunks * nh * d * dv,), f32))
-        else:
-            o = o[:ops.retention_parts(d, dv, v, v_ld, batch)]
-            ops.retention_recurrence(qk, v, v_ld, self.decay, cache.tensor, batch, o, nh, d, dv)
         og = rt.buffer("ret.og", (T, nh * dv))
-        ops.retention_output(o, proj[:, 2 * nh * d + nh * dv:], ld, self.eps, og, nh, dv, self.norm_w,
-                             self.output_norm == "whole", self.gate_act)
+        gate = proj[:, 2 * nh * d + nh * dv:]
+        for kind, part, t0, t1 in ops.retention_groups(batch, nh, d, dv, v, v_ld, cache.tensor):
+            own = o if kind == "serial" else o[:1]
+            if kind == "chunks":
+                chunks = ops.retention_chunks(part, nh, d, dv, v, v_ld, cache.tensor)
+                ops.retention_chunked(qk, v, v_ld, self.decay, cache.tensor, part, own, nh, d, dv, chunks,
+                                      rt.buffer("ret.states", (chunks * nh * d * dv,), f32))
+            else:
+                ops.retention_recurrence(qk, v, v_ld, self.decay, cache.tensor, part, own, nh, d, dv)
+            rows = (own, gate, og) if t1 - t0 == T else (own[:, t0:t1], gate[t0:t1], og[t0:t1])
+            ops.retention_output(rows[0], rows[1], ld, self.eps, rows[2], nh, dv, self.norm_w, self.output_norm == "whole",
+                                 self.gate_act)
         return rt.linear(og, self.w_o, rt.buffer("ret.delta", (T, self.hidden), f32 if self.out_f32 else None))

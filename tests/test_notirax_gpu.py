@@ -851,6 +851,7 @@ def test_delta_runs_keep_what_is_not_finite_from_earlier_tokens(t, what, dim, vd
 
 RECURRENT = {
     "channel_delta": {"n_kv_heads": 2, "conv": 4, "decay_rank": 16, "gate_rank": 16},
+    "retention": {"rotary_dim": 128, "rope_base": 1e4, "decay": [0.97, 0.999]},
 }
 
 
