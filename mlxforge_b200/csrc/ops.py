@@ -448,6 +448,13 @@ def retention_groups(batch, n_heads: int, dim: int, vdim: int, v: torch.Tensor, 
     return sequence_groups(batch, kind, cost, RETENTION_CHUNKED_MAX_FLOATS)
 
 
+def retention_chunks_room(tokens: int, n_heads: int, dim: int, vdim: int) -> int:
+    """Floats of scratch that no group of a step of ``tokens`` tokens goes beyond: whole chunks, and a broken one behind
+    every portion."""
+    chunks = tokens // RETENTION_CHUNK + tokens // RETENTION_CHUNKED_MIN_TOKENS
+    return min(chunks * n_heads * dim * vdim, RETENTION_CHUNKED_MAX_FLOATS)
+
+
 def retention_chunks(batch, n_heads: int, dim: int, vdim: int, v: torch.Tensor, v_ld: int, state: torch.Tensor) -> int:
     """Chunks with which ``retention_chunked`` takes the step, or 0 where ``retention_recurrence`` is the way: short
     portions, other head sizes, operands that are not whole 16-byte pieces, too much scratch."""
@@ -928,6 +935,13 @@ def delta_groups(batch, n_heads: int, dim: int, vdim: int):
         return -(-n // DELTA_RUN) * per_run if n >= DELTA_RUNS_MIN_TOKENS else 0
 
     return sequence_groups(batch, kind, cost, DELTA_RUNS_MAX_FLOATS)
+
+
+def delta_runs_room(tokens: int, n_heads: int, dim: int, vdim: int) -> int:
+    """Floats of scratch that no group of a step of ``tokens`` tokens goes beyond: whole runs, and a broken one behind
+    every portion."""
+    runs = tokens // DELTA_RUN + tokens // DELTA_RUNS_MIN_TOKENS
+    return min(runs * _delta_sizes(n_heads, dim, vdim)[1], DELTA_RUNS_MAX_FLOATS)
 
 
 def delta_runs(batch, n_heads: int, dim: int, vdim: int):

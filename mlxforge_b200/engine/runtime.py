@@ -56,9 +56,10 @@ class Runtime:
         self.fused_swiglu_min_rows = 256
 
     # ------------------------------------------------------------------ scratch
-    def buffer(self, name: str, shape: Tuple[int, ...], dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+    def buffer(self, name: str, shape: Tuple[int, ...], dtype: Optional[torch.dtype] = None, room: int = 0) -> torch.Tensor:
         """A contiguous scratch tensor of ``shape``; the storage behind ``name``
-        only ever grows, so steady-state steps allocate nothing."""
+        only ever grows, so steady-state steps allocate nothing.  ``room``: elements to make it for at first, where
+        the shape's rows are not the step's tokens."""
         dtype = dtype or self.dtype
         # the same view is asked for step after step: keep it, as long as no buffer has moved
         vkey = (name, shape, dtype)
@@ -74,7 +75,7 @@ class Runtime:
             cap = n
             if len(shape) >= 2 and self.reserve_rows > shape[0]:
                 cap = n // int(shape[0]) * self.reserve_rows
-            buf = torch.empty(max(cap, 1), dtype=dtype, device=self.device)
+            buf = torch.empty(max(cap, room, 1), dtype=dtype, device=self.device)
             self._buffers[key] = buf
             self.generation += 1
         view = buf[:n].view(shape)

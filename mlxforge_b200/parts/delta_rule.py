@@ -171,7 +171,7 @@ class ChannelDeltaMixer(Mixer):
             if kind == "runs":
                 runs, floats = ops.delta_runs(part, nh, d, dv)
                 ops.delta_recurrence_runs(qkv, beta, ag, state, part, o, nh, nkv, d, dv, runs,
-                                          rt.buffer("delta.runs", (floats,), f32))
+                                          rt.buffer("delta.runs", (floats,), f32, room=ops.delta_runs_room(rt.reserve_rows, nh, d, dv)))
             else:
                 ops.delta_recurrence(qkv, beta, ag, state, part, o, nh, nkv, d, dv)
         og = rt.buffer("delta.og", (T, nh * dv))

@@ -121,7 +121,8 @@ class Retention(Mixer):
             if kind == "chunks":
                 chunks = ops.retention_chunks(part, nh, d, dv, v, v_ld, cache.tensor)
                 ops.retention_chunked(qk, v, v_ld, self.decay, cache.tensor, part, own, nh, d, dv, chunks,
-                                      rt.buffer("ret.states", (chunks * nh * d * dv,), f32))
+                                      rt.buffer("ret.states", (chunks * nh * d * dv,), f32,
+                                                room=ops.retention_chunks_room(rt.reserve_rows, nh, d, dv)))
             else:
                 ops.retention_recurrence(qk, v, v_ld, self.decay, cache.tensor, part, own, nh, d, dv)
             rows = (own, gate, og) if t1 - t0 == T else (own[:, t0:t1], gate[t0:t1], og[t0:t1])

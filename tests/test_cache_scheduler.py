@@ -545,3 +545,21 @@ def test_sequences_are_grouped_by_their_own_length():
     most = ops.DELTA_RUNS_MAX_FLOATS // ops.library().mf_delta_runs_scratch(1, 64, 128, 128) * 16      # tokens
     n = most // 2 - 16
     assert [(k, len(l)) for k, l, *_ in groups([n, n, n, most + 16, 64], heads=64)] == [("runs", 2), ("runs", 1), ("serial", 1), ("runs", 1)]
+
+
+def test_room_for_runs_and_chunks_holds_every_step_of_the_budget():
+    """Against the scratch that drawn steps of at most the budget's tokens ask for."""
+    import random
+    from types import SimpleNamespace
+    from mlxforge_b200.csrc import ops
+    rng, budget, heads = random.Random(0), 1024, 2
+    runs_room, chunks_room = ops.delta_runs_room(budget, heads, 128, 64), ops.retention_chunks_room(budget, heads, 128, 64)
+    per_run, worst = ops.delta_runs_room(16, heads, 128, 64), [0, 0]
+    for _ in range(2000):
+        lens, left = [], budget
+        while left > 0 and len(lens) < 40:
+            lens.append(min(left, rng.choice([48, 49, 64, 65, 256, 257, 320, 321, rng.randint(1, 400)])))
+            left -= lens[-1]
+        worst[0] = max(worst[0], sum(-(-n // 16) for n in lens if n >= ops.DELTA_RUNS_MIN_TOKENS) * per_run)
+        worst[1] = max(worst[1], sum(-(-n // 64) for n in lens if n >= ops.RETENTION_CHUNKED_MIN_TOKENS) * heads * 128 * 64)
+    assert 0.8 * runs_room < worst[0] <= runs_room and 0.8 * chunks_room < worst[1] <= chunks_room, (worst, runs_room, chunks_room)

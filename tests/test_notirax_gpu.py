@@ -902,3 +902,22 @@ def test_a_sequence_has_the_same_bits_alone_and_beside_others(kind):
     (together, s_together), (alone, s_alone) = results
     differ = [lens[i] for i in range(len(lens)) if not (torch.equal(together[i], alone[i]) and torch.equal(s_together[i], s_alone[i]))]
     assert not differ, differ
+
+
+@pytest.mark.parametrize("kind", list(RECURRENT))
+def test_scratch_of_runs_and_chunks_does_not_move_within_the_token_budget(kind):
+    """A buffer that moves makes every captured decode graph void: the first long portion makes room for all that the budget allows."""
+    import torch
+    from mlxforge_b200.engine.runtime import Runtime
+    from mlxforge_b200.engine.step import StepEntry
+    rt = Runtime(torch.bfloat16)
+    rt.reserve_rows = 2048
+    part = recurrent_part(kind, rt, np.random.default_rng(0))
+    seen = []
+    for lens in ([300], [1, 40], [2048], [48] * 42, [257] * 7 + [1] * 3, [600, 1400]):
+        runner, seqs, _ = recurrent_runner(part, len(lens))
+        entries = [StepEntry(s, [0] * n, []) for s, n in zip(seqs, lens)]
+        runner.cache.reserve([(e.seq, len(e.tokens)) for e in entries])
+        part.forward(dev(rand(np.random.default_rng(1), sum(lens), 64), torch.bfloat16), runner._build(entries), runner.cache.lane(0))
+        seen.append(rt.generation)
+    assert len(set(seen)) == 1, seen
