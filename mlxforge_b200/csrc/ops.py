@@ -877,7 +877,7 @@ def delta_prepare(proj: torch.Tensor, conv_w: torch.Tensor, taps: int, state: to
     """Convolutions, SiLU and unit norms of the step's projections; the slots' convolution tails move on."""
     _need_cuda(proj, conv_w, state, qkv_out, beta_out, low)
     # the kernel's accesses are 16 bytes wide: operands off that boundary take the plain one, which never moves the history
-    moves = int(max(batch.q_len) == 1 and not (proj.data_ptr() | state.data_ptr() | qkv_out.data_ptr() | conv_w.data_ptr()) % 16
+    moves = int(min(batch.q_len) == 1 == max(batch.q_len) and not (proj.data_ptr() | state.data_ptr() | qkv_out.data_ptr() | conv_w.data_ptr()) % 16
                 and library().mf_delta_prepare_moves(proj.shape[0], taps, dim, vdim, proj.shape[1], state.stride(0), conv_off))
     check(library().mf_delta_prepare(proj.data_ptr(), proj.shape[1], conv_w.data_ptr(), taps, state.data_ptr(),
                                      state.stride(0), conv_off, batch.positions.data_ptr(),

@@ -921,3 +921,22 @@ def test_scratch_of_runs_and_chunks_does_not_move_within_the_token_budget(kind):
         part.forward(dev(rand(np.random.default_rng(1), sum(lens), 64), torch.bfloat16), runner._build(entries), runner.cache.lane(0))
         seen.append(rt.generation)
     assert len(set(seen)) == 1, seen
+
+
+def test_delta_prepare_takes_a_sequence_without_a_token_beside_single_ones():
+    """Its history stays as it is, the others' move on."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    rng = np.random.default_rng(3)
+    lens, heads, dim, taps = [1, 0, 1], 2, 64, 4
+    C = 3 * heads * dim
+    proj, w = rng.standard_normal((2, C + 4)).astype(np.float32), rng.standard_normal((C, taps)).astype(np.float32)
+    state = rng.standard_normal((3, 3, C)).astype(np.float32)
+    i32 = lambda a: dev(np.asarray(a, np.int32))
+    batch = SimpleNamespace(q_len=lens, n_seqs=3, positions=i32([0, 0]), slots=i32([2, 1, 0]), seq_of_token=i32([0, 2]),
+                            seq_q_start=i32([0, 1, 1]), seq_q_len=i32(lens))
+    st, qkv, beta, low = dev(state.reshape(3, -1)), *(torch.empty((2, n), device="cuda") for n in (C, heads, 2))
+    ops.delta_prepare(dev(proj), dev(w), taps, st, 0, batch, qkv, beta, low, heads, heads, dim, dim)
+    for slot, t in ((2, 0), (0, 1)):
+        state[slot] = np.concatenate([state[slot, 1:], proj[t:t + 1, :C]])
+    assert np.array_equal(st.cpu().numpy(), state.reshape(3, -1)) and torch.isfinite(qkv).all()
