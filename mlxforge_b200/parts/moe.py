@@ -25,8 +25,8 @@ The experts' matrices are stacked at load time (``[E, 2, ff, H]`` gate rows then
 ``[E, H, ff]``).  Few tokens (and the 32-bit path) take the kernel with a block per (token, chosen
 expert), which streams that expert's matrices once; many tokens in bfloat16 are sorted by expert and go
 through the tcgen05 products over the sorted pairs (``MLXFORGE_MOE_TILES=1``: the mma.sync tiles).  Either way a
-token's chosen experts are added in the order of the choice, so its result does not depend on what
-else is in the batch.
+token's chosen experts are added in the order of the choice; what else is in the step moves its result only
+by which of the two paths the step's size takes, and by the type of a pair's result in a step of many tokens (``wide_y``).
 """
 from __future__ import annotations
 
@@ -86,7 +86,7 @@ class RoutedExperts(FeedForward):
             raise ValueError("routed_experts: a shared gate without a shared branch")
         # tokens from which the sorted, tiled path is taken (bfloat16 only)
         self.grouped_min_tokens = int(p.get("grouped_min_tokens", 64))
-        # tokens from which a pair's result goes to the weighted sum in bfloat16
+        # tokens from which a prompt's pairs go to the weighted sum in bfloat16 (``forward_grouped``)
         self.wide_y_tokens = 512
         self.w_router = self.w_gu = self.w_down = self.choice_bias = self.logit_bias = None
 
@@ -166,7 +166,7 @@ class RoutedExperts(FeedForward):
         out = rt.buffer("moe.delta", (T, self.hidden))
         if (x.dtype == torch.bfloat16 and T >= self.grouped_min_tokens and self.n_experts
                 and ops.moe_grouped_ok(self.hidden, self.ff, self.n_experts)):
-            return self.forward_grouped(x, ids, weights, out, z, shared)
+            return self.forward_grouped(x, batch, ids, weights, out, z, shared)
         slices = ops.moe_rows_slices(self.ff)
         y = rt.buffer("moe.y", (T, self.top * slices, self.hidden), torch.float32)
         if self.n_experts:
@@ -174,7 +174,15 @@ class RoutedExperts(FeedForward):
         self._combine(y, weights, None, out, slices, ids, x, z, shared)
         return out
 
-    def forward_grouped(self, x, ids, weights, out, z, shared):
+    def wide_y(self, T, batch) -> bool:
+        """Whether a pair's result goes to the weighted sum in 32-bit: in steps of few tokens, in every step that decodes
+        (recorded or not) and with the ``tcgen05`` backend.  Long prompts hand it on in bfloat16, as the library's grouped product gave it,
+        because its way through memory is long there (the mixture with 6 of 64 experts of 768 x 2,048 in bfloat16 and in 32-bit:
+        2,048 tokens 202 and 269 us, 1,024 175 and 206, 513 163 and 179, 256 159 and 165, 64 155 and 157)."""
+        return (T < self.wide_y_tokens or getattr(self.rt, "gemm_backend", "auto") == "tcgen05"
+                or getattr(batch, "n_decode", None) == T or torch.cuda.is_current_stream_capturing())
+
+    def forward_grouped(self, x, batch, ids, weights, out, z, shared):
         """Many tokens: pairs ordered by expert, the two products over the sorted rows, the weighted sum in
         the order of the choice."""
         rt, T = self.rt, x.shape[0]
@@ -195,9 +203,7 @@ class RoutedExperts(FeedForward):
             ops.moe_sort(ids, self.n_experts, slot_of, row_token, meta, tiles, tile_rows=ops.moe_tc_rows())
             ops.moe_tc_up(x, row_token, rt.buffer("moe.xg", (n, self.hidden)), self.w_gu, meta, tiles, act, self.limit,
                           self.alpha, self.up_offset, self.expert_act)
-            # a pair's result in 32-bit where its way through memory is short (and in a recorded step, whatever its size)
-            wide = T < self.wide_y_tokens or torch.cuda.is_current_stream_capturing()
-            y = rt.buffer("moe.y", (n, self.hidden), torch.float32 if wide else None)
+            y = rt.buffer("moe.y", (n, self.hidden), torch.float32 if self.wide_y(T, batch) else None)
             ops.moe_tc_down(act, self.w_down, meta, tiles, y)
         self._combine(y, weights, slot_of, out, 1, ids, x, z, shared)
         return out

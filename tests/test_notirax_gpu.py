@@ -940,3 +940,27 @@ def test_delta_prepare_takes_a_sequence_without_a_token_beside_single_ones():
     for slot, t in ((2, 0), (0, 1)):
         state[slot] = np.concatenate([state[slot, 1:], proj[t:t + 1, :C]])
     assert np.array_equal(st.cpu().numpy(), state.reshape(3, -1)) and torch.isfinite(qkv).all()
+
+
+@pytest.mark.parametrize("gemm", ["auto", "tcgen05"])
+def test_the_type_of_an_experts_result(gemm):
+    """32-bit in every step that decodes, recorded or not, of few tokens or many, and for prompts too with the ``tcgen05`` backend:
+    a token's result then has the same bits in a step of 511 tokens and of 600, and in a replayed one."""
+    import torch
+    from mlxforge_b200.engine.runtime import Runtime
+    from mlxforge_b200.parts.base import FEED_FORWARDS, PartSpec, build_part
+    rng, rt = np.random.default_rng(0), Runtime(torch.bfloat16)
+    rt.gemm_backend = gemm
+    part = build_part(FEED_FORWARDS, PartSpec("routed_experts", {"hidden_size": 128, "intermediate_size": 64, "n_experts": 8, "top": 4,
+                                                                "n_groups": 0, "keep_groups": 0, "limit": 7.0}, prefix="f."), rt)
+    part.bind({n: dev(rand(rng, *s.shape, std=s.shape[-1] ** -0.5)) for n, s in part.tensor_specs().items()})
+    x = dev(rand(rng, 600, 128), torch.bfloat16)
+    decode = lambda n: SimpleNamespace(n_decode=n) if gemm == "auto" else None
+    few, many = part.forward(x[:511], decode(511)).clone(), part.forward(x, decode(600)).clone()
+    prompt = part.forward(x, SimpleNamespace(n_decode=0)).clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = part.forward(x, decode(600))
+    graph.replay()
+    assert torch.equal(few, many[:511]) and torch.equal(out, many)
+    assert torch.equal(prompt, many) == (gemm == "tcgen05")
