@@ -76,6 +76,9 @@ __device__ __forceinline__ void tt_pieces(float x, float y, uint32_t (&p)[3]) {
   }
 }
 #define TT_LOG2E 1.4426950408889634f
+// a maximum in powers of two, rounded once: the weights, what moves older sums to a new maximum and the merge of the splits all
+// go by this number, so that its rounding (1e-3 of a weight at scores of 20,000) drops out
+__device__ __forceinline__ float tt_max_log2(float m) { return __fmul_rn(m, TT_LOG2E); }
 __device__ __forceinline__ float tt_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -128,7 +131,7 @@ struct TtArgs {
   int splits;               // 0: every block walks all its keys; else gridDim.z splits of split_tiles tiles
   int split_tiles;
   float* part_o;            // [rows, splits, H, VDIM] unnormalised outputs of the splits
-  float* part_ml;           // [rows, splits, H, 2]    running maximum and sum
+  float* part_ml;           // [rows, splits, H, 2]    maximum (in powers of two) and sum
 };
 
 template <int VDIM, int MAXH>
@@ -312,8 +315,8 @@ talking_attention_tc_kernel(const TtArgs a) {
         mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 1));
         mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 2));
         const float m_new = fmaxf(m_run[e], mx[e]);
-        m_log2[e] = m_new == -INFINITY ? 0.f : m_new * TT_LOG2E;
-        alpha[e] = tt_exp2(fmaf(m_run[e], TT_LOG2E, -m_log2[e]));
+        m_log2[e] = m_new == -INFINITY ? 0.f : tt_max_log2(m_new);
+        alpha[e] = tt_exp2(tt_max_log2(m_run[e]) - m_log2[e]);
         m_run[e] = m_new;
       }
       float sum[2] = {0.f, 0.f};
@@ -372,7 +375,7 @@ talking_attention_tc_kernel(const TtArgs a) {
             *reinterpret_cast<float2*>(a.part_o + slot * VDIM + nt * 8 + c2) =
                 make_float2(o[nt][2 * half], o[nt][2 * half + 1]);
           if (c2 == 0) {
-            a.part_ml[slot * 2] = m_run[half];
+            a.part_ml[slot * 2] = tt_max_log2(m_run[half]);
             a.part_ml[slot * 2 + 1] = l_run[half];
           }
         }
@@ -406,7 +409,7 @@ MF_API int mf_attention_talking_tc_ok(int n_heads, int n_kv, int dim, int vdim, 
   return tt_smem_bytes(n_heads, n_kv, dim, vdim) <= 200 * 1024 ? 1 : 0;
 }
 
-// out[t, h] = sum_z o_z e^{m_z - m} / sum_z l_z e^{m_z - m}, the splits in their order; a warp per (token, head), VDIM / 32
+// out[t, h] = sum_z o_z 2^{m_z - m} / sum_z l_z 2^{m_z - m}, the splits in their order; a warp per (token, head), VDIM / 32
 // neighbouring channels a lane
 template <int VDIM>
 __global__ void __launch_bounds__(256)
@@ -426,7 +429,7 @@ talking_attention_merge_kernel(const float* __restrict__ part_o, const float* __
   for (int z = 0; z < splits; z++) {
     const float2 x = ml[(long long)z * H];
     if (x.x == -INFINITY) continue;
-    const float w = __expf(x.x - m);
+    const float w = tt_exp2(x.x - m);
     l += x.y * w;
 #pragma unroll
     for (int i = 0; i < N; i++) acc[i] += po[(long long)z * H * VDIM + i] * w;
@@ -561,12 +564,12 @@ talking_decode_kernel(const TtArgs a) {
     float m = fmaxf(x.x, x.y);
 #pragma unroll
     for (int off = 16; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-    const float m_log2 = m == -INFINITY ? 0.f : m * TT_LOG2E;
+    const float m_log2 = m == -INFINITY ? 0.f : tt_max_log2(m);
     const float p0 = tt_exp2(fmaf(x.x, TT_LOG2E, -m_log2)), p1 = tt_exp2(fmaf(x.y, TT_LOG2E, -m_log2));
     const float l = warp_sum(p0 + p1);
     *reinterpret_cast<uint32_t*>(Ps + h * p_ld + lane * 2) = tt_pack(p0, p1);
     if (lane == 0) {
-      a.part_ml[(slot0 + h) * 2] = m;
+      a.part_ml[(slot0 + h) * 2] = tt_max_log2(m);
       a.part_ml[(slot0 + h) * 2 + 1] = l;
     }
   }
@@ -630,7 +633,7 @@ talking_decode_merge_kernel(const float* __restrict__ part_o, const float* __res
   for (int z = warp; z < splits; z += 8) {
     const float2 x = ml[(long long)z * H];
     const bool some = x.x != -INFINITY;                       // a split without a key has no output
-    const float w = some ? __expf(x.x - m) : 0.f;
+    const float w = some ? tt_exp2(x.x - m) : 0.f;
     l += x.y * w;
 #pragma unroll
     for (int i = 0; i < N; i++) acc[i] += (some ? po[(long long)z * H * VDIM + i * 32] : 0.f) * w;

@@ -964,3 +964,52 @@ def test_the_type_of_an_experts_result(gemm):
     graph.replay()
     assert torch.equal(few, many[:511]) and torch.equal(out, many)
     assert torch.equal(prompt, many) == (gemm == "tcgen05")
+
+
+def talking_case(seqs, heads, kv, k, v, q, scale, talk=None):
+    """(tensor-core kernels, block-per-token kernel) [T, heads, vdim] over sequences of (new tokens, context) with the keys and values
+    k[i], v[i] [context, kv, .]."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    from mlxforge_b200.engine.runtime import Runtime
+    from mlxforge_b200.parts.talking_attention import talking_paged_attention
+    bf, page, T, dim, vdim = torch.bfloat16, 16, sum(n for n, _ in seqs), k[0].shape[2], v[0].shape[2]
+    blocks = [-(-c // page) for _, c in seqs]
+    table, at = np.full((len(seqs), max(blocks)), -1, np.int32), 0
+    kp, vp = (np.zeros((sum(blocks), kv, page, d), np.float32) for d in (dim, vdim))
+    for i, (n, c) in enumerate(seqs):
+        for b in range(blocks[i]):
+            table[i, b], m = at, min(page, c - b * page)
+            kp[at, :, :m], vp[at, :, :m] = (x[i][b * page:b * page + m].transpose(1, 0, 2) for x in (k, v))
+            at += 1
+    i32 = lambda a: dev(np.asarray(a, np.int32))
+    lens, ctx = [n for n, _ in seqs], [c for _, c in seqs]
+    starts = np.cumsum([0] + lens[:-1])
+    batch = SimpleNamespace(n_decode=sum(n == 1 for n in lens), n_tokens=T, max_ctx=max(ctx), q_len=lens, block_table=lambda g: dev(table),
+                            seq_q_start=i32(starts), seq_q_len=i32(lens), seq_ctx_len=i32(ctx))
+    lane = SimpleNamespace(group=0, k=dev(kp, bf), v=dev(vp, bf), page_size=page)
+    m = SimpleNamespace(n_heads=heads, n_kv=kv, dim=dim, vdim=vdim, scale=scale, softcap=0.0, window=0, chunk=0, talk=talk)
+    got, want = (torch.full((T, heads * vdim), float("nan"), device="cuda", dtype=bf) for _ in range(2))
+    talking_paged_attention(Runtime(bf), batch, dev(q.reshape(T, -1), bf), lane, got, m)
+    pos = np.concatenate([np.arange(c - n, c) for n, c in seqs])
+    ops.attention_talking(dev(q.reshape(T, -1), bf), lane.k, lane.v, want, i32(pos), i32(np.repeat(np.arange(len(seqs)), lens)), dev(table),
+                          page, heads, kv, dim, vdim, scale, 0.0, talk, 0, 0)
+    return host(got).reshape(T, heads, vdim), host(want).reshape(T, heads, vdim)
+
+
+@pytest.mark.parametrize("seqs", [[(1, 300)], [(2, 300)], [(16, 2000)]])
+@pytest.mark.parametrize("base", [3.0, 2.0 ** 20])
+def test_talking_weights_of_large_scores(seqs, base):
+    """Scores of base + j / 4 (exact in every type used), the maximum rising from tile to tile: however large they are, a weight is
+    e^(j / 4).  Weights and results are rounded to bfloat16 (2^-8 each); a maximum rounded in one place and not in another moves a weight
+    by up to 2^-4.5 at the larger base."""
+    heads, kv, dim, vdim = 2, 1, 16, 32
+    n, c = seqs[0]
+    k, v, q = np.zeros((c, kv, dim), np.float32), np.zeros((c, kv, vdim), np.float32), np.zeros((n, heads, dim), np.float32)
+    k[:, 0, 0], k[:, 0, 1], q[:, :, :2] = base, np.arange(c) // 32 % 8 * 0.25, 1.0
+    v[np.arange(c), 0, np.arange(c) // 32 % vdim] = 1.0
+    got, other = talking_case(seqs, heads, kv, [k], [v], q, 1.0)
+    for i in range(n):
+        p = np.exp(k[:c - n + 1 + i, 0, 1].astype(np.float64))
+        want = p @ v[:c - n + 1 + i, 0].astype(np.float64) / p.sum()
+        assert np.all(np.abs(got[i] - want) <= 2.0 ** -7 * 1.02 * want) and np.all(np.abs(other[i] - want) <= 2.0 ** -8 * 1.02 * want)
