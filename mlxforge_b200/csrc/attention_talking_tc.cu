@@ -94,7 +94,7 @@ __device__ __forceinline__ float tt_tanh(float x) {
 // and the next, zero beyond H
 __device__ __forceinline__ void tt_talk_pieces(const float* talk, int H, int reg, int lane, uint32_t* tk) {
   const int h = (lane >> 2) + (reg & 1) * 8, g = (lane & 3) * 2 + (reg >> 1) * 8;
-  auto at = [&](int g) { return h < H && g < H ? (talk ? talk[h * H + g] : (h == g ? 1.f : 0.f)) : 0.f; };
+  auto at = [&](int g) { return h < H && g < H ? (talk ? talk[h * H + g] : 0.f) : 0.f; };
   uint32_t p[3];
   tt_pieces(at(g), at(g + 1), p);
 #pragma unroll
@@ -270,7 +270,7 @@ talking_attention_tc_kernel(const TtArgs a) {
     else tt_cp_async_commit();
 
     // 2. the heads mixed and the mask: a warp one query and eight keys at a time
-    {
+    if (a.talk) {
       uint32_t t[3][4];
 #pragma unroll
       for (int i = 0; i < 3; i++)
@@ -289,6 +289,12 @@ talking_attention_tc_kernel(const TtArgs a) {
         if (r0 + 8 < H)
           *reinterpret_cast<float2*>(to + (size_t)(r0 + 8) * sc_hd) =
               make_float2(ok0 ? c[2] : -INFINITY, ok1 ? c[3] : -INFINITY);
+      }
+    } else {
+      // no matrix: the mask alone (the identity's zeros would let what is not finite in one head into all of them)
+      for (int i = tid; i < H * rows * TT_BN; i += nthreads) {
+        const int h = i / (rows * TT_BN), r = (i - h * rows * TT_BN) / TT_BN, key = i % TT_BN, pj = k0 + key;
+        if (pj < first_s[r] || pj > pos0 + r) sc[(size_t)h * sc_hd + r * sc_ld + key] = -INFINITY;
       }
     }
     tt_cp_async_wait<1>();      // the values are there; the next keys may still be on their way
@@ -547,7 +553,12 @@ talking_decode_kernel(const TtArgs a) {
 #pragma unroll
       for (int e = 0; e < 4; e++) t[i][e] = tk[(i * 4 + e) * 32 + lane];
     float c[4];
-    tt_mix(t, sc + n0 + r0, sc_ld, H, c2, c);
+    if (a.talk) {
+      tt_mix(t, sc + n0 + r0, sc_ld, H, c2, c);
+    } else {                     // no matrix: a head's own scores (the identity's zeros would let what is not finite into all heads)
+#pragma unroll
+      for (int e = 0; e < 4; e++) c[e] = r0 + (e & 2) * 4 < H ? sc[(r0 + (e & 2) * 4) * sc_ld + n0 + c2 + (e & 1)] : 0.f;
+    }
     const int pj = k0 + n0 + c2;
     const bool ok0 = pj >= k_lo && pj <= k_hi, ok1 = pj + 1 >= k_lo && pj + 1 <= k_hi;
     float* to = sc + n0 + c2;

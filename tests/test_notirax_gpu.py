@@ -1013,3 +1013,18 @@ def test_talking_weights_of_large_scores(seqs, base):
         p = np.exp(k[:c - n + 1 + i, 0, 1].astype(np.float64))
         want = p @ v[:c - n + 1 + i, 0].astype(np.float64) / p.sum()
         assert np.all(np.abs(got[i] - want) <= 2.0 ** -7 * 1.02 * want) and np.all(np.abs(other[i] - want) <= 2.0 ** -8 * 1.02 * want)
+
+
+@pytest.mark.parametrize("seqs", [[(1, 200)], [(20, 200)]])
+@pytest.mark.parametrize("heads,kv", [(4, 2), (16, 4)])
+def test_talking_heads_without_a_mixing_matrix_stay_apart(heads, kv, seqs):
+    """A query that is not finite in one head leaves the others as they are."""
+    rng = np.random.default_rng(0)
+    f = lambda *s: rng.standard_normal(s).astype(np.float32)
+    k, v, q = f(200, kv, 64), f(200, kv, 64), f(seqs[0][0], heads, 64)
+    clean, _ = talking_case(seqs, heads, kv, [k], [v], q, 0.125)
+    q[:, 1, 5] = np.nan
+    got, want = talking_case(seqs, heads, kv, [k], [v], q, 0.125)
+    others = np.arange(heads) != 1
+    assert np.isfinite(want[:, others]).all() and np.array_equal(got[:, others], clean[:, others])
+    assert not np.isfinite(want[:, 1]).any() and not np.isfinite(got[:, 1]).any()
