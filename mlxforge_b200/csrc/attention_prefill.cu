@@ -81,7 +81,7 @@ attn_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   // all heads before any lighter tile
   const int tile = (int)gridDim.y - 1 - (int)blockIdx.y, head = blockIdx.x, s = blockIdx.z;
   const int q_len = seq_q_len[s];
-  if (tile * BM >= q_len) return;
+  if (tile * BM >= q_len || (opt.below > 0 && q_len >= opt.below)) return;
   const int q_start = seq_q_start[s], ctx = seq_ctx_len[s];
   const int seq_row = table_row0 + s;
   const int p0 = ctx - q_len;                              // position of the portion's first token
@@ -355,7 +355,8 @@ int launch_prefill_tc(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const
 int launch_prefill_tc_ex(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __nv_bfloat16* v_pool,
                          __nv_bfloat16* out, const int* seq_q_start, const int* seq_q_len, const int* seq_ctx_len,
                          int table_row0, int n_seqs, int max_q_len, int n_tokens, int n_heads, PagedView pv,
-                         float scale, int window, const AttnOptions& opt, int* status, cudaStream_t stream);
+                         float scale, int window, const AttnOptions& opt, int min_len, int* status, cudaStream_t stream);
+int prefill_tc_rows();
 
 // q, out: [T, n_heads * hd] of the whole step.  The n_seqs sequences start at row
 // `table_row0` of the block table; seq_q_start / seq_q_len / seq_ctx_len are their
@@ -394,26 +395,32 @@ MF_API int mf_attention_prefill(const void* q, const void* k_pool, const void* v
 // The same with the options of AttnOptions (value width, values inside the keys, kept first keys, sink,
 // output gate): the tcgen05 kernels where they take the form (portions of at least 128 tokens; head size 128 with kept
 // keys, sink and gate, or values inside keys of 65 to 256 channels), else the mma.sync kernel.  `out` and the gate are
-// [T, n_heads * vd], `n_tokens` is T.
+// [T, n_heads * vd], `n_tokens` is T.  `min_q_len`: the shortest portion, or 0 where it is not known.  A step of portions on
+// both sides of 128 tokens takes a launch of each kernel, so that a portion's numbers do not depend on what else is in the step.
 MF_API int mf_attention_prefill_ex(const void* q, const void* k_pool, const void* v_pool, void* out,
                                    const int* seq_q_start, const int* seq_q_len, const int* seq_ctx_len,
-                                   int table_row0, int n_seqs, int max_q_len, int n_tokens, int n_heads, int n_kv, int hd,
-                                   const int* block_table, int bt_stride, int page_size, float scale, int window,
-                                   int vd, int v_in_k, int keep_first, const float* sink, const void* gate,
+                                   int table_row0, int n_seqs, int min_q_len, int max_q_len, int n_tokens, int n_heads,
+                                   int n_kv, int hd, const int* block_table, int bt_stride, int page_size, float scale,
+                                   int window, int vd, int v_in_k, int keep_first, const float* sink, const void* gate,
                                    long long gate_ld, float softcap, int* status, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
   if (hd < 16 || hd > 256 || hd % 16 || n_kv <= 0 || n_heads % n_kv) return MF_ERR_BAD_ARG;
   if (vd <= 0 || vd > hd || vd % 16 || keep_first < 0) return MF_ERR_BAD_ARG;
   if (n_heads > 65535 || n_seqs > 65535) return MF_ERR_BAD_ARG;
   PagedView pv{block_table, bt_stride, page_size, n_kv, hd};
-  const AttnOptions opt{vd, v_in_k, keep_first, sink, (const __nv_bfloat16*)gate, gate_ld, softcap};
+  AttnOptions opt{vd, v_in_k, keep_first, sink, (const __nv_bfloat16*)gate, gate_ld, softcap, 0};
   const __nv_bfloat16 *qq = (const __nv_bfloat16*)q, *kk = (const __nv_bfloat16*)k_pool,
                       *vv = (const __nv_bfloat16*)v_pool;
   __nv_bfloat16* oo = (__nv_bfloat16*)out;
   {
+    const bool apart = min_q_len > 0 && min_q_len < prefill_tc_rows() && max_q_len >= prefill_tc_rows();
     const int rc = launch_prefill_tc_ex(qq, kk, vv, oo, seq_q_start, seq_q_len, seq_ctx_len, table_row0, n_seqs, max_q_len,
-                                        n_tokens, n_heads, pv, scale, window, opt, status, stream);
-    if (rc != MF_ERR_BAD_ARG) return rc;
+                                        n_tokens, n_heads, pv, scale, window, opt, apart ? prefill_tc_rows() : 0, status, stream);
+    if (rc != MF_ERR_BAD_ARG && (rc || !apart)) return rc;
+    if (rc == 0) {
+      opt.below = prefill_tc_rows();
+      max_q_len = opt.below - 1;
+    }
   }
   if (hd <= 64)
     return launch_prefill<64>(qq, kk, vv, oo, seq_q_start, seq_q_len, seq_ctx_len, table_row0, n_seqs, max_q_len,

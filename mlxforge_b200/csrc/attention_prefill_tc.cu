@@ -250,6 +250,7 @@ struct TcOptions {
   const float* sink;
   const __nv_bfloat16* gate;
   long long gate_ld;
+  int min_len;              // only portions of at least so many tokens
 };
 // eight results of a row times sigmoid of eight gates (16-byte aligned)
 __device__ __forceinline__ void apply_gate(float* v, const __nv_bfloat16* g) {
@@ -285,7 +286,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   // all heads before any lighter tile
   const int tile = (int)gridDim.y - 1 - (int)blockIdx.y, head = blockIdx.x, s = blockIdx.z;
   const int q_len = seq_q_len[s];
-  if (tile * BM >= q_len) return;
+  if (tile * BM >= q_len || (EX && q_len < opt.min_len)) return;
   if (q_u & 1023u) {                                       // never seen; refused rather than computed wrongly
     if (threadIdx.x == 0 && status) atomicExch(status, 40);
     return;
@@ -784,7 +785,7 @@ __global__ void __launch_bounds__(192, 1)
 attn_prefill_latent_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                            __nv_bfloat16* __restrict__ out, const int* __restrict__ seq_q_start,
                            const int* __restrict__ seq_q_len, const int* __restrict__ seq_ctx_len, int table_row0, PagedView pv,
-                           int n_heads, int vd, float scale_log2, int window, int* __restrict__ status) {
+                           int n_heads, int vd, float scale_log2, int window, int min_len, int* __restrict__ status) {
   using namespace latent;
   constexpr int RING = ring(SPANS), STAGE_BYTES = SPANS * K_SPAN_BYTES, Q_BYTES = SPANS * Q_SPAN_BYTES;
   constexpr int COLS = 2 * SUB + VSPANS * 64 <= 256 ? 256 : 512;
@@ -799,7 +800,7 @@ attn_prefill_latent_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tile = (int)gridDim.y - 1 - (int)blockIdx.y, head = blockIdx.x, s = blockIdx.z;
   const int q_len = seq_q_len[s];
-  if (tile * BM >= q_len) return;
+  if (tile * BM >= q_len || q_len < min_len) return;
   if (q_u & 1023u) {
     if (threadIdx.x == 0 && status) atomicExch(status, 40);
     return;
@@ -995,7 +996,7 @@ attn_prefill_latent_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 template <int SPANS, int VSPANS>
 int launch_latent(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, __nv_bfloat16* out, const int* seq_q_start,
                   const int* seq_q_len, const int* seq_ctx_len, int table_row0, int n_seqs, int max_q_len, int n_tokens,
-                  int n_heads, PagedView pv, int vd, float scale, int window, int* status, cudaStream_t stream) {
+                  int n_heads, PagedView pv, int vd, float scale, int window, int min_len, int* status, cudaStream_t stream) {
   CUtensorMap mq, mk;
   int rc = tma_host::bf16_map(q, n_tokens, (long long)n_heads * pv.head_dim, BM, 64, &mq);
   if (rc) return rc;
@@ -1013,7 +1014,7 @@ int launch_latent(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, __nv_bflo
   dim3 grid(n_heads, (max_q_len + BM - 1) / BM, n_seqs);
   mf_count(MF_K_ATTN_PREFILL_TC);
   attn_prefill_latent_kernel<SPANS, VSPANS><<<grid, 192, latent::smem(SPANS), stream>>>(
-      mq, mk, out, seq_q_start, seq_q_len, seq_ctx_len, table_row0, pv, n_heads, vd, scale * LOG2E, window, status);
+      mq, mk, out, seq_q_start, seq_q_len, seq_ctx_len, table_row0, pv, n_heads, vd, scale * LOG2E, window, min_len, status);
   return (int)cudaGetLastError();
 }
 
@@ -1043,20 +1044,23 @@ int launch_prefill_tc(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const
   return MF_ERR_BAD_ARG;
 }
 
-// The same for attention with options; MF_ERR_BAD_ARG where the mma.sync kernel is the way: portions below 128 tokens, a soft
+// Tokens of a tile of queries, and of the portions from which these kernels are taken.
+int prefill_tc_rows() { return BM; }
+
+// The same for attention with options; portions below `min_len` tokens are left out.  MF_ERR_BAD_ARG where the mma.sync kernel is the way: portions below 128 tokens, a soft
 // cap, separate values of another size than head size 128, values inside the keys together with kept keys, a sink or
 // a gate, a gate off its 16-byte boundary.
 int launch_prefill_tc_ex(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __nv_bfloat16* v_pool,
                          __nv_bfloat16* out, const int* seq_q_start, const int* seq_q_len, const int* seq_ctx_len,
                          int table_row0, int n_seqs, int max_q_len, int n_tokens, int n_heads, PagedView pv,
-                         float scale, int window, const AttnOptions& opt, int* status, cudaStream_t stream) {
+                         float scale, int window, const AttnOptions& opt, int min_len, int* status, cudaStream_t stream) {
   if (!g_prefill_tc || pv.page_size % 16 || max_q_len < BM || n_tokens <= 0 || opt.softcap > 0.f) return MF_ERR_BAD_ARG;
   if ((((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool) & 15) != 0 || (max_q_len + BM - 1) / BM > 65535) return MF_ERR_BAD_ARG;
   const int hd = pv.head_dim, vd = opt.vd;
   if (!opt.v_in_k) {
     if (hd != 128 || vd != 128 || ((uintptr_t)v_pool & 15) || (opt.gate && (((uintptr_t)opt.gate & 15) || opt.gate_ld % 8)))
       return MF_ERR_BAD_ARG;
-    const TcOptions o{opt.keep_first, opt.sink, opt.gate, opt.gate_ld};
+    const TcOptions o{opt.keep_first, opt.sink, opt.gate, opt.gate_ld, min_len};
     return launch_tc<128, 64, true>(q, k_pool, v_pool, out, seq_q_start, seq_q_len, seq_ctx_len, table_row0, n_seqs, max_q_len,
                                     n_tokens, n_heads, pv, scale, window, status, o, stream);
   }
@@ -1064,7 +1068,7 @@ int launch_prefill_tc_ex(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, co
 #define LATENT_GO(S, V)                                                                                                     \
   if ((hd + 63) / 64 == S && (vd + 63) / 64 == V)                                                                           \
   return launch_latent<S, V>(q, k_pool, out, seq_q_start, seq_q_len, seq_ctx_len, table_row0, n_seqs, max_q_len, n_tokens,  \
-                             n_heads, pv, vd, scale, window, status, stream)
+                             n_heads, pv, vd, scale, window, min_len, status, stream)
   LATENT_GO(2, 1);
   LATENT_GO(2, 2);
   LATENT_GO(3, 1);

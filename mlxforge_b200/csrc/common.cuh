@@ -157,6 +157,7 @@ struct AttnOptions {
   const __nv_bfloat16* gate;
   long long gate_ld;
   float softcap;
+  int below;         // portions of prompts: only those of fewer tokens (0: all)
 };
 // A raw dot product d (not yet scaled) under a soft cap, returned in the same unscaled units, so that
 // the kernel's own multiplication by the scale gives cap * tanh(d * scale / cap).

@@ -236,15 +236,17 @@ def attention_prefill_ex(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Te
                          table_row0: int, max_q_len: int, block_table: torch.Tensor, page_size: int, n_heads: int,
                          n_kv: int, head_dim: int, scale: float, window: int, v_dim: int, v_in_k: bool,
                          keep_first: int = 0, sink: Optional[torch.Tensor] = None,
-                         gate: Optional[torch.Tensor] = None, gate_ld: int = 0, softcap: float = 0.0) -> None:
+                         gate: Optional[torch.Tensor] = None, gate_ld: int = 0, softcap: float = 0.0,
+                         min_q_len: int = 0) -> None:
     """``attention_prefill`` with options: values ``v_dim`` wide (``v_in_k``: the first channels of the keys),
-    kept first keys, a sink per head, the output times sigmoid(``gate``).  bfloat16."""
+    kept first keys, a sink per head, the output times sigmoid(``gate``).  bfloat16.  ``min_q_len``: the shortest portion, where it
+    is known; portions on both sides of 128 tokens then go through a kernel each."""
     _need_cuda(q, k_pool, v_pool, out, seq_q_start, seq_q_len, seq_ctx_len, block_table, sink)
     if q.dtype != torch.bfloat16 or k_pool.dtype != torch.bfloat16:
         raise KernelError("attention_prefill_ex: bfloat16 only")
     check(library().mf_attention_prefill_ex(q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(),
                                             seq_q_start.data_ptr(), seq_q_len.data_ptr(), seq_ctx_len.data_ptr(),
-                                            table_row0, seq_q_len.shape[0], max_q_len, q.shape[0], n_heads, n_kv, head_dim,
+                                            table_row0, seq_q_len.shape[0], min_q_len, max_q_len, q.shape[0], n_heads, n_kv, head_dim,
                                             block_table.data_ptr(), block_table.shape[1], page_size, scale, window,
                                             v_dim, int(v_in_k), keep_first, _ptr(sink), _ptr(gate), gate_ld,
                                             float(softcap or 0.0), kernel_status(q.device).data_ptr(), _stream()),

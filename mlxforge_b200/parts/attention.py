@@ -158,7 +158,7 @@ def options_paged_attention(rt, batch, q, lane, out, n_heads: int, scale: float,
         ops.attention_prefill_ex(q, lane.k, lane.v, out, batch.seq_q_start[nd:], batch.seq_q_len[nd:],
                                  batch.seq_ctx_len[nd:], nd, max(batch.q_len[nd:]), table, lane.page_size, n_heads,
                                  need.n_kv_heads, need.head_dim, scale, window, vd, in_k, keep_first, sink, gate,
-                                 gate_ld, softcap)
+                                 gate_ld, softcap, min(n for n in batch.q_len[nd:] if n))
 
 
 _SINK_NAMES = {"q": "q", "k": "k", "v": "v", "g": "g", "o": "o", "sink": "sink"}

@@ -1067,3 +1067,45 @@ def test_attention_f32_a_token_alone_and_beside_a_portion():
         ops.attention_f32(q, k, v, o, batch, dev(table), page, heads, kv, hd, hd ** -0.5, 0, hd, hd)
         out.append(o[:3])
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("lens", [[40, 300], [20, 130, 64, 500], [127, 128]])
+@pytest.mark.parametrize("hd,vd,in_k,window,keep,softcap", [(128, 128, False, 100, 4, 0.0), (224, 192, True, 0, 0, 0.0), (64, 64, False, 50, 0, 0.0),
+                                                            (128, 128, False, 0, 0, 9.0)])
+def test_a_portion_has_the_same_bits_alone_and_beside_longer_ones(lens, hd, vd, in_k, window, keep, softcap):
+    """Attention with options: portions below 128 tokens take the mma.sync kernel and the others the tcgen05 one whatever the step
+    holds (sizes and options that the latter does not take go through the former whole)."""
+    import torch
+    from types import SimpleNamespace
+    from mlxforge_b200.csrc import binding, ops
+    from mlxforge_b200.engine.runtime import Runtime
+    from mlxforge_b200.parts.attention import options_paged_attention
+    rng, bf, page, heads, kv = np.random.default_rng(hd), torch.bfloat16, 16, 4, 1 if in_k else 2
+    i32 = lambda a: dev(np.asarray(a, np.int32))
+    blocks = [-(-c // page) for c in lens]
+    table, at = np.full((len(lens), max(blocks)), -1, np.int32), 0
+    for i, b in enumerate(blocks):
+        table[i, :b], at = np.arange(at, at + b), at + b
+    k = dev(rng.standard_normal((at, kv, page, hd)).astype(np.float32), bf)
+    v = k if in_k else dev(rng.standard_normal((at, kv, page, vd)).astype(np.float32), bf)
+    q = dev(rng.standard_normal((sum(lens), heads * hd)).astype(np.float32), bf)
+    lane = SimpleNamespace(need=SimpleNamespace(n_kv_heads=kv, head_dim=hd, value_dim=vd, values_in_keys=in_k), group=0, k=k, v=v, page_size=page)
+    starts = np.cumsum([0] + lens[:-1])
+
+    def run(which):
+        own = [lens[i] for i in which]
+        batch = SimpleNamespace(n_decode=0, n_tokens=sum(own), n_seqs=len(own), q_len=own, seq_q_start=i32(np.cumsum([0] + own[:-1])),
+                                seq_q_len=i32(own), seq_ctx_len=i32(own), block_table=lambda g: dev(table[which]))
+        out = torch.full((sum(own), heads * vd), float("nan"), dtype=bf, device="cuda")
+        options_paged_attention(Runtime(bf), batch, torch.cat([q[starts[i]:starts[i] + lens[i]] for i in which]), lane, out, heads,
+                                hd ** -0.5, window, keep, softcap=softcap)
+        return out
+
+    before = binding.kernel_launches()
+    together = run(list(range(len(lens))))
+    ran = {n: c - before[n] for n, c in binding.kernel_launches().items() if c - before[n]}
+    both = hd > 64 and not softcap
+    assert ran == {"attn_prefill_mma": 1, **({"attn_prefill_tc": 1} if both else {})}, ran
+    ops.check_kernel_status()
+    for i, n in enumerate(lens):
+        assert torch.equal(run([i]), together[starts[i]:starts[i] + n]), n
