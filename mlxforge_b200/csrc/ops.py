@@ -205,9 +205,10 @@ def attention_generic_ex(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Te
 
 
 def attention_f32_ok(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, n_heads: int, n_kv: int, head_dim: int,
-                     v_dim: int, v_ld: int) -> bool:
-    """Whether ``attention_f32`` takes these operands: 32-bit, rows in whole 16-byte pieces, at most 256 channels."""
-    return (q.dtype == torch.float32 and k_pool.dtype == torch.float32
+                     v_dim: int, v_ld: int, n_seqs: int = 1) -> bool:
+    """Whether ``attention_f32`` takes these operands: 32-bit, rows in whole 16-byte pieces, at most 256 channels, at most
+    65,535 sequences."""
+    return (q.dtype == torch.float32 and k_pool.dtype == torch.float32 and n_seqs <= 65535
             and not (q.data_ptr() | k_pool.data_ptr() | v_pool.data_ptr()) % 16
             and bool(library().mf_attention_f32_ok(n_heads, n_kv, head_dim, v_dim, v_ld)))
 

@@ -26,7 +26,8 @@ def paged_attention(rt, batch, q, lane, out, n_heads: int, scale: float, window:
     prefill kernel.  float32: the tiled 32-bit kernel for all, the generic one at sizes it does not take."""
     need = lane.need
     table = batch.block_table(lane.group)
-    if ops.attention_f32_ok(q, lane.k, lane.v, n_heads, need.n_kv_heads, need.head_dim, need.head_dim, need.head_dim):
+    if ops.attention_f32_ok(q, lane.k, lane.v, n_heads, need.n_kv_heads, need.head_dim, need.head_dim, need.head_dim,
+                            batch.n_seqs):
         ops.attention_f32(q, lane.k, lane.v, out, batch, table, lane.page_size, n_heads, need.n_kv_heads, need.head_dim,
                           scale, window, need.head_dim, need.head_dim)
         return
@@ -137,7 +138,7 @@ def options_paged_attention(rt, batch, q, lane, out, n_heads: int, scale: float,
     table = batch.block_table(lane.group)
     vd, in_k = need.value_dim, need.values_in_keys
     v_ld = need.head_dim if in_k else vd
-    if ops.attention_f32_ok(q, lane.k, lane.v, n_heads, need.n_kv_heads, need.head_dim, vd, v_ld):
+    if ops.attention_f32_ok(q, lane.k, lane.v, n_heads, need.n_kv_heads, need.head_dim, vd, v_ld, batch.n_seqs):
         ops.attention_f32(q, lane.k, lane.v, out, batch, table, lane.page_size, n_heads, need.n_kv_heads, need.head_dim,
                           scale, window, vd, v_ld, keep_first, sink, gate, gate_ld, softcap)
         return

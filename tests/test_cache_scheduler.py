@@ -563,3 +563,11 @@ def test_room_for_runs_and_chunks_holds_every_step_of_the_budget():
         worst[0] = max(worst[0], sum(-(-n // 16) for n in lens if n >= ops.DELTA_RUNS_MIN_TOKENS) * per_run)
         worst[1] = max(worst[1], sum(-(-n // 64) for n in lens if n >= ops.RETENTION_CHUNKED_MIN_TOKENS) * heads * 128 * 64)
     assert 0.8 * runs_room < worst[0] <= runs_room and 0.8 * chunks_room < worst[1] <= chunks_room, (worst, runs_room, chunks_room)
+
+
+def test_float32_attention_over_more_sequences_than_a_grid_holds_goes_token_by_token():
+    import torch
+    from mlxforge_b200.csrc import ops
+    q, k = torch.zeros(4, 64), torch.zeros(2, 1, 16, 64)
+    assert ops.attention_f32_ok(q, k, k, 1, 1, 64, 64, 64, 65535)
+    assert not ops.attention_f32_ok(q, k, k, 1, 1, 64, 64, 64, 65536)
