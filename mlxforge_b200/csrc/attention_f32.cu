@@ -310,6 +310,7 @@ MF_API int mf_attention_f32(const float* q, const float* k_pool, const float* v_
       (((uintptr_t)k_pool) & 15) || (((uintptr_t)v_pool) & 15))
     return MF_ERR_BAD_ARG;
   mf_count(MF_K_ATTN_GENERIC);
+  mf_count(MF_K_ATTN_F32);
   const int rep = n_heads / n_kv, vc = (vd + 63) / 64;
   // where 16 rows hold all there is, as in decoding, a tile does a quarter of the work
   const bool few = (long long)max_q_len * rep <= 16;

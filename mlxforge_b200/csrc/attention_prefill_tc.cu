@@ -1013,6 +1013,7 @@ int launch_latent(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, __nv_bflo
   }
   dim3 grid(n_heads, (max_q_len + BM - 1) / BM, n_seqs);
   mf_count(MF_K_ATTN_PREFILL_TC);
+  mf_count(MF_K_ATTN_PREFILL_LATENT);
   attn_prefill_latent_kernel<SPANS, VSPANS><<<grid, 192, latent::smem(SPANS), stream>>>(
       mq, mk, out, seq_q_start, seq_q_len, seq_ctx_len, table_row0, pv, n_heads, vd, scale * LOG2E, window, min_len, status);
   return (int)cudaGetLastError();

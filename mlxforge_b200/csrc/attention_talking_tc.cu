@@ -676,6 +676,7 @@ static int tt_decode(const TtArgs& a, int n_seqs, cudaStream_t stream) {
     if (e != cudaSuccess) return (int)e;
     once.done[d] = true;
   }
+  mf_count(MF_K_ATTN_TALKING_DECODE);
   int rc = (int)launch_dep(talking_decode_kernel<VDIM>, dim3(a.splits, n_seqs), dim3(256), smem, stream, a);
   if (rc != 0) return rc;
   mf_count(MF_K_ATTN_TALKING_MERGE);

@@ -212,7 +212,8 @@ def count_launches(n: int) -> None:
 
 def kernel_launches() -> dict:
     """How often each kind of kernel has been launched by this process, by name (a launch
-    recorded into a CUDA graph counts once, its replays do not).  Tests of whole models use
+    recorded into a CUDA graph counts once, its replays do not; the last names are kernels that are
+    counted under their kind as well).  Tests of whole models use
     the difference of two readings to say which kernels a model's steps went through."""
     lib = library()
     return {lib.mf_kernel_name(i).decode(): int(lib.mf_kernel_launches(i)) for i in range(lib.mf_kernel_kinds())}

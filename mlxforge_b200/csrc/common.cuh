@@ -269,6 +269,14 @@ enum MfKernel {
   MF_K_POST_NORM,             // a sublayer's output through a norm of its own into the stream, and the stream's next norm
   MF_K_QKV_CONV,              // convolved projections: norm per head, rotation, the cache write
   MF_K_SOFT_CAP,              // cap tanh(x / cap) on rows of logits
+  // kernels of a kind above that a test has to tell from the kind's others: counted there and here
+  MF_K_ATTN_F32,              // attn_generic: the tiled 32-bit kernel
+  MF_K_ATTN_PREFILL_LATENT,   // attn_prefill_tc: values inside the keys
+  MF_K_ATTN_TALKING_DECODE,   // attn_talking_tc: one token of every sequence, query heads as rows
+  MF_K_DELTA_RUNS,            // delta_recurrence: over runs of tokens as products
+  MF_K_DELTA_STEP,            // delta_recurrence: one token of every sequence
+  MF_K_RETENTION_STEP,        // retention_recurrence: one token of every sequence
+  MF_K_MOE_GROUPED_TC,        // moe_grouped: the tcgen05 products
   MF_K_COUNT
 };
 extern unsigned long long g_mf_kernel_launches[MF_K_COUNT];

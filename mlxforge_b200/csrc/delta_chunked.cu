@@ -478,6 +478,7 @@ MF_API int mf_delta_recurrence_runs(const float* qkv, const float* beta, const f
   if (!mf_delta_runs_ok(dim, vdim) || n_kv <= 0 || n_heads % n_kv || n_heads > 65535 || ((uintptr_t)scratch & 15))
     return MF_ERR_BAD_ARG;
   mf_count(MF_K_DELTA_RECURRENCE);
+  mf_count(MF_K_DELTA_RUNS);
   // blocks of 8 columns where blocks of 16 would leave half of the SMs without one (a run takes 0.83 us instead of
   // 1.12 us, so two blocks of 8 after one another are slower than one of 16)
   const int nc = (long long)n_seqs * n_heads * (vdim / 16) * 2 <= mf_sm_count() ? 8 : 16;

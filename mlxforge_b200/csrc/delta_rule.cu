@@ -628,6 +628,7 @@ MF_API int mf_delta_recurrence(const float* qkv, const float* beta, const float*
   dim3 grid(n_seqs, n_heads, (vdim + DR_COLS - 1) / DR_COLS);
   mf_count(MF_K_DELTA_RECURRENCE);
   if (one_each && mf_delta_step_ok(dim, vdim)) {
+    mf_count(MF_K_DELTA_STEP);
     const dim3 step_grid(n_seqs, n_heads, vdim / 32);
     return (int)launch_dep(dim == 64 ? delta_step_kernel<64> : delta_step_kernel<128>, step_grid, dim3(128), 0, stream, qkv, beta,
                            ag, ag_ld, state, state_stride, seq_q_start, slots, o_out, n_heads, n_kv, vdim);

@@ -266,6 +266,7 @@ int launch(const void* w, long long w_rows, const void* b, int n_pairs, const in
     once.done[dev] = true;
   }
   mf_count(MF_K_MOE_GROUPED);
+  mf_count(MF_K_MOE_GROUPED_TC);
   moe_tc_kernel<MODE><<<max_units < n_sms ? max_units : n_sms, 320, Ring<MODE>::SMEM, stream>>>(
       mw, mb, meta, tiles, out, rows_w, stride_w, K, act_kind, ec, status);
   return (int)cudaGetLastError();

@@ -337,6 +337,7 @@ MF_API int mf_retention_recurrence(const float* qk, const void* v, int v_dtype, 
     if (!mf_retention_step_ok(dim, vdim)) return MF_ERR_BAD_ARG;
     if (v_dtype != MF_F32 && v_dtype != MF_BF16) return MF_ERR_BAD_DTYPE;
     mf_count(MF_K_RETENTION_RECURRENCE);
+    mf_count(MF_K_RETENTION_STEP);
     const dim3 step_grid(n_seqs, n_heads, vdim / 32);
     if (v_dtype == MF_F32)
       return (int)launch_dep(dim == 64 ? retention_step_kernel<float, 64> : retention_step_kernel<float, 128>, step_grid,

@@ -210,7 +210,7 @@ def test_attention_f32_against_the_block_per_token_kernel(form):
     largest result."""
     import torch
     from types import SimpleNamespace
-    from mlxforge_b200.csrc import ops
+    from mlxforge_b200.csrc import binding, ops
     heads, kv, hd, vd, in_k, seqs, window, keep, has_sink, has_gate, cap = form
     rng = np.random.default_rng(hd + heads)
     page, T = 16, sum(n for n, _ in seqs)
@@ -244,8 +244,10 @@ def test_attention_f32_against_the_block_per_token_kernel(form):
     of = np.concatenate([np.full(n, i) for i, (n, _) in enumerate(seqs)])
     got, want = (torch.full((T, heads * vd), float("nan"), device="cuda") for _ in range(2))
     assert ops.attention_f32_ok(q, k_pool, v_pool, heads, kv, hd, vd, v_ld)
+    before = binding.kernel_launches()["attn_f32"]
     ops.attention_f32(q, k_pool, v_pool, got, batch, dev(table), page, heads, kv, hd, hd ** -0.5, window, vd, v_ld, keep, sink,
                       gate, gate_ld, cap)
+    assert binding.kernel_launches()["attn_f32"] == before + 1
     ops.attention_generic_ex(q, k_pool, v_pool, want, i32(pos), i32(of), dev(table), page, heads, kv, hd, hd ** -0.5, window, vd,
                              v_ld, keep, sink, gate, gate_ld, cap)
     assert torch.isfinite(want).all()
@@ -998,11 +1000,12 @@ def test_prefill_options_on_tcgen05(form):
     gate, gate_ld = (gates[:, 8:], heads * vd + 8) if has_gate else (None, 0)
     starts = np.cumsum([0] + [n for n, _ in seqs[:-1]])
     got, want = (torch.full((T, heads * vd), float("nan"), device="cuda", dtype=bf) for _ in range(2))
-    before = binding.kernel_launches()["attn_prefill_tc"]
+    before, latent = (binding.kernel_launches()[n] for n in ("attn_prefill_tc", "attn_prefill_latent"))
     ops.attention_prefill_ex(q, k_pool, v_pool, got, i32(starts), i32([n for n, _ in seqs]), i32([c for _, c in seqs]), 0,
                              max(n for n, _ in seqs), dev(table), page, heads, kv, hd, hd ** -0.5, window, vd, in_k, keep, sink,
                              gate, gate_ld)
     assert binding.kernel_launches()["attn_prefill_tc"] == before + 1
+    assert binding.kernel_launches()["attn_prefill_latent"] == latent + in_k
     ops.check_kernel_status()
     pos = np.concatenate([np.arange(c - n, c) for n, c in seqs])
     of = np.concatenate([np.full(n, i) for i, (n, _) in enumerate(seqs)])
@@ -1104,8 +1107,8 @@ def test_a_portion_has_the_same_bits_alone_and_beside_longer_ones(lens, hd, vd, 
     before = binding.kernel_launches()
     together = run(list(range(len(lens))))
     ran = {n: c - before[n] for n, c in binding.kernel_launches().items() if c - before[n]}
-    both = hd > 64 and not softcap
-    assert ran == {"attn_prefill_mma": 1, **({"attn_prefill_tc": 1} if both else {})}, ran
+    both = {"attn_prefill_tc": 1, **({"attn_prefill_latent": 1} if in_k else {})} if hd > 64 and not softcap else {}
+    assert ran == {"attn_prefill_mma": 1, **both}, ran
     ops.check_kernel_status()
     for i, n in enumerate(lens):
         assert torch.equal(run([i]), together[starts[i]:starts[i] + n]), n

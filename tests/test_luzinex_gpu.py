@@ -582,7 +582,7 @@ def test_retention_over_chunks_and_of_one_token_each(lens, heads, dim, vdim, dty
     a chain of at most ~350 roundings of 2^-24, which add like a random walk: 2e-6 of the norm of what was added up."""
     import torch
     from types import SimpleNamespace
-    from mlxforge_b200.csrc import ops
+    from mlxforge_b200.csrc import binding, ops
     rng = np.random.default_rng(sum(lens))
     T, ld = sum(lens), heads * vdim + 24
     dev = lambda a, t=None: torch.from_numpy(np.ascontiguousarray(a)).cuda().to(t or torch.from_numpy(a).dtype)
@@ -598,7 +598,9 @@ def test_retention_over_chunks_and_of_one_token_each(lens, heads, dim, vdim, dty
     chunks = ops.retention_chunks(batch, heads, dim, vdim, v, ld, st)
     if max(lens) == 1:
         assert chunks == 0 and ops.retention_parts(dim, vdim, v, ld, batch) == 1
+        before = binding.kernel_launches()["retention_step"]
         ops.retention_recurrence(dev(qk), v, ld, dev(decay), st, batch, o, heads, dim, vdim)
+        assert binding.kernel_launches()["retention_step"] == before + 1
     else:
         assert chunks == sum(-(-n // 64) for n in lens)
         ops.retention_chunked(dev(qk), v, ld, dev(decay), st, batch, o, heads, dim, vdim, chunks,

@@ -399,8 +399,8 @@ def test_router_kernel(E, groups, keep, top):
 @pytest.mark.parametrize("H,ff,E,groups,keep,top,T", [(40, 24, 6, 3, 2, 2, 9), (64, 64, 8, 0, 0, 3, 150),
                                                        (128, 32, 16, 4, 2, 4, 300), (72, 20, 5, 0, 0, 1, 70)])
 def test_routed_experts_part(dtype, H, ff, E, groups, keep, top, T, own_tiles, monkeypatch):
-    """``own_tiles``: many tokens in bfloat16 through this engine's own tensor-core tiles instead of the
-    library's grouped product (the other cases take the same kernels either way)."""
+    """``own_tiles``: many tokens in bfloat16 through the mma.sync tiles instead of the tcgen05 products (the other
+    cases take the same kernels either way)."""
     from mlxforge_b200.csrc import binding
     from mlxforge_b200.engine.runtime import Runtime
     if own_tiles and (dtype != "bfloat16" or T < 64 or H % 8 or ff % 8):
@@ -427,7 +427,8 @@ def test_routed_experts_part(dtype, H, ff, E, groups, keep, top, T, own_tiles, m
     assert np.max(np.abs(got - want)) < tol(dtype, np.abs(want).max())
     ran = {k: v - before[k] for k, v in binding.kernel_launches().items() if v - before[k]}
     if dtype == "bfloat16" and T >= 64 and H % 8 == 0 and ff % 8 == 0:
-        assert ran.get("moe_grouped", 0) == (2 if own_tiles else 2) and ran.get("moe_sort", 0) == 1, ran
+        assert ran.get("moe_grouped", 0) == 2 and ran.get("moe_sort", 0) == 1, ran
+        assert ran.get("moe_grouped_tc", 0) == (0 if own_tiles else 2), ran
     else:
         assert ran.get("moe_rows", 0) == 1, ran
     # each token alone gives the same as inside the batch
@@ -524,7 +525,7 @@ def test_every_request_decoded_from_its_first_token(models, which, dtype, tmp_pa
 @pytest.mark.parametrize("own_tiles", [False, True])
 def test_serving_shapes_take_the_fast_kernels(models, tmp_path, own_tiles, monkeypatch):
     """Configuration C in bfloat16: which kernels its prompts and its decoding go through, with the experts of
-    many tokens through the library's grouped product and through this engine's own tiles."""
+    many tokens through the tcgen05 products and through the mma.sync tiles."""
     monkeypatch.setenv("MLXFORGE_MOE_TILES", "1" if own_tiles else "0")
     reqs = models[("C", False)][2]
     ran = _check(models, "C", False, "bfloat16", TT.decode_tail(reqs, tail=8), tmp_path)
@@ -532,6 +533,7 @@ def test_serving_shapes_take_the_fast_kernels(models, tmp_path, own_tiles, monke
         assert ran.get(k, 0) > 0, (k, ran)
     assert ran.get("attn_talking_tc", 0) > 0 and ran.get("attn_talking_merge", 0) > 0, ran
     assert ran.get("moe_grouped", 0) > 0 and ran.get("moe_rows", 0) > 0, ran
+    assert (ran.get("moe_grouped_tc", 0) > 0) != own_tiles, ran
 
 
 # ----------------------------------------------------------------------------- generation through the entry point
@@ -722,6 +724,9 @@ def test_talking_kernels_mix_in_32_bits(heads, kv, dim, vdim, chunk, window, cap
     before = dict(ops_launches())
     talking_paged_attention(Runtime(bf), batch, q, lane, got, m)
     assert ops_launches()["attn_talking_tc"] > before["attn_talking_tc"]
+    fits = kv * 64 * (vdim + 8) * 2 + heads * (68 * 4 + 72 * 2) <= 200 * 1024        # the values of a split of 64 keys, scores, weights
+    decode = ops_launches()["attn_talking_decode"] - before["attn_talking_decode"]
+    assert decode == (1 if batch.n_decode and fits else 0)
     pos = np.concatenate([np.arange(c - n, c) for n, c in seqs])
     ops.attention_talking(q, lane.k, lane.v, want, i32(pos), i32(np.repeat(np.arange(len(seqs)), lens)), dev(table), page, heads, kv,
                           dim, vdim, m.scale, cap, m.talk, window, chunk)
@@ -800,7 +805,9 @@ def test_delta_step_against_the_rule(n, heads, n_kv, dim, vdim):
     slots = np.arange(n)[::-1]
     st, o = dev(state), torch.full((n, heads * vdim), np.nan, device="cuda")
     batch = SimpleNamespace(q_len=[1] * n, n_seqs=n, seq_q_start=i32(np.arange(n)), seq_q_len=i32(np.ones(n)), slots=i32(slots))
+    before = ops_launches()["delta_step"]
     ops.delta_recurrence(dev(qkv), dev(beta), dev(ag), st, batch, o, heads, n_kv, dim, vdim)
+    assert ops_launches()["delta_step"] == before + 1
     d, rep = lambda a: a.astype(np.float64), heads // n_kv
     for t in range(n):
         q, k = (np.repeat(d(qkv[t, i * n_kv * dim:(i + 1) * n_kv * dim]).reshape(n_kv, dim), rep, axis=0) for i in (0, 1))
