@@ -856,7 +856,7 @@ LEDINEX_SIZES = {
               context=4096),
 }
 LEDINEX_KERNELS = ("embed", "conv_input", "postnorm_add", "qk_norm_rope", "rotate_rows", "attention_prefill_ex",
-                   "attention_decode_ex", "attention_generic_ex", "retention_prepare", "retention_recurrence",
+                   "attention_decode_ex", "attention_generic_ex", "retention_prepare", "retention_recurrence", "retention_chunked",
                    "retention_output", "gdelta_prepare", "gdelta_recurrence", "delta_gates_ex", "delta_prepare",
                    "delta_recurrence", "delta_recurrence_runs", "delta_output", "moe_route", "moe_rows", "moe_combine", "moe_sort",
                    "moe_grouped_up", "moe_grouped_down", "moe_tc_up", "moe_tc_down", "unary_act", "add_rmsnorm",
