@@ -1077,7 +1077,7 @@ def test_attention_f32_a_token_alone_and_beside_a_portion():
                                                             (128, 128, False, 0, 0, 9.0)])
 def test_a_portion_has_the_same_bits_alone_and_beside_longer_ones(lens, hd, vd, in_k, window, keep, softcap):
     """Attention with options: portions below 128 tokens take the mma.sync kernel and the others the tcgen05 one whatever the step
-    holds (sizes and options that the latter does not take go through the former whole)."""
+    holds (sizes and options that the latter does not take go through the former whole), behind 500 tokens each."""
     import torch
     from types import SimpleNamespace
     from mlxforge_b200.csrc import binding, ops
@@ -1085,7 +1085,8 @@ def test_a_portion_has_the_same_bits_alone_and_beside_longer_ones(lens, hd, vd, 
     from mlxforge_b200.parts.attention import options_paged_attention
     rng, bf, page, heads, kv = np.random.default_rng(hd), torch.bfloat16, 16, 4, 1 if in_k else 2
     i32 = lambda a: dev(np.asarray(a, np.int32))
-    blocks = [-(-c // page) for c in lens]
+    ctx = [n + 500 for n in lens]
+    blocks = [-(-c // page) for c in ctx]
     table, at = np.full((len(lens), max(blocks)), -1, np.int32), 0
     for i, b in enumerate(blocks):
         table[i, :b], at = np.arange(at, at + b), at + b
@@ -1098,7 +1099,7 @@ def test_a_portion_has_the_same_bits_alone_and_beside_longer_ones(lens, hd, vd, 
     def run(which):
         own = [lens[i] for i in which]
         batch = SimpleNamespace(n_decode=0, n_tokens=sum(own), n_seqs=len(own), q_len=own, seq_q_start=i32(np.cumsum([0] + own[:-1])),
-                                seq_q_len=i32(own), seq_ctx_len=i32(own), block_table=lambda g: dev(table[which]))
+                                seq_q_len=i32(own), seq_ctx_len=i32([ctx[i] for i in which]), block_table=lambda g: dev(table[which]))
         out = torch.full((sum(own), heads * vd), float("nan"), dtype=bf, device="cuda")
         options_paged_attention(Runtime(bf), batch, torch.cat([q[starts[i]:starts[i] + lens[i]] for i in which]), lane, out, heads,
                                 hd ** -0.5, window, keep, softcap=softcap)
