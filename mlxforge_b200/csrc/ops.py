@@ -365,25 +365,41 @@ def set_retention_rows(rows: int) -> None:
 
 
 def sequence_groups(batch, kind, cost=None, limit: int = 0):
-    """The step's sequences in groups of neighbours that ``kind(tokens)`` names alike, as ``(kind, batch, first token, end)``
-    with a batch of the group's own sequences.  Kernels that are chosen by the length of a portion are given a group each, so that
-    a sequence's numbers are a matter of its own tokens and not of what else is in the step.  Sequences without a token are left
-    out.  ``cost(tokens)``: a group ends where its costs would add up to more than ``limit``."""
-    groups, t = [], 0                 # [kind, first sequence, end, first token, end, cost]
-    for i, n in enumerate(batch.q_len):
+    """The step's sequences in groups that ``kind(tokens)`` names alike, as ``(kind, batch, rows)`` with a batch of the group's own
+    sequences and the ranges of the step's tokens that are theirs.  Kernels that are chosen by the length of a portion are given a
+    group each, so that a sequence's numbers are a matter of its own tokens and not of what else is in the step.  A group is
+    neighbours in the order of length where the batch has its arrays in that order (``by_length``), else neighbours in the step.
+    Sequences without a token are left out.  ``cost(tokens)``: a group ends where its costs would add up to more than ``limit``."""
+    lens, arrays = batch.q_len, getattr(batch, "by_length", None)
+    order = range(len(lens)) if arrays is None else arrays.order
+    groups = []                       # [kind, first place in the order, end, cost]
+    for place, i in enumerate(order):
+        n = lens[i]
         if n:
             k, c = kind(n), cost(n) if cost else 0
             g = groups[-1] if groups else None
-            if g is None or g[0] != k or g[2] != i or g[5] + c > limit:
-                groups.append([k, i, i + 1, t, t + n, c])
+            if g is None or g[0] != k or g[2] != place or g[3] + c > limit:
+                groups.append([k, place, place + 1, c])
             else:
-                g[2], g[4], g[5] = i + 1, t + n, g[5] + c
-            t += n
+                g[2], g[3] = place + 1, g[3] + c
     if len(groups) == 1 and groups[0][2] - groups[0][1] == batch.n_seqs:
-        return [(groups[0][0], batch, 0, t)]
-    return [(k, SimpleNamespace(q_len=batch.q_len[a:b], n_seqs=b - a, seq_q_start=batch.seq_q_start[a:b],
-                                seq_q_len=batch.seq_q_len[a:b], slots=batch.slots[a:b]), t0, t1)
-            for k, a, b, t0, t1, _ in groups]
+        return [(groups[0][0], batch, [(0, sum(lens))])]
+    starts, t = [], 0
+    for n in lens:
+        starts.append(t)
+        t += n
+    arrays = batch if arrays is None else arrays
+    out = []
+    for k, a, b, _ in groups:
+        own, rows = [order[p] for p in range(a, b)], []
+        for i in sorted(own):
+            if rows and rows[-1][1] == starts[i]:
+                rows[-1] = (rows[-1][0], starts[i] + lens[i])
+            else:
+                rows.append((starts[i], starts[i] + lens[i]))
+        out.append((k, SimpleNamespace(q_len=[lens[i] for i in own], n_seqs=b - a, seq_q_start=arrays.seq_q_start[a:b],
+                                       seq_q_len=arrays.seq_q_len[a:b], slots=arrays.slots[a:b]), rows))
+    return out
 
 
 @lru_cache(maxsize=None)

@@ -15,6 +15,7 @@ from __future__ import annotations
 import gc
 from collections import OrderedDict
 from dataclasses import dataclass
+from types import SimpleNamespace
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -42,7 +43,10 @@ class StepBatch:
     (decoding) come first, and ``n_decode`` says how many there are: a fact about the
     layout that a mixer may use (the attention mixer gives those rows to its decode
     kernel) or ignore.  ``positions[t]`` is the token's index in its sequence,
-    ``seq_of_token[t]`` the row of its sequence in the block tables and in ``slots``."""
+    ``seq_of_token[t]`` the row of its sequence in the block tables and in ``slots``.  Where the
+    sequences do not stand in the order of their number of tokens, ``by_length`` has the
+    per-sequence arrays in that order (``order[p]`` is the row at place p): mixers whose kernels
+    are chosen by it take each kind in one launch."""
 
     def __init__(self):
         self.n_tokens = 0
@@ -62,6 +66,7 @@ class StepBatch:
         self.seq_q_start = None           # [R] device copies of the three lists
         self.seq_q_len = None
         self.seq_ctx_len = None
+        self.by_length = None
         self._block_tables: Dict[int, torch.Tensor] = {}
         self.max_ctx = 0
 
@@ -283,6 +288,9 @@ class ModelRunner:
                  np.asarray(b.slot_ids, dtype=np.int32), np.asarray(b.q_start, dtype=np.int32),
                  np.asarray(b.q_len, dtype=np.int32), np.asarray(b.ctx_len, dtype=np.int32)]
         parts += [tab.reshape(-1) for tab in tables]
+        by_length = sorted(range(R), key=b.q_len.__getitem__)
+        if by_length != list(range(R)):
+            parts += [np.asarray([of[i] for i in by_length], dtype=np.int32) for of in (b.q_start, b.q_len, b.slot_ids)]
         # every part starts on a 16-byte boundary
         offsets, total = [], 0
         for p in parts:
@@ -304,6 +312,8 @@ class ModelRunner:
         b.meta_tokens = b.tokens
         for g, tab in enumerate(tables):
             b._block_tables[g] = views[8 + g].view(tab.shape)
+        if len(views) > 8 + len(tables):
+            b.by_length = SimpleNamespace(order=by_length, seq_q_start=views[-3], seq_q_len=views[-2], slots=views[-1])
         if pad_tables and self._plain_groups:
             def hv(i):
                 return host[offsets[i]:offsets[i] + parts[i].size]

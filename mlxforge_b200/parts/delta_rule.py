@@ -167,7 +167,7 @@ class ChannelDeltaMixer(Mixer):
             ops.delta_gates_ex(decay_in, decay_ld, self.decay_per_head, 0, 0.0, self.a_log, self.dt_bias, gate_in, gate_ld,
                                self.gate_act, ag, nh, d, nh * dv)
         o = rt.buffer("delta.o", (T, nh * dv), f32)
-        for kind, part, _, _ in ops.delta_groups(batch, nh, d, dv):
+        for kind, part, _ in ops.delta_groups(batch, nh, d, dv):
             if kind == "runs":
                 runs, floats = ops.delta_runs(part, nh, d, dv)
                 ops.delta_recurrence_runs(qkv, beta, ag, state, part, o, nh, nkv, d, dv, runs,

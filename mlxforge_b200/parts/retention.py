@@ -116,7 +116,7 @@ class Retention(Mixer):
         o = rt.buffer("ret.o", (T, parts * nh * dv), f32).view(parts, T, nh * dv)
         og = rt.buffer("ret.og", (T, nh * dv))
         gate = proj[:, 2 * nh * d + nh * dv:]
-        for kind, part, t0, t1 in ops.retention_groups(batch, nh, d, dv, v, v_ld, cache.tensor):
+        for kind, part, rows in ops.retention_groups(batch, nh, d, dv, v, v_ld, cache.tensor):
             own = o if kind == "serial" else o[:1]
             if kind == "chunks":
                 chunks = ops.retention_chunks(part, nh, d, dv, v, v_ld, cache.tensor)
@@ -125,7 +125,8 @@ class Retention(Mixer):
                                                 room=ops.retention_chunks_room(rt.reserve_rows, nh, d, dv)))
             else:
                 ops.retention_recurrence(qk, v, v_ld, self.decay, cache.tensor, part, own, nh, d, dv)
-            rows = (own, gate, og) if t1 - t0 == T else (own[:, t0:t1], gate[t0:t1], og[t0:t1])
-            ops.retention_output(rows[0], rows[1], ld, self.eps, rows[2], nh, dv, self.norm_w, self.output_norm == "whole",
-                                 self.gate_act)
+            for t0, t1 in rows:
+                at = (own, gate, og) if t1 - t0 == T else (own[:, t0:t1], gate[t0:t1], og[t0:t1])
+                ops.retention_output(at[0], at[1], ld, self.eps, at[2], nh, dv, self.norm_w, self.output_norm == "whole",
+                                     self.gate_act)
         return rt.linear(og, self.w_o, rt.buffer("ret.delta", (T, self.hidden), f32 if self.out_f32 else None))

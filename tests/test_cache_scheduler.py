@@ -523,25 +523,34 @@ def test_a_kernel_that_gave_up_ends_every_request_with_error(pipeline):
 
 
 def test_sequences_are_grouped_by_their_own_length():
-    """Neighbours of one kind share a launch, sequences without a token are left out, a group ends at the limit of scratch, and a
-    portion too long for the scratch by itself goes another way whatever stands beside it."""
+    """One kind shares a launch (neighbours in the order of length where the batch has it, else in the step), sequences without a token
+    are left out, a group ends at the limit of scratch, and a portion too long for the scratch by itself goes another way whatever
+    stands beside it."""
     from types import SimpleNamespace
     import torch
     from mlxforge_b200.csrc import ops
 
-    def batch(lens):
-        i = torch.arange(len(lens))
-        return SimpleNamespace(q_len=lens, n_seqs=len(lens), seq_q_start=i, seq_q_len=i + 10, slots=i + 20)
+    def batch(lens, sort=False):
+        i, by = torch.arange(len(lens)), None
+        if sort:
+            order = sorted(range(len(lens)), key=lens.__getitem__)
+            o = torch.tensor(order)
+            by = SimpleNamespace(order=order, seq_q_start=o, seq_q_len=o + 10, slots=o + 20)
+        return SimpleNamespace(q_len=lens, n_seqs=len(lens), seq_q_start=i, seq_q_len=i + 10, slots=i + 20, by_length=by)
 
-    def groups(lens, dim=128, vdim=128, heads=2):
-        return [(k, b.q_len, t0, t1, b.slots.tolist()) for k, b, t0, t1 in ops.delta_groups(batch(lens), heads, dim, vdim)]
+    def groups(lens, dim=128, vdim=128, heads=2, sort=False):
+        return [(k, b.q_len, rows, b.slots.tolist()) for k, b, rows in ops.delta_groups(batch(lens, sort), heads, dim, vdim)]
 
     assert groups([1, 1, 300, 48, 47, 2, 0, 700, 1]) == [
-        ("one", [1, 1], 0, 2, [20, 21]), ("runs", [300, 48], 2, 350, [22, 23]), ("serial", [47, 2], 350, 399, [24, 25]),
-        ("runs", [700], 399, 1099, [27]), ("one", [1], 1099, 1100, [28])]
-    assert groups([1, 300], dim=48) == [("serial", [1, 300], 0, 301, [20, 21])]
-    whole = batch([1] * 5)
-    assert [(k, b is whole, t0, t1) for k, b, t0, t1 in ops.delta_groups(whole, 2, 128, 128)] == [("one", True, 0, 5)]
+        ("one", [1, 1], [(0, 2)], [20, 21]), ("runs", [300, 48], [(2, 350)], [22, 23]), ("serial", [47, 2], [(350, 399)], [24, 25]),
+        ("runs", [700], [(399, 1099)], [27]), ("one", [1], [(1099, 1100)], [28])]
+    assert groups([1, 1, 300, 48, 47, 2, 0, 700, 1], sort=True) == [
+        ("one", [1, 1, 1], [(0, 2), (1099, 1100)], [20, 21, 28]), ("serial", [2, 47], [(350, 399)], [25, 24]),
+        ("runs", [48, 300, 700], [(2, 350), (399, 1099)], [23, 22, 27])]
+    assert groups([1, 300], dim=48) == [("serial", [1, 300], [(0, 301)], [20, 21])]
+    for sort in (False, True):
+        whole = batch([1] * 5, sort)
+        assert [(k, b is whole, rows) for k, b, rows in ops.delta_groups(whole, 2, 128, 128)] == [("one", True, [(0, 5)])]
     most = ops.DELTA_RUNS_MAX_FLOATS // ops.library().mf_delta_runs_scratch(1, 64, 128, 128) * 16      # tokens
     n = most // 2 - 16
     assert [(k, len(l)) for k, l, *_ in groups([n, n, n, most + 16, 64], heads=64)] == [("runs", 2), ("runs", 1), ("serial", 1), ("runs", 1)]
