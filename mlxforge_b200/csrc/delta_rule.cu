@@ -12,8 +12,10 @@
 // Every column of S is independent of the others: u_c = beta (v_c - S[:, c] . k) touches
 // column c only.  So the recurrence runs in parallel over (sequence, head, column) and is
 // serial in time only; a column is shared by 8 lanes that hold dim/8 rows each in registers.
-// The state after a token is the same however the prompt was cut: a step continues from the
-// state in the request's slot.
+// A step continues from the state in the request's slot.  Which kernel takes a sequence is a matter
+// of its own portion: one token, token after token, or runs of 16 tokens (delta_chunked.cu); they
+// add in other orders, so another cut of a prompt moves a result within 32-bit rounding, and what
+// else is in the step does not.
 //
 // The slot also keeps the last taps-1 inputs of the convolutions, [(taps-1), C] after S.
 #include "common.cuh"

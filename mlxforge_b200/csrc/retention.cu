@@ -11,8 +11,10 @@
 //  * retention_recurrence: every column of S is independent, so the recurrence is parallel over
 //    (sequence, head, column) and serial in time only.  Eight lanes share a column and hold
 //    dim/8 of its rows in registers; q and k of the coming tokens are staged in shared memory,
-//    eight tokens at a time.  A step continues from the slot's state, so the result does not
-//    depend on how a prompt was cut.  Portions of many tokens: retention_chunked.cu.
+//    eight tokens at a time.  A step continues from the slot's state, and which kernel takes a
+//    sequence is a matter of its own portion: one token, token after token, or chunks of 64
+//    (retention_chunked.cu).  The three add a read-out in other orders, so another cut of a prompt moves
+//    it within 32-bit rounding; what else is in the step does not.
 //  * retention_output: per token and head the read-out (summed over the row groups that a staged
 //    launch spreads a head's state over) over its root mean square, times silu(gate).
 #include "rotary.cuh"

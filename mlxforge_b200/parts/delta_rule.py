@@ -21,8 +21,8 @@ per head); ``gate_rank`` 0 makes the gate a direct projection ``Wg x`` (role ``g
 ``generalized_delta`` (below) is the rule with a removal term beside the decay.
 
 The request's slot keeps ``S`` of every head and the last ``conv - 1`` inputs of every convolution,
-so a step goes on from where the step before ended, however the prompt was cut.  All projections
-that read the mixer's input are one product; the two low-rank second factors are one product with a
+so a step goes on from where the step before ended, however the prompt was cut (to the rounding of
+sums in another order).  All projections that read the mixer's input are one product; the two low-rank second factors are one product with a
 block-diagonal matrix.  Everything after the projections is 32-bit.
 """
 from __future__ import annotations

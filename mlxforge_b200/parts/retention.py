@@ -18,7 +18,8 @@ ONE root mean square over all of them instead of one per head; ``norm_weight`` n
 SiLU; ``out_f32`` writes the output projection in 32-bit.
 
 The request's slot keeps ``S`` of every head, so a step goes on from where the step before ended,
-however the prompt was cut.  All projections that read the mixer's input are one product;
+however the prompt was cut (to the rounding of sums in another order).  All projections that read the
+mixer's input are one product;
 everything after them is 32-bit.  ``names`` maps the tensors' roles to their names.
 """
 from __future__ import annotations
