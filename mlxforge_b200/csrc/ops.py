@@ -437,9 +437,9 @@ def retention_recurrence(qk: torch.Tensor, v: torch.Tensor, v_ld: int, decay: to
           "retention_recurrence")
 
 
-# Tokens of the longest portion from which retention goes over chunks of tokens side by side (8 heads of 128, chunks against
+# Tokens of a portion from which retention goes over chunks of tokens side by side (8 heads of 128, chunks against
 # token after token: 36 and 17 us for 96 tokens, 37 and 37 for 256, 64 and 244 for 1,777), and the most scratch for that,
-# 1 GB (a step that needs more goes token after token).
+# 1 GB (a group of sequences ends there; a portion that needs more by itself goes token after token).
 RETENTION_CHUNK = 64
 RETENTION_CHUNKED_MIN_TOKENS = 256
 RETENTION_CHUNKED_MAX_FLOATS = 1 << 28
@@ -924,9 +924,9 @@ def delta_recurrence(qkv: torch.Tensor, beta: torch.Tensor, ag: torch.Tensor, st
                                         _stream()), "delta_recurrence")
 
 
-# Tokens of the longest portion from which the delta rule goes over runs of tokens (16 heads of 128, runs against token
+# Tokens of a portion from which the delta rule goes over runs of tokens (16 heads of 128, runs against token
 # after token: 18.7 and 15.2 us for 32 tokens, 16.7 and 18.9 for 48 of 8 heads, 20.8 and 24.9 for 64), and the most
-# scratch for that, 1 GB (a step that needs more goes token after token).
+# scratch for that, 1 GB (a group of sequences ends there; a portion that needs more by itself goes token after token).
 DELTA_RUN = 16
 DELTA_RUNS_MIN_TOKENS = 48
 DELTA_RUNS_MAX_FLOATS = 1 << 28
