@@ -82,7 +82,7 @@ _SIGNATURES = {
                         _P, _P, _P, _P, c_int, c_float, c_double, _P, _P, _P, c_int, c_int, _P, _P, _P, c_int, _P],
     "mf_rotate_rows": [_P, c_int, c_int, c_int, c_int, c_int, _P, _P, _P, c_float, _P],
     "mf_moe_route": [_P, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, _P, _P, _P, _P, _P],
-    "mf_moe_rows": [_P, _P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, _P],
+    "mf_moe_rows": [_P, _P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, _P, _P],
     "mf_moe_combine": [_P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P, _P, _P, c_int, _P],
     "mf_moe_rows_slices": [c_int],
     "mf_attention_talking_tc_ok": [c_int, c_int, c_int, c_int, c_int],

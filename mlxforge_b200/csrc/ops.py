@@ -1292,8 +1292,8 @@ def moe_rows(x: torch.Tensor, w_gu: torch.Tensor, w_down: torch.Tensor, ids: tor
     T, H = x.shape
     check(library().mf_moe_rows(x.data_ptr(), w_gu.data_ptr(), w_down.data_ptr(), dtype_code(x), ids.data_ptr(),
                                 y.data_ptr(), T, H, w_down.shape[2], ids.shape[1], limit, alpha, up_offset,
-                                w_down.shape[0], -1 if act is None else activation_code(act), _stream()),
-          "moe_rows")
+                                w_down.shape[0], -1 if act is None else activation_code(act),
+                                kernel_status(x.device).data_ptr(), _stream()), "moe_rows")
 
 
 def moe_rows_slices(ff: int) -> int:

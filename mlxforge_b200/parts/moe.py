@@ -22,8 +22,8 @@ branch every token takes; it is added times ``sigmoid(w_sg . x)`` where ``shared
 vector (its product rides along with the router's), else as it is.
 
 The experts' matrices are stacked at load time (``[E, 2, ff, H]`` gate rows then up rows, and
-``[E, H, ff]``).  Few tokens (and the 32-bit path) take the kernel with a block per (token, chosen
-expert), which streams that expert's matrices once; many tokens in bfloat16 are sorted by expert and go
+``[E, H, ff]``).  Few tokens read every chosen expert's matrices once and multiply them with all its
+tokens (the 32-bit path: a block per (token, chosen expert)); many tokens in bfloat16 are sorted by expert and go
 through the tcgen05 products over the sorted pairs (``MLXFORGE_MOE_TILES=1``: the mma.sync tiles).  Either way a
 token's chosen experts are added in the order of the choice; what else is in the step moves its result only
 by which of the two paths the step's size takes, and by the type of a pair's result in a step of many tokens (``wide_y``).

@@ -1,0 +1,125 @@
+"""Kernels of single layers at the sizes where they can go wrong: edges of tiles, remainders, the smallest and largest of
+their range, against 64-bit references."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _ran(before):
+    from mlxforge_b200.csrc import binding
+    return {k: v - before[k] for k, v in binding.kernel_launches().items() if v - before[k]}
+
+
+# ----------------------------------------------------------------------------- experts, few tokens
+
+@pytest.mark.parametrize("H,ff,E,top,T,act", [
+    (2048, 768, 64, 6, 8, None), (64, 64, 4, 1, 1, None), (72, 24, 5, 2, 9, None), (136, 200, 7, 3, 17, "silu"),
+    (256, 128, 2, 2, 63, None), (4160, 64, 3, 2, 20, None), (128, 72, 3, 3, 33, "relu2"), (1024, 512, 1024, 8, 63, None)])
+def test_experts_few_tokens(H, ff, E, top, T, act):
+    """Every chosen expert's matrices once; passes of 8 and 16 tokens, experts with more than one pass, identity experts
+    (a choice beyond the matrices), ragged rows and slices."""
+    import torch
+    from mlxforge_b200.csrc import binding, ops
+    g = torch.Generator(device="cuda").manual_seed(H + ff + T)
+    bf = torch.bfloat16
+    x = torch.randn((T, H), generator=g, device="cuda").to(bf)
+    w_gu = (torch.randn((E, 1 if act else 2, ff, H), generator=g, device="cuda") * H ** -0.5).to(bf)
+    w_down = (torch.randn((E, H, ff), generator=g, device="cuda") * ff ** -0.5).to(bf)
+    # a choice without repetition out of the experts and one identity expert behind them
+    ids = torch.rand((T, E + 1), generator=g, device="cuda").topk(top, 1).indices.to(torch.int32).contiguous()
+    slices = ops.moe_rows_slices(ff)
+    y = torch.full((T, top * slices, H), float("nan"), device="cuda")
+    before = binding.kernel_launches()
+    ops.moe_rows(x, w_gu, w_down, ids, y, 7.0, 1.702, 1.0, act)
+    assert _ran(before).get("moe_rows_mma", 0) == 1
+    got = y.view(T, top, slices, H).double().sum(2)
+    for t in range(T):
+        for k in range(top):
+            e = int(ids[t, k])
+            if e >= E:
+                assert bool(torch.isnan(y.view(T, top, slices, H)[t, k]).all())
+                continue
+            r = w_gu[e].double() @ x[t].double()
+            if act == "silu":
+                a = r[0] * torch.sigmoid(r[0])
+            elif act == "relu2":
+                a = r[0].clamp(min=0) ** 2
+            else:
+                gate, up = r[0].clamp(max=7.0), r[1].clamp(-7.0, 7.0)
+                a = gate * torch.sigmoid(1.702 * gate) * (up + 1.0)
+            a = a.to(bf).double()
+            terms = w_down[e].double() * a
+            # an activation next to a tie of its rounding may fall on the other side (a bfloat16 step, 2^-8 of it, in at most
+            # a few of ff: 32-bit sums differ by 1e-6 of a step's 4e-3); the rest is 32-bit summation
+            bound = 4 * 2 ** -8 * terms.abs().amax(1) + 1e-5 * terms.abs().sum(1)
+            assert bool(((got[t, k] - terms.sum(1)).abs() <= bound).all()), (t, k)
+    alone = torch.empty((1, top * slices, H), device="cuda")
+    ops.moe_rows(x[T // 2:T // 2 + 1].contiguous(), w_gu, w_down, ids[T // 2:T // 2 + 1].contiguous(), alone, 7.0, 1.702, 1.0, act)
+    here = (ids[T // 2] < E).repeat_interleave(slices)
+    assert torch.equal(alone[0][here], y[T // 2][here]), "a token's result depends on what else is in the step"
+
+
+@pytest.mark.parametrize("E,groups,keep,top", [(64, 8, 4, 6), (33, 0, 0, 5), (6, 3, 1, 2), (200, 0, 0, 9)])
+def test_router_ties_and_values_that_are_not_finite(E, groups, keep, top):
+    """Equal scores go to the lower expert (groups: the higher one leaves first); a score that is not a number is never chosen
+    and its group never leaves."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    rng = np.random.default_rng(E)
+    T = 37
+    z = rng.integers(-2, 3, (T, E)).astype(np.float32)
+    z[3, :] = 0.0
+    z[5, 1] = np.nan
+    z[6, 2] = -np.inf
+    z[7, 4] = np.inf
+    bias = rng.integers(-1, 2, E).astype(np.float32) if groups == 0 else None
+    ids = torch.empty((T, top), dtype=torch.int32, device="cuda")
+    wts = torch.empty((T, top), dtype=torch.float32, device="cuda")
+    ops.moe_route(torch.from_numpy(z).cuda(), groups, keep, top, 1.0, ids, wts,
+                  bias=None if bias is None else torch.from_numpy(bias).cuda())
+    s = torch.sigmoid(torch.from_numpy(z)).numpy()          # equal inputs, equal scores: all that the choice needs
+    for t in range(T):
+        sel = s[t] + (bias if bias is not None else 0)
+        if groups:
+            pairs = np.sort(s[t].reshape(groups, -1), 1)[:, -2:].sum(1)
+            left = list(range(groups))
+            for _ in range(groups - keep):
+                low = [g for g in left if not np.isnan(pairs[g])]
+                left.remove(max(g for g in low if pairs[g] == min(pairs[h] for h in low)))
+            sel = np.where(np.isin(np.arange(E) // (E // groups), left), sel, -np.inf)
+        if t == 5 and groups:
+            continue                                        # which two of a group's scores count when one is NaN is not defined
+        order = sorted((e for e in range(E) if sel[e] > -np.inf), key=lambda e: (-sel[e], e))[:top]
+        assert ids[t].tolist()[:len(order)] == order, t
+
+
+@pytest.mark.parametrize("H,top,slices,T,kind", [(2048, 6, 12, 8, 0), (132, 9, 3, 5, 1), (1028, 2, 1, 70, 2), (128, 17, 2, 3, 3),
+                                                  (130, 3, 2, 4, 3), (2048, 6, 1, 100, 3)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_weighted_sum_of_experts(H, top, slices, T, kind, dtype):
+    """kind 0: plain; 1: identity experts; 2: rows by slot; 3: a shared branch with its gate as well."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    dt = getattr(torch, dtype)
+    g = torch.Generator(device="cuda").manual_seed(H + top)
+    y = torch.randn((T * top, slices, H), generator=g, device="cuda")
+    w = torch.rand((T, top), generator=g, device="cuda")
+    x, shared = (torch.randn((T, H), generator=g, device="cuda").to(dt) for _ in range(2))
+    gate = torch.randn((T, 3), generator=g, device="cuda")
+    ids = torch.randint(0, 6, (T, top), generator=g, device="cuda", dtype=torch.int32)
+    slot = torch.randperm(T * top, generator=g, device="cuda").to(torch.int32)
+    out = torch.empty((T, H), dtype=dt, device="cuda")
+    ops.moe_combine(y.view(T, top * slices, H) if kind != 2 else y, w, slot if kind >= 2 else None, out, slices,
+                    ids if kind in (1, 3) else None, 4, x if kind in (1, 3) else None, shared if kind == 3 else None,
+                    gate[:, 2:] if kind == 3 else None, 3)
+    rows = (slot.long() if kind >= 2 else torch.arange(T * top, device="cuda")).view(T, top)
+    parts = y.double().sum(1)[rows]
+    if kind in (1, 3):
+        parts = torch.where((ids >= 4)[..., None], x.double()[:, None], parts)
+    want = (w.double()[..., None] * parts).sum(1)
+    if kind == 3:
+        want = want + torch.sigmoid(gate[:, 2:].double()) * shared.double()
+    mag = (w.double()[..., None] * y.double().abs().sum(1)[rows]).sum(1) + x.double().abs() * top + shared.double().abs()
+    bound = (top + slices + 4) * 2 ** -24 * mag + (want.abs() * 2 ** -8 if dtype == "bfloat16" else 0)
+    assert bool(((out.double() - want).abs() <= bound).all())
