@@ -57,7 +57,9 @@ class PagePool:
         return out
 
     def give_back(self, pages: List[int]) -> None:
-        for p in pages:
+        # the last one first: whoever takes them next gets them in the order in which they were held, so that pages that
+        # follow one another go on doing so
+        for p in reversed(pages):
             if not (0 <= p < self.n_pages) or not self._held[p]:
                 raise RuntimeError(f"page {p} given back but not held")
             self._held[p] = False

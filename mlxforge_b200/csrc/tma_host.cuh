@@ -101,4 +101,31 @@ inline int bf16_map_chunked(const void* ptr, long long rows, long long cols, int
   return 0;
 }
 
+// A pool of pages, [pages][page_rows][cols] bfloat16, with boxes of 16 rows and 64 columns of n_pages pages that follow one another,
+// laid out as one tile of 16 n_pages rows with 128-byte swizzle.  The number of pages only bounds the unit's own range check.
+inline int bf16_map_pages(const void* ptr, int page_rows, long long cols, int n_pages, CUtensorMap* out) {
+  static std::unordered_map<Key, CUtensorMap, Hash> cache;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  const Key key{ptr, page_rows, cols, 16, n_pages};
+  auto it = cache.find(key);
+  if (it != cache.end()) {
+    *out = it->second;
+    return 0;
+  }
+  EncodeTiled enc = encoder();
+  if (!enc) return MF_ERR_BAD_ARG;
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)page_rows, 1ull << 24};
+  const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)cols * 2 * page_rows};
+  const cuuint32_t box[3] = {64, 16, (cuuint32_t)n_pages};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return 20000 + (int)r;
+  if (cache.size() > 4096) cache.clear();
+  cache.emplace(key, *out);
+  return 0;
+}
+
 }  // namespace tma_host

@@ -123,3 +123,68 @@ def test_weighted_sum_of_experts(H, top, slices, T, kind, dtype):
     mag = (w.double()[..., None] * y.double().abs().sum(1)[rows]).sum(1) + x.double().abs() * top + shared.double().abs()
     bound = (top + slices + 4) * 2 ** -24 * mag + (want.abs() * 2 ** -8 if dtype == "bfloat16" else 0)
     assert bool(((out.double() - want).abs() <= bound).all())
+
+
+# ----------------------------------------------------------------------------- attention of prompts: pages that follow one another
+
+@pytest.mark.parametrize("form", ["plain", "options", "latent"])
+@pytest.mark.parametrize("lens,held", [([128, 191], [0, 0]), ([129, 300], [63, 500]), ([257], [1000])])
+def test_prefill_attention_does_not_depend_on_where_the_pages_are(form, lens, held):
+    """A tile of keys whose pages follow one another comes as one copy, any other page by page: the same bits from a cache laid
+    out in order, one in reverse and one with every page elsewhere (what the kernel does not fetch is NaN), near a 64-bit result."""
+    import torch
+    from mlxforge_b200.csrc import binding, ops
+    nh, nkv, hd, vd, window, keep = {"plain": (4, 2, 128, 128, 0, 0), "options": (4, 2, 128, 128, 150, 4), "latent": (3, 1, 160, 128, 0, 0)}[form]
+    g = torch.Generator(device="cuda").manual_seed(sum(lens) + hd)
+    bf, T, ctx = torch.bfloat16, sum(lens), [n + h for n, h in zip(lens, held)]
+    q = torch.randn((T, nh * hd), generator=g, device="cuda").to(bf)
+    gate = torch.randn((T, nh * vd), generator=g, device="cuda").to(bf) if form == "options" else None
+    sink = torch.randn(nh, generator=g, device="cuda") if form == "options" else None
+    ks = [torch.randn((c, nkv, hd), generator=g, device="cuda").to(bf) for c in ctx]
+    vs = [k[..., :vd] if form == "latent" else torch.randn((c, nkv, vd), generator=g, device="cuda").to(bf) for k, c in zip(ks, ctx)]
+    per = [-(-c // 16) for c in ctx]
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    outs = []
+    for order in ("in order", "reverse", "elsewhere"):
+        ids = {"in order": np.arange(sum(per)), "reverse": np.arange(sum(per))[::-1],
+               "elsewhere": np.random.default_rng(1).permutation(3 * sum(per))[:sum(per)]}[order]
+        kp = torch.full((3 * sum(per) + 1, nkv, 16, hd), float("nan"), device="cuda", dtype=bf)
+        vp = torch.full((3 * sum(per) + 1, nkv, 16, vd), float("nan"), device="cuda", dtype=bf)
+        table, at = np.full((len(lens), max(per)), -1, np.int32), 0
+        for s, n in enumerate(per):
+            table[s, :n] = ids[at:at + n]
+            at += n
+            for b in range(n):
+                k, v = ks[s][b * 16:b * 16 + 16], vs[s][b * 16:b * 16 + 16]
+                kp[int(table[s, b]), :, :k.shape[0]] = k.transpose(0, 1)
+                vp[int(table[s, b]), :, :k.shape[0]] = v.transpose(0, 1)
+        out = torch.full((T, nh * vd), float("nan"), device="cuda", dtype=bf)
+        before = binding.kernel_launches()
+        args = (i32(np.cumsum([0] + lens[:-1]).tolist()), i32(lens), i32(ctx), 0, max(lens), torch.from_numpy(table).cuda(), 16, nh, nkv, hd, hd ** -0.5)
+        if form == "plain":
+            ops.attention_prefill(q, kp, vp, out, *args, 0)
+        else:
+            ops.attention_prefill_ex(q, kp, kp if form == "latent" else vp, out, *args, window, vd, form == "latent", keep, sink, gate, nh * vd,
+                                     0.0, min(lens))
+        ops.check_kernel_status()
+        assert _ran(before).get("attn_prefill_tc", 0) == 1
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    at = 0
+    for n, h, k, v in zip(lens, held, ks, vs):
+        i, j = torch.arange(h, h + n, device="cuda")[:, None], torch.arange(h + n, device="cuda")[None]
+        seen = (j <= i) & ((i - j < window) | (j < keep)) if window else j <= i
+        for head in range(nh):
+            kv = head // (nh // nkv)
+            s = (q[at:at + n, head * hd:(head + 1) * hd].double() @ k[:, kv].double().T * hd ** -0.5).masked_fill_(~seen, -np.inf)
+            if sink is not None:
+                s = torch.cat((s, sink[head].double().expand(n, 1)), 1)
+            p = torch.softmax(s, 1)[:, :h + n]
+            want, mag = p @ v[:, kv].double(), p @ v[:, kv].double().abs()
+            if gate is not None:
+                sg = torch.sigmoid(gate[at:at + n, head * vd:(head + 1) * vd].double())
+                want, mag = want * sg, mag * sg
+            # a probability is rounded to 8 bits once, the result once more
+            got = outs[0][at:at + n, head * vd:(head + 1) * vd].double()
+            assert bool(((got - want).abs() <= 2 ** -8 * mag + 2 ** -8 * want.abs() + 1e-6).all()), (head, n)
+        at += n
