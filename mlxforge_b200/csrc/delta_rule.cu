@@ -538,6 +538,32 @@ delta_output_kernel(const float* __restrict__ o, const float* __restrict__ gate,
   for (int c = lane; c < vdim; c += 32) out[(long long)item * vdim + c] = from_f32<TO>(row[c] * inv * wh[c] * g[c]);
 }
 
+// The same for heads of 32 N columns in whole pieces, N neighbouring columns a lane, read once and kept.  2,048 tokens of 16 heads of
+// 128: 11.0 -> 8.2 us.
+template <typename TO, int N>
+__global__ void __launch_bounds__(256)
+delta_output_vec_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_ld, const float* __restrict__ w,
+                        float eps, TO* __restrict__ out, int n_heads, int total, int w_per_head) {
+  constexpr int V = 32 * N;
+  pdl_launch();
+  pdl_wait();
+  const int item = blockIdx.x * 8 + (threadIdx.x >> 5), c = (threadIdx.x & 31) * N;
+  if (item >= total) return;
+  const int t = item / n_heads, h = item - t * n_heads;
+  float x[N], g[N], wh[N];
+  dp_get(x, o + (long long)item * V + c);
+  dp_get(g, gate + (long long)t * gate_ld + h * V + c);
+  dp_get(wh, w + (w_per_head ? h * V : 0) + c);
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; i++) ss = fmaf(x[i], x[i], ss);
+  const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)V + eps);
+  struct alignas(sizeof(TO) * N) R { TO v[N]; } r;
+#pragma unroll
+  for (int i = 0; i < N; i++) r.v[i] = from_f32<TO>(x[i] * inv * wh[i] * g[i]);
+  *reinterpret_cast<R*>(out + (long long)item * V + c) = r;
+}
+
 // ------------------------------------------------------------------ entry points
 static bool delta_prepare_heads_ok(int taps, int dim, int vdim, int ld, long long state_stride, long long conv_off) {
   return taps <= 4 && (dim == 64 || dim == 128) && (vdim == 64 || vdim == 128) && ld % 4 == 0 && state_stride % 4 == 0 &&
@@ -680,6 +706,19 @@ MF_API int mf_delta_output(const float* o, const float* gate, int gate_ld, const
   const int total = T * n_heads;
   const unsigned blocks = (unsigned)((total + 7) / 8);
   mf_count(MF_K_DELTA_OUTPUT);
+  if ((vdim == 64 || vdim == 128) && gate_ld % 4 == 0 && (out_dtype == MF_F32 || out_dtype == MF_BF16) &&
+      !(((uintptr_t)o | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)out) & 15)) {
+#define DO_GO(TO, N)                                                                                                      \
+  return (int)launch_small(T, delta_output_vec_kernel<TO, N>, dim3(blocks), dim3(256), 0, stream, o, gate, gate_ld, w, eps, \
+                           (TO*)out, n_heads, total, w_per_head)
+    if (out_dtype == MF_F32) {
+      if (vdim == 64) DO_GO(float, 2);
+      DO_GO(float, 4);
+    }
+    if (vdim == 64) DO_GO(__nv_bfloat16, 2);
+    DO_GO(__nv_bfloat16, 4);
+#undef DO_GO
+  }
   if (out_dtype == MF_F32)
     return (int)launch_small(T, delta_output_kernel<float>, dim3(blocks), dim3(256), 0, stream, o, gate, gate_ld, w, eps,
                              (float*)out, n_heads, vdim, total, w_per_head);

@@ -188,3 +188,97 @@ def test_prefill_attention_does_not_depend_on_where_the_pages_are(form, lens, he
             got = outs[0][at:at + n, head * vd:(head + 1) * vd].double()
             assert bool(((got - want).abs() <= 2 ** -8 * mag + 2 ** -8 * want.abs() + 1e-6).all()), (head, n)
         at += n
+
+
+# ----------------------------------------------------------------------------- rotations, biases and norms of prompts
+
+def _store_case(kind, T, g, pages):
+    """A launch of ``kind`` for tokens a..b of T tokens: a function of (a, b) that returns the outputs of those tokens' rows."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    bf, f32 = torch.bfloat16, torch.float32
+    r = lambda *s, dt=bf: torch.randn(s, generator=g, device="cuda").to(dt)
+    pos = torch.randint(0, 5000, (T,), generator=g, device="cuda", dtype=torch.int32)
+    table = torch.arange(T, device="cuda", dtype=torch.int32)[:, None].repeat(1, 5000 // 16 + 1).contiguous()       # a page a token
+    seq = torch.arange(T, device="cuda", dtype=torch.int32)
+    inv = 50000.0 ** (-torch.arange(32, device="cuda", dtype=f32) / 32)
+    pool = lambda heads, d: torch.full((T, heads, 16, d), float("nan"), device="cuda", dtype=bf)
+
+    def kv(p, a, b):
+        return p[torch.arange(a, b, device="cuda"), :, pos[a:b].long() % 16]
+
+    if kind == "pairs":
+        x, nh, nkv, hd = r(T, 8 * 128), 4, 2, 128
+        def go(a, b):
+            q, k, v = r(b - a, nh * hd), pool(nkv, hd), pool(nkv, hd)
+            ops.rope_store(x[a:b], pos[a:b], seq[a:b], table, 16, inv[:24].contiguous(), None, q, k, v, nh, nkv, hd, 48, True, True, True, ld=8 * 128)
+            return q, kv(k, a, b), kv(v, a, b)
+    elif kind == "halves":
+        nh, nkv, hd = 6, 2, 64
+        x, freqs = r(T, (nh + 2 * nkv) * hd), (1 / inv[:16]).contiguous()
+        def go(a, b):
+            q, k, v = r(b - a, nh * hd), pool(nkv, hd), pool(nkv, hd)
+            ops.rope_kv_write(x[a:b], pos[a:b], seq[a:b], table, 16, freqs, q, k, v, nh, nkv, hd, 32, True, False)
+            return q, kv(k, a, b), kv(v, a, b)
+    elif kind == "retention":
+        x = r(T, 1000)
+        def go(a, b):
+            qk = r(b - a, 2 * 3 * 64, dt=f32)
+            ops.retention_prepare(x[a:b], 3, 64, 48, 0.125, pos[a:b], inv[:24].contiguous(), None, qk, silu=True)
+            return (qk,)
+    elif kind == "biases":
+        nh, nkv, d, dv = 5, 1, 36, 20
+        x, bias = r(T, nh * d + d + dv, dt=f32), r(nh * d + d + dv, dt=f32)
+        def go(a, b):
+            q, k, v = r(b - a, nh * d), pool(nkv, d), pool(nkv, dv)
+            ops.biased_kv_store(x[a:b], bias, pos[a:b], seq[a:b], table, 16, q, k, v, nh, nkv, d, dv, True)
+            return q, kv(k, a, b), kv(v, a, b)
+    else:
+        x, wq, wkv = r(T, 1208), r(1032, dt=f32), r(104, dt=f32)
+        def go(a, b):
+            cq, k = r(b - a, 1032), pool(1, 104 + 64)
+            ops.latent_prepare(x[a:b], 1032, 1040, 104, 64, wq, wkv, 1e-6, pos[a:b], seq[a:b], table, 16, inv, None, cq, k, True)
+            return cq, kv(k, a, b)
+        xd = x.double()
+        want = xd[:, :1032] / (xd[:, :1032].square().mean(1, keepdim=True) + 1e-6).sqrt() * wq.double()
+        assert bool(((go(0, T)[0].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all())         # one rounding
+    return go
+
+
+@pytest.mark.parametrize("kind", ["pairs", "halves", "retention", "biases", "latent"])
+def test_several_tokens_a_block(kind):
+    """Steps of so many tokens that a block takes several, with a last block that has fewer: every token's bits are those it has
+    in a step of few."""
+    import torch
+    T = 8 * torch.cuda.get_device_properties(0).multi_processor_count + 3
+    g = torch.Generator(device="cuda").manual_seed(len(kind))
+    go = _store_case(kind, T, g, None)
+    many = go(0, T)
+    assert all(not bool(torch.isnan(m).any()) for m in many)
+    for a, b in ((0, 1), (5, 9), (T - 2, T)):
+        for m, f in zip(many, go(a, b)):
+            assert torch.equal(m[a:b], f), (kind, a)
+
+
+@pytest.mark.parametrize("V,heads,T,parts", [(64, 3, 5, 1), (128, 5, 3, 4), (128, 1, 1, 1)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_read_out_norms(V, heads, T, parts, dtype):
+    """Retention's and the delta rule's norms over whole heads, broken last blocks, several partial read-outs."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    dt, n = getattr(torch, dtype), heads * V
+    g = torch.Generator(device="cuda").manual_seed(V + T)
+    o = torch.randn((parts, T, n), generator=g, device="cuda")
+    x = torch.randn((T, n + 8), generator=g, device="cuda").to(dt)
+    out = torch.empty((T, n), dtype=dt, device="cuda")
+    ops.retention_output(o, x[:, 8:], n + 8, 1e-6, out, heads, V)
+    rms = lambda a: (a / (a.view(T, heads, V).square().mean(-1, keepdim=True) + 1e-6).sqrt().expand(T, heads, V).reshape(T, n))
+    gd = x[:, 8:].double()
+    # sums of up to 128 squares and a few roundings of 2^-24, one of the result's type
+    tol = 2 ** -8 if dtype == "bfloat16" else 2 ** -19
+    want = rms(o.double().sum(0)) * gd * torch.sigmoid(gd)
+    assert bool(((out.double() - want).abs() <= tol * want.abs() + 2 ** -20 * gd.abs() * parts).all())
+    gate, w = torch.randn((T, n + 4), generator=g, device="cuda"), torch.randn(V, generator=g, device="cuda")
+    ops.delta_output(o[0].contiguous(), gate[:, 4:], n + 4, w, 1e-6, out, heads, V)
+    want = rms(o[0].double()) * w.double().repeat(heads) * gate[:, 4:].double()
+    assert bool(((out.double() - want).abs() <= tol * want.abs() + 1e-12).all())
