@@ -15,8 +15,9 @@
 //   3. warp h:  online softmax of its mixed scores (32-bit), P_h rounded to bfloat16 as the
 //               A operand, O_h += P_h V_g(h).
 //
-// Keys and values of a tile come in by cp.async (16 bytes a copy): the next tile's keys while heads are mixed and the
-// softmax runs, its values while its own scores are made, so one buffer of each is enough and no step waits for memory.
+// Keys and values of a tile come in by tensor copies (other head sizes than 64 and 128 by cp.async): the next tile's keys while heads
+// are mixed and the softmax runs, its values while its own scores are made, so one buffer of each is enough and no step waits for
+// memory.
 //
 // Decoding (one query per sequence) has a kernel of its own further down: the keys are cut into splits of
 // TT_SPLIT_TILES tiles that start at multiples of that many tiles, a block per (sequence, split)
@@ -26,11 +27,13 @@
 // long prompt would otherwise walk all its keys alone while the blocks of the first tiles are
 // long done), the tiles with the most keys first.
 //
-// What bounds it: the tensor pipe and the special function unit (a tanh and an exponential per score) take turns
-// between the three barriers of a tile, and one block of 16 heads fills an SM's shared memory.  2,048 tokens of 16 / 4 heads
-// of 128 in one chunk: 458 -> 223 us (6.4 us a tile; 13 of them before, with the mixing as 32-bit multiplications by 256 of the 512
-// threads, waits for every copy and a block that walked 64 tiles), merge 53 -> 18.
+// What bounds it: 1,400 mma.sync a tile (13 cycles each and scheduler, 4,700 of a tile's cycles), then the arithmetic beside them, in three
+// phases that one block of 16 heads goes through together.  2,048 tokens of 16 / 4 heads of 128 in one chunk: 224 -> 202 us, 9,400 cycles
+// a tile: its copies as cp.async, 64 KB through the warps' own load path, were 2,700 of 10,300 cycles by a block's clock, whether or
+// not they looked pages up; the tensor copies need the products' addresses to fold (the head size as a constant), else
+// their swizzle costs what they save (234 us).  Two score tiles and two barriers instead of three were no faster (247 us).
 #include "common.cuh"
+#include "tma_host.cuh"
 
 #define TT_BM 16
 #define TT_BN 32
@@ -46,21 +49,41 @@ __device__ __forceinline__ void tt_mma(float (&c)[4], const uint32_t (&a)[4], ui
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void tt_ldmatrix_x4(uint32_t (&r)[4], const void* p) {
-  const uint32_t addr = (uint32_t)__cvta_generic_to_shared(p);
+__device__ __forceinline__ uint32_t tt_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void tt_ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
-__device__ __forceinline__ void tt_ldmatrix_x4_trans(uint32_t (&r)[4], const void* p) {
-  const uint32_t addr = (uint32_t)__cvta_generic_to_shared(p);
+__device__ __forceinline__ void tt_ldmatrix_x4(uint32_t (&r)[4], const void* p) { tt_ldmatrix_x4(r, tt_addr(p)); }
+__device__ __forceinline__ void tt_ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
+__device__ __forceinline__ void tt_ldmatrix_x4_trans(uint32_t (&r)[4], const void* p) { tt_ldmatrix_x4_trans(r, tt_addr(p)); }
 __device__ __forceinline__ void tt_cp_async16(void* smem, const void* gmem) {
   const uint32_t addr = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(addr), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void tt_cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void tt_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tt_wait(uint32_t bar, uint32_t parity, int* status, int code) {
+  for (unsigned i = 0; i < 1u << 24; i++) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done) return;
+  }
+  if (status) atomicExch(status, code);
+}
+__device__ __forceinline__ void tt_tensor_copy(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
+               ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
 template <int N>
 __device__ __forceinline__ void tt_cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 __device__ __forceinline__ uint32_t tt_pack(float lo, float hi) {
@@ -76,6 +99,7 @@ __device__ __forceinline__ void tt_pieces(float x, float y, uint32_t (&p)[3]) {
     y -= __uint_as_float(p[i] & 0xffff0000u);
   }
 }
+#define TT_GRANULES (2 * (TT_PREFILL_SPLIT_TILES + 2))      // of 16 keys, the most of a block whose keys are cut
 #define TT_LOG2E 1.4426950408889634f
 // a maximum in powers of two, rounded once: the weights, what moves older sums to a new maximum and the merge of the splits all
 // go by this number, so that its rounding (1e-3 of a weight at scores of 20,000) drops out
@@ -85,10 +109,12 @@ __device__ __forceinline__ float tt_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// tanh in 32-bit arithmetic through one exponential: (1 - e^{-2|x|}) / (1 + e^{-2|x|})
+// tanh in 32-bit arithmetic through one exponential and one reciprocal: (1 - e^{-2|x|}) / (1 + e^{-2|x|})
 __device__ __forceinline__ float tt_tanh(float x) {
-  const float t = __expf(-2.0f * fabsf(x));
-  return copysignf(__fdividef(1.0f - t, 1.0f + t), x);
+  const float t = tt_exp2(-2.0f * TT_LOG2E * fabsf(x));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + t));
+  return copysignf((1.0f - t) * r, x);
 }
 
 // register `reg` of the mixing matrix as A fragments of its three pieces, [piece][register][lane]: rows r0 (+ 8), columns c2 (+ 8)
@@ -133,13 +159,18 @@ struct TtArgs {
   int split_tiles;
   float* part_o;            // [rows, splits, H, VDIM] unnormalised outputs of the splits
   float* part_ml;           // [rows, splits, H, 2]    maximum (in powers of two) and sum
+  int* status;              // codes 91 (keys) and 92 (values): a wait for a copy ran out
 };
 
-template <int VDIM, int MAXH>
+// DIM: the head size, where keys and values come by tensor copies (64 or 128, and values of whole 64-wide spans), [head][span][32 keys]
+// [128 bytes], 128-byte swizzle; 0: by cp.async in padded rows.
+template <int VDIM, int MAXH, int DIM>
 __global__ void __launch_bounds__(32 * MAXH)
-talking_attention_tc_kernel(const TtArgs a) {
-  extern __shared__ __align__(16) unsigned char tt_smem[];
-  const int H = a.n_heads, G = a.n_kv, dim = a.dim;
+talking_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                            const TtArgs a) {
+  extern __shared__ __align__(1024) unsigned char tt_smem[];
+  constexpr bool TENSOR = DIM > 0;
+  const int H = a.n_heads, G = a.n_kv, dim = TENSOR ? DIM : a.dim;
   const int rep = H / G;
   const int seq = blockIdx.y;
   const int q_len = a.seq_q_len[seq];
@@ -153,10 +184,11 @@ talking_attention_tc_kernel(const TtArgs a) {
 
   const int qs_ld = dim + 8, vs_ld = VDIM + 8;
   constexpr int sc_ld = TT_BN + TT_SPAD, sc_hd = TT_BM * sc_ld + 4;         // a head's rows: heads in other banks
-  __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(tt_smem);            // [H][16][qs_ld]
-  __nv_bfloat16* Ks = Qs + (size_t)H * TT_BM * qs_ld;                       // [G][32][qs_ld]
-  __nv_bfloat16* Vs = Ks + (size_t)G * TT_BN * qs_ld;                       // [G][32][vs_ld]
-  float* sc = reinterpret_cast<float*>(Vs + (size_t)G * TT_BN * vs_ld);     // [H][sc_hd]
+  const int k_ld = TENSOR ? dim : qs_ld, v_ld = TENSOR ? VDIM : vs_ld;      // a key's share
+  __nv_bfloat16* Ks = reinterpret_cast<__nv_bfloat16*>(tt_smem);           // [G][32][k_ld]
+  __nv_bfloat16* Vs = Ks + (size_t)G * TT_BN * k_ld;                        // [G][32][v_ld]
+  __nv_bfloat16* Qs = Vs + (size_t)G * TT_BN * v_ld;                        // [H][16][qs_ld]
+  float* sc = reinterpret_cast<float*>(Qs + (size_t)H * TT_BM * qs_ld);     // [H][sc_hd]
   // the mixing matrix as A fragments of its three pieces: [piece][register][lane], zero beyond H
   uint32_t* tk = reinterpret_cast<uint32_t*>(sc + (size_t)H * sc_hd);
 
@@ -172,6 +204,13 @@ talking_attention_tc_kernel(const TtArgs a) {
     uint4 v = make_uint4(0, 0, 0, 0);
     if (r < rows) v = *reinterpret_cast<const uint4*>(a.q + ((long long)(q_start + row0 + r) * H + h) * dim + c);
     *reinterpret_cast<uint4*>(Qs + ((size_t)h * TT_BM + r) * qs_ld + c) = v;
+  }
+  __shared__ __align__(8) unsigned long long bars[2];      // the keys, the values of a tile are there
+  const uint32_t k_full = tt_addr(bars), v_full = k_full + 8;
+  if (TENSOR && tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(k_full));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(v_full));
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __shared__ int first_s[TT_BM];       // the first key that each query sees
   if (tid < TT_BM) {
@@ -203,20 +242,28 @@ talking_attention_tc_kernel(const TtArgs a) {
     k_first = max(k_first, (first_split + (int)blockIdx.z) * span);
     k_last = min(k_last, (first_split + (int)blockIdx.z + 1) * span - 1);
   }
-  // keys or values of a tile: a thread takes 16-byte pieces (key, column), of every head the same, so that page and slot
-  // are worked out once for all of them
-  const long long head_step = (long long)a.page_size;
+  // where the granules of 16 keys of this block's range stand in the pools (rows before heads; -1: no query sees one), looked up once
+  __shared__ long long granule_s[TT_GRANULES];
+  const int g_first = k_first / 16, n_granules = k_first <= k_last ? (k_last - k_first) / TT_BN * (TT_BN / 16) + TT_BN / 16 : 0;
+  auto granule = [&](int i) {
+    const int p0 = (g_first + i) * 16, blk = p0 / a.page_size;
+    return p0 + 15 >= lo0 && p0 <= pos_last ? (long long)table[blk] * G * a.page_size + (p0 - blk * a.page_size) : -1;
+  };
+  for (int i = tid; i < min(n_granules, TT_GRANULES); i += nthreads) granule_s[i] = granule(i);
+  __syncthreads();
+  // keys or values of a tile: a thread takes 16-byte pieces (key, column), of every head the same
   auto copy_pieces = [&](int k0, __nv_bfloat16* dst, const __nv_bfloat16* pool, int width, int pieces, int ld) {
+    const long long head_step = (long long)a.page_size * width;
     for (int i = tid; i < TT_BN * pieces; i += nthreads) {
-      const int j = i / pieces, c = (i - j * pieces) * 8;
-      const int pj = k0 + j, p0 = pj & ~15, blk = p0 / a.page_size;
+      const int j = i / pieces, c = (i - j * pieces) * 8, pj = k0 + j;
+      const int at = (pj >> 4) - g_first;
+      const long long row = at < TT_GRANULES ? granule_s[at] : granule(at);
       __nv_bfloat16* to = dst + (size_t)j * ld + c;
-      const bool in = pj >= lo0 && pj <= pos_last;
-      const long long page = in ? (long long)table[blk] : -1;
-      const __nv_bfloat16* from = pool + (page * G * head_step + (pj - blk * a.page_size)) * width + c;
-      for (int g = 0; g < G; g++, to += (size_t)TT_BN * ld, from += head_step * width) {
-        if (page >= 0) tt_cp_async16(to, from);
-        else *reinterpret_cast<uint4*>(to) = make_uint4(0, 0, 0, 0);
+      if (row >= 0 && pj >= lo0 && pj <= pos_last) {
+        const __nv_bfloat16* from = pool + (row + (pj & 15)) * width + c;
+        for (int g = 0; g < G; g++, to += (size_t)TT_BN * ld, from += head_step) tt_cp_async16(to, from);
+      } else {
+        for (int g = 0; g < G; g++, to += (size_t)TT_BN * ld) *reinterpret_cast<uint4*>(to) = make_uint4(0, 0, 0, 0);
       }
     }
     tt_cp_async_commit();
@@ -225,12 +272,47 @@ talking_attention_tc_kernel(const TtArgs a) {
     if (values) copy_pieces(k0, Vs, a.v_pool, VDIM, VDIM / 8, vs_ld);
     else copy_pieces(k0, Ks, a.k_pool, dim, dv8, qs_ld);
   };
-  if (k_first <= k_last) copy(k_first, false);
+  // The same by tensor copies of 16 keys x 64 channels of a head.  One thread says how many bytes are coming (before the barrier that frees
+  // the buffer), then every warp sends for some of them, so that no warp stands long at the unit, which takes 67 cycles a copy.
+  // A granule that no query sees is not fetched: its scores are masked, its values cleared.
+  auto expect = [&](int k0, bool values) {
+    if (tid) return;
+    int n = 0;
+#pragma unroll
+    for (int i = 0; i < TT_BN / 16; i++) n += k0 + 16 * i + 15 >= lo0 && k0 + 16 * i <= pos_last;
+    tt_expect(values ? v_full : k_full, (uint32_t)(n * G * 16 * 2 * (values ? VDIM : dim)));
+  };
+  auto fetch = [&](int k0, bool values) {
+    if (lane) return;
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");        // what was read there, before it is written
+    const int spans = (values ? VDIM : dim) / 64, per = (TT_BN / 16) * spans;
+    for (int i = warp; i < G * per; i += nthreads >> 5) {
+      const int g = i / per, gran = (i - g * per) / spans, span = i % spans, at = k0 / 16 + gran - g_first;
+      const long long row = at < TT_GRANULES ? granule_s[at] : granule(at);
+      if (row < 0) continue;
+      tt_tensor_copy(tt_addr(values ? Vs : Ks) + ((g * spans + span) * TT_BN + gran * 16) * 128, values ? &map_v : &map_k, span * 64,
+                     (int)row + g * a.page_size, values ? v_full : k_full);
+    }
+  };
+  if (TENSOR) {
+    if (k_first <= k_last) expect(k_first, false);
+    __syncthreads();
+    if (k_first <= k_last) fetch(k_first, false);
+  } else if (k_first <= k_last) {
+    copy(k_first, false);
+  }
   const float cap_scale = a.softcap > 0.f ? a.scale / a.softcap : a.scale;
   for (int k0 = k_first; k0 <= k_last; k0 += TT_BN) {
-    tt_cp_async_wait<0>();
-    __syncthreads();       // the keys are there for all; the tile before is done with Vs and sc (and Qs, tk are written)
-    copy(k0, true);
+    const uint32_t parity = (uint32_t)((k0 - k_first) / TT_BN) & 1;
+    if (TENSOR) expect(k0, true);
+    else tt_cp_async_wait<0>();
+    __syncthreads();       // the tile before is done with Vs and sc (and Qs, tk are written); copied rows are there for all
+    if (TENSOR) {
+      fetch(k0, true);
+      tt_wait(k_full, parity, a.status, 91);
+    } else {
+      copy(k0, true);
+    }
 
     // 1. raw scores of this warp's head
     if (has_head) {
@@ -241,15 +323,32 @@ talking_attention_tc_kernel(const TtArgs a) {
       // columns kk and kk + 8, then the next eight
       const __nv_bfloat16* qh = Qs + ((size_t)warp * TT_BM + (lane & 15)) * qs_ld + (lane >> 4) * 8;
       const __nv_bfloat16* kg = Ks + ((size_t)g_own * TT_BN + (lane >> 4) * 8 + (lane & 7)) * qs_ld + (lane >> 3 & 1) * 8;
-#pragma unroll 4
-      for (int kk = 0; kk < dim; kk += 16) {
-        uint32_t af[4], bf[4];
-        tt_ldmatrix_x4(af, qh + kk);
+      if constexpr (TENSOR) {
+        // a piece's place is its number exchanged with the row's: one exclusive or an address
+        const uint32_t ka = tt_addr(Ks) + (uint32_t)(g_own * (DIM / 64) * TT_BN + (lane >> 4) * 8 + (lane & 7)) * 128 +
+                            (((lane >> 3 & 1) ^ (lane & 7)) << 4);
 #pragma unroll
-        for (int nt = 0; nt < TT_BN / 8; nt += 2) {
-          tt_ldmatrix_x4(bf, kg + (size_t)nt * 8 * qs_ld + kk);
-          tt_mma(s[nt], af, bf[0], bf[1]);
-          tt_mma(s[nt + 1], af, bf[2], bf[3]);
+        for (int kk = 0; kk < DIM; kk += 16) {
+          uint32_t af[4], bf[4];
+          tt_ldmatrix_x4(af, qh + kk);
+#pragma unroll
+          for (int nt = 0; nt < TT_BN / 8; nt += 2) {
+            tt_ldmatrix_x4(bf, (ka ^ ((kk & 63) >> 3 << 4)) + ((kk >> 6) * TT_BN + nt * 8) * 128);
+            tt_mma(s[nt], af, bf[0], bf[1]);
+            tt_mma(s[nt + 1], af, bf[2], bf[3]);
+          }
+        }
+      } else {
+#pragma unroll 4
+        for (int kk = 0; kk < dim; kk += 16) {
+          uint32_t af[4], bf[4];
+          tt_ldmatrix_x4(af, qh + kk);
+#pragma unroll
+          for (int nt = 0; nt < TT_BN / 8; nt += 2) {
+            tt_ldmatrix_x4(bf, kg + (size_t)nt * 8 * qs_ld + kk);
+            tt_mma(s[nt], af, bf[0], bf[1]);
+            tt_mma(s[nt + 1], af, bf[2], bf[3]);
+          }
         }
       }
       float* sh = sc + (size_t)warp * sc_hd;
@@ -264,11 +363,18 @@ talking_attention_tc_kernel(const TtArgs a) {
         *reinterpret_cast<float2*>(sh + (size_t)(r0 + 8) * sc_ld + nt * 8 + c2) = make_float2(s[nt][2], s[nt][3]);
       }
     }
+    const bool more = k0 + TT_BN <= k_last;
+    if (TENSOR && more) expect(k0 + TT_BN, false);
     __syncthreads();
 
     // the scores are written and the keys read: the next tile's keys may come
-    if (k0 + TT_BN <= k_last) copy(k0 + TT_BN, false);
-    else tt_cp_async_commit();
+    if (TENSOR) {
+      if (more) fetch(k0 + TT_BN, false);
+    } else if (more) {
+      copy(k0 + TT_BN, false);
+    } else {
+      tt_cp_async_commit();
+    }
 
     // 2. the heads mixed and the mask: a warp one query and eight keys at a time
     if (a.talk) {
@@ -298,7 +404,17 @@ talking_attention_tc_kernel(const TtArgs a) {
         if (pj < first_s[r] || pj > pos0 + r) sc[(size_t)h * sc_hd + r * sc_ld + key] = -INFINITY;
       }
     }
-    tt_cp_async_wait<1>();      // the values are there; the next keys may still be on their way
+    if (TENSOR) {
+      tt_wait(v_full, parity, a.status, 92);
+      // values of keys that no query of the tile sees are stale memory: a weight of zero times them has to be zero
+      if (k0 < lo0 || k0 + TT_BN - 1 > pos_last)
+        for (int i = tid; i < G * TT_BN * (VDIM / 8); i += nthreads) {
+          const int key = k0 + i / 8 % TT_BN;
+          if (key < lo0 || key > pos_last) reinterpret_cast<uint4*>(Vs)[i] = make_uint4(0, 0, 0, 0);
+        }
+    } else {
+      tt_cp_async_wait<1>();      // the values are there; the next keys may still be on their way
+    }
     __syncthreads();
 
     // 3. softmax of the mixed scores and the product with the values
@@ -346,6 +462,7 @@ talking_attention_tc_kernel(const TtArgs a) {
         }
       }
       const __nv_bfloat16* vg = Vs + (size_t)g_own * TT_BN * vs_ld;
+      const uint32_t va = tt_addr(Vs) + (uint32_t)(g_own * (VDIM / 64) * TT_BN + (lane & 15)) * 128 + (((lane >> 4) ^ (lane & 7)) << 4);
 #pragma unroll
       for (int ks = 0; ks < TT_BN / 16; ks++) {
         uint32_t pf[4];
@@ -356,7 +473,10 @@ talking_attention_tc_kernel(const TtArgs a) {
 #pragma unroll
         for (int nt = 0; nt < VDIM / 8; nt += 2) {
           uint32_t bf[4];        // keys 0-7 and 8-15 of the step at eight columns, then at the next eight
-          tt_ldmatrix_x4_trans(bf, vg + (size_t)(ks * 16 + (lane & 15)) * vs_ld + nt * 8 + (lane >> 4) * 8);
+          if (TENSOR)
+            tt_ldmatrix_x4_trans(bf, (va ^ ((nt & 7) << 4)) + ((nt >> 3) * TT_BN + ks * 16) * 128);
+          else
+            tt_ldmatrix_x4_trans(bf, vg + (size_t)(ks * 16 + (lane & 15)) * vs_ld + nt * 8 + (lane >> 4) * 8);
           tt_mma(o[nt], pf, bf[0], bf[1]);
           tt_mma(o[nt + 1], pf, bf[2], bf[3]);
         }
@@ -706,22 +826,37 @@ static int tt_prefill_split_tiles(int window, int chunk) {
   return most > 0 && most <= 4096 ? TT_PREFILL_SPLIT_TILES / 2 : TT_PREFILL_SPLIT_TILES;
 }
 
-template <int VDIM, int MAXH>
-static int tt_launch(const TtArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
+template <int VDIM, int MAXH, int DIM>
+static int tt_launch_as(const CUtensorMap& mk, const CUtensorMap& mv, const TtArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
   const size_t smem = tt_smem_bytes(a.n_heads, a.n_kv, a.dim, VDIM);
   static DeviceOnce once;
   const int d = mf_current_device();
   if (d < 0) return MF_ERR_BAD_ARG;
   if (!once.done[d]) {
-    cudaError_t e = cudaFuncSetAttribute(talking_attention_tc_kernel<VDIM, MAXH>,
+    cudaError_t e = cudaFuncSetAttribute(talking_attention_tc_kernel<VDIM, MAXH, DIM>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return (int)e;
     once.done[d] = true;
   }
   dim3 grid((max_q_len + TT_BM - 1) / TT_BM, n_seqs, a.splits > 0 ? a.splits : 1);
   const int warps = a.n_heads < 4 ? 4 : a.n_heads;       // at least four warps for the loads and the mixing
-  talking_attention_tc_kernel<VDIM, MAXH><<<grid, 32 * warps, smem, stream>>>(a);
+  talking_attention_tc_kernel<VDIM, MAXH, DIM><<<grid, 32 * warps, smem, stream>>>(mk, mv, a);
   return (int)cudaGetLastError();
+}
+
+template <int VDIM, int MAXH>
+static int tt_launch(const TtArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
+  CUtensorMap mk = {}, mv = {};
+  if constexpr (VDIM % 64 == 0) {
+    if ((a.dim == 64 || a.dim == 128) && !(((uintptr_t)a.k_pool | (uintptr_t)a.v_pool) & 15)) {
+      int rc = tma_host::bf16_map(a.k_pool, 1ll << 28, a.dim, 16, 64, &mk);
+      if (rc == 0) rc = tma_host::bf16_map(a.v_pool, 1ll << 28, VDIM, 16, 64, &mv);
+      if (rc) return rc;
+      if (a.dim == 64) return tt_launch_as<VDIM, MAXH, 64>(mk, mv, a, n_seqs, max_q_len, stream);
+      return tt_launch_as<VDIM, MAXH, 128>(mk, mv, a, n_seqs, max_q_len, stream);
+    }
+  }
+  return tt_launch_as<VDIM, MAXH, 0>(mk, mv, a, n_seqs, max_q_len, stream);
 }
 
 // The sequences described by the three per-sequence arrays start at row `table_row0` of the
@@ -731,13 +866,13 @@ MF_API int mf_attention_talking_tc(const void* q, const void* k_pool, const void
                                    int table_row0, int n_seqs, int max_q_len, int n_heads, int n_kv, int dim, int vdim,
                                    const int* block_table, int bt_stride, int page_size, float scale, float softcap,
                                    const float* talk, int window, int chunk, int splits, float* part_o, float* part_ml,
-                                   int first_row, int n_rows, cudaStream_t stream) {
+                                   int first_row, int n_rows, int* status, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
   if (!mf_attention_talking_tc_ok(n_heads, n_kv, dim, vdim, page_size) || n_seqs > 65535 || splits < 0 || splits > 65535)
     return MF_ERR_BAD_ARG;
   TtArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out,
            seq_q_start, seq_q_len, seq_ctx_len, block_table, talk, table_row0, bt_stride, page_size, n_heads, n_kv, dim,
-           scale, softcap, window, chunk, splits, tt_prefill_split_tiles(window, chunk), part_o, part_ml};
+           scale, softcap, window, chunk, splits, tt_prefill_split_tiles(window, chunk), part_o, part_ml, status};
   mf_count(MF_K_ATTN_TALKING_TC);
   int rc = MF_ERR_BAD_ARG;
 #define TT_CASE(VD)                                                         \
@@ -773,13 +908,13 @@ MF_API int mf_attention_talking_decode(const void* q, const void* k_pool, const 
                                        const int* seq_q_start, const int* seq_q_len, const int* seq_ctx_len, int n_seqs,
                                        int n_heads, int n_kv, int dim, int vdim, const int* block_table, int bt_stride,
                                        int page_size, float scale, float softcap, const float* talk, int window,
-                                       int chunk, int splits, float* part_o, float* part_ml, cudaStream_t stream) {
+                                       int chunk, int splits, float* part_o, float* part_ml, int* status, cudaStream_t stream) {
   if (n_seqs <= 0) return 0;
   if (!mf_attention_talking_tc_ok(n_heads, n_kv, dim, vdim, page_size) || n_seqs > 65535 || splits < 1 || splits > 65535)
     return MF_ERR_BAD_ARG;
   TtArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out,
            seq_q_start, seq_q_len, seq_ctx_len, block_table, talk, 0, bt_stride, page_size, n_heads, n_kv, dim,
-           scale, softcap, window, chunk, splits, TT_SPLIT_TILES, part_o, part_ml};
+           scale, softcap, window, chunk, splits, TT_SPLIT_TILES, part_o, part_ml, status};
   mf_count(MF_K_ATTN_TALKING_TC);
   // the values of all key heads of a split have to fit in shared memory; what is wider takes the kernel of the prompts
   if (tt_decode_smem(n_heads, n_kv, vdim) <= 200 * 1024) {

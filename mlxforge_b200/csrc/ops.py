@@ -1346,7 +1346,7 @@ def attention_talking_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Te
                                             table_row0, seq_q_len.shape[0], max_q_len, n_heads, n_kv, dim, vdim,
                                             block_table.data_ptr(), block_table.shape[1], page_size, scale, softcap,
                                             _ptr(talk), window, chunk, splits, _ptr(part_o), _ptr(part_ml), first_row,
-                                            T - first_row, _stream()), "attention_talking_tc",
+                                            T - first_row, kernel_status(q.device).data_ptr(), _stream()), "attention_talking_tc",
           launches=2 if splits else 1)
 
 
@@ -1378,7 +1378,8 @@ def attention_talking_decode(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torc
                                                 seq_q_start.data_ptr(), seq_q_len.data_ptr(), seq_ctx_len.data_ptr(),
                                                 n, n_heads, n_kv, dim, vdim, block_table.data_ptr(),
                                                 block_table.shape[1], page_size, scale, softcap, _ptr(talk), window,
-                                                chunk, splits, part_o.data_ptr(), part_ml.data_ptr(), _stream()),
+                                                chunk, splits, part_o.data_ptr(), part_ml.data_ptr(), kernel_status(q.device).data_ptr(),
+                                                _stream()),
           "attention_talking_decode", launches=2)
 
 

@@ -282,3 +282,52 @@ def test_read_out_norms(V, heads, T, parts, dtype):
     ops.delta_output(o[0].contiguous(), gate[:, 4:], n + 4, w, 1e-6, out, heads, V)
     want = rms(o[0].double()) * w.double().repeat(heads) * gate[:, 4:].double()
     assert bool(((out.double() - want).abs() <= tol * want.abs() + 1e-12).all())
+
+
+# ----------------------------------------------------------------------------- talking heads: keys and values by tensor copies
+
+@pytest.mark.parametrize("H,G,dim,vdim,page,lens,held,window,chunk", [
+    (16, 4, 128, 128, 16, [33, 17], [0, 700], 0, 0), (8, 2, 128, 64, 32, [48], [15], 0, 32), (6, 3, 64, 128, 16, [70], [1100], 40, 0),
+    (4, 4, 64, 64, 48, [1, 31, 64], [5, 0, 0], 0, 0), (16, 1, 128, 128, 16, [130], [2000], 0, 2048), (4, 2, 80, 96, 16, [40], [9], 0, 0)])
+def test_talking_heads_portions(H, G, dim, vdim, page, lens, held, window, chunk):
+    """Head sizes with and without tensor copies, pages of other sizes, first and last granules that are partly unseen (NaN stands
+    wherever no key is), windows and chunks that begin inside a granule, key ranges that are cut."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(H + dim + sum(lens))
+    bf, T, ctx = torch.bfloat16, sum(lens), [n + h for n, h in zip(lens, held)]
+    q = torch.randn((T, H * dim), generator=g, device="cuda").to(bf)
+    talk = torch.eye(H, device="cuda") + 0.1 * torch.randn((H, H), generator=g, device="cuda")
+    per = [-(-c // page) for c in ctx]
+    ids = np.random.default_rng(0).permutation(sum(per) + 3)[:sum(per)]
+    kp, vp = (torch.full((sum(per) + 3, G, page, d), float("nan"), device="cuda", dtype=bf) for d in (dim, vdim))
+    table, ks, vs, at = np.full((len(lens), max(per)), -1, np.int32), [], [], 0
+    for s, (n, c) in enumerate(zip(per, ctx)):
+        table[s, :n] = ids[at:at + n]
+        at += n
+        ks.append(torch.randn((c, G, dim), generator=g, device="cuda").to(bf))
+        vs.append(torch.randn((c, G, vdim), generator=g, device="cuda").to(bf))
+        for b in range(n):
+            for pool, x in ((kp, ks[-1]), (vp, vs[-1])):
+                x = x[b * page:(b + 1) * page]
+                pool[int(table[s, b]), :, :x.shape[0]] = x.transpose(0, 1)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    out = torch.full((T, H * vdim), float("nan"), device="cuda", dtype=bf)
+    seen = max(min(c, chunk or c, window or c) for c in ctx) + 64
+    splits = ops.attention_talking_prefill_splits(seen, window, chunk)
+    f = lambda n: torch.full((max(n, 1),), float("nan"), device="cuda")
+    ops.attention_talking_tc(q, kp, vp, out, i32(np.cumsum([0] + lens[:-1]).tolist()), i32(lens), i32(ctx), 0, max(lens), torch.from_numpy(table).cuda(),
+                             page, H, G, dim, vdim, dim ** -0.5, 30.0, talk, window, chunk, splits, f(T * splits * H * vdim), f(T * splits * H * 2))
+    ops.check_kernel_status()
+    at = 0
+    for n, h, k, v in zip(lens, held, ks, vs):
+        i, j = torch.arange(h, h + n, device="cuda")[:, None], torch.arange(h + n, device="cuda")[None]
+        ok = (j <= i) & ((i - j < window) if window else True) & ((i // chunk == j // chunk) if chunk else True)
+        s = torch.einsum("ihd,jhd->hij", q[at:at + n].double().view(n, H, dim), k.double().repeat_interleave(H // G, 1)) * dim ** -0.5
+        s = torch.einsum("hg,gij->hij", talk.double(), 30.0 * torch.tanh(s / 30.0))
+        p = torch.softmax(s.masked_fill(~ok, -np.inf), 2)
+        vv = v.double().repeat_interleave(H // G, 1)
+        want, mag = torch.einsum("hij,jhd->ihd", p, vv).flatten(1), torch.einsum("hij,jhd->ihd", p, vv.abs()).flatten(1)
+        # a probability is rounded to 8 bits once, the result once more
+        assert bool(((out[at:at + n].double() - want).abs() <= 2 ** -8 * mag + 2 ** -8 * want.abs() + 1e-6).all()), n
+        at += n
