@@ -331,3 +331,20 @@ def test_talking_heads_portions(H, G, dim, vdim, page, lens, held, window, chunk
         # a probability is rounded to 8 bits once, the result once more
         assert bool(((out[at:at + n].double() - want).abs() <= 2 ** -8 * mag + 2 ** -8 * want.abs() + 1e-6).all()), n
         at += n
+
+
+# ----------------------------------------------------------------------------- 32-bit products
+
+@pytest.mark.parametrize("M,N,K", [(300, 3001, 36), (449, 1409, 67), (150, 2900, 52), (45, 700, 20)])
+def test_gemm_f32_every_tile(M, N, K):
+    """Sizes that choose 64 x 128, 48 x 128, 64 x 64 and 32 x 64 results a block, with broken tiles on both sides: rows have the bits
+    they have alone; sums of K products of unit normals in four chains within 2^-22 sqrt(K) of their norm sqrt(K)."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, w = torch.randn((M, K), generator=g, device="cuda"), torch.randn((N, K), generator=g, device="cuda")
+    out, few = torch.full((M, N), float("nan"), device="cuda"), torch.empty((5, N), device="cuda")
+    ops.gemm_f32(a, w, out)
+    assert bool(((out.double() - a.double() @ w.double().T).abs() < 2.0 ** -22 * K).all())
+    ops.gemm_f32(a[M - 5:].contiguous(), w, few)
+    assert torch.equal(few, out[M - 5:])
