@@ -12,9 +12,9 @@
 // the tiles instead (while they are copied, before a tile's product, behind it) cost the finite ones 1 to 27 %.
 //
 // The block per (token, head) of attention_generic.cu read every key row again for each of them, a lane a row of its own.
-// The layers around the two (projections included; us before -> now): 32 / 8 heads of 64, 300 tokens 964 -> 309; 384 tokens of
-// three sequences behind 1,000 keys 4,245 -> 538; a latent of 192 + 32 under 16 heads, 300 tokens 1,378 -> 608; one token behind
-// 8,000 keys 3,386 -> 1,289 (a block per KV head walks all of them: bound by the tiles' way through shared memory).
+// The layers around the two (projections included; us before -> now): 32 / 8 heads of 64, 300 tokens 964 -> 251; a latent of 192 + 32
+// under 16 heads, 150 tokens behind 300 keys 619 -> 334 with rows of keys looked up once a tile, values on their way while the
+// scores are made and tiles of 32 and 16 rows (8 tokens behind 1,000 keys 420 -> 261; 32 / 8 heads of 128 514 -> 268).
 // That kernel stays for bfloat16 at sizes the tensor-core kernels do not take and for rows that are no whole 16-byte pieces.
 #include "common.cuh"
 
@@ -183,26 +183,47 @@ attention_f32_kernel(const F32Args a) {
       for (int j = 0; j < CPT; j++) o[v][i][j] = 0.f;
 
   const int first_win = lo / KT * KT;
-  for (int k0 = keep > 0 ? 0 : first_win; k0 <= last; k0 += KT) {
-    if (k0 < first_win && k0 >= keep) {            // from the kept keys on to the window
-      k0 = first_win - KT;
-      continue;
-    }
-    // keys transposed, values as they are; keys that no row sees are zero and not read
-    for (int i = tid; i < KT * (dp / 4); i += 128) {
-      const int quad = i % 4, key = i / 4 % KT, d = i / (4 * KT) * 16 + quad * 4, j = k0 + key;
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (d < hd && j <= last && (j >= lo || j < keep)) x = load4(a.k_pool + paged_offset(a.pv, seq, j, kvh) + d);
-      float* dst = kt + d * KT + (key ^ quad * 8);
-      dst[0] = x.x; dst[KT] = x.y; dst[2 * KT] = x.z; dst[3 * KT] = x.w;
-    }
+  // where the keys of a tile stand in the pools, in rows (-1: no row of the tile sees the key), looked up a tile ahead: the table and
+  // the divisions for every piece of a key or value were most of a tile's time
+  __shared__ long long row_s[KT];
+  auto row_of = [&](int k0) {
+    const int j = k0 + tid;
+    if (tid >= KT || j > last || !(j >= lo || j < keep)) return -1ll;
+    return paged_offset(a.pv, seq, j, kvh) / hd;
+  };
+  auto after = [&](int k0) { return k0 + KT < first_win && k0 + KT >= keep ? first_win : k0 + KT; };      // from the kept keys on to the window
+  int k0 = keep > 0 ? 0 : first_win;
+  if (tid < KT) row_s[tid] = row_of(k0);
+  __syncthreads();
+  for (; k0 <= last;) {
+    // values as they are, on their way while the scores are made; keys transposed, eight pieces at a time; keys that no row sees are
+    // zero and not read
     for (int i = tid; i < KT * VW / 4; i += 128) {
-      const int key = i / (VW / 4), c = i % (VW / 4) * 4, j = k0 + key;
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c < a.vd && j <= last && (j >= lo || j < keep))
-        x = load4(a.v_pool + paged_offset(a.pv, seq, j, kvh) / hd * a.v_ld + c);
-      *reinterpret_cast<float4*>(vs + key * VW + c) = x;
+      const int key = i / (VW / 4), c = i % (VW / 4) * 4;
+      const long long row = row_s[key];
+      const bool in = c < a.vd && row >= 0;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(vs + key * VW + c)),
+                   "l"(in ? a.v_pool + row * a.v_ld + c : a.v_pool), "r"(in ? 16 : 0) : "memory");
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    for (int i0 = tid; i0 < KT * (dp / 4); i0 += 8 * 128) {
+      float4 x[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int i = i0 + u * 128, quad = i % 4, key = i / 4 % KT, d = i / (4 * KT) * 16 + quad * 4;
+        x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (d < hd && row_s[key] >= 0) x[u] = load4(a.k_pool + row_s[key] * hd + d);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int i = i0 + u * 128, quad = i % 4, key = i / 4 % KT, d = i / (4 * KT) * 16 + quad * 4;
+        if (d >= dp) break;
+        float* dst = kt + d * KT + (key ^ quad * 8);
+        dst[0] = x[u].x; dst[KT] = x[u].y; dst[2 * KT] = x[u].z; dst[3 * KT] = x[u].w;
+      }
+    }
+    const int k_next = after(k0);
+    const long long row_next = row_of(k_next);
     __syncthreads();
     float s[RPT][CPT];
 #pragma unroll
@@ -275,6 +296,8 @@ attention_f32_kernel(const F32Args a) {
       if constexpr (RPT == 4) *reinterpret_cast<float4*>(dst) = make_float4(s[0][j], s[1][j], s[RPT - 2][j], s[RPT - 1][j]);
       else *reinterpret_cast<float2*>(dst) = make_float2(s[0][j], s[1][j]);
     }
+    if (tid < KT) row_s[tid] = row_next;
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     // keys behind the last one any row sees have weight zero
     const int keys = min(KT, (last - k0 + 16) / 16 * 16);
@@ -299,6 +322,7 @@ attention_f32_kernel(const F32Args a) {
       }
     }
     __syncthreads();
+    k0 = k_next;
   }
 #pragma unroll
   for (int i = 0; i < RPT; i++) {
@@ -373,10 +397,16 @@ MF_API int mf_attention_f32(const float* q, const float* k_pool, const float* v_
   mf_count(MF_K_ATTN_GENERIC);
   mf_count(MF_K_ATTN_F32);
   const int rep = n_heads / n_kv, vc = (vd + 63) / 64;
-  // where 16 rows hold all there is, as in decoding, a tile does a quarter of the work
-  const bool few = (long long)max_q_len * rep <= 16;
+  // The tallest tile that leaves an SM a block and a half: a block is a warp a scheduler, which waits for itself; 16 rows where they hold
+  // all there is, as in decoding.  Heads of 128, 150 tokens behind 300 keys: 32 / 8 heads 202 us in 80 blocks of 64 rows, 102 in 152 of 32,
+  // 104 in 304 of 16; 16 / 4 heads 212 in 40, 99 in 76, 75 in 152.
+  const int sms = mf_sm_count();
+  auto crowded = [&](int rows) {
+    return rep <= rows && (long long)((max_q_len + rows / rep - 1) / (rows / rep)) * n_kv * n_seqs * 2 > 3ll * sms;
+  };
+  const int height = (long long)max_q_len * rep <= 16 ? 16 : crowded(64) ? 64 : crowded(32) ? 32 : rep <= 16 ? 16 : rep <= 32 ? 32 : 64;
   F32Args a{q, k_pool, v_pool, out, q_start, q_len, ctx_len, PagedView{block_table, bt_stride, page_size, n_kv, hd},
-            n_heads, rep, (few ? 16 : 64) / rep, scale, window, vd, v_ld, keep_first, sink, gate, gate_ld, softcap};
+            n_heads, rep, height / rep, scale, window, vd, v_ld, keep_first, sink, gate, gate_ld, softcap};
 #define F32_GO(RT)                                              \
   do {                                                          \
     if (vc == 1) return launch<RT, 1>(a, n_seqs, max_q_len, stream); \
@@ -384,7 +414,8 @@ MF_API int mf_attention_f32(const float* q, const float* k_pool, const float* v_
     if (vc == 3) return launch<RT, 3>(a, n_seqs, max_q_len, stream); \
     return launch<RT, 4>(a, n_seqs, max_q_len, stream);         \
   } while (0)
-  if (few) F32_GO(16);
+  if (height == 16) F32_GO(16);
+  if (height == 32) F32_GO(32);
   F32_GO(64);
 #undef F32_GO
 }

@@ -348,3 +348,38 @@ def test_gemm_f32_every_tile(M, N, K):
     assert bool(((out.double() - a.double() @ w.double().T).abs() < 2.0 ** -22 * K).all())
     ops.gemm_f32(a[M - 5:].contiguous(), w, few)
     assert torch.equal(few, out[M - 5:])
+
+
+@pytest.mark.parametrize("nh,nkv,hd,vd,n", [(8, 2, 64, 64, 40), (16, 4, 128, 128, 100), (3, 1, 96, 192, 70), (20, 1, 32, 32, 9)])
+def test_attention_f32_tiles_of_every_height(nh, nkv, hd, vd, n):
+    """A portion alone (tiles of 16 or 32 rows), beside a few and beside so many others that tiles of 64 rows are taken: the same bits,
+    within 2^-18 of a 64-bit result's weighted magnitudes (chains of at most 64 roundings of 2^-24 a tile, few tiles)."""
+    import torch
+    from types import SimpleNamespace
+    from mlxforge_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(n)
+    held, per = 130, -(-(130 + n) // 16)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    q = torch.randn((n, nh * hd), generator=g, device="cuda")
+    kp, vp = (torch.randn((per + 2, nkv, 16, d), generator=g, device="cuda") for d in (hd, vd))
+    order = np.random.default_rng(n).permutation(per + 2)[:per].astype(np.int32)
+    outs = []
+    for copies in (1, 6, 60):
+        out = torch.full((copies * n, nh * vd), float("nan"), device="cuda")
+        batch = SimpleNamespace(seq_q_start=i32([c * n for c in range(copies)]), seq_q_len=i32([n] * copies), seq_ctx_len=i32([held + n] * copies),
+                                n_seqs=copies, q_len=[n] * copies)
+        table = torch.from_numpy(np.tile(order, (copies, 1))).cuda()
+        if vd == hd:
+            ops.attention_f32(q.repeat(copies, 1), kp, vp, out, batch, table, 16, nh, nkv, hd, hd ** -0.5, 0, vd, vd)
+        else:
+            ops.attention_f32(q.repeat(copies, 1), kp, vp, out, batch, table, 16, nh, nkv, hd, hd ** -0.5, 90, vd, vd, 20)
+        outs.append(out[-n:])
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    k, v = (p[torch.from_numpy(order).long().cuda()].transpose(1, 2).reshape(per * 16, nkv, -1)[:held + n].double() for p in (kp, vp))
+    i, j = torch.arange(held, held + n, device="cuda")[:, None], torch.arange(held + n, device="cuda")[None]
+    seen = j <= i if vd == hd else (j <= i) & ((i - j < 90) | (j < 20))
+    for h in range(nh):
+        s = (q[:, h * hd:(h + 1) * hd].double() @ k[:, h // (nh // nkv)].T * hd ** -0.5).masked_fill(~seen, -np.inf)
+        p = torch.softmax(s, 1)
+        want, mag = p @ v[:, h // (nh // nkv)], p @ v[:, h // (nh // nkv)].abs()
+        assert bool(((outs[0][:, h * vd:(h + 1) * vd].double() - want).abs() <= 2 ** -18 * mag).all())
