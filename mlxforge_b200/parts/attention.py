@@ -19,6 +19,13 @@ from ..csrc import ops
 from .base import POSITIONS, FixedState, Mixer, PagedKV, PartSpec, TensorSpec, build_part, register_mixer
 
 
+def portions(batch):
+    """(start, length, context) of the sequences behind those that bring one token: the batch's own arrays where there are none of
+    those (a slice costs as much of the host's time as half a launch)."""
+    nd, arrays = batch.n_decode, (batch.seq_q_start, batch.seq_q_len, batch.seq_ctx_len)
+    return tuple(a[nd:] for a in arrays) if nd else arrays
+
+
 def paged_attention(rt, batch, q, lane, out, n_heads: int, scale: float, window: int) -> None:
     """Attention of the step's queries over ``lane``; the kernel is chosen by dtype and by how
     many tokens each sequence brings.  bfloat16: the sequences that bring one token (the batch
@@ -44,8 +51,7 @@ def paged_attention(rt, batch, q, lane, out, n_heads: int, scale: float, window:
                              batch.positions[:nd], batch.seq_of_token[:nd], table, lane.page_size, n_heads,
                              need.n_kv_heads, need.head_dim, scale, window, batch.max_ctx, unequal)
     if nd < batch.n_tokens and q.dtype == torch.bfloat16:
-        ops.attention_prefill(q, lane.k, lane.v, out, batch.seq_q_start[nd:], batch.seq_q_len[nd:],
-                              batch.seq_ctx_len[nd:], nd, max(batch.q_len[nd:]), table, lane.page_size,
+        ops.attention_prefill(q, lane.k, lane.v, out, *portions(batch), nd, max(batch.q_len[nd:]), table, lane.page_size,
                               n_heads, need.n_kv_heads, need.head_dim, scale, window)
     elif nd < batch.n_tokens:
         ops.attention_generic(q[nd:], lane.k, lane.v, out[nd:], batch.positions[nd:],
@@ -156,8 +162,7 @@ def options_paged_attention(rt, batch, q, lane, out, n_heads: int, scale: float,
                                 need.head_dim, scale, window, batch.max_ctx, vd, in_k, keep_first, sink, gate, gate_ld,
                                 softcap)
     if nd < batch.n_tokens:
-        ops.attention_prefill_ex(q, lane.k, lane.v, out, batch.seq_q_start[nd:], batch.seq_q_len[nd:],
-                                 batch.seq_ctx_len[nd:], nd, max(batch.q_len[nd:]), table, lane.page_size, n_heads,
+        ops.attention_prefill_ex(q, lane.k, lane.v, out, *portions(batch), nd, max(batch.q_len[nd:]), table, lane.page_size, n_heads,
                                  need.n_kv_heads, need.head_dim, scale, window, vd, in_k, keep_first, sink, gate,
                                  gate_ld, softcap, min(n for n in batch.q_len[nd:] if n))
 

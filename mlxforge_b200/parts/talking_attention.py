@@ -24,6 +24,7 @@ from typing import Dict
 import torch
 
 from ..csrc import ops
+from .attention import portions
 from .base import Mixer, PagedKV, TensorSpec, register_mixer
 
 _NAMES = {"q": "q", "k": "k", "v": "v", "o": "o", "talk": "talk", "bias": ".b"}
@@ -141,7 +142,6 @@ def talking_paged_attention(rt, batch, q, lane, out, m: TalkingAttention) -> Non
         if splits:
             part_o = rt.buffer("tattn.part_o", (T * splits * m.n_heads * m.vdim,), torch.float32)
             part_ml = rt.buffer("tattn.part_ml", (T * splits * m.n_heads * 2,), torch.float32)
-        ops.attention_talking_tc(q, lane.k, lane.v, out, batch.seq_q_start[nd:], batch.seq_q_len[nd:],
-                                 batch.seq_ctx_len[nd:], nd, max(batch.q_len[nd:]), table, lane.page_size,
+        ops.attention_talking_tc(q, lane.k, lane.v, out, *portions(batch), nd, max(batch.q_len[nd:]), table, lane.page_size,
                                  m.n_heads, m.n_kv, m.dim, m.vdim, m.scale, m.softcap, m.talk, m.window, m.chunk,
                                  splits, part_o, part_ml, nd)
