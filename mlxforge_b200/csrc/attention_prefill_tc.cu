@@ -42,7 +42,7 @@ constexpr float LOG2E = 1.4426950408889634f;
 constexpr float MAX_SLACK_LOG2 = 8.0f;
 // With options and over a latent the reference IS the maximum: the largest probability of a row is then a 1 that bfloat16
 // holds exactly, as in the mma.sync kernel that had these forms before, and the error against 64 bits is the same (a windowed
-// layer 0.00369 of the result; 0.00379 with the slack, which would take 49 instead of 53 us at 2,237 tokens).
+// layer 0.00369 of the result; 0.00379 with the slack, which took 49 instead of 53 us at 2,237 tokens with one chain a block).
 constexpr float EXACT_MAX_LOG2 = 0.0f;
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
