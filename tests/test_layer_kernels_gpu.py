@@ -383,3 +383,36 @@ def test_attention_f32_tiles_of_every_height(nh, nkv, hd, vd, n):
         p = torch.softmax(s, 1)
         want, mag = p @ v[:, h // (nh // nkv)], p @ v[:, h // (nh // nkv)].abs()
         assert bool(((outs[0][:, h * vd:(h + 1) * vd].double() - want).abs() <= 2 ** -18 * mag).all())
+
+
+# ----------------------------------------------------------------------------- experts, many tokens
+
+@pytest.mark.parametrize("T,top,E", [(1, 1, 1), (37, 3, 33), (2048, 8, 1024), (16385, 1, 64), (5001, 7, 200), (4099, 12, 2)])
+def test_sorted_pairs_and_gathered_rows(T, top, E):
+    """Pairs that a thread holds in registers (up to 16,384) and those beyond, experts in part of a warp up to all of the block's
+    threads, identity experts in between, gathers whose last block has a rest: whole numbers and copies, so equality."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    rng, H = np.random.default_rng(T + E), 64
+    ids = rng.integers(0, E + max(E // 4, 1), (T, top)).astype(np.int32)
+    ids[0, 0] = 0
+    n, tile_rows, bf = T * top, ops.moe_tc_rows(), torch.bfloat16
+    empty = lambda m: torch.full((m,), -7, dtype=torch.int32, device="cuda")
+    slot, row_token, meta, tiles = empty(n), empty(n), empty(4), empty(3 * ops.moe_grouped_max_tiles(T, top, E))
+    ops.moe_sort(torch.from_numpy(ids).cuda(), E, slot, row_token, meta, tiles, tile_rows)
+    slots, tokens = slot.cpu().numpy().reshape(T, top), row_token.cpu().numpy()
+    real = ids < E
+    m = int(real.sum())
+    assert np.all(slots[~real] == -1) and np.array_equal(np.sort(slots[real]), np.arange(m)) and np.all(tokens[m:] == 0)
+    assert np.array_equal(tokens[slots[real]], np.nonzero(real)[0])
+    of_row = np.empty(m, np.int64)
+    of_row[slots[real]] = ids[real]
+    assert np.all(np.diff(of_row) >= 0)                       # the experts' rows one expert after another
+    cuts = tiles.cpu().numpy()[:3 * int(meta[0])].reshape(-1, 3)
+    assert all(np.all(of_row[r:r + k] == e) and 0 < k <= tile_rows for e, r, k in cuts) and cuts[:, 2].sum() == m
+    x = torch.from_numpy(rng.standard_normal((T, H)).astype(np.float32)).cuda().to(bf)
+    xg, act = torch.zeros((n, H), dtype=bf, device="cuda"), torch.empty((n, 64), dtype=bf, device="cuda")
+    wg = torch.zeros((E, 2, 64, H), dtype=bf, device="cuda")
+    ops.moe_tc_up(x, row_token, xg, wg, meta, tiles, act, 1.5, 1.702, 1.0, None)
+    ops.check_kernel_status()
+    assert torch.equal(xg, x[row_token.long()])
