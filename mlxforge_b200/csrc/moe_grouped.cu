@@ -28,6 +28,7 @@
 #define MG_LD (MG_BK + 8)
 #define MG_STAGES 2
 #define MG_MAX_EXPERTS 1024
+#define MG_SORT_STAGED 32768       // pairs whose tokens the sort keeps in shared memory
 
 __device__ __forceinline__ void mg_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -39,11 +40,13 @@ __device__ __forceinline__ void mg_mma(float (&c)[4], const uint32_t (&a)[4], ui
 // meta: [0] number of tiles; tiles: [max_tiles][3] = expert, first row, rows.  An expert's rows are cut into as few tiles of at
 // most `tile_rows` as hold them: full ones and a rest (64 rows), or for larger tiles equal ones in steps of 16.  A thread per
 // expert: offsets by a scan over the block (a thread that walked the experts alone took most of 21 us for 64 of them).
-// A pair is counted once and its place kept (12,288 pairs of 64 experts: 11.0 -> 10.4 us); with the gather below and both launched
+// A pair is counted once and its place kept (12,288 pairs of 64 experts: 11.0 -> 10.4 us), and the rows' tokens are put in order in
+// shared memory where they fit, since a warp's 32 scattered words are 32 stores to memory (10.4 -> 7.2); with the gather below and both launched
 // behind their predecessor's end, the mixture of 2,048 tokens 207 -> 202.5 us.
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int* __restrict__ ids, int n_pairs, int E, int top, int tile_rows, int* __restrict__ slot_of,
-                int* __restrict__ row_token, int* __restrict__ meta, int* __restrict__ tiles) {
+                int* __restrict__ row_token, int* __restrict__ meta, int* __restrict__ tiles, int staged) {
+  extern __shared__ int tokens[];            // staged: [n_pairs], a row's token
   __shared__ int count[MG_MAX_EXPERTS], first[MG_MAX_EXPERTS];
   __shared__ int2 warp_total[32];
   __shared__ int used_rows;
@@ -111,7 +114,8 @@ moe_sort_kernel(const int* __restrict__ ids, int n_pairs, int E, int top, int ti
     }
     const int row = first[id] + at;
     slot_of[i] = row;
-    row_token[row] = i / top;
+    if (staged) tokens[row] = i / top;
+    else row_token[row] = i / top;
   };
 #pragma unroll
   for (int k = 0; k < HELD; k++) put(e + k * 1024, own[k], place[k]);
@@ -125,6 +129,10 @@ moe_sort_kernel(const int* __restrict__ ids, int n_pairs, int E, int top, int ti
 #pragma unroll
     for (int k = 0; k < HELD; k++) put(i0 + k * 1024, id[k], at[k]);
   }
+  if (staged) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < used_rows; i += blockDim.x) row_token[i] = tokens[i];
+  }
   // rows that no pair took (pairs of identity experts have none) name token 0, so that a gather over all
   // n_pairs rows stays inside x
   for (int i = used_rows + threadIdx.x; i < n_pairs; i += blockDim.x) row_token[i] = 0;
@@ -135,8 +143,18 @@ MF_API int mf_moe_sort(const int* ids, int T, int E, int top, int tile_rows, int
   if (T <= 0) return 0;
   if (E < 1 || E > MG_MAX_EXPERTS || tile_rows < MG_BM || tile_rows % 16) return MF_ERR_BAD_ARG;
   mf_count(MF_K_MOE_SORT);
-  return (int)launch_dep(moe_sort_kernel, dim3(1), dim3(1024), 0, stream, ids, T * top, E, top, tile_rows, slot_of, row_token,
-                         meta, tiles);
+  // rows' tokens are put in order in shared memory where they fit
+  const int n = T * top, staged = n <= MG_SORT_STAGED;
+  static DeviceOnce once;
+  const int dev = mf_current_device();
+  if (dev < 0) return MF_ERR_BAD_ARG;
+  if (!once.done[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(moe_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SORT_STAGED * 4);
+    if (e != cudaSuccess) return (int)e;
+    once.done[dev] = true;
+  }
+  return (int)launch_dep(moe_sort_kernel, dim3(1), dim3(1024), staged ? n * sizeof(int) : 0, stream, ids, n, E, top, tile_rows,
+                         slot_of, row_token, meta, tiles, staged);
 }
 
 __device__ __forceinline__ void mg_ldmatrix_x4(uint32_t (&r)[4], const void* p) {
