@@ -14,6 +14,7 @@
 // The split size is fixed (it depends on the head size only), so a token's result
 // does not depend on what else is in the batch.  Formula: src/model/sdpa.cpp:71-95.
 #include "common.cuh"
+#include "tma_host.cuh"
 
 namespace {
 
@@ -394,7 +395,7 @@ int launch_decode(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __n
 // attention_decode_tma.cu: the first kernel with keys and values brought in by the TMA unit
 int launch_decode_tma(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __nv_bfloat16* v_pool,
                       __nv_bfloat16* out, float* part_o, float* part_ml, int n_tokens, int n_heads, PagedView pv,
-                      long long pool_rows, const int* positions, const int* seq_of_token, float scale, int window,
+                      const int* positions, const int* seq_of_token, float scale, int window,
                       int max_ctx, int unequal, int* status, int* split_out, int* merged_out, cudaStream_t stream);
 extern int g_merge_inside;
 
@@ -447,27 +448,27 @@ MF_API int mf_attention_decode_ex_split(int hd, int window) {
 // Scratch: part_o  [n_tokens * n_heads * max_splits * hd] floats,
 //          part_ml [n_tokens * n_heads * max_splits * 2] floats, max_splits = ceil(max_ctx / split).
 // `max_ctx` bounds position + 1 of every token; a larger value only costs idle blocks.
+// `pool_rows`: rows of hd numbers that each pool holds (pages x KV heads x page size); the tensor copies' maps end there.
 // `unequal_contexts` != 0: the caller knows that the tokens' contexts differ widely in length (the
 // kernels read the lengths on the device, the launcher cannot); with many work items to a block
 // the kernel whose blocks the hardware deals out is then taken instead of the persistent one.
 MF_API int mf_attention_decode_hinted(const void* q, const void* k_pool, const void* v_pool, void* out, float* part_o,
                                       float* part_ml, int n_tokens, int n_heads, int n_kv, int hd, const int* positions,
                                       const int* seq_of_token, const int* block_table, int bt_stride, int page_size,
-                                      float scale, int window, int max_ctx, int unequal_contexts, cudaStream_t stream) {
+                                      long long pool_rows, float scale, int window, int max_ctx, int unequal_contexts,
+                                      cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (hd < 16 || hd > 256 || hd % 16 || n_kv <= 0 || n_heads % n_kv || max_ctx <= 0) return MF_ERR_BAD_ARG;
   if (n_tokens > 65535) return MF_ERR_BAD_ARG;
-  PagedView pv{block_table, bt_stride, page_size, n_kv, hd};
+  PagedView pv{block_table, bt_stride, page_size, n_kv, hd, pool_rows};
   g_last_decode_launches = 2;
   const __nv_bfloat16 *qq = (const __nv_bfloat16*)q, *kk = (const __nv_bfloat16*)k_pool,
                       *vv = (const __nv_bfloat16*)v_pool;
   __nv_bfloat16* oo = (__nv_bfloat16*)out;
   if ((hd == 64 || hd == 128) && g_decode_tma) {
-    // the map's row count only bounds the unit's own range check; rows beyond the pool are never asked for
     int split = SPLIT_KEYS, merged = 0;
-    const int rc = launch_decode_tma(qq, kk, vv, oo, part_o, part_ml, n_tokens, n_heads, pv, 1ll << 28, positions,
-                                     seq_of_token, scale, window, max_ctx, unequal_contexts, g_decode_status, &split,
-                                     &merged, stream);
+    const int rc = launch_decode_tma(qq, kk, vv, oo, part_o, part_ml, n_tokens, n_heads, pv, positions, seq_of_token, scale, window,
+                                     max_ctx, unequal_contexts, g_decode_status, &split, &merged, stream);
     if (rc == 0 && merged) {
       mf_count(MF_K_ATTN_DECODE_TMA_MERGED);
       g_last_decode_launches = 1;
@@ -526,8 +527,14 @@ MF_API int mf_attention_decode(const void* q, const void* k_pool, const void* v_
                                float* part_ml, int n_tokens, int n_heads, int n_kv, int hd, const int* positions,
                                const int* seq_of_token, const int* block_table, int bt_stride, int page_size,
                                float scale, int window, int max_ctx, cudaStream_t stream) {
+  // this caller does not say how long its pools are: as far as the memory they stand in goes
+  long long rows = 0;
+  if (hd == 64 || hd == 128) {
+    const long long k_rows = tma_host::mapped_rows(k_pool, 2ll * hd), v_rows = tma_host::mapped_rows(v_pool, 2ll * hd);
+    rows = k_rows < v_rows ? k_rows : v_rows;
+  }
   return mf_attention_decode_hinted(q, k_pool, v_pool, out, part_o, part_ml, n_tokens, n_heads, n_kv, hd, positions,
-                                    seq_of_token, block_table, bt_stride, page_size, scale, window, max_ctx, 0, stream);
+                                    seq_of_token, block_table, bt_stride, page_size, rows, scale, window, max_ctx, 0, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

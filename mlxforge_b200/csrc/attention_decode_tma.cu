@@ -493,14 +493,14 @@ namespace {
 
 template <int HD, int STAGES, int BLOCKS_PER_SM>
 int launch_for(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __nv_bfloat16* v_pool, __nv_bfloat16* out,
-               float* part_o, float* part_ml, int n_tokens, int n_heads, PagedView pv, long long pool_rows,
+               float* part_o, float* part_ml, int n_tokens, int n_heads, PagedView pv,
                const int* positions, const int* seq_of_token, float scale, int window, int max_ctx, int unequal,
                int* status, int* split_out, int* merged_out, cudaStream_t stream) {
   constexpr int STAGE_BYTES = 2 * 8 * (HD / 64) * BOX_BYTES, Q_BYTES = 16 * HD * 2;
   CUtensorMap mk, mv;
-  int rc = tma_host::bf16_map(k_pool, pool_rows, HD, 16, 64, &mk);
+  int rc = tma_host::bf16_map(k_pool, pv.pool_rows, HD, 16, 64, &mk);
   if (rc) return rc;
-  rc = tma_host::bf16_map(v_pool, pool_rows, HD, 16, 64, &mv);
+  rc = tma_host::bf16_map(v_pool, pv.pool_rows, HD, 16, 64, &mv);
   if (rc) return rc;
   const int G0 = n_heads / pv.n_kv_heads;
   const int comb_rows = G0 < 16 ? G0 : 16;
@@ -559,19 +559,19 @@ int launch_for(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __nv_b
 // Returns MF_ERR_BAD_ARG when this path does not apply.
 int launch_decode_tma(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __nv_bfloat16* v_pool,
                       __nv_bfloat16* out, float* part_o, float* part_ml, int n_tokens, int n_heads, PagedView pv,
-                      long long pool_rows, const int* positions, const int* seq_of_token, float scale, int window,
+                      const int* positions, const int* seq_of_token, float scale, int window,
                       int max_ctx, int unequal, int* status, int* split_out, int* merged_out, cudaStream_t stream) {
-  if (pv.page_size % 16) return MF_ERR_BAD_ARG;
+  if (pv.page_size % 16 || pv.pool_rows <= 0) return MF_ERR_BAD_ARG;
   if (pv.head_dim == 64)
-    return launch_for<64, 3, 2>(q, k_pool, v_pool, out, part_o, part_ml, n_tokens, n_heads, pv, pool_rows, positions,
+    return launch_for<64, 3, 2>(q, k_pool, v_pool, out, part_o, part_ml, n_tokens, n_heads, pv, positions,
                                 seq_of_token, scale, window, max_ctx, unequal, status, split_out, merged_out, stream);
   if (pv.head_dim == 128) {
     // one block per SM with three stages of 64 KB; groups of many heads need a combine buffer that
     // leaves room for two stages only
-    const int rc = launch_for<128, 3, 1>(q, k_pool, v_pool, out, part_o, part_ml, n_tokens, n_heads, pv, pool_rows,
-                                         positions, seq_of_token, scale, window, max_ctx, unequal, status, split_out, merged_out, stream);
+    const int rc = launch_for<128, 3, 1>(q, k_pool, v_pool, out, part_o, part_ml, n_tokens, n_heads, pv, positions,
+                                         seq_of_token, scale, window, max_ctx, unequal, status, split_out, merged_out, stream);
     if (rc != MF_ERR_BAD_ARG) return rc;
-    return launch_for<128, 2, 1>(q, k_pool, v_pool, out, part_o, part_ml, n_tokens, n_heads, pv, pool_rows, positions,
+    return launch_for<128, 2, 1>(q, k_pool, v_pool, out, part_o, part_ml, n_tokens, n_heads, pv, positions,
                                  seq_of_token, scale, window, max_ctx, unequal, status, split_out, merged_out, stream);
   }
   return MF_ERR_BAD_ARG;

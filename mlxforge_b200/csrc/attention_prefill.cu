@@ -361,18 +361,19 @@ int prefill_tc_rows();
 // q, out: [T, n_heads * hd] of the whole step.  The n_seqs sequences start at row
 // `table_row0` of the block table; seq_q_start / seq_q_len / seq_ctx_len are their
 // first token's index in q, their number of new tokens and their length after the
-// step.  `max_q_len` bounds seq_q_len (it sizes the grid); `n_tokens` is T.  `status`: a device int
+// step.  `max_q_len` bounds seq_q_len (it sizes the grid); `n_tokens` is T.  `pool_rows`: rows (pages x KV heads x page
+// size) of either pool, where the tensor copies' maps end.  `status`: a device int
 // (may be null) for the bounded waits of the tcgen05 kernel (attention_prefill_tc.cu), which
 // takes head size 64 when a portion has at least 128 tokens.
 MF_API int mf_attention_prefill(const void* q, const void* k_pool, const void* v_pool, void* out,
                                 const int* seq_q_start, const int* seq_q_len, const int* seq_ctx_len,
                                 int table_row0, int n_seqs, int max_q_len, int n_tokens, int n_heads, int n_kv,
-                                int hd, const int* block_table, int bt_stride, int page_size, float scale,
+                                int hd, const int* block_table, int bt_stride, int page_size, long long pool_rows, float scale,
                                 int window, int* status, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
   if (hd < 16 || hd > 256 || hd % 16 || n_kv <= 0 || n_heads % n_kv) return MF_ERR_BAD_ARG;
   if (n_heads > 65535 || n_seqs > 65535) return MF_ERR_BAD_ARG;
-  PagedView pv{block_table, bt_stride, page_size, n_kv, hd};
+  PagedView pv{block_table, bt_stride, page_size, n_kv, hd, pool_rows};
   const __nv_bfloat16 *qq = (const __nv_bfloat16*)q, *kk = (const __nv_bfloat16*)k_pool,
                       *vv = (const __nv_bfloat16*)v_pool;
   __nv_bfloat16* oo = (__nv_bfloat16*)out;
@@ -400,14 +401,14 @@ MF_API int mf_attention_prefill(const void* q, const void* k_pool, const void* v
 MF_API int mf_attention_prefill_ex(const void* q, const void* k_pool, const void* v_pool, void* out,
                                    const int* seq_q_start, const int* seq_q_len, const int* seq_ctx_len,
                                    int table_row0, int n_seqs, int min_q_len, int max_q_len, int n_tokens, int n_heads,
-                                   int n_kv, int hd, const int* block_table, int bt_stride, int page_size, float scale,
+                                   int n_kv, int hd, const int* block_table, int bt_stride, int page_size, long long pool_rows, float scale,
                                    int window, int vd, int v_in_k, int keep_first, const float* sink, const void* gate,
                                    long long gate_ld, float softcap, int* status, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
   if (hd < 16 || hd > 256 || hd % 16 || n_kv <= 0 || n_heads % n_kv) return MF_ERR_BAD_ARG;
   if (vd <= 0 || vd > hd || vd % 16 || keep_first < 0) return MF_ERR_BAD_ARG;
   if (n_heads > 65535 || n_seqs > 65535) return MF_ERR_BAD_ARG;
-  PagedView pv{block_table, bt_stride, page_size, n_kv, hd};
+  PagedView pv{block_table, bt_stride, page_size, n_kv, hd, pool_rows};
   AttnOptions opt{vd, v_in_k, keep_first, sink, (const __nv_bfloat16*)gate, gate_ld, softcap, 0};
   const __nv_bfloat16 *qq = (const __nv_bfloat16*)q, *kk = (const __nv_bfloat16*)k_pool,
                       *vv = (const __nv_bfloat16*)v_pool;

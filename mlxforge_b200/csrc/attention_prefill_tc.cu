@@ -502,9 +502,9 @@ int launch_tc_ahead(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const _
   CUtensorMap mq, mk, mv;
   int rc = tma_host::bf16_map(q, n_tokens, (long long)n_heads * ahead::HD, BM, 64, &mq);
   if (rc) return rc;
-  rc = tma_host::bf16_map(k_pool, 1ll << 28, ahead::HD, 16, 64, &mk);
+  rc = tma_host::bf16_map(k_pool, pv.pool_rows, ahead::HD, 16, 64, &mk);
   if (rc) return rc;
-  rc = tma_host::bf16_map(v_pool, 1ll << 28, ahead::HD, 16, 64, &mv);
+  rc = tma_host::bf16_map(v_pool, pv.pool_rows, ahead::HD, 16, 64, &mv);
   if (rc) return rc;
   static DeviceOnce once;
   const int dev_ = mf_current_device();
@@ -896,11 +896,10 @@ int launch_pair(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __nv_
   CUtensorMap mq, mk, mv, mk4, mv4;
   int rc = tma_host::bf16_map(q, n_tokens, (long long)n_heads * pv.head_dim, BM, 64, &mq);
   if (rc) return rc;
-  // the maps' row count only bounds the unit's own range check; rows beyond the pool are never asked for
-  rc = tma_host::bf16_map(k_pool, 1ll << 28, pv.head_dim, 16, 64, &mk);
+  rc = tma_host::bf16_map(k_pool, pv.pool_rows, pv.head_dim, 16, 64, &mk);
   if (rc) return rc;
   if (OWN_V) {
-    rc = tma_host::bf16_map(v_pool, 1ll << 28, vd, 16, 64, &mv);
+    rc = tma_host::bf16_map(v_pool, pv.pool_rows, vd, 16, 64, &mv);
     if (rc) return rc;
   } else {
     mv = mk;
@@ -908,9 +907,10 @@ int launch_pair(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __nv_
   // four pages of 16 tokens at once: [pages][rows of a page][channels]
   mk4 = mk, mv4 = mv;
   if (pv.page_size == 16) {
-    rc = tma_host::bf16_map_pages(k_pool, pv.n_kv_heads * 16, pv.head_dim, 4, &mk4);
+    const long long pages = pv.pool_rows / (pv.n_kv_heads * 16);
+    rc = tma_host::bf16_map_pages(k_pool, pages, pv.n_kv_heads * 16, pv.head_dim, 4, &mk4);
     if (rc) return rc;
-    rc = OWN_V ? tma_host::bf16_map_pages(v_pool, pv.n_kv_heads * 16, vd, 4, &mv4) : 0;
+    rc = OWN_V ? tma_host::bf16_map_pages(v_pool, pages, pv.n_kv_heads * 16, vd, 4, &mv4) : 0;
     if (rc) return rc;
   }
   constexpr size_t smem = pair::smem(SPANS, VSPANS, OWN_V);
@@ -1163,7 +1163,7 @@ int launch_latent(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, __nv_bflo
   CUtensorMap mq, mk;
   int rc = tma_host::bf16_map(q, n_tokens, (long long)n_heads * pv.head_dim, BM, 64, &mq);
   if (rc) return rc;
-  rc = tma_host::bf16_map(k_pool, 1ll << 28, pv.head_dim, 16, 64, &mk);
+  rc = tma_host::bf16_map(k_pool, pv.pool_rows, pv.head_dim, 16, 64, &mk);
   if (rc) return rc;
   static DeviceOnce once;
   const int dev_ = mf_current_device();
@@ -1197,7 +1197,7 @@ int launch_prefill_tc(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const
                       __nv_bfloat16* out, const int* seq_q_start, const int* seq_q_len, const int* seq_ctx_len,
                       int table_row0, int n_seqs, int max_q_len, int n_tokens, int n_heads, PagedView pv,
                       float scale, int window, int* status, cudaStream_t stream) {
-  if (!g_prefill_tc || pv.page_size % 16 || max_q_len < BM || n_tokens <= 0) return MF_ERR_BAD_ARG;
+  if (!g_prefill_tc || pv.page_size % 16 || max_q_len < BM || n_tokens <= 0 || pv.pool_rows <= 0) return MF_ERR_BAD_ARG;
   if ((((uintptr_t)q | (uintptr_t)out) & 15) != 0) return MF_ERR_BAD_ARG;
   if (pv.head_dim == 64)
     return launch_tc_ahead(q, k_pool, v_pool, out, seq_q_start, seq_q_len, seq_ctx_len, table_row0, n_seqs, max_q_len,
@@ -1218,7 +1218,7 @@ int launch_prefill_tc_ex(const __nv_bfloat16* q, const __nv_bfloat16* k_pool, co
                          __nv_bfloat16* out, const int* seq_q_start, const int* seq_q_len, const int* seq_ctx_len,
                          int table_row0, int n_seqs, int max_q_len, int n_tokens, int n_heads, PagedView pv,
                          float scale, int window, const AttnOptions& opt, int min_len, int* status, cudaStream_t stream) {
-  if (!g_prefill_tc || pv.page_size % 16 || max_q_len < BM || n_tokens <= 0 || opt.softcap > 0.f) return MF_ERR_BAD_ARG;
+  if (!g_prefill_tc || pv.page_size % 16 || max_q_len < BM || n_tokens <= 0 || pv.pool_rows <= 0 || opt.softcap > 0.f) return MF_ERR_BAD_ARG;
   if ((((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool) & 15) != 0 || (max_q_len + BM - 1) / BM > 65535) return MF_ERR_BAD_ARG;
   const int hd = pv.head_dim, vd = opt.vd;
   if (!opt.v_in_k) {

@@ -160,6 +160,7 @@ struct TtArgs {
   float* part_o;            // [rows, splits, H, VDIM] unnormalised outputs of the splits
   float* part_ml;           // [rows, splits, H, 2]    maximum (in powers of two) and sum
   int* status;              // codes 91 (keys) and 92 (values): a wait for a copy ran out
+  long long pool_rows;      // rows (pages x KV heads x page size) of either pool
 };
 
 // DIM: the head size, where keys and values come by tensor copies (64 or 128, and values of whole 64-wide spans), [head][span][32 keys]
@@ -848,9 +849,9 @@ template <int VDIM, int MAXH>
 static int tt_launch(const TtArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
   CUtensorMap mk = {}, mv = {};
   if constexpr (VDIM % 64 == 0) {
-    if ((a.dim == 64 || a.dim == 128) && !(((uintptr_t)a.k_pool | (uintptr_t)a.v_pool) & 15)) {
-      int rc = tma_host::bf16_map(a.k_pool, 1ll << 28, a.dim, 16, 64, &mk);
-      if (rc == 0) rc = tma_host::bf16_map(a.v_pool, 1ll << 28, VDIM, 16, 64, &mv);
+    if ((a.dim == 64 || a.dim == 128) && a.pool_rows > 0 && !(((uintptr_t)a.k_pool | (uintptr_t)a.v_pool) & 15)) {
+      int rc = tma_host::bf16_map(a.k_pool, a.pool_rows, a.dim, 16, 64, &mk);
+      if (rc == 0) rc = tma_host::bf16_map(a.v_pool, a.pool_rows, VDIM, 16, 64, &mv);
       if (rc) return rc;
       if (a.dim == 64) return tt_launch_as<VDIM, MAXH, 64>(mk, mv, a, n_seqs, max_q_len, stream);
       return tt_launch_as<VDIM, MAXH, 128>(mk, mv, a, n_seqs, max_q_len, stream);
@@ -864,7 +865,7 @@ static int tt_launch(const TtArgs& a, int n_seqs, int max_q_len, cudaStream_t st
 MF_API int mf_attention_talking_tc(const void* q, const void* k_pool, const void* v_pool, void* out,
                                    const int* seq_q_start, const int* seq_q_len, const int* seq_ctx_len,
                                    int table_row0, int n_seqs, int max_q_len, int n_heads, int n_kv, int dim, int vdim,
-                                   const int* block_table, int bt_stride, int page_size, float scale, float softcap,
+                                   const int* block_table, int bt_stride, int page_size, long long pool_rows, float scale, float softcap,
                                    const float* talk, int window, int chunk, int splits, float* part_o, float* part_ml,
                                    int first_row, int n_rows, int* status, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
@@ -872,7 +873,7 @@ MF_API int mf_attention_talking_tc(const void* q, const void* k_pool, const void
     return MF_ERR_BAD_ARG;
   TtArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out,
            seq_q_start, seq_q_len, seq_ctx_len, block_table, talk, table_row0, bt_stride, page_size, n_heads, n_kv, dim,
-           scale, softcap, window, chunk, splits, tt_prefill_split_tiles(window, chunk), part_o, part_ml, status};
+           scale, softcap, window, chunk, splits, tt_prefill_split_tiles(window, chunk), part_o, part_ml, status, pool_rows};
   mf_count(MF_K_ATTN_TALKING_TC);
   int rc = MF_ERR_BAD_ARG;
 #define TT_CASE(VD)                                                         \
@@ -907,14 +908,14 @@ MF_API int mf_attention_talking_splits(int max_keys) {
 MF_API int mf_attention_talking_decode(const void* q, const void* k_pool, const void* v_pool, void* out,
                                        const int* seq_q_start, const int* seq_q_len, const int* seq_ctx_len, int n_seqs,
                                        int n_heads, int n_kv, int dim, int vdim, const int* block_table, int bt_stride,
-                                       int page_size, float scale, float softcap, const float* talk, int window,
+                                       int page_size, long long pool_rows, float scale, float softcap, const float* talk, int window,
                                        int chunk, int splits, float* part_o, float* part_ml, int* status, cudaStream_t stream) {
   if (n_seqs <= 0) return 0;
   if (!mf_attention_talking_tc_ok(n_heads, n_kv, dim, vdim, page_size) || n_seqs > 65535 || splits < 1 || splits > 65535)
     return MF_ERR_BAD_ARG;
   TtArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out,
            seq_q_start, seq_q_len, seq_ctx_len, block_table, talk, 0, bt_stride, page_size, n_heads, n_kv, dim,
-           scale, softcap, window, chunk, splits, TT_SPLIT_TILES, part_o, part_ml, status};
+           scale, softcap, window, chunk, splits, TT_SPLIT_TILES, part_o, part_ml, status, pool_rows};
   mf_count(MF_K_ATTN_TALKING_TC);
   // the values of all key heads of a split have to fit in shared memory; what is wider takes the kernel of the prompts
   if (tt_decode_smem(n_heads, n_kv, vdim) <= 200 * 1024) {

@@ -38,14 +38,14 @@ _SIGNATURES = {
     "mf_set_stream_tensor_copies": [c_int],
     "mf_stream_linear": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_float, _P, _P],
     "mf_attention_prefill": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int,
-                             c_int, c_float, c_int, _P, _P],
+                             c_int, c_longlong, c_float, c_int, _P, _P],
     "mf_set_prefill_tcgen05": [c_int],
     "mf_attention_decode_split": [c_int],
     "mf_attention_decode_ex_split": [c_int, c_int],
     "mf_attention_decode": [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P, c_int, c_int,
                             c_float, c_int, c_int, _P],
     "mf_attention_decode_hinted": [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P, c_int, c_int,
-                                   c_float, c_int, c_int, c_int, _P],
+                                   c_longlong, c_float, c_int, c_int, c_int, _P],
     "mf_apply_penalties": [_P, c_int, c_longlong, _P, _P, _P, _P, _P, _P, _P],
     "mf_filter_logits": [_P, c_int, c_int, c_longlong, _P, _P, _P, _P, _P],
     "mf_kernel_kinds": [],
@@ -87,11 +87,11 @@ _SIGNATURES = {
     "mf_moe_rows_slices": [c_int],
     "mf_attention_talking_tc_ok": [c_int, c_int, c_int, c_int, c_int],
     "mf_attention_talking_tc": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int,
-                                c_int, c_float, c_float, _P, c_int, c_int, c_int, _P, _P, c_int, c_int, _P, _P],
+                                c_int, c_longlong, c_float, c_float, _P, c_int, c_int, c_int, _P, _P, c_int, c_int, _P, _P],
     "mf_attention_talking_prefill_splits": [c_int, c_int, c_int],
     "mf_attention_talking_splits": [c_int],
     "mf_attention_talking_decode": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, c_int, c_int,
-                                    c_float, c_float, _P, c_int, c_int, c_int, _P, _P, _P, _P],
+                                    c_longlong, c_float, c_float, _P, c_int, c_int, c_int, _P, _P, _P, _P],
     "mf_moe_sort": [_P, c_int, c_int, c_int, c_int, _P, _P, _P, _P, _P],
     "mf_moe_tc_rows": [],
     "mf_moe_tc_up": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, _P, _P],
@@ -102,7 +102,7 @@ _SIGNATURES = {
                           _P],
     "mf_moe_grouped_down": [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P],
     "mf_attention_prefill_ex": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int, c_int,
-                                c_float, c_int, c_int, c_int, c_int, _P, _P, c_longlong, c_float, _P, _P],
+                                c_longlong, c_float, c_int, c_int, c_int, c_int, _P, _P, c_longlong, c_float, _P, _P],
     "mf_attention_decode_ex": [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P, c_int, c_int,
                                c_float, c_int, c_int, c_int, c_int, c_int, _P, _P, c_longlong, c_float, _P],
     "mf_gated_act": [_P, _P, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, _P],

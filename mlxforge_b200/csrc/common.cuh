@@ -135,6 +135,7 @@ struct PagedView {
   int page_size;
   int n_kv_heads;
   int head_dim;
+  long long pool_rows;      // rows of head_dim numbers that a pool holds (pages x KV heads x page size), for the tensor copies' maps
 };
 __device__ __forceinline__ long long paged_offset(const PagedView& pv, int seq, int pos, int kv_head) {
   const int blk = pos / pv.page_size, slot = pos - blk * pv.page_size;

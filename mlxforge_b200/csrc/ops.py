@@ -249,8 +249,8 @@ def attention_prefill_ex(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Te
     check(library().mf_attention_prefill_ex(q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(),
                                             seq_q_start.data_ptr(), seq_q_len.data_ptr(), seq_ctx_len.data_ptr(),
                                             table_row0, seq_q_len.shape[0], min_q_len, max_q_len, q.shape[0], n_heads, n_kv, head_dim,
-                                            block_table.data_ptr(), block_table.shape[1], page_size, scale, window,
-                                            v_dim, int(v_in_k), keep_first, _ptr(sink), _ptr(gate), gate_ld,
+                                            block_table.data_ptr(), block_table.shape[1], page_size, k_pool.numel() // head_dim, scale,
+                                            window, v_dim, int(v_in_k), keep_first, _ptr(sink), _ptr(gate), gate_ld,
                                             float(softcap or 0.0), kernel_status(q.device).data_ptr(), _stream()),
           "attention_prefill_ex")
 
@@ -543,8 +543,8 @@ def attention_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tenso
     check(library().mf_attention_prefill(q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(),
                                          seq_q_start.data_ptr(), seq_q_len.data_ptr(), seq_ctx_len.data_ptr(),
                                          table_row0, seq_q_len.shape[0], max_q_len, q.shape[0], n_heads, n_kv,
-                                         head_dim, block_table.data_ptr(), block_table.shape[1], page_size, scale,
-                                         window, kernel_status(q.device).data_ptr(), _stream()), "attention_prefill")
+                                         head_dim, block_table.data_ptr(), block_table.shape[1], page_size,
+                                         k_pool.numel() // head_dim, scale, window, kernel_status(q.device).data_ptr(), _stream()), "attention_prefill")
 
 
 def set_prefill_tcgen05(on: bool) -> None:
@@ -757,7 +757,7 @@ def attention_decode(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor
     check(library().mf_attention_decode_hinted(q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(),
                                                part_o.data_ptr(), part_ml.data_ptr(), n, n_heads, n_kv, head_dim,
                                                positions.data_ptr(), seq_of_token.data_ptr(), block_table.data_ptr(),
-                                               block_table.shape[1], page_size, scale, window, max_ctx,
+                                               block_table.shape[1], page_size, k_pool.numel() // head_dim, scale, window, max_ctx,
                                                1 if unequal_contexts else 0, _stream()),
           "attention_decode", launches=0)
     # one kernel when the TMA kernel merged its splits itself, two when a merge kernel followed
@@ -1345,8 +1345,8 @@ def attention_talking_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Te
     check(library().mf_attention_talking_tc(q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(),
                                             seq_q_start.data_ptr(), seq_q_len.data_ptr(), seq_ctx_len.data_ptr(),
                                             table_row0, seq_q_len.shape[0], max_q_len, n_heads, n_kv, dim, vdim,
-                                            block_table.data_ptr(), block_table.shape[1], page_size, scale, softcap,
-                                            _ptr(talk), window, chunk, splits, _ptr(part_o), _ptr(part_ml), first_row,
+                                            block_table.data_ptr(), block_table.shape[1], page_size, k_pool.numel() // dim, scale,
+                                            softcap, _ptr(talk), window, chunk, splits, _ptr(part_o), _ptr(part_ml), first_row,
                                             T - first_row, kernel_status(q.device).data_ptr(), _stream()), "attention_talking_tc",
           launches=2 if splits else 1)
 
@@ -1378,7 +1378,7 @@ def attention_talking_decode(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torc
     check(library().mf_attention_talking_decode(q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(),
                                                 seq_q_start.data_ptr(), seq_q_len.data_ptr(), seq_ctx_len.data_ptr(),
                                                 n, n_heads, n_kv, dim, vdim, block_table.data_ptr(),
-                                                block_table.shape[1], page_size, scale, softcap, _ptr(talk), window,
+                                                block_table.shape[1], page_size, k_pool.numel() // dim, scale, softcap, _ptr(talk), window,
                                                 chunk, splits, part_o.data_ptr(), part_ml.data_ptr(), kernel_status(q.device).data_ptr(),
                                                 _stream()),
           "attention_talking_decode", launches=2)

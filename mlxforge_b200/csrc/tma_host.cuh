@@ -43,8 +43,28 @@ struct Hash {
   }
 };
 
+// Rows of `row_bytes` from `ptr` to the end of the memory that is mapped there without a gap, for callers that do not say how long
+// their pool is: a map must not reach beyond it.  0 where the driver does not know the address.
+inline long long mapped_rows(const void* ptr, long long row_bytes) {
+  typedef CUresult (*Range)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static Range fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<Range>(p);
+  });
+  CUdeviceptr at = (CUdeviceptr)ptr, base = 0;
+  size_t size = 0;
+  for (int i = 0; fn && i < 256 && fn(&base, &size, at) == CUDA_SUCCESS && base + size > at; i++) at = base + size;
+  return (long long)(at - (CUdeviceptr)ptr) / row_bytes;
+}
+
 // A [rows, cols] row-major bfloat16 matrix as a tiled map with boxes of box_rows x box_cols
-// (box_cols * 2 bytes = 128: one swizzle span) and 128-byte swizzle.  0 on success.
+// (box_cols * 2 bytes = 128: one swizzle span) and 128-byte swizzle.  0 on success.  `rows` is what is allocated, of a cache pool
+// too: copies by a map of 2^28 rows over a pool of 60 KB were an illegal memory access where the pool stood within 80 KB of the end of what
+// was mapped, although every box lay inside the pool; with the pool's own rows the same copies run.
 inline int bf16_map(const void* ptr, long long rows, long long cols, int box_rows, int box_cols, CUtensorMap* out) {
   static std::unordered_map<Key, CUtensorMap, Hash> cache;
   static std::mutex mu;
@@ -102,12 +122,12 @@ inline int bf16_map_chunked(const void* ptr, long long rows, long long cols, int
 }
 
 // A pool of pages, [pages][page_rows][cols] bfloat16, with boxes of 16 rows and 64 columns of n_pages pages that follow one another,
-// laid out as one tile of 16 n_pages rows with 128-byte swizzle.  The number of pages only bounds the unit's own range check.
-inline int bf16_map_pages(const void* ptr, int page_rows, long long cols, int n_pages, CUtensorMap* out) {
+// laid out as one tile of 16 n_pages rows with 128-byte swizzle.
+inline int bf16_map_pages(const void* ptr, long long pages, int page_rows, long long cols, int n_pages, CUtensorMap* out) {
   static std::unordered_map<Key, CUtensorMap, Hash> cache;
   static std::mutex mu;
   std::lock_guard<std::mutex> lock(mu);
-  const Key key{ptr, page_rows, cols, 16, n_pages};
+  const Key key{ptr, pages, cols, page_rows, n_pages};
   auto it = cache.find(key);
   if (it != cache.end()) {
     *out = it->second;
@@ -115,7 +135,7 @@ inline int bf16_map_pages(const void* ptr, int page_rows, long long cols, int n_
   }
   EncodeTiled enc = encoder();
   if (!enc) return MF_ERR_BAD_ARG;
-  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)page_rows, 1ull << 24};
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)page_rows, (cuuint64_t)pages};
   const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)cols * 2 * page_rows};
   const cuuint32_t box[3] = {64, 16, (cuuint32_t)n_pages};
   const cuuint32_t estr[3] = {1, 1, 1};
