@@ -432,7 +432,8 @@ attn_prefill_tc_ahead_kernel(const __grid_constant__ CUtensorMap map_q, const __
                       : row_scores_max<false>(s_addr, sc, key0, my_pos, my_lo);
       mx *= scale_log2;
       const float m_cand = fmaxf(m_row, mx);
-      const bool moved = __any_sync(0xffffffffu, m_cand - m_row > MAX_SLACK_LOG2);      // also from -inf
+      // also from -inf; rows past the portion (another's queries, keys that were not fetched) have no say in it
+      const bool moved = __any_sync(0xffffffffu, r < rows && m_cand - m_row > MAX_SLACK_LOG2);
       const float m_new = moved ? m_cand : m_row;
       const float m_off = (m_new == -INFINITY) ? 0.f : m_new;
       const float alpha = !moved ? 1.f : ((m_row == -INFINITY) ? 0.f : ex2(m_row - m_off));
@@ -782,7 +783,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       if (lane == 0) mbar_arrive(s_free);
       mx *= scale_log2;                                      // scale > 0: the max commutes with it
       const float m_cand = fmaxf(m_row, mx);
-      const bool moved = __any_sync(0xffffffffu, m_cand - m_row > (EX ? EXACT_MAX_LOG2 : MAX_SLACK_LOG2));      // also from -inf
+      // also from -inf; rows past the portion (another's queries, keys that were not fetched) have no say in it
+      const bool moved = __any_sync(0xffffffffu, r < rows && m_cand - m_row > (EX ? EXACT_MAX_LOG2 : MAX_SLACK_LOG2));
       const float m_new = moved ? m_cand : m_row;
       const float m_off = (m_new == -INFINITY) ? 0.f : m_new;
       const float alpha = !moved ? 1.f : ((m_row == -INFINITY) ? 0.f : ex2(m_row - m_off));

@@ -190,6 +190,34 @@ def test_prefill_attention_does_not_depend_on_where_the_pages_are(form, lens, he
         at += n
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("n,held", [(137, 0), (130, 200), (161, 1000)])
+def test_prefill_attention_does_not_depend_on_the_next_portion(hd, n, held):
+    """A portion whose last tile of queries is partly another portion's, whose scores are hundreds of times as large: the bits that it
+    has alone."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(n + hd)
+    nh, nkv, bf, other = 4, 2, torch.bfloat16, 140
+    per, per2 = -(-(n + held) // 16), -(-other // 16)
+    q = torch.randn((n + other, nh * hd), generator=g, device="cuda")
+    q[n:] *= 300.0
+    q = q.to(bf)
+    kp, vp = (torch.randn((per + per2, nkv, 16, hd), generator=g, device="cuda").to(bf) for _ in range(2))
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    table = torch.full((2, max(per, per2)), -1, dtype=torch.int32, device="cuda")
+    table[0, :per], table[1, :per2] = torch.arange(per), per + torch.arange(per2)
+    outs = []
+    for seqs in (1, 2):
+        T = n if seqs == 1 else n + other
+        out = torch.empty((T, nh * hd), device="cuda", dtype=bf)
+        ops.attention_prefill(q[:T].contiguous(), kp, vp, out, i32([0, n][:seqs]), i32([n, other][:seqs]), i32([n + held, other][:seqs]), 0,
+                              max(n, other if seqs == 2 else 0), table[:seqs].contiguous(), 16, nh, nkv, hd, hd ** -0.5, 0)
+        outs.append(out[:n].clone())
+    ops.check_kernel_status()
+    assert torch.equal(outs[0], outs[1])
+
+
 # ----------------------------------------------------------------------------- rotations, biases and norms of prompts
 
 def _store_case(kind, T, g, pages):
