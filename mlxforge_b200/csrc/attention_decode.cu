@@ -56,10 +56,10 @@ constexpr int NSTAGE = 2;               // tiles in flight per warp: NSTAGE - 1 
 
 template <int HD_MAX>
 __global__ void __launch_bounds__(Tile<HD_MAX>::W * 32)
-attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_pool,
-                   const __nv_bfloat16* __restrict__ v_pool, float* __restrict__ part_o,
-                   float* __restrict__ part_ml, const int* __restrict__ positions,
-                   const int* __restrict__ seq_of_token, PagedView pv, int n_heads, float scale_log2,
+attn_decode_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k_pool,
+                   const __nv_bfloat16* v_pool, float* __restrict__ part_o,
+                   float* __restrict__ part_ml, const int* positions,
+                   const int* seq_of_token, PagedView pv, int n_heads, float scale_log2,
                    int window, int max_splits, int split_keys, AttnOptions opt) {
   constexpr int KPW = Tile<HD_MAX>::KPW;
   constexpr int WARPS = Tile<HD_MAX>::W;
@@ -299,8 +299,8 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 // One block per (token, head): merge the partials of the splits that saw keys.  `hd` is the width of
 // an output row.  With kept first keys the splits that hold some of them count beside the window's;
 // a sink joins the denominator here; a gate multiplies the result.
-__global__ void attn_decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                         __nv_bfloat16* __restrict__ out, const int* __restrict__ positions,
+__global__ void attn_decode_merge_kernel(const float* part_o, const float* part_ml,
+                                         __nv_bfloat16* __restrict__ out, const int* positions,
                                          int n_heads, int hd, int window, int max_splits, int split_keys,
                                          AttnOptions opt) {
   pdl_wait();

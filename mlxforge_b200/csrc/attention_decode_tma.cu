@@ -130,8 +130,8 @@ __device__ __forceinline__ Item make_item(int item, int rows, int groups, int hg
 template <int HD, int STAGES>
 __global__ void __launch_bounds__((CW + 1) * 32)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                       const __nv_bfloat16* __restrict__ q, float* __restrict__ part_o, float* __restrict__ part_ml,
-                       __nv_bfloat16* __restrict__ out, const int* __restrict__ positions, const int* __restrict__ seq_of_token, PagedView pv,
+                       const __nv_bfloat16* q, float* part_o, float* part_ml,
+                       __nv_bfloat16* __restrict__ out, const int* positions, const int* seq_of_token, PagedView pv,
                        int n_heads, int n_tokens, float scale_log2, int window, int max_splits, int comb_rows,
                        int split_keys, int* __restrict__ status) {
   constexpr int HALVES = HD / 64;                   // spans of 64 columns per row of the cache

@@ -191,8 +191,8 @@ MF_API int mf_attention_talking(const void* q, const void* k_pool, const void* v
 // go to page block_table[seq, p / page_size], slot p % page_size, p = positions[t].
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256)
-biased_kv_store_kernel(const TI* __restrict__ qkv, const float* __restrict__ bias, const int* __restrict__ positions,
-                       const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int bt_stride,
+biased_kv_store_kernel(const TI* qkv, const float* __restrict__ bias, const int* positions,
+                       const int* seq_of_token, const int* block_table, int bt_stride,
                        int page_size, TO* __restrict__ q_out, TO* __restrict__ k_pool, TO* __restrict__ v_pool,
                        int n_heads, int n_kv, int dim, int vdim, int write_kv) {
   pdl_launch();
@@ -223,8 +223,8 @@ biased_kv_store_kernel(const TI* __restrict__ qkv, const float* __restrict__ bia
 // per token, 8.5 here.
 template <int TOK>
 __global__ void __launch_bounds__(256)
-biased_kv_store_vec_kernel(const float* __restrict__ qkv, const float* __restrict__ bias, const int* __restrict__ positions,
-                           const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int bt_stride,
+biased_kv_store_vec_kernel(const float* qkv, const float* __restrict__ bias, const int* positions,
+                           const int* seq_of_token, const int* block_table, int bt_stride,
                            int page_size, __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_pool,
                            __nv_bfloat16* __restrict__ v_pool, int T, int n_heads, int n_kv, int dim, int vdim, int write_kv) {
   __shared__ long long row_s[TOK];         // of the cache, before heads

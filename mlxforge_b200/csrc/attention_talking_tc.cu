@@ -742,7 +742,7 @@ talking_decode_kernel(const TtArgs a) {
 // eighth split each.
 template <int VDIM>
 __global__ void __launch_bounds__(256)
-talking_decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, __nv_bfloat16* __restrict__ out,
+talking_decode_merge_kernel(const float* part_o, const float* part_ml, __nv_bfloat16* __restrict__ out,
                             int splits, int H) {
   constexpr int N = VDIM / 32;
   __shared__ float m_s[8], l_s[8], o_s[8][VDIM];

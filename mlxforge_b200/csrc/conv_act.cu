@@ -16,9 +16,9 @@ __device__ __forceinline__ float ca_act(float v, int silu) { return silu ? v / (
 // any number of taps and channels: a thread per (token, channel)
 template <typename T2>
 __global__ void __launch_bounds__(256)
-conv_act_kernel(const float* __restrict__ x, int ld, int C, const float* __restrict__ w, const float* __restrict__ bias,
-                int taps, int silu, float* __restrict__ state, long long state_stride, long long tail_off,
-                const int* __restrict__ seq_of_token, const int* __restrict__ seq_q_start, const int* __restrict__ slots,
+conv_act_kernel(const float* x, int ld, int C, const float* __restrict__ w, const float* __restrict__ bias,
+                int taps, int silu, float* state, long long state_stride, long long tail_off,
+                const int* seq_of_token, const int* seq_q_start, const int* slots,
                 float* __restrict__ out, T2* __restrict__ out2, int move_tail) {
   pdl_launch();
   pdl_wait();
@@ -46,10 +46,10 @@ conv_act_kernel(const float* __restrict__ x, int ld, int C, const float* __restr
 // time) and handed on in registers
 template <typename T2, int TAPS>
 __global__ void __launch_bounds__(128)
-conv_act_vec_kernel(const float* __restrict__ x, int ld, int C, const float* __restrict__ w,
-                    const float* __restrict__ bias, int silu, float* __restrict__ state, long long state_stride,
-                    long long tail_off, const int* __restrict__ seq_of_token, const int* __restrict__ seq_q_start,
-                    const int* __restrict__ slots, float* __restrict__ out, T2* __restrict__ out2, int T, int run,
+conv_act_vec_kernel(const float* x, int ld, int C, const float* __restrict__ w,
+                    const float* __restrict__ bias, int silu, float* state, long long state_stride,
+                    long long tail_off, const int* seq_of_token, const int* seq_q_start,
+                    const int* slots, float* __restrict__ out, T2* __restrict__ out2, int T, int run,
                     int move_tail) {
   pdl_launch();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
@@ -116,9 +116,9 @@ conv_act_vec_kernel(const float* __restrict__ x, int ld, int C, const float* __r
 
 // After the step the slot keeps the last taps-1 inputs of every channel.
 __global__ void __launch_bounds__(256)
-conv_act_tail_kernel(const float* __restrict__ x, int ld, int C, int taps, float* __restrict__ state,
-                     long long state_stride, long long tail_off, const int* __restrict__ seq_q_start,
-                     const int* __restrict__ seq_q_len, const int* __restrict__ slots) {
+conv_act_tail_kernel(const float* x, int ld, int C, int taps, float* state,
+                     long long state_stride, long long tail_off, const int* seq_q_start,
+                     const int* seq_q_len, const int* slots) {
   pdl_launch();
   pdl_wait();
   const int seq = blockIdx.x;

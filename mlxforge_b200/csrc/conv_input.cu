@@ -17,10 +17,10 @@
 // ------------------------------------------------------------------ h = x + conv(x)
 template <typename TO>
 __global__ void __launch_bounds__(256)
-conv_input_kernel(const float* __restrict__ x, int H, const float* __restrict__ w, int taps,
-                  float* __restrict__ state, long long state_stride, long long tail_off,
-                  const int* __restrict__ seq_of_token, const int* __restrict__ seq_q_start,
-                  const int* __restrict__ slots, TO* __restrict__ out, int move_tail) {
+conv_input_kernel(const float* x, int H, const float* __restrict__ w, int taps,
+                  float* state, long long state_stride, long long tail_off,
+                  const int* seq_of_token, const int* seq_q_start,
+                  const int* slots, TO* __restrict__ out, int move_tail) {
   pdl_launch();
   pdl_wait();
   const int t = blockIdx.x;
@@ -44,10 +44,10 @@ conv_input_kernel(const float* __restrict__ x, int H, const float* __restrict__ 
 // four channels a thread: 16-byte loads of x and of the tail (H a multiple of 4)
 template <typename TO, int TAPS>
 __global__ void __launch_bounds__(256)
-conv_input_vec_kernel(const float* __restrict__ x, int H, const float* __restrict__ w,
-                      float* __restrict__ state, long long state_stride, long long tail_off,
-                      const int* __restrict__ seq_of_token, const int* __restrict__ seq_q_start,
-                      const int* __restrict__ slots, TO* __restrict__ out, int move_tail) {
+conv_input_vec_kernel(const float* x, int H, const float* __restrict__ w,
+                      float* state, long long state_stride, long long tail_off,
+                      const int* seq_of_token, const int* seq_q_start,
+                      const int* slots, TO* __restrict__ out, int move_tail) {
   pdl_launch();
   pdl_wait();
   const int t = blockIdx.x;
@@ -84,9 +84,9 @@ conv_input_vec_kernel(const float* __restrict__ x, int H, const float* __restric
 
 // After the step the slot keeps the last taps-1 rows of x that the convolution has read.
 __global__ void __launch_bounds__(256)
-conv_input_tail_kernel(const float* __restrict__ x, int H, int taps, float* __restrict__ state, long long state_stride,
-                       long long tail_off, const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len,
-                       const int* __restrict__ slots) {
+conv_input_tail_kernel(const float* x, int H, int taps, float* state, long long state_stride,
+                       long long tail_off, const int* seq_q_start, const int* seq_q_len,
+                       const int* slots) {
   pdl_launch();
   pdl_wait();
   const int seq = blockIdx.x;
@@ -142,7 +142,7 @@ MF_API int mf_conv_input(const float* x, int T, int H, const float* w, int taps,
 // One block per token.  y1, y2 [T, H] in the dtype T1 (32-bit or bfloat16); y2 may be null.
 template <typename T1>
 __global__ void __launch_bounds__(256)
-postnorm_add_kernel(float* __restrict__ x, int H, const T1* __restrict__ y1, float s1, const T1* __restrict__ y2,
+postnorm_add_kernel(float* x, int H, const T1* y1, float s1, const T1* y2,
                     float s2, const float* __restrict__ g, float eps) {
   extern __shared__ float pn_y[];      // [H]
   __shared__ float red[32];
@@ -164,7 +164,7 @@ postnorm_add_kernel(float* __restrict__ x, int H, const T1* __restrict__ y1, flo
 // four channels a thread with 16-byte accesses to the stream (H a multiple of 4): the sums stay in registers
 template <typename T1, int PER>
 __global__ void __launch_bounds__(256)
-postnorm_add_vec_kernel(float* __restrict__ x, int H, const T1* __restrict__ y1, float s1, const T1* __restrict__ y2,
+postnorm_add_vec_kernel(float* x, int H, const T1* y1, float s1, const T1* y2,
                         float s2, const float* __restrict__ g, float eps) {
   __shared__ float red[32];
   pdl_launch();

@@ -345,8 +345,8 @@ decay_recurrence_kernel(DecayRec p) {
 
 // seg_state[0] <- the slot's state; seg_state[i] <- decay[i-1] seg_state[i-1] + (local end state of segment i-1)
 __global__ void __launch_bounds__(256)
-decay_combine_kernel(float* __restrict__ seg_state, const float* __restrict__ seg_decay, const float* __restrict__ state,
-                     long long state_stride, const int* __restrict__ seq_q_len, const int* __restrict__ slots,
+decay_combine_kernel(float* seg_state, const float* seg_decay, const float* state,
+                     long long state_stride, const int* seq_q_len, const int* slots,
                      int seg_len, int n_seg, int n_heads, int dim, int vdim, int per_channel) {
   pdl_launch();
   pdl_wait();
@@ -506,7 +506,7 @@ MF_API int mf_decay_recurrence(const float* q, int q_ld, const float* k, int k_l
 // gate_first: the gate multiplies before the norm, else after it.  WARPS warps share a (token, group).
 template <typename TO, int WARPS, int VEC>
 __global__ void __launch_bounds__(256)
-gated_norm_kernel(const float* __restrict__ x, int n_parts, long long part_stride, const float* __restrict__ gate,
+gated_norm_kernel(const float* x, int n_parts, long long part_stride, const float* gate,
                   long long gate_ld, const float* __restrict__ w, int w_len, float eps, TO* __restrict__ out, int width,
                   int groups, int gate_first, long long total) {
   extern __shared__ __align__(16) float gn_sm[];       // [items of the block][group size]

@@ -217,7 +217,7 @@ static int delta_prepare_heads(const DeltaPrepare& a, void* low, int n_low, cuda
 // the rest sigmoid(x), in place.  N neighbouring columns a thread, a row of blocks per token.
 template <int N>
 __global__ void __launch_bounds__(256)
-delta_gates_kernel(float* __restrict__ ag, const float* __restrict__ a_log, const float* __restrict__ dt_bias, int n_decay,
+delta_gates_kernel(float* ag, const float* __restrict__ a_log, const float* __restrict__ dt_bias, int n_decay,
                    int dim, int width) {
   pdl_launch();
   pdl_wait();
@@ -467,9 +467,9 @@ delta_recurrence_staged_kernel(const float* __restrict__ qkv, const float* __res
 // of a row at a time and set up a ring for one token: 8 sequences of 16 heads of 128 x 128 (17 MB there and back) 12.8 -> 4.3 us.
 template <int DIM>
 __global__ void __launch_bounds__(128)
-delta_step_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ ag, int ag_ld,
-                  float* __restrict__ state, long long state_stride, const int* __restrict__ seq_q_start,
-                  const int* __restrict__ slots, float* __restrict__ o_out, int n_heads, int n_kv, int vdim) {
+delta_step_kernel(const float* qkv, const float* beta, const float* ag, int ag_ld,
+                  float* state, long long state_stride, const int* seq_q_start,
+                  const int* slots, float* __restrict__ o_out, int n_heads, int n_kv, int vdim) {
   constexpr int ROWS = DIM / 4;
   __shared__ float q_s[DIM], k_s[DIM], g_s[DIM], part[4][32];
   pdl_launch();
@@ -519,7 +519,7 @@ delta_step_kernel(const float* __restrict__ qkv, const float* __restrict__ beta,
 // w_per_head: the weight is [n_heads * vdim] (a row of its own for every head) instead of [vdim].
 template <typename TO>
 __global__ void __launch_bounds__(256)
-delta_output_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_ld,
+delta_output_kernel(const float* o, const float* gate, int gate_ld,
                     const float* __restrict__ w, float eps, TO* __restrict__ out, int n_heads, int vdim, int total,
                     int w_per_head) {
   pdl_launch();
@@ -542,7 +542,7 @@ delta_output_kernel(const float* __restrict__ o, const float* __restrict__ gate,
 // 128: 11.0 -> 8.2 us.
 template <typename TO, int N>
 __global__ void __launch_bounds__(256)
-delta_output_vec_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_ld, const float* __restrict__ w,
+delta_output_vec_kernel(const float* o, const float* gate, int gate_ld, const float* __restrict__ w,
                         float eps, TO* __restrict__ out, int n_heads, int total, int w_per_head) {
   constexpr int V = 32 * N;
   pdl_launch();

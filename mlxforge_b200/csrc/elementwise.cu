@@ -26,7 +26,7 @@ __global__ void embed_kernel(const T* __restrict__ table, const int* __restrict_
 }
 
 // bfloat16 rows in 16-byte pieces (H a multiple of 8)
-__global__ void embed_bf16_vec_kernel(const __nv_bfloat16* __restrict__ table, const int* __restrict__ tokens,
+__global__ void embed_bf16_vec_kernel(const __nv_bfloat16* __restrict__ table, const int* tokens,
                                       float* __restrict__ out, int H, float scale) {
   pdl_wait();
   pdl_launch();
@@ -95,9 +95,9 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ resid, const TD* __restri
 // most 8 * 256 * NV, every value held in registers between the two passes.
 template <int NV>
 __global__ void __launch_bounds__(256)
-add_rmsnorm_bf16_vec_kernel(float* __restrict__ resid, const __nv_bfloat16* __restrict__ delta,
+add_rmsnorm_bf16_vec_kernel(float* resid, const __nv_bfloat16* delta,
                             const float* __restrict__ w, float eps, __nv_bfloat16* __restrict__ out,
-                            const int* __restrict__ rows, int H) {
+                            const int* rows, int H) {
   __shared__ float red[32];
   pdl_launch();              // the product after this one fetches its weights meanwhile
   pdl_wait();
@@ -240,8 +240,8 @@ __global__ void rope_kv_write_kernel(const T* __restrict__ qkv, int n_heads, int
 // (25 MB) took 8.8 us, with four 7.5 (a block's angles side by side, more pieces on their way at once).
 template <int TOK>
 __global__ void __launch_bounds__(256)
-rope_kv_write_bf16_vec_kernel(const __nv_bfloat16* __restrict__ qkv, int T, int n_heads, int n_kv, int hd, int rot,
-                              const int* __restrict__ positions, const int* __restrict__ seq_of_token,
+rope_kv_write_bf16_vec_kernel(const __nv_bfloat16* qkv, int T, int n_heads, int n_kv, int hd, int rot,
+                              const int* positions, const int* seq_of_token,
                               PagedView pv, const float* __restrict__ freqs, __nv_bfloat16* __restrict__ q_out,
                               __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool,
                               int write_kv) {
@@ -404,7 +404,7 @@ MF_API int mf_gated_act(const void* gu, void* out, int dtype, int T, int I, int 
 // ------------------------------------------------------------------ activation without a gate
 // out[i] = act(in[i]) in 32-bit, rounded once (in place where out == in)
 template <typename T>
-__global__ void unary_act_kernel(const T* __restrict__ in, T* __restrict__ out, long long n, int act) {
+__global__ void unary_act_kernel(const T* in, T* out, long long n, int act) {
   pdl_launch();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -412,7 +412,7 @@ __global__ void unary_act_kernel(const T* __restrict__ in, T* __restrict__ out, 
 }
 
 // bfloat16, 8 elements a thread
-__global__ void unary_act_bf16_vec_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, long long n8, int act) {
+__global__ void unary_act_bf16_vec_kernel(const uint4* in, uint4* out, long long n8, int act) {
   pdl_launch();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -456,10 +456,10 @@ MF_API int mf_swiglu(const void* gu, void* out, int dtype, int T, int I, int gro
 // out1 = rmsnorm(resid) * w1 and, if asked for, out2 = rmsnorm(resid) * w2: one pass over the row,
 // one sum of squares.  With `rows` only those rows are produced and resid is left as it is.
 template <typename TD, typename TO>
-__global__ void add_rmsnorm_pair_kernel(float* __restrict__ resid, const TD* __restrict__ d1,
-                                        const TD* __restrict__ d2, const float* __restrict__ w1,
+__global__ void add_rmsnorm_pair_kernel(float* resid, const TD* d1,
+                                        const TD* d2, const float* __restrict__ w1,
                                         const float* __restrict__ w2, float eps, TO* __restrict__ out1,
-                                        TO* __restrict__ out2, const int* __restrict__ rows, int H) {
+                                        TO* __restrict__ out2, const int* rows, int H) {
   __shared__ float red[32];
   pdl_launch();
   pdl_wait();
@@ -499,10 +499,10 @@ __global__ void add_rmsnorm_pair_kernel(float* __restrict__ resid, const TD* __r
 // 8 * 256 * NV, every value held in registers between the two passes.
 template <int NV>
 __global__ void __launch_bounds__(256)
-add_rmsnorm_pair_bf16_vec_kernel(float* __restrict__ resid, const __nv_bfloat16* __restrict__ d1,
-                                 const __nv_bfloat16* __restrict__ d2, const float* __restrict__ w1,
+add_rmsnorm_pair_bf16_vec_kernel(float* resid, const __nv_bfloat16* d1,
+                                 const __nv_bfloat16* d2, const float* __restrict__ w1,
                                  const float* __restrict__ w2, float eps, __nv_bfloat16* __restrict__ out1,
-                                 __nv_bfloat16* __restrict__ out2, const int* __restrict__ rows, int H) {
+                                 __nv_bfloat16* __restrict__ out2, const int* rows, int H) {
   __shared__ float red[32];
   pdl_launch();              // the products after this one fetch their weights meanwhile
   pdl_wait();
@@ -605,14 +605,14 @@ MF_API int mf_add_rmsnorm_pair(float* resid, const void* d1, const void* d2, int
 
 // ------------------------------------------------------------------ soft cap
 // x[i] = cap tanh(x[i] / cap), in place, 32-bit (logits that a library product wrote)
-__global__ void __launch_bounds__(256) soft_cap_kernel(float* __restrict__ x, long long n, float cap) {
+__global__ void __launch_bounds__(256) soft_cap_kernel(float* x, long long n, float cap) {
   pdl_launch();
   pdl_wait();
   const long long step = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) x[i] = soft_cap(x[i], cap);
 }
 
-__global__ void __launch_bounds__(256) soft_cap_vec_kernel(float4* __restrict__ x, long long n4, float cap) {
+__global__ void __launch_bounds__(256) soft_cap_vec_kernel(float4* x, long long n4, float cap) {
   pdl_launch();
   pdl_wait();
   const long long step = (long long)gridDim.x * blockDim.x;

@@ -145,7 +145,7 @@ __device__ __forceinline__ void store16(OutT* __restrict__ out, const float (&v)
 template <int MODE, int CHUNKS, typename OutT>
 __global__ void __launch_bounds__(192, 1)
 mid_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                OutT* __restrict__ out, float* __restrict__ scratch, int M, int N, int K, int NT, int stages,
+                OutT* __restrict__ out, float* scratch, int M, int N, int K, int NT, int stages,
                 int* __restrict__ status) {
   extern __shared__ unsigned char raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);

@@ -93,7 +93,7 @@ __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;\
 
 template <int NB, int ROWS, typename OutT>
 __global__ void __launch_bounds__((CW + 1) * 32)
-stream_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ W, OutT* __restrict__ out,
+stream_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W, OutT* __restrict__ out,
               int M, int N, int K, int mode, EpiConst ec, int* __restrict__ status) {
   constexpr int STAGES = Ring<ROWS>::STAGES;
   constexpr int STAGE_BYTES = ROWS * ROW_BYTES;
@@ -165,7 +165,7 @@ stream_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
 #pragma unroll
         for (int nb = 0; nb < NB; nb++) {
           const int m = nb * 8 + g;
-          xv[c][nb] = (k < K && m < M) ? __ldg(reinterpret_cast<const uint4*>(x + (long long)m * K + k)) : zero;
+          xv[c][nb] = (k < K && m < M) ? *reinterpret_cast<const uint4*>(x + (long long)m * K + k) : zero;
         }
       }
       mbar_wait(bars_u + 8 * s, round & 1, status, 2);
@@ -247,7 +247,7 @@ __device__ __forceinline__ void tma_load_3d(unsigned dst, const CUtensorMap* map
 
 template <int NB, int ROWS, int T_STAGES, typename OutT>
 __global__ void __launch_bounds__((CW + 1) * 32)
-stream_tmap_kernel(const __nv_bfloat16* __restrict__ x, const __grid_constant__ CUtensorMap map,
+stream_tmap_kernel(const __nv_bfloat16* x, const __grid_constant__ CUtensorMap map,
                    OutT* __restrict__ out, int M, int N, int K, int mode, EpiConst ec, int* __restrict__ status) {
   constexpr int SUB = 16 / ROWS;                 // chunks of 64 per warp and stage (1 or 2)
   constexpr int KSTAGE = 512 * SUB;              // elements of K per stage
@@ -312,7 +312,7 @@ stream_tmap_kernel(const __nv_bfloat16* __restrict__ x, const __grid_constant__ 
 #pragma unroll
           for (int nb = 0; nb < NB; nb++) {
             const int m = nb * 8 + g;
-            xv[h][c][nb] = (k < K && m < M) ? __ldg(reinterpret_cast<const uint4*>(x + (long long)m * K + k)) : zero;
+            xv[h][c][nb] = (k < K && m < M) ? *reinterpret_cast<const uint4*>(x + (long long)m * K + k) : zero;
           }
         }
       mbar_wait(bars_u + 8 * s, round & 1, status, 2);

@@ -33,7 +33,7 @@ struct HsPair {
 
 template <typename T>
 __global__ void __launch_bounds__(HS_THREADS)
-embed_positions_kernel(const T* __restrict__ table, const int* __restrict__ tokens, const int* __restrict__ positions,
+embed_positions_kernel(const T* __restrict__ table, const int* tokens, const int* positions,
                        const double* __restrict__ freqs, float* __restrict__ out, int H, int copies, int precise) {
   pdl_wait();
   pdl_launch();
@@ -78,11 +78,11 @@ MF_API int mf_embed_positions(const void* table, int table_dtype, const int* tok
 // ones (the single residual sum); `win` null means ones (the plain sum of the streams).
 template <typename TD, typename TO>
 __global__ void __launch_bounds__(HS_THREADS)
-hyper_update_norm_kernel(float* __restrict__ streams, const TD* __restrict__ delta,
+hyper_update_norm_kernel(float* streams, const TD* delta,
                          const float* __restrict__ delta_bias, const float* __restrict__ mix,
                          const float* __restrict__ wout, const float* __restrict__ win,
                          const float* __restrict__ w, float eps, int groups, TO* __restrict__ out,
-                         const int* __restrict__ rows, int H, int S, HsPair pair) {
+                         const int* rows, int H, int S, HsPair pair) {
   extern __shared__ float u[];      // [H]
   __shared__ float red[32];
   __shared__ float cm[HS_MAX_STREAMS * HS_MAX_STREAMS], co[HS_MAX_STREAMS], ci[HS_MAX_STREAMS];
@@ -175,11 +175,11 @@ __device__ __forceinline__ void hs_load4(const __nv_bfloat16* p, float* y) {
 // accesses to the streams, and each thread keeps its values of u in registers between the passes.
 template <typename TD, typename TO, int NV, bool PAIR>
 __global__ void __launch_bounds__(HS_THREADS)
-hyper_update_norm_vec_kernel(float* __restrict__ streams, const TD* __restrict__ delta,
+hyper_update_norm_vec_kernel(float* streams, const TD* delta,
                              const float* __restrict__ delta_bias, const float* __restrict__ mix,
                              const float* __restrict__ wout, const float* __restrict__ win,
                              const float* __restrict__ w, float eps, int groups, TO* __restrict__ out,
-                             const int* __restrict__ rows, int H, int S, HsPair pair) {
+                             const int* rows, int H, int S, HsPair pair) {
   __shared__ float red[32];
   __shared__ float cm[HS_MAX_STREAMS * HS_MAX_STREAMS], co[HS_MAX_STREAMS], ci[HS_MAX_STREAMS];
   __shared__ float gsum[HS_MAX_GROUPS];

@@ -43,9 +43,9 @@ __device__ __forceinline__ void rotate_part(const T* __restrict__ src, T* __rest
 }
 
 template <typename T>
-__global__ void latent_prepare_kernel(const T* __restrict__ proj, int ld, int q_rank, int kv_off, int rank, int rot,
+__global__ void latent_prepare_kernel(const T* proj, int ld, int q_rank, int kv_off, int rank, int rot,
                                       const float* __restrict__ wq, const float* __restrict__ wkv, float eps,
-                                      const int* __restrict__ positions, const int* __restrict__ seq_of_token,
+                                      const int* positions, const int* seq_of_token,
                                       PagedView pv, const float* __restrict__ inv_f, const double* __restrict__ inv_d,
                                       T* __restrict__ cq_out, T* __restrict__ k_pool, int write_kv, int layout,
                                       int rot_dims, float mag) {
@@ -85,9 +85,9 @@ __global__ void latent_prepare_kernel(const T* __restrict__ proj, int ld, int q_
 // of 768 and 192: 8.8 us with a block per token and four barriers, 5.8 here.
 template <int Q>
 __global__ void __launch_bounds__(256)
-latent_prepare_vec_kernel(const __nv_bfloat16* __restrict__ proj, int T, int ld, int q_rank, int kv_off, int rank, int rot,
+latent_prepare_vec_kernel(const __nv_bfloat16* proj, int T, int ld, int q_rank, int kv_off, int rank, int rot,
                           const float* __restrict__ wq, const float* __restrict__ wkv, float eps,
-                          const int* __restrict__ positions, const int* __restrict__ seq_of_token, PagedView pv,
+                          const int* positions, const int* seq_of_token, PagedView pv,
                           const float* __restrict__ inv_f, const double* __restrict__ inv_d,
                           __nv_bfloat16* __restrict__ cq_out, __nv_bfloat16* __restrict__ k_pool, int write_kv, int layout,
                           int rot_dims, float mag) {
@@ -179,8 +179,8 @@ MF_API int mf_latent_prepare(const void* proj, int dtype, int T, int ld, int q_r
 
 // q [T, heads, dim + rot] in rows q_ld apart -> q_full[t, h, rank : rank + rot] = rotation of q[t, h, dim : dim + rot]
 template <typename T>
-__global__ void latent_query_kernel(const T* __restrict__ q, long long q_ld, int n_heads, int dim, int rot, int rank,
-                                    const int* __restrict__ positions, const float* __restrict__ inv_f,
+__global__ void latent_query_kernel(const T* q, long long q_ld, int n_heads, int dim, int rot, int rank,
+                                    const int* positions, const float* __restrict__ inv_f,
                                     const double* __restrict__ inv_d, T* __restrict__ q_full, int layout, int rot_dims,
                                     float mag) {
   pdl_launch();
@@ -218,8 +218,8 @@ constexpr int HL_WARPS = 8;
 
 template <typename T>
 __global__ void __launch_bounds__(HL_WARPS * 32)
-head_linear_kernel(const T* __restrict__ x, long long x_ld, int x_hs, const T* __restrict__ w, T* __restrict__ out,
-                   long long out_ld, int out_hs, int N, int K, const T* __restrict__ gate, long long gate_ld, int gate_hs,
+head_linear_kernel(const T* x, long long x_ld, int x_hs, const T* __restrict__ w, T* __restrict__ out,
+                   long long out_ld, int out_hs, int N, int K, const T* gate, long long gate_ld, int gate_hs,
                    int gate_ns) {
   extern __shared__ float xs[];          // [K]
   pdl_launch();
@@ -271,9 +271,9 @@ __device__ __forceinline__ void hm_mma(float (&c)[4], const unsigned (&a)[4], un
 }  // namespace
 
 __global__ void __launch_bounds__(HM_WARPS * 32)
-head_linear_mma_kernel(const __nv_bfloat16* __restrict__ x, long long x_ld, int x_hs, const __nv_bfloat16* __restrict__ w,
+head_linear_mma_kernel(const __nv_bfloat16* x, long long x_ld, int x_hs, const __nv_bfloat16* __restrict__ w,
                        __nv_bfloat16* __restrict__ out, long long out_ld, int out_hs, int T, int N, int K,
-                       const __nv_bfloat16* __restrict__ gate, long long gate_ld, int gate_hs, int gate_ns, int vec) {
+                       const __nv_bfloat16* gate, long long gate_ld, int gate_hs, int gate_ns, int vec) {
   extern __shared__ __align__(16) unsigned char hm_smem[];
   const int ld = K + 8, chunks = K >> 3;
   __nv_bfloat16* x_s = reinterpret_cast<__nv_bfloat16*>(hm_smem);      // [HM_BM][ld]

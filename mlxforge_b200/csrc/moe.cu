@@ -38,7 +38,7 @@ constexpr unsigned KEY_NONE = 0x007fffffu;      // of minus infinity; NaN and wh
 // and two reductions of whole numbers in hardware (the largest key, then the lowest index that has it): 6.1 us for 6 of 64 experts
 // in 8 groups at any number of tokens up to 400, 8.0 with a chain of shuffles for each.
 __global__ void __launch_bounds__(128)
-moe_route_kernel(const float* __restrict__ z, int ldz, int E, int n_groups, int keep, int top, float route_scale,
+moe_route_kernel(const float* z, int ldz, int E, int n_groups, int keep, int top, float route_scale,
                  int mode, const float* __restrict__ logit_bias, const float* __restrict__ bias, int* __restrict__ ids, float* __restrict__ weights, int T) {
   extern __shared__ float sm[];
   const unsigned all = 0xffffffffu;
@@ -150,8 +150,8 @@ MF_API int mf_moe_route(const float* z, int ldz, int T, int E, int n_groups, int
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-moe_rows_kernel(const T* __restrict__ x, const T* __restrict__ w_gu, const T* __restrict__ w_down,
-                const int* __restrict__ ids, float* __restrict__ y, int H, int ff, int top, float limit, float alpha,
+moe_rows_kernel(const T* x, const T* __restrict__ w_gu, const T* __restrict__ w_down,
+                const int* ids, float* __restrict__ y, int H, int ff, int top, float limit, float alpha,
                 float up_off, int n_real, int act_kind) {
   extern __shared__ float sm[];
   float* xs = sm;            // [H]
@@ -214,8 +214,8 @@ __device__ __forceinline__ float moe_dot8(const uint4 w, const float* xv) {
 }
 
 __global__ void __launch_bounds__(256)
-moe_rows_bf16_vec_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w_gu,
-                         const __nv_bfloat16* __restrict__ w_down, const int* __restrict__ ids, float* __restrict__ y,
+moe_rows_bf16_vec_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ w_gu,
+                         const __nv_bfloat16* __restrict__ w_down, const int* ids, float* __restrict__ y,
                          int H, int ff, int top, float limit, float alpha, float up_off, int n_real, int act_kind) {
   extern __shared__ __align__(16) float sm[];
   float* xs = sm;            // [H]
@@ -325,7 +325,7 @@ struct MoeExtras {
 
 template <typename TO, typename TY>
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const TY* __restrict__ y, const float* __restrict__ weights, const int* __restrict__ slot_of,
+moe_combine_kernel(const TY* y, const float* weights, const int* slot_of,
                    TO* __restrict__ out, int H, int top, int slices, MoeExtras ex) {
   pdl_launch();
   pdl_wait();
@@ -353,8 +353,8 @@ moe_combine_kernel(const TY* __restrict__ y, const float* __restrict__ weights, 
 // bfloat16 rows in 16-byte pieces (H a multiple of 8, one partial sum per pair): 8 columns a thread;
 // identity experts and the shared branch as in the kernel above
 __global__ void __launch_bounds__(256)
-moe_combine_bf16_vec_kernel(const __nv_bfloat16* __restrict__ y, const float* __restrict__ weights,
-                            const int* __restrict__ slot_of, __nv_bfloat16* __restrict__ out, int H, int top,
+moe_combine_bf16_vec_kernel(const __nv_bfloat16* y, const float* weights,
+                            const int* slot_of, __nv_bfloat16* __restrict__ out, int H, int top,
                             MoeExtras ex) {
   pdl_launch();
   pdl_wait();
@@ -406,7 +406,7 @@ moe_combine_bf16_vec_kernel(const __nv_bfloat16* __restrict__ y, const float* __
 // tokens of 2,048 columns 15.2 -> 7.3 us).
 template <typename TO, int KS>
 __global__ void __launch_bounds__(256)
-moe_combine_f32_vec_kernel(const float* __restrict__ y, const float* __restrict__ weights, const int* __restrict__ slot_of,
+moe_combine_f32_vec_kernel(const float* y, const float* weights, const int* slot_of,
                            TO* __restrict__ out, int H, int top, int slices, MoeExtras ex) {
   __shared__ float4 parts[KS][32];
   pdl_launch();

@@ -44,7 +44,7 @@ __device__ __forceinline__ void mg_mma(float (&c)[4], const uint32_t (&a)[4], ui
 // shared memory where they fit, since a warp's 32 scattered words are 32 stores to memory (10.4 -> 7.2); with the gather below and both launched
 // behind their predecessor's end, the mixture of 2,048 tokens 207 -> 202.5 us.
 __global__ void __launch_bounds__(1024)
-moe_sort_kernel(const int* __restrict__ ids, int n_pairs, int E, int top, int tile_rows, int* __restrict__ slot_of,
+moe_sort_kernel(const int* ids, int n_pairs, int E, int top, int tile_rows, int* slot_of,
                 int* __restrict__ row_token, int* __restrict__ meta, int* __restrict__ tiles, int staged) {
   extern __shared__ int tokens[];            // staged: [n_pairs], a row's token
   __shared__ int count[MG_MAX_EXPERTS], first[MG_MAX_EXPERTS];
@@ -362,7 +362,7 @@ MF_API int mf_moe_grouped_down(const void* act, const void* w_down, const int* m
 // writes alone are 7.7 at the copy rate).
 constexpr int GATHER_ROWS = 4;
 __global__ void __launch_bounds__(256)
-moe_gather_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ row_token, uint4* __restrict__ xg, int n_rows, int h8) {
+moe_gather_rows_kernel(const uint4* x, const int* row_token, uint4* __restrict__ xg, int n_rows, int h8) {
   pdl_launch();
   pdl_wait();
   const int row0 = blockIdx.x * GATHER_ROWS;

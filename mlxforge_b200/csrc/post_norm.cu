@@ -27,8 +27,8 @@ __device__ __forceinline__ float slot_sum(float v, float* slot) {
 // ------------------------------------------------------------------ any sizes and dtypes
 template <typename TY, typename TO>
 __global__ void __launch_bounds__(256)
-post_norm_kernel(float* __restrict__ resid, const TY* __restrict__ y, const float* __restrict__ w1, int kind1, float eps1,
-                 const float* __restrict__ w2, int kind2, float eps2, TO* __restrict__ out, const int* __restrict__ rows,
+post_norm_kernel(float* resid, const TY* y, const float* __restrict__ w1, int kind1, float eps1,
+                 const float* __restrict__ w2, int kind2, float eps2, TO* __restrict__ out, const int* rows,
                  int H) {
   extern __shared__ float pn_row[];      // [H]
   __shared__ float red[32];
@@ -84,9 +84,9 @@ post_norm_kernel(float* __restrict__ resid, const TY* __restrict__ y, const floa
 // 8 * NT * NV: every value stays in registers between the sums.
 template <int NT, int NV>
 __global__ void __launch_bounds__(NT)
-post_norm_bf16_vec_kernel(float* __restrict__ resid, const __nv_bfloat16* __restrict__ y, const float* __restrict__ w1,
+post_norm_bf16_vec_kernel(float* resid, const __nv_bfloat16* y, const float* __restrict__ w1,
                           int kind1, float eps1, const float* __restrict__ w2, int kind2, float eps2,
-                          __nv_bfloat16* __restrict__ out, const int* __restrict__ rows, int H) {
+                          __nv_bfloat16* __restrict__ out, const int* rows, int H) {
   __shared__ float red[4][8];
   pdl_launch();              // the product after this one fetches its weights meanwhile
   pdl_wait();

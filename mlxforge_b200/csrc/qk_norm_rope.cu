@@ -36,8 +36,8 @@ struct QkPrepare {
 
 template <typename TP, typename T>
 __global__ void __launch_bounds__(256)
-qk_norm_rope_kernel(const TP* __restrict__ proj, int ld, QkPrepare p, const int* __restrict__ positions,
-                    const int* __restrict__ seq_of_token, PagedView pk, PagedView pvv, T* __restrict__ q_out,
+qk_norm_rope_kernel(const TP* proj, int ld, QkPrepare p, const int* positions,
+                    const int* seq_of_token, PagedView pk, PagedView pvv, T* __restrict__ q_out,
                     T* __restrict__ k_pool, T* __restrict__ v_pool, int write_kv) {
   extern __shared__ float qs[];     // row [nq + nk + nv], then cos/sin of the keys' and of the values' rotation
   __shared__ float red[32];
@@ -176,7 +176,7 @@ MF_API int mf_qk_norm_rope(const void* proj, int ld, int dtype, int out_dtype, i
 // sign * position * inv[m].
 template <typename T>
 __global__ void __launch_bounds__(256)
-rotate_rows_kernel(T* __restrict__ x, int n_heads, int d, int rot, const int* __restrict__ positions,
+rotate_rows_kernel(T* x, int n_heads, int d, int rot, const int* positions,
                    const float* __restrict__ inv_f, const double* __restrict__ inv_d, float sign) {
   extern __shared__ float rr_cs[];
   pdl_launch();

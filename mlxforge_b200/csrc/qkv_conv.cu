@@ -47,9 +47,9 @@ constexpr int MAXT = 4;      // taps a lane holds; fewer are padded with zeros i
 // R: tokens of a run; NC: pieces of 64 channels a head has at most
 template <typename TO, int R, int NC>
 __global__ void __launch_bounds__(WARPS * 32, 2)
-qkv_conv_kernel(const float* __restrict__ proj, int ld, QkvConv p, const float* __restrict__ w, int taps,
-                float* __restrict__ state, long long state_stride, long long tail_off, const int* __restrict__ positions,
-                const int* __restrict__ seq_of_token, const int* __restrict__ seq_q_start, const int* __restrict__ slots,
+qkv_conv_kernel(const float* proj, int ld, QkvConv p, const float* __restrict__ w, int taps,
+                float* state, long long state_stride, long long tail_off, const int* positions,
+                const int* seq_of_token, const int* seq_q_start, const int* slots,
                 PagedView pk, PagedView pvv, TO* __restrict__ q_out, TO* __restrict__ k_pool, TO* __restrict__ v_pool,
                 int T, int move_tail) {
   extern __shared__ float qc_sm[];         // cos and sin of the run's positions, then R rows of a head per warp

@@ -29,8 +29,8 @@ constexpr int RT_CHUNK = 8;                 // tokens staged at a time
 // act 1: SiLU of every query and key channel before anything else.  v_out (optional): the row's `nv`
 // channels from column `v_off` on, through the same activation, in 32-bit [T, nv].
 template <typename T>
-__global__ void retention_prepare_kernel(const T* __restrict__ proj, int ld, int n_heads, int dim, int rot,
-                                         float k_scale, const int* __restrict__ positions,
+__global__ void retention_prepare_kernel(const T* proj, int ld, int n_heads, int dim, int rot,
+                                         float k_scale, const int* positions,
                                          const float* __restrict__ inv_f, const double* __restrict__ inv_d,
                                          float* __restrict__ qk, int act, float* __restrict__ v_out, int v_off, int nv) {
   extern __shared__ float cs[];            // [half] cos, [half] sin
@@ -73,8 +73,8 @@ __global__ void retention_prepare_kernel(const T* __restrict__ proj, int ld, int
 // 7.7 here.
 template <int TOK>
 __global__ void __launch_bounds__(256)
-retention_prepare_vec_kernel(const __nv_bfloat16* __restrict__ proj, int ld, int n_heads, int dim, int rot, int T, float k_scale,
-                             const int* __restrict__ positions, const float* __restrict__ inv_f,
+retention_prepare_vec_kernel(const __nv_bfloat16* proj, int ld, int n_heads, int dim, int rot, int T, float k_scale,
+                             const int* positions, const float* __restrict__ inv_f,
                              const double* __restrict__ inv_d, float* __restrict__ qk, int act) {
   extern __shared__ float cs[];            // [TOK][half] cos, then sin
   pdl_launch();
@@ -159,10 +159,10 @@ MF_API int mf_retention_prepare(const void* proj, int dtype, int T, int ld, int 
 // state [slots, heads, dim, vdim] with `state_stride` floats per slot.  o_out [T, heads * vdim] 32-bit.
 template <typename T, int RPL>
 __global__ void __launch_bounds__(RT_THREADS)
-retention_recurrence_kernel(const float* __restrict__ qk, const T* __restrict__ v, long long v_ld,
-                            const float* __restrict__ decay, float* __restrict__ state, long long state_stride,
-                            const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len,
-                            const int* __restrict__ slots, float* __restrict__ o_out, int n_heads, int dim, int vdim) {
+retention_recurrence_kernel(const float* qk, const T* v, long long v_ld,
+                            const float* __restrict__ decay, float* state, long long state_stride,
+                            const int* seq_q_start, const int* seq_q_len,
+                            const int* slots, float* __restrict__ o_out, int n_heads, int dim, int vdim) {
   extern __shared__ float sm[];            // [RT_CHUNK][2 dim] q then k of a token, [RT_CHUNK][RT_COLS] v
   float* v_s = sm + RT_CHUNK * 2 * dim;
   pdl_launch();
@@ -238,10 +238,10 @@ __device__ __forceinline__ void rs_cp_async_16(void* smem, const void* gmem) {
 
 template <typename T, int RS_ROWS>
 __global__ void __launch_bounds__(RT_THREADS)
-retention_recurrence_staged_kernel(const float* __restrict__ qk, const T* __restrict__ v, long long v_ld,
-                                   const float* __restrict__ decay, float* __restrict__ state, long long state_stride,
-                                   const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len,
-                                   const int* __restrict__ slots, float* __restrict__ o_part, long long part_stride,
+retention_recurrence_staged_kernel(const float* qk, const T* v, long long v_ld,
+                                   const float* __restrict__ decay, float* state, long long state_stride,
+                                   const int* seq_q_start, const int* seq_q_len,
+                                   const int* slots, float* __restrict__ o_part, long long part_stride,
                                    int n_heads, int dim, int vdim) {
   constexpr int RS_RPL = RS_ROWS / RT_LANES;
   constexpr int V_PIECES = RT_COLS * sizeof(T) / 16;               // 16-byte pieces of a token's values
@@ -333,9 +333,9 @@ retention_recurrence_staged_kernel(const float* __restrict__ qk, const T* __rest
 // and back).
 template <typename T, int DIM>
 __global__ void __launch_bounds__(128)
-retention_step_kernel(const float* __restrict__ qk, const T* __restrict__ v, long long v_ld, const float* __restrict__ decay,
-                      float* __restrict__ state, long long state_stride, const int* __restrict__ seq_q_start,
-                      const int* __restrict__ slots, float* __restrict__ o_out, int n_heads, int vdim) {
+retention_step_kernel(const float* qk, const T* v, long long v_ld, const float* __restrict__ decay,
+                      float* state, long long state_stride, const int* seq_q_start,
+                      const int* slots, float* __restrict__ o_out, int n_heads, int vdim) {
   constexpr int ROWS = DIM / 4;
   __shared__ float q_s[DIM], k_s[DIM], part[4][32];
   pdl_launch();
@@ -462,8 +462,8 @@ MF_API int mf_retention_recurrence(const float* qk, const void* v, int v_dtype, 
 // whole: one root mean square over all heads of the token instead of one per head.  weight (optional):
 // [n_heads * vdim], multiplied in.  gate_act 1: the gate passes a sigmoid instead of SiLU.
 template <typename T>
-__global__ void retention_output_kernel(const float* __restrict__ o, int n_parts, long long part_stride,
-                                        const T* __restrict__ gate, long long gate_ld, float eps, T* __restrict__ out,
+__global__ void retention_output_kernel(const float* o, int n_parts, long long part_stride,
+                                        const T* gate, long long gate_ld, float eps, T* __restrict__ out,
                                         int n_heads, int vdim, const float* __restrict__ weight, int whole,
                                         int gate_act) {
   extern __shared__ float ro_ss[];      // [n_heads] sums of squares
@@ -509,7 +509,7 @@ __global__ void retention_output_kernel(const float* __restrict__ o, int n_parts
 // lane, read once and kept.  1,777 tokens of 8 heads of 128: 8.9 us with a block per token that reads twice, 5.6 here.
 template <typename T, int N>
 __global__ void __launch_bounds__(256)
-retention_output_vec_kernel(const float* __restrict__ o, int n_parts, long long part_stride, const T* __restrict__ gate,
+retention_output_vec_kernel(const float* o, int n_parts, long long part_stride, const T* gate,
                             long long gate_ld, float eps, T* __restrict__ out, int n_heads, int total,
                             const float* __restrict__ weight, int gate_act) {
   constexpr int V = 32 * N;

@@ -10,8 +10,8 @@
 #include "rotary.cuh"
 
 template <typename T>
-__global__ void rope_store_kernel(const T* __restrict__ qk, int ld, int n_heads, int n_kv, int hd, int rot, int layout,
-                                  const int* __restrict__ positions, const int* __restrict__ seq_of_token,
+__global__ void rope_store_kernel(const T* qk, int ld, int n_heads, int n_kv, int hd, int rot, int layout,
+                                  const int* positions, const int* seq_of_token,
                                   PagedView pv, const float* __restrict__ inv_f, const double* __restrict__ inv_d,
                                   T* __restrict__ q_out, T* __restrict__ k_pool, T* __restrict__ v_pool,
                                   int write_kv, int v_from_k) {
@@ -61,8 +61,8 @@ __global__ void rope_store_kernel(const T* __restrict__ qk, int ld, int n_heads,
 // bfloat16 with adjacent pairs (2i, 2i + 1), an even head size: a pair is one 32-bit word, and so
 // are two channels that pass; every thread moves whole words.
 __global__ void __launch_bounds__(256)
-rope_store_pairs_bf16_kernel(const __nv_bfloat16* __restrict__ qk, int ld, int n_heads, int n_kv, int hd, int rot,
-                             const int* __restrict__ positions, const int* __restrict__ seq_of_token, PagedView pv,
+rope_store_pairs_bf16_kernel(const __nv_bfloat16* qk, int ld, int n_heads, int n_kv, int hd, int rot,
+                             const int* positions, const int* seq_of_token, PagedView pv,
                              const float* __restrict__ inv_f, __nv_bfloat16* __restrict__ q_out,
                              __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool, int write_kv) {
   extern __shared__ float cs[];            // [half] cos, [half] sin
@@ -99,8 +99,8 @@ rope_store_pairs_bf16_kernel(const __nv_bfloat16* __restrict__ qk, int ld, int n
 // (25 MB): 12.3 us with a word a thread and a block per token, 7.5 here.
 template <int TOK>
 __global__ void __launch_bounds__(256)
-rope_store_pairs_vec_kernel(const __nv_bfloat16* __restrict__ qk, int ld, int n_heads, int n_kv, int hd, int rot, int T,
-                            const int* __restrict__ positions, const int* __restrict__ seq_of_token, PagedView pv,
+rope_store_pairs_vec_kernel(const __nv_bfloat16* qk, int ld, int n_heads, int n_kv, int hd, int rot, int T,
+                            const int* positions, const int* seq_of_token, PagedView pv,
                             const float* __restrict__ inv_f, __nv_bfloat16* __restrict__ q_out,
                             __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool, int write_kv) {
   extern __shared__ float cs[];            // [TOK][half] cos, then sin

@@ -235,9 +235,9 @@ selective_scan_kernel(ScanArgs p, TO* __restrict__ out) {
 
 // seg_state[0] <- the slot's state; seg_state[i] <- exp(A sum dt of segment i-1) seg_state[i-1] + (local end state)
 __global__ void __launch_bounds__(256)
-scan_combine_kernel(float* __restrict__ seg_state, const float* __restrict__ seg_dt, const float* __restrict__ A,
-                    const float* __restrict__ state, long long state_stride, const int* __restrict__ seq_q_len,
-                    const int* __restrict__ slots, int seg_len, int n_seg, int channels, int n_state) {
+scan_combine_kernel(float* seg_state, const float* seg_dt, const float* __restrict__ A,
+                    const float* state, long long state_stride, const int* seq_q_len,
+                    const int* slots, int seg_len, int n_seg, int channels, int n_state) {
   pdl_launch();
   pdl_wait();
   const int seq = blockIdx.y;
@@ -384,7 +384,7 @@ __device__ __forceinline__ float lr_act(float x, int f, float inv_tau) {
 
 template <typename TW>
 __global__ void __launch_bounds__(256)
-low_rank_split_kernel(const float* __restrict__ low, int ld, const TW* __restrict__ wt, const float* __restrict__ bias,
+low_rank_split_kernel(const float* low, int ld, const TW* __restrict__ wt, const float* __restrict__ bias,
                       int f, float inv_tau, float* __restrict__ out, int T, int R, int n) {
   __shared__ float part[8][LR_TOK][32];
   __shared__ float ls[LR_TOK][LR_PIECE];
@@ -429,7 +429,7 @@ low_rank_split_kernel(const float* __restrict__ low, int ld, const TW* __restric
 
 template <typename TW>
 __global__ void __launch_bounds__(256)
-low_rank_kernel(const float* __restrict__ low, int ld, const TW* __restrict__ wt, const float* __restrict__ bias, int f,
+low_rank_kernel(const float* low, int ld, const TW* __restrict__ wt, const float* __restrict__ bias, int f,
                 float inv_tau, float* __restrict__ out, int T, int R, int n) {
   extern __shared__ __align__(16) float lr_sm[];       // weights [R][32], then low [8 * LR_TOK][R4]
   const int R4 = (R + 3) & ~3;
