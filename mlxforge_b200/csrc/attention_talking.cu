@@ -218,10 +218,10 @@ biased_kv_store_kernel(const TI* qkv, const float* __restrict__ bias, const int*
   }
 }
 
-// 32-bit projections into bfloat16 in pieces of four channels (16 bytes in, 8 out; head sizes multiples of 4), TOK tokens a block, four
-// pieces a thread on their way at once.  2,048 tokens of 16 + 2 x 4 heads of 128 (38 MB): 14.0 us with a channel a thread and a block
-// per token, 8.5 here.
-template <int TOK>
+// 32-bit projections into bfloat16 in pieces of four channels (16 bytes in, 8 out; head sizes multiples of 4), TOK tokens a block
+// (mf_store_tokens), U pieces a thread on their way at once.  2,048 tokens of 16 + 2 x 4 heads of 128 (38 MB, in L2): 10.2 us with a channel a
+// thread, 5.0 here.
+template <int TOK, int U>
 __global__ void __launch_bounds__(256)
 biased_kv_store_vec_kernel(const float* qkv, const float* __restrict__ bias, const int* positions,
                            const int* seq_of_token, const int* block_table, int bt_stride,
@@ -230,7 +230,7 @@ biased_kv_store_vec_kernel(const float* qkv, const float* __restrict__ bias, con
   __shared__ long long row_s[TOK];         // of the cache, before heads
   __shared__ int slot_s[TOK];
   pdl_launch();
-  const int t0 = blockIdx.x * TOK, nt = min(TOK, T - t0);
+  const int t0 = blockIdx.x * TOK, nt = TOK == 1 ? 1 : min(TOK, T - t0);
   if (threadIdx.x < nt) {
     const int pos = positions[t0 + threadIdx.x], seq = seq_of_token[t0 + threadIdx.x], blk = pos / page_size;
     slot_s[threadIdx.x] = pos - blk * page_size;
@@ -239,21 +239,31 @@ biased_kv_store_vec_kernel(const float* qkv, const float* __restrict__ bias, con
   __syncthreads();
   pdl_wait();
   const int nq = n_heads * dim, nk = n_kv * dim, width = nq + nk + n_kv * vdim, pieces = (write_kv ? width : nq) / 4;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < nt * pieces; i += 256) {
-    const int t = i / pieces, c = (i - t * pieces) * 4;
-    const float4 x = *reinterpret_cast<const float4*>(qkv + (long long)(t0 + t) * width + c);
-    const float4 b = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-    __nv_bfloat16* to;
-    if (c < nq) {
-      to = q_out + (long long)(t0 + t) * nq + c;
-    } else {
-      const bool key = c < nq + nk;
-      const int d = key ? dim : vdim, e = c - nq - (key ? 0 : nk), h = e / d;
-      to = (key ? k_pool : v_pool) + ((row_s[t] + h) * page_size + slot_s[t]) * d + e - h * d;
+  // U pieces a thread are on their way before the first is stored
+  for (int i0 = threadIdx.x; i0 < nt * pieces; i0 += U * 256) {
+    float4 in[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * 256, t = TOK == 1 ? 0 : i / pieces;
+      if (i < nt * pieces) in[u] = *reinterpret_cast<const float4*>(qkv + (long long)(t0 + t) * width + (i - t * pieces) * 4);
     }
-    __nv_bfloat162 o[2] = {__floats2bfloat162_rn(x.x + b.x, x.y + b.y), __floats2bfloat162_rn(x.z + b.z, x.w + b.w)};
-    *reinterpret_cast<uint2*>(to) = *reinterpret_cast<uint2*>(o);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * 256, t = TOK == 1 ? 0 : i / pieces, c = (i - t * pieces) * 4;
+      if (i >= nt * pieces) continue;
+      const float4 x = in[u];
+      const float4 b = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      __nv_bfloat16* to;
+      if (c < nq) {
+        to = q_out + (long long)(t0 + t) * nq + c;
+      } else {
+        const bool key = c < nq + nk;
+        const int d = key ? dim : vdim, e = c - nq - (key ? 0 : nk), h = e / d;
+        to = (key ? k_pool : v_pool) + ((row_s[t] + h) * page_size + slot_s[t]) * d + e - h * d;
+      }
+      __nv_bfloat162 o[2] = {__floats2bfloat162_rn(x.x + b.x, x.y + b.y), __floats2bfloat162_rn(x.z + b.z, x.w + b.w)};
+      *reinterpret_cast<uint2*>(to) = *reinterpret_cast<uint2*>(o);
+    }
   }
 }
 
@@ -265,13 +275,12 @@ MF_API int mf_biased_kv_store(const void* qkv, int in_dtype, const float* bias, 
   mf_count(MF_K_KV_STORE);
   if (in_dtype == MF_F32 && out_dtype == MF_BF16 && dim % 4 == 0 && vdim % 4 == 0 &&
       !(((uintptr_t)qkv | (uintptr_t)bias) & 15) && !(((uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 7)) {
-    // four tokens a block where that leaves two blocks for every SM
-#define KV_GO(TOK)                                                                                                          \
-  return (int)launch_dep(biased_kv_store_vec_kernel<TOK>, dim3((T + TOK - 1) / TOK), dim3(256), 0, stream, (const float*)qkv, \
+#define KV_GO(TOK, U)                                                                                                          \
+  return (int)launch_dep(biased_kv_store_vec_kernel<TOK, U>, dim3((T + TOK - 1) / TOK), dim3(256), 0, stream, (const float*)qkv, \
                          bias, positions, seq_of_token, block_table, bt_stride, page_size, (__nv_bfloat16*)q_out,            \
                          (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, T, n_heads, n_kv, dim, vdim, write_kv)
-    if (T >= 8 * mf_sm_count()) KV_GO(4);
-    KV_GO(1);
+    if (mf_store_tokens(T, (n_heads * dim + (write_kv ? n_kv * (dim + vdim) : 0)) / 4) == 4) KV_GO(4, 4);
+    KV_GO(1, 1);
 #undef KV_GO
   }
 #define KS_LAUNCH(TI, TO)                                                                                          \

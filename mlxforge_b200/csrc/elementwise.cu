@@ -236,9 +236,8 @@ __global__ void rope_kv_write_kernel(const T* __restrict__ qkv, int n_heads, int
 
 // The serving case: bfloat16, rot_dim a multiple of 16, head_dim a multiple of 8.  The
 // cosines and sines of the token's position are computed once (float32, accurate sincosf)
-// and shared by all heads; rows move in 16-byte pieces.  TOK tokens a block: with one, 2,048 tokens of 32 + 2 x 8 heads of 64
-// (25 MB) took 8.8 us, with four 7.5 (a block's angles side by side, more pieces on their way at once).
-template <int TOK>
+// and shared by all heads; rows move in 16-byte pieces, TOK tokens a block (mf_store_tokens), U pieces a thread at a time.
+template <int TOK, int U>
 __global__ void __launch_bounds__(256)
 rope_kv_write_bf16_vec_kernel(const __nv_bfloat16* qkv, int T, int n_heads, int n_kv, int hd, int rot,
                               const int* positions, const int* seq_of_token,
@@ -250,7 +249,7 @@ rope_kv_write_bf16_vec_kernel(const __nv_bfloat16* qkv, int T, int n_heads, int 
   pdl_launch();              // the attention after this one fetches older keys and values meanwhile
   // positions and the frequency table are in place before the step's first kernel starts and do not
   // change during it: the angles are computed before the wait, off the path between two kernels
-  const int t0 = blockIdx.x * TOK, nt = min(TOK, T - t0), half = rot >> 1;
+  const int t0 = blockIdx.x * TOK, nt = TOK == 1 ? 1 : min(TOK, T - t0), half = rot >> 1;
   if (threadIdx.x < nt) {
     pos_s[threadIdx.x] = positions[t0 + threadIdx.x];
     seq_s[threadIdx.x] = seq_of_token[t0 + threadIdx.x];
@@ -269,42 +268,55 @@ rope_kv_write_bf16_vec_kernel(const __nv_bfloat16* qkv, int T, int n_heads, int 
   const int pc = (hd - rot) >> 3;          // pass-through pieces per head
   const int per_head = rc + pc, vc = hd >> 3;
   const int rotated = (n_heads + (write_kv ? n_kv : 0)) * per_head, per_token = rotated + (write_kv ? n_kv * vc : 0);
-#pragma unroll 2
-  for (int i = threadIdx.x; i < nt * per_token; i += 256) {
-    const int t = i / per_token, idx = i - t * per_token;
-    const __nv_bfloat16* row = qkv + (long long)(t0 + t) * width;
-    if (idx >= rotated) {                  // a piece of a value
-      const int h = (idx - rotated) / vc, c = idx - rotated - h * vc;
-      *reinterpret_cast<uint4*>(v_pool + paged_offset(pv, seq_s[t], pos_s[t], h) + c * 8) =
-          *reinterpret_cast<const uint4*>(row + (long long)(n_heads + n_kv + h) * hd + c * 8);
-      continue;
-    }
-    const int h = idx / per_head, c = idx - h * per_head;
-    const __nv_bfloat16* src = row + (long long)h * hd;
-    __nv_bfloat16* dst = h < n_heads ? q_out + ((long long)(t0 + t) * n_heads + h) * hd
-                                     : k_pool + paged_offset(pv, seq_s[t], pos_s[t], h - n_heads);
-    if (c < rc) {
-      const int j = c * 8;
-      const uint4 a = *reinterpret_cast<const uint4*>(src + j), b = *reinterpret_cast<const uint4*>(src + j + half);
-      const __nv_bfloat162* ap = reinterpret_cast<const __nv_bfloat162*>(&a);
-      const __nv_bfloat162* bp = reinterpret_cast<const __nv_bfloat162*>(&b);
-      const float *co = cs + t * half + j, *si = cs + (TOK + t) * half + j;
-      uint4 oa, ob;
-      __nv_bfloat162* oap = reinterpret_cast<__nv_bfloat162*>(&oa);
-      __nv_bfloat162* obp = reinterpret_cast<__nv_bfloat162*>(&ob);
+  // U pieces a thread are on their way before the first is stored
+  for (int i0 = threadIdx.x; i0 < nt * per_token; i0 += U * 256) {
+    uint4 in[U], in2[U];
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const float2 x1 = __bfloat1622float2(ap[e]), x2 = __bfloat1622float2(bp[e]);
-        const float c0 = co[2 * e], c1 = co[2 * e + 1];
-        const float s0 = si[2 * e], s1 = si[2 * e + 1];
-        oap[e] = __floats2bfloat162_rn(x1.x * c0 - x2.x * s0, x1.y * c1 - x2.y * s1);
-        obp[e] = __floats2bfloat162_rn(x1.x * s0 + x2.x * c0, x1.y * s1 + x2.y * c1);
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * 256, t = TOK == 1 ? 0 : i / per_token, idx = i - t * per_token;
+      if (i >= nt * per_token) continue;
+      const __nv_bfloat16* row = qkv + (long long)(t0 + t) * width;
+      if (idx >= rotated) {                  // a piece of a value
+        in[u] = *reinterpret_cast<const uint4*>(row + (long long)(n_heads + n_kv) * hd + (idx - rotated) * 8);
+        continue;
       }
-      *reinterpret_cast<uint4*>(dst + j) = oa;
-      *reinterpret_cast<uint4*>(dst + j + half) = ob;
-    } else {
-      const int ch = rot + (c - rc) * 8;
-      *reinterpret_cast<uint4*>(dst + ch) = *reinterpret_cast<const uint4*>(src + ch);
+      const int h = idx / per_head, c = idx - h * per_head, at = c < rc ? c * 8 : rot + (c - rc) * 8;
+      in[u] = *reinterpret_cast<const uint4*>(row + (long long)h * hd + at);
+      if (c < rc) in2[u] = *reinterpret_cast<const uint4*>(row + (long long)h * hd + at + half);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * 256, t = TOK == 1 ? 0 : i / per_token, idx = i - t * per_token;
+      if (i >= nt * per_token) continue;
+      if (idx >= rotated) {
+        const int h = (idx - rotated) / vc, c = idx - rotated - h * vc;
+        *reinterpret_cast<uint4*>(v_pool + paged_offset(pv, seq_s[t], pos_s[t], h) + c * 8) = in[u];
+        continue;
+      }
+      const int h = idx / per_head, c = idx - h * per_head;
+      __nv_bfloat16* dst = h < n_heads ? q_out + ((long long)(t0 + t) * n_heads + h) * hd
+                                       : k_pool + paged_offset(pv, seq_s[t], pos_s[t], h - n_heads);
+      if (c < rc) {
+        const int j = c * 8;
+        const __nv_bfloat162* ap = reinterpret_cast<const __nv_bfloat162*>(&in[u]);
+        const __nv_bfloat162* bp = reinterpret_cast<const __nv_bfloat162*>(&in2[u]);
+        const float *co = cs + t * half + j, *si = cs + (TOK + t) * half + j;
+        uint4 oa, ob;
+        __nv_bfloat162* oap = reinterpret_cast<__nv_bfloat162*>(&oa);
+        __nv_bfloat162* obp = reinterpret_cast<__nv_bfloat162*>(&ob);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const float2 x1 = __bfloat1622float2(ap[e]), x2 = __bfloat1622float2(bp[e]);
+          const float c0 = co[2 * e], c1 = co[2 * e + 1];
+          const float s0 = si[2 * e], s1 = si[2 * e + 1];
+          oap[e] = __floats2bfloat162_rn(x1.x * c0 - x2.x * s0, x1.y * c1 - x2.y * s1);
+          obp[e] = __floats2bfloat162_rn(x1.x * s0 + x2.x * c0, x1.y * s1 + x2.y * c1);
+        }
+        *reinterpret_cast<uint4*>(dst + j) = oa;
+        *reinterpret_cast<uint4*>(dst + j + half) = ob;
+      } else {
+        *reinterpret_cast<uint4*>(dst + rot + (c - rc) * 8) = in[u];
+      }
     }
   }
 }
@@ -318,12 +330,12 @@ MF_API int mf_rope_kv_write(const void* qkv, int dtype, int T, int n_heads, int 
   PagedView pv{block_table, bt_stride, page_size, n_kv, hd};
   if (dtype == MF_BF16 && !precise && rot_dim % 16 == 0 && hd % 8 == 0 &&
       (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0) {
-    // four tokens a block where that leaves two blocks for every SM
-    if (T >= 8 * mf_sm_count())
-      return (int)launch_dep(rope_kv_write_bf16_vec_kernel<4>, dim3((T + 3) / 4), dim3(256), (size_t)4 * rot_dim * sizeof(float),
+    const int pieces = (n_heads + (write_kv ? n_kv : 0)) * ((hd - rot_dim / 2) / 8) + (write_kv ? n_kv * hd / 8 : 0);
+    if (mf_store_tokens(T, pieces) == 4 && 4 * rot_dim * sizeof(float) <= 48 * 1024)
+      return (int)launch_dep(rope_kv_write_bf16_vec_kernel<4, 2>, dim3((T + 3) / 4), dim3(256), (size_t)4 * rot_dim * sizeof(float),
                              stream, (const __nv_bfloat16*)qkv, T, n_heads, n_kv, hd, rot_dim, positions, seq_of_token, pv, freqs,
                              (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, write_kv);
-    return (int)launch_dep(rope_kv_write_bf16_vec_kernel<1>, dim3(T), dim3(256), (size_t)rot_dim * sizeof(float), stream,
+    return (int)launch_dep(rope_kv_write_bf16_vec_kernel<1, 1>, dim3(T), dim3(256), (size_t)rot_dim * sizeof(float), stream,
                            (const __nv_bfloat16*)qkv, T, n_heads, n_kv, hd, rot_dim, positions, seq_of_token, pv, freqs,
                            (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, write_kv);
   }

@@ -68,17 +68,16 @@ __global__ void retention_prepare_kernel(const T* proj, int ld, int n_heads, int
 }
 
 // The same for bfloat16 rows in pieces of eight channels and of the eight they pair with (head size and half of the rotated channels
-// multiples of 8, 16-byte aligned rows, no v_out), TOK tokens a block: the angles of all of them side by side, then the pieces with two
-// loads each on their way at once.  1,777 tokens of 8 heads of 128 (22 MB): 12.2 us with a channel a thread and a block per token,
-// 7.7 here.
-template <int TOK>
+// multiples of 8, 16-byte aligned rows, no v_out), TOK tokens a block (mf_store_tokens), the angles of all of them side by side.
+// 1,777 tokens of 8 heads of 128 (22 MB, in L2): 10.3 us with a channel a thread, 5.5 here.
+template <int TOK, int U>
 __global__ void __launch_bounds__(256)
 retention_prepare_vec_kernel(const __nv_bfloat16* proj, int ld, int n_heads, int dim, int rot, int T, float k_scale,
                              const int* positions, const float* __restrict__ inv_f,
                              const double* __restrict__ inv_d, float* __restrict__ qk, int act) {
   extern __shared__ float cs[];            // [TOK][half] cos, then sin
   pdl_launch();
-  const int t0 = blockIdx.x * TOK, nt = min(TOK, T - t0), half = rot >> 1;
+  const int t0 = blockIdx.x * TOK, nt = TOK == 1 ? 1 : min(TOK, T - t0), half = rot >> 1;
   for (int i = threadIdx.x; i < nt * half; i += 256) {
     const int t = i / half, j = i - t * half;
     rotary_cs(positions[t0 + t], j, inv_f, inv_d, cs[i], cs[TOK * half + i]);
@@ -99,32 +98,47 @@ retention_prepare_vec_kernel(const __nv_bfloat16* proj, int ld, int n_heads, int
     *reinterpret_cast<float4*>(p + 4) = make_float4(x[4], x[5], x[6], x[7]);
   };
   const int turned = half >> 3, per_head = turned + ((dim - rot) >> 3), per_token = 2 * n_heads * per_head;
-#pragma unroll 2
-  for (int i = threadIdx.x; i < nt * per_token; i += 256) {
-    const int t = i / per_token, rest = i - t * per_token, h = rest / per_head, c = rest - h * per_head;
-    const __nv_bfloat16* src = proj + (long long)(t0 + t) * ld + (long long)h * dim;
-    float* dst = qk + ((long long)(t0 + t) * 2 * n_heads + h) * dim;      // heads 0..n-1: queries, n..2n-1: keys
-    const float f = h >= n_heads ? k_scale : 1.0f;
-    float u[8], v[8];
-    if (c < turned) {
-      const int j = c * 8;
-      unpack(*reinterpret_cast<const uint4*>(src + j), u);
-      unpack(*reinterpret_cast<const uint4*>(src + j + half), v);
+  // U pieces a thread are on their way before the first is stored
+  for (int i0 = threadIdx.x; i0 < nt * per_token; i0 += U * 256) {
+    uint4 in[U], in2[U];
 #pragma unroll
-      for (int e = 0; e < 8; e++) {
-        const float co = cs[t * half + j + e], si = cs[(TOK + t) * half + j + e];
-        const float a = (u[e] * co - v[e] * si) * f, b = (v[e] * co + u[e] * si) * f;
-        u[e] = a;
-        v[e] = b;
+    for (int w = 0; w < U; w++) {
+      const int i = i0 + w * 256, t = TOK == 1 ? 0 : i / per_token, rest = i - t * per_token;
+      const int h = rest / per_head, c = rest - h * per_head;
+      if (i >= nt * per_token) continue;
+      const __nv_bfloat16* src =
+          proj + (long long)(t0 + t) * ld + (long long)h * dim + (c < turned ? c * 8 : rot + (c - turned) * 8);
+      in[w] = *reinterpret_cast<const uint4*>(src);
+      if (c < turned) in2[w] = *reinterpret_cast<const uint4*>(src + half);
+    }
+#pragma unroll
+    for (int w = 0; w < U; w++) {
+      const int i = i0 + w * 256, t = TOK == 1 ? 0 : i / per_token, rest = i - t * per_token;
+      const int h = rest / per_head, c = rest - h * per_head;
+      if (i >= nt * per_token) continue;
+      float* dst = qk + ((long long)(t0 + t) * 2 * n_heads + h) * dim;      // heads 0..n-1: queries, n..2n-1: keys
+      const float f = h >= n_heads ? k_scale : 1.0f;
+      float u[8], v[8];
+      if (c < turned) {
+        const int j = c * 8;
+        unpack(in[w], u);
+        unpack(in2[w], v);
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+          const float co = cs[t * half + j + e], si = cs[(TOK + t) * half + j + e];
+          const float a = (u[e] * co - v[e] * si) * f, b = (v[e] * co + u[e] * si) * f;
+          u[e] = a;
+          v[e] = b;
+        }
+        put(dst + j, u);
+        put(dst + j + half, v);
+      } else {
+        const int ch = rot + (c - turned) * 8;
+        unpack(in[w], u);
+#pragma unroll
+        for (int e = 0; e < 8; e++) u[e] *= f;
+        put(dst + ch, u);
       }
-      put(dst + j, u);
-      put(dst + j + half, v);
-    } else {
-      const int ch = rot + (c - turned) * 8;
-      unpack(*reinterpret_cast<const uint4*>(src + ch), u);
-#pragma unroll
-      for (int e = 0; e < 8; e++) u[e] *= f;
-      put(dst + ch, u);
     }
   }
 }
@@ -138,11 +152,10 @@ MF_API int mf_retention_prepare(const void* proj, int dtype, int T, int ld, int 
   mf_count(MF_K_RETENTION_PREPARE);
   if (dtype == MF_BF16 && !v_out && dim % 8 == 0 && rot % 16 == 0 && ld % 8 == 0 && 4 * smem <= 48 * 1024 &&
       !(((uintptr_t)proj | (uintptr_t)qk) & 15)) {
-    // four tokens a block where that leaves two blocks for every SM
-    if (T >= 8 * mf_sm_count())
-      return (int)launch_dep(retention_prepare_vec_kernel<4>, dim3((T + 3) / 4), dim3(256), 4 * smem, stream,
+    if (mf_store_tokens(T, 2 * n_heads * ((dim - rot / 2) / 8)) == 4)
+      return (int)launch_dep(retention_prepare_vec_kernel<4, 2>, dim3((T + 3) / 4), dim3(256), 4 * smem, stream,
                              (const __nv_bfloat16*)proj, ld, n_heads, dim, rot, T, k_scale, positions, inv_f, inv_d, qk, act);
-    return (int)launch_dep(retention_prepare_vec_kernel<1>, dim3(T), dim3(256), smem, stream, (const __nv_bfloat16*)proj, ld,
+    return (int)launch_dep(retention_prepare_vec_kernel<1, 1>, dim3(T), dim3(256), smem, stream, (const __nv_bfloat16*)proj, ld,
                            n_heads, dim, rot, T, k_scale, positions, inv_f, inv_d, qk, act);
   }
   if (dtype == MF_F32)

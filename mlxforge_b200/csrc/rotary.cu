@@ -94,10 +94,10 @@ rope_store_pairs_bf16_kernel(const __nv_bfloat16* qk, int ld, int n_heads, int n
   }
 }
 
-// The same in pieces of 16 bytes (head size and rotated channels multiples of 8, 16-byte aligned rows), TOK tokens a block: the
-// angles of all of them side by side, then up to four pieces a thread on their way at once.  2,237 tokens of 16 + 4 heads of 128
-// (25 MB): 12.3 us with a word a thread and a block per token, 7.5 here.
-template <int TOK>
+// The same in pieces of 16 bytes (head size and rotated channels multiples of 8, 16-byte aligned rows), TOK tokens a block
+// (mf_store_tokens), the angles of all of them side by side.  2,048 tokens of 16 + 4 heads of 128 (23 MB, in L2): 9.5 us with a word a thread,
+// 5.2 here.  One token a block has nothing to gain from several pieces a thread at once (5.2 with one, 6.5 with four).
+template <int TOK, int U>
 __global__ void __launch_bounds__(256)
 rope_store_pairs_vec_kernel(const __nv_bfloat16* qk, int ld, int n_heads, int n_kv, int hd, int rot, int T,
                             const int* positions, const int* seq_of_token, PagedView pv,
@@ -106,7 +106,7 @@ rope_store_pairs_vec_kernel(const __nv_bfloat16* qk, int ld, int n_heads, int n_
   extern __shared__ float cs[];            // [TOK][half] cos, then sin
   __shared__ int pos_s[TOK], seq_s[TOK];
   pdl_launch();
-  const int t0 = blockIdx.x * TOK, nt = min(TOK, T - t0), half = rot >> 1;
+  const int t0 = blockIdx.x * TOK, nt = TOK == 1 ? 1 : min(TOK, T - t0), half = rot >> 1;
   if (threadIdx.x < nt) {
     pos_s[threadIdx.x] = positions[t0 + threadIdx.x];
     seq_s[threadIdx.x] = seq_of_token[t0 + threadIdx.x];
@@ -118,27 +118,37 @@ rope_store_pairs_vec_kernel(const __nv_bfloat16* qk, int ld, int n_heads, int n_
   __syncthreads();
   pdl_wait();
   const int pieces = hd >> 3, per_token = (n_heads + (write_kv ? n_kv : 0)) * pieces;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < nt * per_token; i += 256) {
-    const int t = i / per_token, rest = i - t * per_token, h = rest / pieces, ch = (rest - h * pieces) * 8;
-    const uint4 in = *reinterpret_cast<const uint4*>(qk + (long long)(t0 + t) * ld + (long long)h * hd + ch);
-    uint4 o = in;
-    if (ch < rot) {
-      const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&in);
-      __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&o);
+  // U pieces a thread are on their way before the first is stored
+  for (int i0 = threadIdx.x; i0 < nt * per_token; i0 += U * 256) {
+    uint4 in[U];
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const float2 f = __bfloat1622float2(a[e]);
-        const float c = cs[t * half + ch / 2 + e], s = cs[(TOK + t) * half + ch / 2 + e];
-        b[e] = __floats2bfloat162_rn(f.x * c - f.y * s, f.y * c + f.x * s);
-      }
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * 256, t = TOK == 1 ? 0 : i / per_token;
+      if (i < nt * per_token) in[u] = *reinterpret_cast<const uint4*>(qk + (long long)(t0 + t) * ld + (i - t * per_token) * 8);
     }
-    if (h < n_heads) {
-      *reinterpret_cast<uint4*>(q_out + ((long long)(t0 + t) * n_heads + h) * hd + ch) = o;
-    } else {
-      const long long off = paged_offset(pv, seq_s[t], pos_s[t], h - n_heads) + ch;
-      *reinterpret_cast<uint4*>(k_pool + off) = o;
-      *reinterpret_cast<uint4*>(v_pool + off) = in;          // the values are the keys as projected
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * 256, t = TOK == 1 ? 0 : i / per_token, rest = i - t * per_token;
+      const int h = rest / pieces, ch = (rest - h * pieces) * 8;
+      if (i >= nt * per_token) continue;
+      uint4 o = in[u];
+      if (ch < rot) {
+        const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&in[u]);
+        __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const float2 f = __bfloat1622float2(a[e]);
+          const float c = cs[t * half + ch / 2 + e], s = cs[(TOK + t) * half + ch / 2 + e];
+          b[e] = __floats2bfloat162_rn(f.x * c - f.y * s, f.y * c + f.x * s);
+        }
+      }
+      if (h < n_heads) {
+        *reinterpret_cast<uint4*>(q_out + ((long long)(t0 + t) * n_heads + h) * hd + ch) = o;
+      } else {
+        const long long off = paged_offset(pv, seq_s[t], pos_s[t], h - n_heads) + ch;
+        *reinterpret_cast<uint4*>(k_pool + off) = o;
+        *reinterpret_cast<uint4*>(v_pool + off) = in[u];       // the values are the keys as projected
+      }
     }
   }
 }
@@ -155,13 +165,12 @@ MF_API int mf_rope_store(const void* qk, int ld, int dtype, int T, int n_heads, 
   mf_count(MF_K_ROPE_STORE);
   if (dtype == MF_BF16 && layout == MF_ROT_PAIRS && v_from_k && !inv_d && hd % 8 == 0 && rot % 8 == 0 && ld % 8 == 0 &&
       4 * smem <= 48 * 1024 && (((uintptr_t)qk | (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0) {
-    // four tokens a block where that leaves two blocks for every SM
-#define PAIRS_GO(TOK)                                                                                                 \
-  return (int)launch_dep(rope_store_pairs_vec_kernel<TOK>, dim3((T + TOK - 1) / TOK), dim3(256), TOK * smem, stream,  \
+#define PAIRS_GO(TOK, U)                                                                                                 \
+  return (int)launch_dep(rope_store_pairs_vec_kernel<TOK, U>, dim3((T + TOK - 1) / TOK), dim3(256), TOK * smem, stream,  \
                          (const __nv_bfloat16*)qk, ld, n_heads, n_kv, hd, rot, T, positions, seq_of_token, pv, inv_f, \
                          (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, write_kv)
-    if (T >= 8 * mf_sm_count()) PAIRS_GO(4);
-    PAIRS_GO(1);
+    if (mf_store_tokens(T, (n_heads + (write_kv ? n_kv : 0)) * hd / 8) == 4) PAIRS_GO(4, 4);
+    PAIRS_GO(1, 1);
 #undef PAIRS_GO
   }
   if (dtype == MF_BF16 && layout == MF_ROT_PAIRS && v_from_k && !inv_d && hd % 2 == 0 && ld % 2 == 0 &&

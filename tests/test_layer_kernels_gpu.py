@@ -288,6 +288,104 @@ def test_several_tokens_a_block(kind):
             assert torch.equal(m[a:b], f), (kind, a)
 
 
+@pytest.mark.parametrize("kind,sizes,per_sm", [
+    ("pairs", (4, 2, 128, 48), 8), ("pairs", (16, 4, 128, 128), 24), ("pairs", (17, 4, 128, 64), 40), ("pairs", (3, 1, 72, 0), 8),
+    ("halves", (6, 2, 64, 32), 8), ("halves", (16, 4, 128, 128), 24), ("halves", (32, 16, 64, 16), 40), ("halves", (1, 1, 4096, 4096), 40),
+    ("retention", (3, 64, 48), 8), ("retention", (8, 128, 64), 24), ("retention", (16, 128, 128), 40), ("retention", (1, 72, 0), 8),
+    ("biases", (5, 1, 36, 20), 8), ("biases", (9, 1, 112, 128), 24), ("biases", (16, 4, 128, 128), 40),
+    ("latent", (1032, 104, 64, 32), 8), ("latent", (0, 256, 32, 32), 8), ("latent", (2048, 8, 16, 0), 8)])
+def test_stored_rows(kind, sizes, per_sm):
+    """Steps around the sizes from which a block takes several tokens, of rows that start on a 16-byte boundary and of rows that do not
+    (the general kernels): both stay within the roundings of the same in 64 bits, and what is only copied or added keeps its bits."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    bf, f32, f64 = torch.bfloat16, torch.float32, torch.float64
+    edge = per_sm * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(sum(sizes))
+    page = 16
+
+    def rows(T, width, dt, off):              # [T, width], `off` elements behind a 16-byte boundary
+        x = torch.empty(T * width + 8, device="cuda", dtype=dt)[off:off + T * width].view(T, width)
+        return x.copy_(torch.randn((T, width), generator=g, device="cuda"))
+
+    def turned(x, cos, sin, pairs):           # 64 bits; also the size of what was added up
+        r, n = 2 * cos.shape[-1], cos.shape[-1]
+        a, b = (x[..., 0:r:2], x[..., 1:r:2]) if pairs else (x[..., :n], x[..., n:r])
+        y, m = x.clone(), x.abs()
+        ya, yb, size = a * cos - b * sin, b * cos + a * sin, a.abs() + b.abs()
+        for z, u, v in ((y, ya, yb), (m, size, size)):
+            if pairs:
+                z[..., 0:r:2], z[..., 1:r:2] = u, v
+            else:
+                z[..., :n], z[..., n:r] = u, v
+        return y, m
+
+    def near(got, want, size, slack=0.0):
+        # sine and cosine to 2 ulp, three roundings of 2^-24 each, what the caller adds; a rounding to the result's type
+        tol = (2 ** -21 + slack) * size + (2 ** -8 * want.abs() if got.dtype == bf else 0)
+        assert bool(((got.double() - want).abs() <= tol).all())
+
+    for T, off in ((1, 0), (3, 1), (edge - 1, 0), (edge, 0), (edge + 3, 0), (edge + 3, 1)):
+        pages = -(-T // page)
+        table = torch.randperm(pages + 1, generator=g, device="cuda")[:pages].to(torch.int32)[None].contiguous()
+        pos, seq = torch.arange(T, device="cuda", dtype=torch.int32), torch.zeros(T, device="cuda", dtype=torch.int32)
+        pool = lambda heads, d: torch.full((pages + 1, heads, page, d), float("nan"), device="cuda", dtype=bf)
+        kept = lambda p: p[table[0, (pos // page).long()].long(), :, (pos % page).long()]          # [T, heads, d]
+        table_f = lambda n: 50000.0 ** (-torch.arange(n, device="cuda", dtype=f32) / max(n, 1))
+        turn = lambda angles: (angles.double().cos()[:, None], angles.double().sin()[:, None])
+        if kind in ("pairs", "halves"):
+            nh, nkv, hd, rot = sizes
+            pairs, heads = kind == "pairs", nh + (1 if kind == "pairs" else 2) * nkv
+            x, q, k, v = rows(T, heads * hd, bf, off), torch.full((T, nh * hd), float("nan"), device="cuda", dtype=bf), pool(nkv, hd), pool(nkv, hd)
+            inv = table_f(rot // 2)
+            if pairs:
+                ops.rope_store(x, pos, seq, table, page, inv, None, q, k, v, nh, nkv, hd, rot, True, True, True, ld=heads * hd)
+                angles = pos.to(f32)[:, None] * inv
+            else:
+                ops.rope_kv_write(x, pos, seq, table, page, 1 / inv, q, k, v, nh, nkv, hd, rot, True, False)
+                angles = pos.to(f32)[:, None] / (1 / inv)
+            xs = x.view(T, heads, hd)
+            want, size = turned(xs[:, :nh + nkv].double(), *turn(angles), pairs)
+            got = torch.cat([q.view(T, nh, hd), kept(k)], 1)
+            near(got[..., :rot], want[..., :rot], size[..., :rot])
+            assert torch.equal(got[..., rot:], xs[:, :nh + nkv, rot:]) and torch.equal(kept(v), xs[:, -nkv:])
+        elif kind == "retention":
+            nh, d, rot = sizes
+            x, qk, inv = rows(T, 3 * nh * d, bf, off), torch.full((T, 2 * nh * d), float("nan"), device="cuda"), table_f(rot // 2)
+            ops.retention_prepare(x, nh, d, rot, 0.3, pos, inv, None, qk, silu=True)
+            xd = x.view(T, 3 * nh, d)[:, :2 * nh].double()
+            y, size = turned(xd * torch.sigmoid(xd), *turn(pos.to(f32)[:, None] * inv), False)
+            f = torch.tensor([1.0] * nh + [0.3] * nh, device="cuda", dtype=f32).double()[None, :, None]
+            near(qk.view(T, 2 * nh, d), y * f, size * f, 2 ** -20)            # the sigmoid: an exponential of 2 ulp, a sum and a quotient
+        elif kind == "biases":
+            nh, nkv, d, dv = sizes
+            w = nh * d + nkv * (d + dv)
+            x, b, q = rows(T, w, f32, off), torch.randn(w, generator=g, device="cuda"), torch.full((T, nh * d), float("nan"), device="cuda", dtype=bf)
+            k, v = pool(nkv, d), pool(nkv, dv)
+            ops.biased_kv_store(x, b, pos, seq, table, page, q, k, v, nh, nkv, d, dv, True)
+            y = (x + b).to(bf)
+            assert torch.equal(q, y[:, :nh * d]) and torch.equal(kept(k).reshape(T, -1), y[:, nh * d:(nh + nkv) * d])
+            assert torch.equal(kept(v).reshape(T, -1), y[:, (nh + nkv) * d:])
+        else:
+            qr, rank, part, rot = sizes
+            x, inv = rows(T, qr + 8 + rank + part, bf, off), table_f(rot // 2)
+            wq, wkv = (torch.randn(max(n, 4), generator=g, device="cuda") for n in (qr, rank))
+            cq, k, pairs = torch.full((T, max(qr, 1)), float("nan"), device="cuda", dtype=bf), pool(1, rank + part), T % 2 == 1
+            ops.latent_prepare(x, qr, qr + 8, rank, part, wq if qr else None, wkv, 1e-6, pos, seq, table, page, inv, None, cq if qr else None, k,
+                               True, pairs=pairs, rot_dims=rot, magnitude=1.25)
+            normed = lambda a, w: a / (a.square().mean(1, keepdim=True) + 1e-6).sqrt() * w.double()
+            xd, row = x.double(), kept(k)[:, 0]
+            if qr:
+                want = normed(xd[:, :qr], wq)
+                near(cq, want, want.abs(), 2 ** -20)                          # the sum of up to 2048 squares, by lanes; root and quotient
+            want = normed(xd[:, qr + 8:qr + 8 + rank], wkv[:rank])
+            near(row[:, :rank], want, want.abs(), 2 ** -20)
+            key = xd[:, None, qr + 8 + rank:]
+            want, size = turned(key, *(1.25 * c for c in turn(pos.to(f32)[:, None] * inv)), pairs)
+            near(row[:, rank:rank + rot], want[:, 0, :rot], 1.25 * size[:, 0, :rot])
+            assert torch.equal(row[:, rank + rot:], x[:, qr + 8 + rank + rot:])
+
+
 @pytest.mark.parametrize("V,heads,T,parts", [(64, 3, 5, 1), (128, 5, 3, 4), (128, 1, 1, 1)])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_read_out_norms(V, heads, T, parts, dtype):
