@@ -28,7 +28,6 @@
 #define MG_LD (MG_BK + 8)
 #define MG_STAGES 2
 #define MG_MAX_EXPERTS 1024
-#define MG_SORT_STAGED 32768       // pairs whose tokens the sort keeps in shared memory
 
 __device__ __forceinline__ void mg_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -40,14 +39,13 @@ __device__ __forceinline__ void mg_mma(float (&c)[4], const uint32_t (&a)[4], ui
 // meta: [0] number of tiles; tiles: [max_tiles][3] = expert, first row, rows.  An expert's rows are cut into as few tiles of at
 // most `tile_rows` as hold them: full ones and a rest (64 rows), or for larger tiles equal ones in steps of 16.  A thread per
 // expert: offsets by a scan over the block (a thread that walked the experts alone took most of 21 us for 64 of them).
-// A pair is counted once and its place kept (12,288 pairs of 64 experts: 11.0 -> 10.4 us), and the rows' tokens are put in order in
-// shared memory where they fit, since a warp's 32 scattered words are 32 stores to memory (10.4 -> 7.2); with the gather below and both launched
-// behind their predecessor's end, the mixture of 2,048 tokens 207 -> 202.5 us.
+// The pairs are counted, then placed: the counts, whose old values nobody asks for, are cheap, and the placing overlaps with its stores.  (Counts
+// that hand out the places at once save the second pass and lose that: 8,192 pairs of 16 experts 6.2 us, 384 of 64 3.3, 12,288 of 64 9.7; here
+// 4.8, 2.7 and 10.0.  Neither is faster with the tokens put in order in shared memory.)
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int* ids, int n_pairs, int E, int top, int tile_rows, int* slot_of,
-                int* __restrict__ row_token, int* __restrict__ meta, int* __restrict__ tiles, int staged) {
-  extern __shared__ int tokens[];            // staged: [n_pairs], a row's token
-  __shared__ int count[MG_MAX_EXPERTS], first[MG_MAX_EXPERTS];
+                int* __restrict__ row_token, int* __restrict__ meta, int* __restrict__ tiles) {
+  __shared__ int count[MG_MAX_EXPERTS], cursor[MG_MAX_EXPERTS];
   __shared__ int2 warp_total[32];
   __shared__ int used_rows;
   const int e = threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -55,21 +53,15 @@ moe_sort_kernel(const int* ids, int n_pairs, int E, int top, int tile_rows, int*
   pdl_wait();
   count[e] = 0;
   __syncthreads();
-  // A pair's place among its expert's rows is what its own count returns; the first HELD pairs of a thread wait for the
-  // offsets in registers, the others in slot_of.  Their loads are on their way together.
-  constexpr int HELD = 16;
-  int own[HELD], place[HELD];
+  // eight pairs a thread at a time: their loads are on their way together
+  constexpr int AT_ONCE = 8;
+  for (int i0 = threadIdx.x; i0 < n_pairs; i0 += AT_ONCE * 1024) {
+    int own[AT_ONCE];
 #pragma unroll
-  for (int k = 0; k < HELD; k++) own[k] = e + k * 1024 < n_pairs ? ids[e + k * 1024] : -1;
+    for (int k = 0; k < AT_ONCE; k++) own[k] = i0 + k * 1024 < n_pairs ? ids[i0 + k * 1024] : E;
 #pragma unroll
-  for (int k = 0; k < HELD; k++) place[k] = own[k] >= 0 && own[k] < E ? atomicAdd(&count[own[k]], 1) : 0;
-  for (int i0 = e + HELD * 1024; i0 < n_pairs; i0 += HELD * 1024) {
-    int id[HELD];
-#pragma unroll
-    for (int k = 0; k < HELD; k++) id[k] = i0 + k * 1024 < n_pairs ? ids[i0 + k * 1024] : -1;
-#pragma unroll
-    for (int k = 0; k < HELD; k++)
-      if (id[k] >= 0 && id[k] < E) slot_of[i0 + k * 1024] = atomicAdd(&count[id[k]], 1);
+    for (int k = 0; k < AT_ONCE; k++)
+      if (own[k] < E) atomicAdd(&count[own[k]], 1);
   }
   __syncthreads();
   {
@@ -92,7 +84,7 @@ moe_sort_kernel(const int* ids, int n_pairs, int E, int top, int tile_rows, int*
     }
     rows += before.x;
     blocks += before.y;
-    first[e] = rows - n;                     // the expert's first row
+    cursor[e] = rows - n;                    // the expert's first row
     if (e == E - 1) {
       meta[0] = blocks;
       used_rows = rows;
@@ -106,32 +98,22 @@ moe_sort_kernel(const int* ids, int n_pairs, int E, int top, int tile_rows, int*
     }
   }
   __syncthreads();
-  auto put = [&](int i, int id, int at) {
-    if (id < 0) return;
-    if (id >= E) {                    // an identity expert: no row
-      slot_of[i] = -1;
-      return;
+  for (int i0 = threadIdx.x; i0 < n_pairs; i0 += AT_ONCE * 1024) {
+    int own[AT_ONCE];
+#pragma unroll
+    for (int k = 0; k < AT_ONCE; k++) own[k] = i0 + k * 1024 < n_pairs ? ids[i0 + k * 1024] : -1;
+#pragma unroll
+    for (int k = 0; k < AT_ONCE; k++) {
+      const int i = i0 + k * 1024;
+      if (own[k] < 0) continue;
+      if (own[k] >= E) {              // an identity expert: no row
+        slot_of[i] = -1;
+        continue;
+      }
+      const int row = atomicAdd(&cursor[own[k]], 1);
+      slot_of[i] = row;
+      row_token[row] = i / top;
     }
-    const int row = first[id] + at;
-    slot_of[i] = row;
-    if (staged) tokens[row] = i / top;
-    else row_token[row] = i / top;
-  };
-#pragma unroll
-  for (int k = 0; k < HELD; k++) put(e + k * 1024, own[k], place[k]);
-  for (int i0 = e + HELD * 1024; i0 < n_pairs; i0 += HELD * 1024) {
-    int id[HELD], at[HELD];
-#pragma unroll
-    for (int k = 0; k < HELD; k++) {
-      id[k] = i0 + k * 1024 < n_pairs ? ids[i0 + k * 1024] : -1;
-      at[k] = i0 + k * 1024 < n_pairs ? slot_of[i0 + k * 1024] : 0;        // this thread's own store, or unused
-    }
-#pragma unroll
-    for (int k = 0; k < HELD; k++) put(i0 + k * 1024, id[k], at[k]);
-  }
-  if (staged) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < used_rows; i += blockDim.x) row_token[i] = tokens[i];
   }
   // rows that no pair took (pairs of identity experts have none) name token 0, so that a gather over all
   // n_pairs rows stays inside x
@@ -143,18 +125,8 @@ MF_API int mf_moe_sort(const int* ids, int T, int E, int top, int tile_rows, int
   if (T <= 0) return 0;
   if (E < 1 || E > MG_MAX_EXPERTS || tile_rows < MG_BM || tile_rows % 16) return MF_ERR_BAD_ARG;
   mf_count(MF_K_MOE_SORT);
-  // rows' tokens are put in order in shared memory where they fit
-  const int n = T * top, staged = n <= MG_SORT_STAGED;
-  static DeviceOnce once;
-  const int dev = mf_current_device();
-  if (dev < 0) return MF_ERR_BAD_ARG;
-  if (!once.done[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(moe_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SORT_STAGED * 4);
-    if (e != cudaSuccess) return (int)e;
-    once.done[dev] = true;
-  }
-  return (int)launch_dep(moe_sort_kernel, dim3(1), dim3(1024), staged ? n * sizeof(int) : 0, stream, ids, n, E, top, tile_rows,
-                         slot_of, row_token, meta, tiles, staged);
+  return (int)launch_dep(moe_sort_kernel, dim3(1), dim3(1024), 0, stream, ids, T * top, E, top, tile_rows, slot_of, row_token,
+                         meta, tiles);
 }
 
 __device__ __forceinline__ void mg_ldmatrix_x4(uint32_t (&r)[4], const void* p) {

@@ -515,7 +515,7 @@ def test_attention_f32_tiles_of_every_height(nh, nkv, hd, vd, n):
 
 @pytest.mark.parametrize("T,top,E", [(1, 1, 1), (37, 3, 33), (2048, 8, 1024), (16385, 1, 64), (5001, 7, 200), (4099, 12, 2)])
 def test_sorted_pairs_and_gathered_rows(T, top, E):
-    """Pairs that a thread holds in registers (up to 16,384) and those beyond, experts in part of a warp up to all of the block's
+    """Pairs that the block loads at once (up to 8,192) and those beyond, experts in part of a warp up to all of the block's
     threads, identity experts in between, gathers whose last block has a rest: whole numbers and copies, so equality."""
     import torch
     from mlxforge_b200.csrc import ops
