@@ -95,7 +95,8 @@ def test_router_ties_and_values_that_are_not_finite(E, groups, keep, top):
 
 
 @pytest.mark.parametrize("H,top,slices,T,kind", [(2048, 6, 12, 8, 0), (132, 9, 3, 5, 1), (1028, 2, 1, 70, 2), (128, 17, 2, 3, 3),
-                                                  (130, 3, 2, 4, 3), (2048, 6, 1, 100, 3)])
+                                                  (130, 3, 2, 4, 3), (2048, 6, 1, 100, 3),
+                                                  (2048, 1, 12, 8, 0), (132, 1, 2, 5, 3), (1028, 1, 1, 70, 1), (132, 2, 2, 5, 3)])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_weighted_sum_of_experts(H, top, slices, T, kind, dtype):
     """kind 0: plain; 1: identity experts; 2: rows by slot; 3: a shared branch with its gate as well."""
