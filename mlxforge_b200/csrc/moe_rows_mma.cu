@@ -245,12 +245,14 @@ moe_rows_mma_kernel(const __grid_constant__ CUtensorMap map_gu, const __grid_con
       if (lane == 0) mbar_arrive(bars + 8 * (STAGES + s));
       if (++s == STAGES) s = 0, round++;
     }
+    // rows beyond ff are zeros, which an input that is not finite turns into NaN
+    const bool real = slice * SLICE + warp * 8 + g < a.ff;
 #pragma unroll
     for (int nb = 0; nb < NB; nb++)
 #pragma unroll
       for (int j = 0; j < 2; j++) {
         const float p = acc[nb][0][j] + acc[nb][1][j], q = acc[nb][0][j + 2] + acc[nb][1][j + 2];
-        const float v = gated ? gated_product(p, q, MF_GATE_CLAMPED, a.ec) : gate_act(p, a.act_kind);
+        const float v = real ? gated ? gated_product(p, q, MF_GATE_CLAMPED, a.ec) : gate_act(p, a.act_kind) : 0.f;
         const int tok = nb * 8 + 2 * t + j;
         const __nv_bfloat16 b = __float2bfloat16_rn(v);
         asm volatile("st.shared.u16 [%0], %1;\n" ::"r"(acts + tok * 128 + ((unsigned)(warp ^ (tok & 7)) << 4) + g * 2),

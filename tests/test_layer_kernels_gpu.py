@@ -60,6 +60,36 @@ def test_experts_few_tokens(H, ff, E, top, T, act):
     assert torch.equal(alone[0][here], y[T // 2][here]), "a token's result depends on what else is in the step"
 
 
+@pytest.mark.parametrize("act", ["silu", "relu2", None])
+@pytest.mark.parametrize("ff", [72, 128, 200])
+@pytest.mark.parametrize("bad", ["nan", "inf"])
+def test_experts_few_tokens_that_are_not_finite(ff, bad, act):
+    """A token that is not finite beside others of its experts' passes: theirs keep their bits, and its own outputs are those of its
+    ff columns, not of the zeros that fill a slice.  An infinity that every column's first factor has, with the sign of ``act``'s case:
+    infinite throughout, zero throughout, or clamped to finite numbers."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(ff)
+    bf, H, E, T, top = torch.bfloat16, 128, 3, 12, 2
+    x = torch.randn((T, H), generator=g, device="cuda").to(bf)
+    w_gu = torch.randn((E, 1 if act else 2, ff, H), generator=g, device="cuda").to(bf)
+    w_gu[:, 0, :, 17] = (w_gu[:, 0, :, 17].abs() + 0.5) * (-1 if act == "relu2" else 1)
+    w_down = (torch.rand((E, H, ff), generator=g, device="cuda") + 0.1).to(bf)
+    ids = torch.rand((T, E), generator=g, device="cuda").topk(top, 1).indices.to(torch.int32).contiguous()
+    slices, ys = ops.moe_rows_slices(ff), []
+    for value in (None, float(bad)):
+        y = torch.full((T, top * slices, H), 7.0, device="cuda")
+        if value is not None:
+            x[5, 17] = value
+        ops.moe_rows(x, w_gu, w_down, ids, y, 7.0, 1.702, 1.0, act)
+        ys.append(y)
+    ops.check_kernel_status()
+    others = torch.arange(T, device="cuda") != 5
+    assert torch.equal(ys[0][others], ys[1][others])
+    if bad == "inf":
+        assert bool(((ys[1][5] == float("inf")) if act == "silu" else (ys[1][5] == 0) if act == "relu2" else ys[1][5].isfinite()).all())
+
+
 @pytest.mark.parametrize("E,groups,keep,top", [(64, 8, 4, 6), (33, 0, 0, 5), (6, 3, 1, 2), (200, 0, 0, 9)])
 def test_router_ties_and_values_that_are_not_finite(E, groups, keep, top):
     """Equal scores go to the lower expert (groups: the higher one leaves first); a score that is not a number is never chosen
