@@ -249,6 +249,59 @@ def test_prefill_attention_does_not_depend_on_the_next_portion(hd, n, held):
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("form", ["plain", "latent"])
+@pytest.mark.parametrize("chain", [0, 1])
+@pytest.mark.parametrize("what", ["value nan", "value inf", "key nan", "tile unseen"])
+def test_prefill_attention_joins_what_is_not_finite(form, chain, what):
+    """Two running results over alternate tiles of 64 keys: a NaN or an infinity that one of them holds is in the joined one where a
+    64-bit softmax has it, one whose scores all are minus infinity has no part, and query tiles that see none of it keep their bits."""
+    import torch
+    from mlxforge_b200.csrc import binding, ops
+    nh, nkv, hd, vd = (4, 2, 128, 128) if form == "plain" else (3, 1, 160, 128)
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    bf, n = torch.bfloat16, 300
+    q = (0.3 * torch.randn((n, nh, hd), generator=g, device="cuda")).to(bf)
+    q[..., -1] = 1
+    k = torch.randn((n, nkv, hd), generator=g, device="cuda").to(bf)
+    v = k[..., :vd] if form == "latent" else torch.randn((n, nkv, vd), generator=g, device="cuda").to(bf)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    per, outs, at = -(-n // 16), [], 64 * (2 + chain) + 5
+    first = 0 if what == "tile unseen" else at            # the first row that sees it
+    for spoilt in (False, True):
+        if spoilt and what == "tile unseen":              # all that this chain has of the first 128 keys
+            k[64 * chain:64 * chain + 64, :, -1] = -float("inf")
+        elif spoilt and what == "key nan":
+            k[at, :, -1] = float("nan")
+        elif spoilt:
+            v[at, :, 7] = float(what.split()[1])
+        kp, vp = (torch.full((per, nkv, 16, x.shape[2]), float("nan"), device="cuda", dtype=bf) for x in (k, v))
+        for b in range(per):
+            for pool, x in ((kp, k), (vp, v)):
+                pool[b, :, :x[b * 16:b * 16 + 16].shape[0]] = x[b * 16:b * 16 + 16].transpose(0, 1)
+        out = torch.full((n, nh * vd), float("nan"), device="cuda", dtype=bf)
+        args = (i32([0]), i32([n]), i32([n]), 0, n, i32([list(range(per))]), 16, nh, nkv, hd, hd ** -0.5)
+        before = binding.kernel_launches()
+        if form == "plain":
+            ops.attention_prefill(q.view(n, -1), kp, vp, out, *args, 0)
+        else:
+            ops.attention_prefill_ex(q.view(n, -1), kp, kp, out, *args, 0, vd, True, 0, None, None, 0, 0.0, n)
+        ops.check_kernel_status()
+        assert _ran(before).get("attn_prefill_tc", 0) == 1
+        outs.append(out)
+    if first >= 128:
+        assert torch.equal(outs[0][:128], outs[1][:128])
+    i, j = torch.arange(n, device="cuda")[:, None], torch.arange(n, device="cuda")[None]
+    for h in range(nh):
+        kd, vd64 = k[:, h // (nh // nkv)].double(), v[:, h // (nh // nkv)].double()
+        p = torch.softmax((q[:, h].double() @ kd.T * hd ** -0.5).masked_fill(j > i, -np.inf), 1)
+        # a row's own keys only: a zero times what is not finite would not be zero
+        for row in range(64 if what == "tile unseen" else first, n, 7):
+            want, mag = p[row, :row + 1] @ vd64[:row + 1], p[row, :row + 1] @ vd64[:row + 1].abs()
+            got, ok = outs[1][row, h * vd:(h + 1) * vd].double(), want.isfinite()
+            assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[~ok & ~want.isnan()], want[~ok & ~want.isnan()])
+            assert bool(((got - want).abs() <= 2 ** -8 * mag + 2 ** -8 * want.abs() + 1e-6)[ok].all()), (h, row)
+
+
 # ----------------------------------------------------------------------------- rotations, biases and norms of prompts
 
 def _store_case(kind, T, g, pages):
