@@ -28,6 +28,7 @@
 #define MG_LD (MG_BK + 8)
 #define MG_STAGES 2
 #define MG_MAX_EXPERTS 1024
+#define MG_SORT_STAGED 32768       // pairs whose tokens the sort keeps in shared memory
 
 __device__ __forceinline__ void mg_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -39,12 +40,14 @@ __device__ __forceinline__ void mg_mma(float (&c)[4], const uint32_t (&a)[4], ui
 // meta: [0] number of tiles; tiles: [max_tiles][3] = expert, first row, rows.  An expert's rows are cut into as few tiles of at
 // most `tile_rows` as hold them: full ones and a rest (64 rows), or for larger tiles equal ones in steps of 16.  A thread per
 // expert: offsets by a scan over the block (a thread that walked the experts alone took most of 21 us for 64 of them).
-// The pairs are counted, then placed: the counts, whose old values nobody asks for, are cheap, and the placing overlaps with its stores.  (Counts
-// that hand out the places at once save the second pass and lose that: 8,192 pairs of 16 experts 6.2 us, 384 of 64 3.3, 12,288 of 64 9.7; here
-// 4.8, 2.7 and 10.0.  Neither is faster with the tokens put in order in shared memory.)
+// The pairs are counted, then placed, the counts' old values asked for by nobody (a count that hands out the places at once has no second pass, but 8,192
+// pairs of 16 experts wait for one another: 6.2 us, 4.7 here).  The rows' tokens are put in order in shared memory where they fit: a warp's 32
+// scattered words are 32 stores to memory (12,288 pairs of 64 experts 9.6 -> 6.6 us, 384 the same 2.6).
+template <bool STAGED>
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int* ids, int n_pairs, int E, int top, int tile_rows, int* slot_of,
                 int* __restrict__ row_token, int* __restrict__ meta, int* __restrict__ tiles) {
+  extern __shared__ int tokens[];            // STAGED: [n_pairs], a row's token
   __shared__ int count[MG_MAX_EXPERTS], cursor[MG_MAX_EXPERTS];
   __shared__ int2 warp_total[32];
   __shared__ int used_rows;
@@ -53,9 +56,15 @@ moe_sort_kernel(const int* ids, int n_pairs, int E, int top, int tile_rows, int*
   pdl_wait();
   count[e] = 0;
   __syncthreads();
-  // eight pairs a thread at a time: their loads are on their way together
+  // eight pairs a thread at a time: their loads are on their way together; the first eight stay in registers
   constexpr int AT_ONCE = 8;
-  for (int i0 = threadIdx.x; i0 < n_pairs; i0 += AT_ONCE * 1024) {
+  int held[AT_ONCE];
+#pragma unroll
+  for (int k = 0; k < AT_ONCE; k++) held[k] = e + k * 1024 < n_pairs ? ids[e + k * 1024] : -1;
+#pragma unroll
+  for (int k = 0; k < AT_ONCE; k++)
+    if (held[k] >= 0 && held[k] < E) atomicAdd(&count[held[k]], 1);
+  for (int i0 = e + AT_ONCE * 1024; i0 < n_pairs; i0 += AT_ONCE * 1024) {
     int own[AT_ONCE];
 #pragma unroll
     for (int k = 0; k < AT_ONCE; k++) own[k] = i0 + k * 1024 < n_pairs ? ids[i0 + k * 1024] : E;
@@ -98,22 +107,29 @@ moe_sort_kernel(const int* ids, int n_pairs, int E, int top, int tile_rows, int*
     }
   }
   __syncthreads();
-  for (int i0 = threadIdx.x; i0 < n_pairs; i0 += AT_ONCE * 1024) {
+  auto put = [&](int i, int id) {
+    if (id < 0) return;
+    if (id >= E) {              // an identity expert: no row
+      slot_of[i] = -1;
+      return;
+    }
+    const int row = atomicAdd(&cursor[id], 1);
+    slot_of[i] = row;
+    if (STAGED) tokens[row] = i / top;
+    else row_token[row] = i / top;
+  };
+#pragma unroll
+  for (int k = 0; k < AT_ONCE; k++) put(e + k * 1024, held[k]);
+  for (int i0 = e + AT_ONCE * 1024; i0 < n_pairs; i0 += AT_ONCE * 1024) {
     int own[AT_ONCE];
 #pragma unroll
     for (int k = 0; k < AT_ONCE; k++) own[k] = i0 + k * 1024 < n_pairs ? ids[i0 + k * 1024] : -1;
 #pragma unroll
-    for (int k = 0; k < AT_ONCE; k++) {
-      const int i = i0 + k * 1024;
-      if (own[k] < 0) continue;
-      if (own[k] >= E) {              // an identity expert: no row
-        slot_of[i] = -1;
-        continue;
-      }
-      const int row = atomicAdd(&cursor[own[k]], 1);
-      slot_of[i] = row;
-      row_token[row] = i / top;
-    }
+    for (int k = 0; k < AT_ONCE; k++) put(i0 + k * 1024, own[k]);
+  }
+  if (STAGED) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < used_rows; i += blockDim.x) row_token[i] = tokens[i];
   }
   // rows that no pair took (pairs of identity experts have none) name token 0, so that a gather over all
   // n_pairs rows stays inside x
@@ -125,8 +141,21 @@ MF_API int mf_moe_sort(const int* ids, int T, int E, int top, int tile_rows, int
   if (T <= 0) return 0;
   if (E < 1 || E > MG_MAX_EXPERTS || tile_rows < MG_BM || tile_rows % 16) return MF_ERR_BAD_ARG;
   mf_count(MF_K_MOE_SORT);
-  return (int)launch_dep(moe_sort_kernel, dim3(1), dim3(1024), 0, stream, ids, T * top, E, top, tile_rows, slot_of, row_token,
-                         meta, tiles);
+  const int n = T * top;
+  if (n > MG_SORT_STAGED)
+    return (int)launch_dep(moe_sort_kernel<false>, dim3(1), dim3(1024), 0, stream, ids, n, E, top, tile_rows, slot_of, row_token,
+                           meta, tiles);
+  static DeviceOnce once;
+  const int dev = mf_current_device();
+  if (dev < 0) return MF_ERR_BAD_ARG;
+  if (!once.done[dev]) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(moe_sort_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SORT_STAGED * 4);
+    if (e != cudaSuccess) return (int)e;
+    once.done[dev] = true;
+  }
+  return (int)launch_dep(moe_sort_kernel<true>, dim3(1), dim3(1024), n * sizeof(int), stream, ids, n, E, top, tile_rows, slot_of,
+                         row_token, meta, tiles);
 }
 
 __device__ __forceinline__ void mg_ldmatrix_x4(uint32_t (&r)[4], const void* p) {
