@@ -216,13 +216,13 @@ int mf_sm_count();
 
 // ---------------------------------------------------------------------------- rows stored piece by piece
 // Tokens a block of 256 threads takes of a step of T, a token being `pieces` of 16 bytes that a thread each loads, turns and stores (in L2,
-// us, one token a block / four).  Four where a token leaves half the threads idle: 2,048 tokens of 4 + 2 heads of 32, 14 pieces, 5.2 / 2.3, of
-// 8 + 2 x 2 heads of 64, 56 pieces, 5.2 / 3.8; 1,200 tokens 3.5 / 2.2 and 3.6 / 3.3; 1,024 of the latter even, 3.5 / 3.5.  One where it fills
-// them, as four leave too few blocks in flight: 2,048 tokens of 32 + 2 x 8 heads of 64, 224 pieces, 5.7 / 7.0, of 16 + 4 heads of 128, 320
-// pieces, 5.2 / 6.5, of 16 + 2 x 4 with biases, 768 pieces, 5.0 / 9.0; until blocks abound: at 4,096 tokens 9.9 / 9.5, 9.1 / 8.9 and
-// 9.3 / 11.7, at 8,192 22.1 / 19.2, 18.5 / 17.9 and 28.4 / 26.1.
-inline int mf_store_tokens(int T, int pieces) {
-  return T >= (pieces <= 128 ? 8 : pieces <= 320 ? 24 : 40) * mf_sm_count() ? 4 : 1;
+// us, one token a block / four).  Four where a token leaves most threads idle: 1,200 tokens of 4 + 2 heads of 32, 14 pieces, 3.5 / 2.2, of 8 + 2 x 2
+// heads of 64, 56 pieces, 3.4 / 3.4, at 2,048 tokens 5.2 / 2.3 and 4.8 / 3.8.  Half of them, later: 16 + 2 x 4 heads of 64, 112 pieces, 1,200 tokens
+// 3.7 / 4.7, 2,048 tokens 5.3 / 5.1.  One where it fills them, as four leave too few blocks in flight: 2,048 tokens of 32 + 2 x 8 heads of 64, 224
+// pieces, 5.7 / 7.0, of 16 + 4 heads of 128, 320 pieces, 5.2 / 6.5, of 16 + 2 x 4 with biases, 768 pieces, 5.0 / 9.0; until blocks abound: at
+// 4,096 tokens 9.9 / 9.5, 9.1 / 8.9 and 9.3 / 11.7, at 8,192 22.1 / 19.2, 18.5 / 17.9 and 28.4 / 26.1.
+inline int mf_store_tokens(int T, int pieces, int few = 56) {
+  return T >= (pieces <= few ? 8 : pieces <= 128 ? 13 : pieces <= 320 ? 24 : 40) * mf_sm_count() ? 4 : 1;
 }
 
 // ---------------------------------------------------------------------------- which kernels ran

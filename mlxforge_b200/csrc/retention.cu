@@ -69,7 +69,7 @@ __global__ void retention_prepare_kernel(const T* proj, int ld, int n_heads, int
 
 // The same for bfloat16 rows in pieces of eight channels and of the eight they pair with (head size and half of the rotated channels
 // multiples of 8, 16-byte aligned rows, no v_out), TOK tokens a block (mf_store_tokens), the angles of all of them side by side.
-// 1,777 tokens of 8 heads of 128 (22 MB, in L2): 10.3 us with a channel a thread, 5.5 here.
+// 1,777 tokens of 8 heads of 128, half of the channels turned (22 MB, in L2): 10.3 us with a channel a thread, 5.5 here; all turned 10.6 and 7.6.
 template <int TOK, int U>
 __global__ void __launch_bounds__(256)
 retention_prepare_vec_kernel(const __nv_bfloat16* proj, int ld, int n_heads, int dim, int rot, int T, float k_scale,
@@ -79,7 +79,7 @@ retention_prepare_vec_kernel(const __nv_bfloat16* proj, int ld, int n_heads, int
   pdl_launch();
   const int t0 = blockIdx.x * TOK, nt = TOK == 1 ? 1 : min(TOK, T - t0), half = rot >> 1;
   for (int i = threadIdx.x; i < nt * half; i += 256) {
-    const int t = i / half, j = i - t * half;
+    const int t = TOK == 1 ? 0 : i / half, j = i - t * half;
     rotary_cs(positions[t0 + t], j, inv_f, inv_d, cs[i], cs[TOK * half + i]);
   }
   __syncthreads();
@@ -152,7 +152,9 @@ MF_API int mf_retention_prepare(const void* proj, int dtype, int T, int ld, int 
   mf_count(MF_K_RETENTION_PREPARE);
   if (dtype == MF_BF16 && !v_out && dim % 8 == 0 && rot % 16 == 0 && ld % 8 == 0 && 4 * smem <= 48 * 1024 &&
       !(((uintptr_t)proj | (uintptr_t)qk) & 15)) {
-    if (mf_store_tokens(T, 2 * n_heads * ((dim - rot / 2) / 8)) == 4)
+    // a piece here is two loads and four stores: four tokens a block from the first size on up to 128 of them (1,777 tokens of 8 heads of 128,
+    // all channels turned, 8.3 / 7.6 us with one / four; 4 heads 6.2 / 5.3)
+    if (mf_store_tokens(T, 2 * n_heads * ((dim - rot / 2) / 8), 128) == 4)
       return (int)launch_dep(retention_prepare_vec_kernel<4, 2>, dim3((T + 3) / 4), dim3(256), 4 * smem, stream,
                              (const __nv_bfloat16*)proj, ld, n_heads, dim, rot, T, k_scale, positions, inv_f, inv_d, qk, act);
     return (int)launch_dep(retention_prepare_vec_kernel<1, 1>, dim3(T), dim3(256), smem, stream, (const __nv_bfloat16*)proj, ld,

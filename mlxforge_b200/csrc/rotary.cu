@@ -112,7 +112,7 @@ rope_store_pairs_vec_kernel(const __nv_bfloat16* qk, int ld, int n_heads, int n_
     seq_s[threadIdx.x] = seq_of_token[t0 + threadIdx.x];
   }
   for (int i = threadIdx.x; i < nt * half; i += 256) {
-    const int t = i / half, j = i - t * half;
+    const int t = TOK == 1 ? 0 : i / half, j = i - t * half;
     sincosf((float)positions[t0 + t] * inv_f[j], &cs[TOK * half + i], &cs[i]);
   }
   __syncthreads();

@@ -373,10 +373,10 @@ def test_several_tokens_a_block(kind):
 
 
 @pytest.mark.parametrize("kind,sizes,per_sm", [
-    ("pairs", (4, 2, 128, 48), 8), ("pairs", (16, 4, 128, 128), 24), ("pairs", (17, 4, 128, 64), 40), ("pairs", (3, 1, 72, 0), 8),
-    ("halves", (6, 2, 64, 32), 8), ("halves", (16, 4, 128, 128), 24), ("halves", (32, 16, 64, 16), 40), ("halves", (1, 1, 4096, 4096), 40),
-    ("retention", (3, 64, 48), 8), ("retention", (8, 128, 64), 24), ("retention", (16, 128, 128), 40), ("retention", (1, 72, 0), 8),
-    ("biases", (5, 1, 36, 20), 8), ("biases", (9, 1, 112, 128), 24), ("biases", (16, 4, 128, 128), 40),
+    ("pairs", (4, 1, 64, 48), 8), ("pairs", (4, 2, 128, 48), 13), ("pairs", (16, 4, 128, 128), 24), ("pairs", (17, 4, 128, 64), 40), ("pairs", (3, 1, 72, 0), 8),
+    ("halves", (4, 2, 64, 32), 8), ("halves", (6, 2, 64, 32), 13), ("halves", (24, 6, 64, 64), 24), ("halves", (16, 4, 128, 128), 24), ("halves", (32, 16, 64, 16), 40), ("halves", (1, 1, 4096, 4096), 40),
+    ("retention", (3, 64, 48), 8), ("retention", (8, 128, 64), 24), ("retention", (16, 128, 64), 40), ("retention", (1, 72, 0), 8), ("retention", (8, 128, 128), 8),
+    ("biases", (3, 1, 36, 20), 8), ("biases", (5, 1, 36, 20), 13), ("biases", (9, 1, 112, 128), 24), ("biases", (16, 4, 128, 128), 40),
     ("latent", (1032, 104, 64, 32), 8), ("latent", (0, 256, 32, 32), 8), ("latent", (2048, 8, 16, 0), 8)])
 def test_stored_rows(kind, sizes, per_sm):
     """Steps around the sizes from which a block takes several tokens, of rows that start on a 16-byte boundary and of rows that do not
