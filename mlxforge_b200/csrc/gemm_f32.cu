@@ -182,7 +182,8 @@ MF_API int mf_gemm_f32(const float* A, const float* W, float* C, int M, int N, i
   if (K <= 0) return MF_ERR_BAD_ARG;
   if (M <= 16) return launch<16, 32, 4, 1>(A, W, C, M, N, K, accumulate, stream);
   // The tile whose blocks go around the SMs in the least time: rounds of blocks times a block's time, which was measured at K 2,048
-  // for at most one block an SM (us); every tile adds an element's terms in the same order.
+  // for at most one block an SM (us); every tile adds an element's terms in the same order.  More blocks of a small tile fit an SM at once, which
+  // the rounds leave out; no M of 17 to 2,048 at eight widths is slower by more than 2 % than with the one tile that all had before.
   const int sms = mf_sm_count();
   if (sms <= 0) return MF_ERR_BAD_ARG;
   auto time = [&](int bm, int bn, float block) {
