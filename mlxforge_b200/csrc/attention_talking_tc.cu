@@ -1,4 +1,5 @@
-// Attention with talking heads for portions of prompts, bfloat16, on the tensor cores.
+// Attention with talking heads for portions of prompts, bfloat16, on the tensor cores (mma.sync): sizes that attention_talking_prompt.cu
+// does not take, and its short sequences.
 //
 // The formulas are those of attention_talking.cu.  The mixing of the heads' scores before the
 // softmax couples all heads of a (query, key) pair, so a block owns a tile of 16 queries of one
@@ -32,6 +33,7 @@
 // a tile: its copies as cp.async, 64 KB through the warps' own load path, were 2,700 of 10,300 cycles by a block's clock, whether or
 // not they looked pages up; the tensor copies need the products' addresses to fold (the head size as a constant), else
 // their swizzle costs what they save (234 us).  Two score tiles and two barriers instead of three were no faster (247 us).
+#include "attention_talking_prompt.cuh"
 #include "common.cuh"
 #include "tma_host.cuh"
 
@@ -161,6 +163,7 @@ struct TtArgs {
   float* part_ml;           // [rows, splits, H, 2]    maximum (in powers of two) and sum
   int* status;              // codes 91 (keys) and 92 (values): a wait for a copy ran out
   long long pool_rows;      // rows (pages x KV heads x page size) of either pool
+  int below_keys;           // > 0: sequences whose queries see as many keys are left out
 };
 
 // DIM: the head size, where keys and values come by tensor copies (64 or 128, and values of whole 64-wide spans), [head][span][32 keys]
@@ -179,6 +182,7 @@ talking_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   if ((int)blockIdx.x >= tiles) return;
   const int row0 = (tiles - 1 - (int)blockIdx.x) * TT_BM;       // the tiles with the most keys first
   const int q_start = a.seq_q_start[seq], ctx = a.seq_ctx_len[seq];
+  if (a.below_keys > 0 && talking_prompt_keys(ctx, a.window, a.chunk) >= a.below_keys) return;
   const int pos0 = ctx - q_len + row0;                       // position of the tile's first query
   const int rows = min(TT_BM, q_len - row0);
   const int* table = a.block_table + (long long)(a.table_row0 + seq) * a.bt_stride;
@@ -549,6 +553,7 @@ talking_attention_merge_kernel(const float* __restrict__ part_o, const float* __
   const int t = first_row + item / H, h = item % H;
   const float2* ml = reinterpret_cast<const float2*>(part_ml) + (long long)t * splits * H + h;
   const float* po = part_o + ((long long)t * splits * H + h) * VDIM + c;
+  if (ml[0].y == -1.f) return;          // keys of one cut: their block has written the row
   float m = -INFINITY;
   for (int z = 0; z < splits; z++) m = fmaxf(m, ml[(long long)z * H].x);
   float l = 0.f, acc[N];
@@ -867,15 +872,31 @@ MF_API int mf_attention_talking_tc(const void* q, const void* k_pool, const void
                                    int table_row0, int n_seqs, int max_q_len, int n_heads, int n_kv, int dim, int vdim,
                                    const int* block_table, int bt_stride, int page_size, long long pool_rows, float scale, float softcap,
                                    const float* talk, int window, int chunk, int splits, float* part_o, float* part_ml,
-                                   int first_row, int n_rows, int* status, cudaStream_t stream) {
+                                   int first_row, int n_rows, int min_ctx, int max_ctx, int* status,
+                                   cudaStream_t stream) {
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
   if (!mf_attention_talking_tc_ok(n_heads, n_kv, dim, vdim, page_size) || n_seqs > 65535 || splits < 0 || splits > 65535)
     return MF_ERR_BAD_ARG;
   TtArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out,
            seq_q_start, seq_q_len, seq_ctx_len, block_table, talk, table_row0, bt_stride, page_size, n_heads, n_kv, dim,
-           scale, softcap, window, chunk, splits, tt_prefill_split_tiles(window, chunk), part_o, part_ml, status, pool_rows};
+           scale, softcap, window, chunk, splits, tt_prefill_split_tiles(window, chunk), part_o, part_ml, status, pool_rows, 0};
   mf_count(MF_K_ATTN_TALKING_TC);
   int rc = MF_ERR_BAD_ARG;
+  // A sequence goes to either kernel by its own length, so that its numbers do not depend on what else is in the step; a kernel that no
+  // sequence goes to is not launched.
+  const int from = talking_prompt_from(n_heads), least = talking_prompt_keys(min_ctx, window, chunk),
+            most = talking_prompt_keys(max_ctx > 0 ? max_ctx : 1 << 30, window, chunk);
+  const bool takes = most >= from && talking_prompt_takes(n_heads, n_kv, dim, vdim, q, k_pool, v_pool, pool_rows);
+  if (takes) {
+    const int cuts = talking_prompt_cuts(splits, chunk);
+    mf_count(MF_K_ATTN_TALKING_PROMPT);
+    rc = talking_prompt_launch(q, k_pool, v_pool, out, seq_q_start, seq_q_len, seq_ctx_len, table_row0, n_seqs, max_q_len, n_heads,
+                               block_table, bt_stride, page_size, pool_rows, scale, softcap, talk, window, chunk, cuts,
+                               from, part_o, part_ml, status, stream);
+    if (rc == 0 && cuts > 1) rc = tt_merge(part_o, part_ml, out, cuts, n_heads, vdim, first_row, n_rows, stream);
+    if (rc != 0 || least >= from) return rc;
+    a.below_keys = from, a.splits = splits = 0;          // of the short ones a block walks all keys
+  }
 #define TT_CASE(VD)                                                         \
   if (vdim == VD)                                                           \
     rc = n_heads <= 8 ? tt_launch<VD, 8>(a, n_seqs, max_q_len, stream) : tt_launch<VD, 16>(a, n_seqs, max_q_len, stream);
@@ -915,7 +936,7 @@ MF_API int mf_attention_talking_decode(const void* q, const void* k_pool, const 
     return MF_ERR_BAD_ARG;
   TtArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out,
            seq_q_start, seq_q_len, seq_ctx_len, block_table, talk, 0, bt_stride, page_size, n_heads, n_kv, dim,
-           scale, softcap, window, chunk, splits, TT_SPLIT_TILES, part_o, part_ml, status, pool_rows};
+           scale, softcap, window, chunk, splits, TT_SPLIT_TILES, part_o, part_ml, status, pool_rows, 0};
   mf_count(MF_K_ATTN_TALKING_TC);
   // the values of all key heads of a split have to fit in shared memory; what is wider takes the kernel of the prompts
   if (tt_decode_smem(n_heads, n_kv, vdim) <= 200 * 1024) {

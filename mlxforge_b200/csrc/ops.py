@@ -1329,12 +1329,14 @@ def attention_talking_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Te
                          table_row0: int, max_q_len: int, block_table: torch.Tensor, page_size: int, n_heads: int,
                          n_kv: int, dim: int, vdim: int, scale: float, softcap: float, talk: Optional[torch.Tensor],
                          window: int, chunk: int, splits: int = 0, part_o: Optional[torch.Tensor] = None,
-                         part_ml: Optional[torch.Tensor] = None, first_row: int = 0) -> None:
+                         part_ml: Optional[torch.Tensor] = None, first_row: int = 0,
+                         min_ctx: int = 0, max_ctx: int = 0) -> None:
     """Talking-heads attention of prompt portions, bfloat16, on the tensor cores.  ``q`` / ``out`` are the
     whole step's rows; the three per-sequence arrays describe the sequences that start at row
     ``table_row0`` of ``block_table``.  ``splits`` > 0 (from ``attention_talking_prefill_splits``): long key
     ranges are cut across blocks and merged; the scratch holds ``T * splits * n_heads * (vdim | 2)`` floats
-    and the portions are the step's rows from ``first_row`` on."""
+    and the portions are the step's rows from ``first_row`` on.  ``min_ctx`` / ``max_ctx``: bounds
+    of the sequences' lengths, 0 where the caller does not know them."""
     _need_cuda(q, k_pool, v_pool, out, seq_q_start, seq_q_len, seq_ctx_len, block_table, talk, part_o, part_ml)
     if q.dtype != torch.bfloat16 or k_pool.dtype != torch.bfloat16:
         raise KernelError("attention_talking_tc: bfloat16 only")
@@ -1347,7 +1349,7 @@ def attention_talking_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Te
                                             table_row0, seq_q_len.shape[0], max_q_len, n_heads, n_kv, dim, vdim,
                                             block_table.data_ptr(), block_table.shape[1], page_size, k_pool.numel() // dim, scale,
                                             softcap, _ptr(talk), window, chunk, splits, _ptr(part_o), _ptr(part_ml), first_row,
-                                            T - first_row, kernel_status(q.device).data_ptr(), _stream()), "attention_talking_tc",
+                                            T - first_row, min_ctx, max_ctx, kernel_status(q.device).data_ptr(), _stream()), "attention_talking_tc",
           launches=2 if splits else 1)
 
 

@@ -144,4 +144,4 @@ def talking_paged_attention(rt, batch, q, lane, out, m: TalkingAttention) -> Non
             part_ml = rt.buffer("tattn.part_ml", (T * splits * m.n_heads * 2,), torch.float32)
         ops.attention_talking_tc(q, lane.k, lane.v, out, *portions(batch), nd, max(batch.q_len[nd:]), table, lane.page_size,
                                  m.n_heads, m.n_kv, m.dim, m.vdim, m.scale, m.softcap, m.talk, m.window, m.chunk,
-                                 splits, part_o, part_ml, nd)
+                                 splits, part_o, part_ml, nd, min(batch.ctx_len[nd:]) if getattr(batch, "ctx_len", None) else 0, batch.max_ctx)

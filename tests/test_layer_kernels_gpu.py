@@ -543,6 +543,62 @@ def test_talking_heads_portions(H, G, dim, vdim, page, lens, held, window, chunk
         at += n
 
 
+@pytest.mark.parametrize("H,page,lens,held,window,chunk,cap,talking", [
+    (16, 16, [33, 17, 250, 1], [0, 700, 0, 0], 0, 0, 30.0, True),          # both kernels in one launch, a sequence each by its own length
+    (8, 48, [70, 24], [1100, 60], 40, 0, 0.0, True),                       # every window short: the other kernel alone
+    (8, 32, [130, 100], [2000, 3], 300, 0, 20.0, True), (16, 16, [130], [2000], 1030, 0, 30.0, True),
+    (16, 16, [600], [1500], 0, 2048, 30.0, True), (8, 16, [70], [250], 0, 300, 30.0, True),       # tiles that begin inside a chunk, cut ranges
+    (16, 16, [20], [3000], 0, 0, 5.0, False), (8, 16, [300], [0], 0, 0, 0.0, False), (16, 64, [256, 192], [0, 0], 0, 0, 0.0, True)])
+def test_talking_heads_prompt_kernel(H, page, lens, held, window, chunk, cap, talking):
+    """Tiles of 16 queries and 128 keys with broken ends on all sides, pages in any order (NaN wherever no key is), keys cut at 1024, the rule
+    by a sequence's own length, with and without cap and matrix."""
+    import torch
+    from mlxforge_b200.csrc import binding, ops
+    g = torch.Generator(device="cuda").manual_seed(H + sum(lens))
+    G, D, bf, T, ctx = H // 4, 128, torch.bfloat16, sum(lens), [n + h for n, h in zip(lens, held)]
+    q = torch.randn((T, H * D), generator=g, device="cuda").to(bf)
+    talk = torch.eye(H, device="cuda") + 0.1 * torch.randn((H, H), generator=g, device="cuda") if talking else None
+    per = [-(-c // page) for c in ctx]
+    ids = np.random.default_rng(1).permutation(sum(per) + 3)[:sum(per)] if T % 2 else np.arange(sum(per))
+    kp, vp = (torch.full((sum(per) + 3, G, page, D), float("nan"), device="cuda", dtype=bf) for _ in range(2))
+    table, ks, vs, at = np.full((len(lens), max(per)), -1, np.int32), [], [], 0
+    for s, (n, c) in enumerate(zip(per, ctx)):
+        table[s, :n] = ids[at:at + n]
+        at += n
+        ks.append(torch.randn((c, G, D), generator=g, device="cuda").to(bf))
+        vs.append(torch.randn((c, G, D), generator=g, device="cuda").to(bf))
+        for b in range(n):
+            for pool, x in ((kp, ks[-1]), (vp, vs[-1])):
+                x = x[b * page:(b + 1) * page]
+                pool[int(table[s, b]), :, :x.shape[0]] = x.transpose(0, 1)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    seen = [min(c, chunk or c, window or c) for c in ctx]
+    splits = ops.attention_talking_prefill_splits(max(seen), window, chunk)
+    f = lambda n: torch.full((max(n, 1),), float("nan"), device="cuda")
+    outs = []
+    for bounds in ((min(ctx), max(ctx)), (0, 0)):
+        out, before = torch.full((T, H * D), float("nan"), device="cuda", dtype=bf), binding.kernel_launches()
+        ops.attention_talking_tc(q, kp, vp, out, i32(np.cumsum([0] + lens[:-1]).tolist()), i32(lens), i32(ctx), 0, max(lens), torch.from_numpy(table).cuda(),
+                                 page, H, G, D, D, D ** -0.5, cap, talk, window, chunk, splits, f(T * splits * H * D), f(T * splits * H * 2), 0, *bounds)
+        ops.check_kernel_status()
+        outs.append(out)
+        assert (_ran(before).get("attn_talking_prompt", 0) == 1) == (max(seen) >= (192 if H == 16 else 80))
+    assert torch.equal(*outs)
+    at = 0
+    for n, h, k, v in zip(lens, held, ks, vs):
+        i, j = torch.arange(h, h + n, device="cuda")[:, None], torch.arange(h + n, device="cuda")[None]
+        ok = (j <= i) & ((i - j < window) if window else True) & ((i // chunk == j // chunk) if chunk else True)
+        s = torch.einsum("ihd,jhd->hij", q[at:at + n].double().view(n, H, D), k.double().repeat_interleave(4, 1)) * D ** -0.5
+        s = cap * torch.tanh(s / cap) if cap else s
+        s = torch.einsum("hg,gij->hij", talk.double(), s) if talking else s
+        p = torch.softmax(s.masked_fill(~ok, -np.inf), 2)
+        vv = v.double().repeat_interleave(4, 1)
+        want, mag = torch.einsum("hij,jhd->ihd", p, vv).flatten(1), torch.einsum("hij,jhd->ihd", p, vv.abs()).flatten(1)
+        # a probability is rounded to 8 bits once, the result once more
+        assert bool(((out[at:at + n].double() - want).abs() <= 2 ** -8 * mag + 2 ** -8 * want.abs() + 1e-6).all()), n
+        at += n
+
+
 # ----------------------------------------------------------------------------- 32-bit products
 
 @pytest.mark.parametrize("M,N,K", [(300, 3001, 36), (449, 1409, 67), (150, 2900, 52), (45, 700, 20)])
