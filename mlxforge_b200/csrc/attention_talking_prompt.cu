@@ -25,9 +25,9 @@
 // sums for the merge of attention_talking_tc.cu.  Blocks with the most keys first.
 //
 // What bounds it: the instructions of the softmax warps, 1,700 a warp, tile and four queries, and their supply: the loop over tiles is larger
-// than the SM's instruction cache (a quarter of the requests miss).  16 heads, one prompt of 2,048 tokens in one chunk, with its merge: 215
-// (mma.sync, tiles of 32 keys) -> 122 us, 16,500 cycles a tile.  Measured on the way: 512 multiply-adds of pairs a pass 122, 1,024 single
-// ones 133, with the matrix in the constant bank 130 either way; four groups, a reference that moves only by 2^8 and no scores kept
+// than the SM's instruction cache.  16 heads, one prompt of 2,048 tokens in one chunk, with its merge: 215
+// (mma.sync, tiles of 32 keys) -> 113 us.  Measured on the way: the loop over a product's stages unrolled 122; so, and 1,024 single multiply-adds
+// instead of 512 of pairs 133, with the matrix in the constant bank 130; four groups, a reference that moves only by 2^8 and no scores kept
 // 125, but results 3 % further from 64 bits; cuts of 512 keys 153; products sent inside `if (lane == 0)` left the tile waiting for them
 // (1,000 cycles a stage beside warps that are busy with multiply-adds, 400 as they are sent now).
 #include <type_traits>
@@ -280,7 +280,7 @@ talking_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         }
       } else {                        // the next stage's barrier is looked at before this one's products are sent: its answer takes as long as two
         bool there = mbar_peek(full0 + 8 * st, phase);
-#pragma unroll
+#pragma unroll 1
         for (int i = 0; i < 2 * G; i++) {
           if (!there) wait(full0 + 8 * st, phase, values ? 98 : 95);
           const int next = st + 1 == RING ? 0 : st + 1;
