@@ -62,16 +62,29 @@ __device__ __forceinline__ unsigned long long smem_desc(unsigned addr) {
   d |= (unsigned long long)2 << 61;                          // 128-byte swizzle
   return d;
 }
+__device__ __forceinline__ bool mbar_peek(unsigned bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done;
+}
 __device__ __forceinline__ void umma(unsigned tmem_c, unsigned long long da, unsigned long long db, unsigned idesc,
                                      unsigned accumulate) {
   asm volatile(
-      "{\n.reg .pred p;\n"
+      "{\n.reg .pred p, e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
       ::"r"(tmem_c), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void umma_commit(unsigned bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+  asm volatile(
+      "{\n.reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(unsigned taddr, unsigned (&r)[32]) {
   asm volatile(
@@ -195,7 +208,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  const unsigned tmem_base = *tmem_slot;
+  const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);      // known to be one number a warp
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -215,29 +228,29 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      // instruction descriptor: D float32, A and B bfloat16, both K-major, N, M
-      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(BM >> 4) << 24);
-      unsigned it = 0, i = 0;
-      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, i++) {
-        const unsigned acc = i & 1, use = i >> 1;
-        if (use > 0) {
-          mbar_wait(acc_empty0 + 8 * acc, (use - 1) & 1, status, 14);     // the epilogue has drained it
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        }
-        const unsigned tmem_c = tmem_base + acc * BN;
-        for (int kt = 0; kt < n_kt; kt++, it++) {
-          const unsigned s = it % STAGES, round = it / STAGES;
-          mbar_wait(full0 + 8 * s, round & 1, status, 12);
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          const unsigned a_addr = smem_u + s * STAGE_BYTES, b_addr = a_addr + A_BYTES;
-#pragma unroll
-          for (int k4 = 0; k4 < BK / 16; k4++)
-            umma(tmem_c, smem_desc(a_addr + k4 * 32), smem_desc(b_addr + k4 * 32), idesc, (kt > 0 || k4 > 0) ? 1u : 0u);
-          umma_commit(empty0 + 8 * s);          // the stage is free once these products have read it
-        }
-        umma_commit(acc_full0 + 8 * acc);        // this tile's accumulator is complete
+    // instruction descriptor: D float32, A and B bfloat16, both K-major, N, M
+    const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(BM >> 4) << 24);
+    unsigned it = 0, i = 0;
+    bool there = false;
+    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, i++) {
+      const unsigned acc = i & 1, use = i >> 1;
+      if (use > 0) {
+        mbar_wait(acc_empty0 + 8 * acc, (use - 1) & 1, status, 14);     // the epilogue has drained it
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       }
+      const unsigned tmem_c = tmem_base + acc * BN;
+      for (int kt = 0; kt < n_kt; kt++, it++) {
+        const unsigned s = it % STAGES, round = it / STAGES;
+        if (!there) mbar_wait(full0 + 8 * s, round & 1, status, 12);
+        there = mbar_peek(full0 + 8 * ((it + 1) % STAGES), (it + 1) / STAGES & 1);      // the answer comes while the products are sent
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const unsigned a_addr = smem_u + s * STAGE_BYTES, b_addr = a_addr + A_BYTES;
+#pragma unroll
+        for (int k4 = 0; k4 < BK / 16; k4++)
+          umma(tmem_c, smem_desc(a_addr + k4 * 32), smem_desc(b_addr + k4 * 32), idesc, (kt > 0 || k4 > 0) ? 1u : 0u);
+        umma_commit(empty0 + 8 * s);          // the stage is free once these products have read it
+      }
+      umma_commit(acc_full0 + 8 * acc);        // this tile's accumulator is complete
     }
   } else {
     // ------------------------------------------------------------ epilogue (4 warps, 32 rows each)
