@@ -599,6 +599,37 @@ def test_talking_heads_prompt_kernel(H, page, lens, held, window, chunk, cap, ta
         at += n
 
 
+# ----------------------------------------------------------------------------- latents: rotated query parts
+
+@pytest.mark.parametrize("T,heads,dim,rot,rank,rot_dims,pairs,extra", [
+    (1, 3, 64, 32, 192, 32, False, 0), (9, 16, 64, 32, 128, 32, False, 8), (17, 5, 16, 64, 24, 32, False, 0), (40, 2, 128, 64, 512, 64, True, 0),
+    (7, 4, 8, 24, 16, 8, True, 16), (12, 3, 64, 24, 64, 24, False, 0), (12, 3, 60, 32, 64, 32, False, 0), (5, 2, 64, 32, 64, 0, False, 0)])
+def test_latent_query_pieces(T, heads, dim, rot, rank, rot_dims, pairs, extra):
+    """Whole pieces in halves and in pairs, parts that pass unturned, broken blocks of tokens, and sizes that are no whole pieces: the rotation
+    in 64 bits to a rounding of bfloat16 of the pair's size, what is not rotated to the bit."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(T + rot)
+    ld = heads * (dim + rot) + extra
+    q = torch.randn((T, ld), generator=g, device="cuda").to(torch.bfloat16)
+    pos = torch.randint(0, 500, (T,), generator=g, device="cuda", dtype=torch.int32)
+    half = rot_dims // 2
+    inv = 100.0 ** (-torch.arange(max(half, 1), device="cuda", dtype=torch.float32) / max(half, 1))
+    out = torch.full((T, heads * (rank + rot)), 7.0, device="cuda", dtype=torch.bfloat16)
+    ops.latent_query(q, heads, dim, rot, rank, pos, inv, None, out, ld, pairs, rot_dims, 1.25)
+    got, src = out.view(T, heads, rank + rot), q[:, :heads * (dim + rot)].view(T, heads, dim + rot)[..., dim:]
+    assert bool((got[..., :rank] == 7).all()) and torch.equal(got[..., rank + rot_dims:], src[..., rot_dims:])
+    x = src[..., :rot_dims].double()
+    u, v = (x[..., 0::2], x[..., 1::2]) if pairs else (x[..., :half], x[..., half:])
+    a = (pos[:, None].float() * inv[None, :half]).double()[:, None]
+    c, s = torch.cos(a) * 1.25, torch.sin(a) * 1.25
+    w = got[..., rank:rank + rot_dims].double()
+    gu, gv = (w[..., 0::2], w[..., 1::2]) if pairs else (w[..., :half], w[..., half:])
+    size = 1.25 * (u.square() + v.square()).sqrt()
+    # one rounding to 8 bits; a few of 24 before it
+    assert bool(((gu - (u * c - v * s)).abs() <= 2.0 ** -8 * size).all()) and bool(((gv - (v * c + u * s)).abs() <= 2.0 ** -8 * size).all())
+
+
 # ----------------------------------------------------------------------------- 32-bit products
 
 @pytest.mark.parametrize("M,N,K", [(300, 3001, 36), (449, 1409, 67), (150, 2900, 52), (45, 700, 20)])
