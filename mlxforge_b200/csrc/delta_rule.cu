@@ -89,7 +89,7 @@ delta_prepare_kernel(const float* __restrict__ proj, int ld, const float* __rest
 // The same for heads of 64 or 128 channels, up to four taps and rows in whole 16-byte pieces: a warp a head (queries, keys,
 // values; a row of blocks for beta and the low-rank columns) over a run of RUN tokens, D/32 neighbouring channels a lane, every
 // input read once.  The kernel above reads each input once per tap, a number at a time, and the weights with a stride of
-// the taps: 2,048 tokens of 16 heads of 128 took 91 us, now 36 (100 MB).  With `moves` every sequence brings one token, so
+// the taps: 2,048 tokens of 16 heads of 128 took 91 us, now 27 (100 MB, 16 us at the copy rate).  With `moves` every sequence brings one token, so
 // a warp is the only reader of its channels' history and moves it on itself.
 template <int N>
 __device__ __forceinline__ void dp_get(float (&x)[N], const float* p) {
@@ -119,10 +119,10 @@ struct DeltaPrepare {
   int T, C, n_heads, n_kv, dim, vdim, moves;
 };
 
-// one head's channels c .. c + CH of a lane; `unit` 0: values, 1: keys, 2: queries
-template <int CH, int TAPS, int RUN>
-__device__ __forceinline__ void delta_prepare_head(const DeltaPrepare& a, int c, int unit, int t0) {
-  float w[CH][TAPS], x[RUN][CH], past[TAPS][CH];       // past[j]: the input taps-1-j tokens back
+// one head's channels c .. c + CH of a lane, token t; `unit` 0: values, 1: keys, 2: queries
+template <int CH, int TAPS>
+__device__ __forceinline__ void delta_prepare_head(const DeltaPrepare& a, int c, int unit, int t) {
+  float w[CH][TAPS], past[TAPS][CH];       // past[j]: the input taps-1-j tokens back
 #pragma unroll
   for (int i = 0; i < CH; i++) {
     if constexpr (TAPS == 4) {
@@ -132,79 +132,158 @@ __device__ __forceinline__ void delta_prepare_head(const DeltaPrepare& a, int c,
       for (int j = 0; j < TAPS; j++) w[i][j] = a.conv_w[(long long)(c + i) * TAPS + j];
     }
   }
+  dp_get(past[TAPS - 1], a.proj + (long long)t * a.ld + c);
+  const int seq = a.seq_of_token[t], rel = t - a.seq_q_start[seq];
+  float* tail = a.state + (long long)a.slots[seq] * a.state_stride + a.conv_off + c;         // [(taps-1), C]
 #pragma unroll
-  for (int r = 0; r < RUN; r++)
-    if (t0 + r < a.T) dp_get(x[r], a.proj + (long long)(t0 + r) * a.ld + c);
+  for (int j = 0; j < TAPS - 1; j++) {
+    const int at = rel - (TAPS - 1) + j;
+    dp_get(past[j], at >= 0 ? a.proj + (long long)(t - (TAPS - 1) + j) * a.ld + c : tail + (long long)(at + TAPS - 1) * a.C);
+  }
+  float y[CH], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < CH; i++) {
+    float v = 0.f;
+#pragma unroll
+    for (int j = 0; j < TAPS; j++) v = fmaf(w[i][j], past[j][i], v);
+    y[i] = v * dr_sigmoid(v);
+    ss = fmaf(y[i], y[i], ss);
+  }
+  if (unit) {
+    ss = warp_sum(ss);
+    float inv = 1.0f / sqrtf(ss + 1e-6f);
+    if (unit == 2) inv *= 1.0f / sqrtf((float)a.dim);
+#pragma unroll
+    for (int i = 0; i < CH; i++) y[i] *= inv;
+  }
+  dp_put(a.qkv_out + (long long)t * a.C + c, y);
+  if (a.moves) {
+#pragma unroll
+    for (int j = 0; j < TAPS - 1; j++) dp_put(tail + (long long)j * a.C, past[j + 1]);
+  }
+}
+
+// The same for eight tokens: one after another they are a chain of loads of their sequence, five steps of a sum over the warp, a root and
+// divisions.  Here a run inside one sequence asks for it once, and the eight sums of squares go over the warp together: a step halves the
+// tokens that a lane has, the pairs and their order being warp_sum's, so that a token's bits are those of a run of one; then a lane has one
+// token's root: 36 -> 31 us; 27 with the row of blocks for the other columns first, where it is no longer the end of the launch, and its
+// tokens' loads together.  The rest is instructions, two thirds of them exponentials and divisions, over loads from L2.
+template <int CH, int TAPS>
+__device__ __forceinline__ void delta_prepare_eight(const DeltaPrepare& a, int c, int unit, int t0) {
+  constexpr int RUN = 8;
+  const int n = min(RUN, a.T - t0), lane = threadIdx.x & 31;
+  float w[CH][TAPS], x[RUN][CH], past[TAPS][CH];       // past[j]: the input taps-1-j tokens back
 #pragma unroll
   for (int r = 0; r < RUN; r++) {
-    const int t = t0 + r;
-    if (t >= a.T) break;
-    const int seq = a.seq_of_token[t], rel = t - a.seq_q_start[seq];
-    float* tail = a.state + (long long)a.slots[seq] * a.state_stride + a.conv_off + c;         // [(taps-1), C]
-    if (TAPS > 1 && (r == 0 || rel == 0)) {            // a run's or a sequence's first token: fetch what stands before it
+    if (r < n) dp_get(x[r], a.proj + (long long)(t0 + r) * a.ld + c);
+    else
 #pragma unroll
-      for (int j = 0; j < TAPS - 1; j++) {
-        const int at = rel - (TAPS - 1) + j;
-        dp_get(past[j], at >= 0 ? a.proj + (long long)(t - (TAPS - 1) + j) * a.ld + c : tail + (long long)(at + TAPS - 1) * a.C);
-      }
+      for (int i = 0; i < CH; i++) x[r][i] = 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < CH; i++) {
+    if constexpr (TAPS == 4) {
+      dp_get(w[i], a.conv_w + (long long)(c + i) * TAPS);
+    } else {
+#pragma unroll
+      for (int j = 0; j < TAPS; j++) w[i][j] = a.conv_w[(long long)(c + i) * TAPS + j];
     }
-    float y[CH], ss = 0.f;
+  }
+  auto before = [&](int t, int seq, int rel) {         // what stands before token t
+    const float* tail = a.state + (long long)a.slots[seq] * a.state_stride + a.conv_off + c;         // [(taps-1), C]
+#pragma unroll
+    for (int j = 0; j < TAPS - 1; j++) {
+      const int at = rel - (TAPS - 1) + j;
+      dp_get(past[j], at >= 0 ? a.proj + (long long)(t - (TAPS - 1) + j) * a.ld + c : tail + (long long)(at + TAPS - 1) * a.C);
+    }
+  };
+  const int seq0 = a.seq_of_token[t0];
+  const bool one = seq0 == a.seq_of_token[t0 + n - 1];
+  if (TAPS > 1) before(t0, seq0, t0 - a.seq_q_start[seq0]);
+  float ss[RUN];
+#pragma unroll
+  for (int r = 0; r < RUN; r++) {
+    if (TAPS > 1 && r > 0 && !one && r < n) {
+      const int seq = a.seq_of_token[t0 + r];
+      if (a.seq_q_start[seq] == t0 + r) before(t0 + r, seq, 0);
+    }
+    ss[r] = 0.f;
 #pragma unroll
     for (int i = 0; i < CH; i++) {
       past[TAPS - 1][i] = x[r][i];
       float v = 0.f;
 #pragma unroll
       for (int j = 0; j < TAPS; j++) v = fmaf(w[i][j], past[j][i], v);
-      y[i] = v * dr_sigmoid(v);
-      ss = fmaf(y[i], y[i], ss);
-    }
-    if (unit) {
-      ss = warp_sum(ss);
-      float inv = 1.0f / sqrtf(ss + 1e-6f);
-      if (unit == 2) inv *= 1.0f / sqrtf((float)a.dim);
+      x[r][i] = v * dr_sigmoid(v);
+      ss[r] = fmaf(x[r][i], x[r][i], ss[r]);
 #pragma unroll
-      for (int i = 0; i < CH; i++) y[i] *= inv;
-    }
-    dp_put(a.qkv_out + (long long)t * a.C + c, y);
-#pragma unroll
-    for (int j = 0; j < TAPS - 1; j++) {
-#pragma unroll
-      for (int i = 0; i < CH; i++) past[j][i] = past[j + 1][i];
-      if (RUN == 1 && a.moves) dp_put(tail + (long long)j * a.C, past[j]);
+      for (int j = 0; j < TAPS - 1; j++) past[j][i] = past[j + 1][i];
     }
   }
+  if (unit) {
+#pragma unroll
+    for (int half = 4; half; half >>= 1) {
+      const bool upper = lane & (half * 4);
+#pragma unroll
+      for (int r = 0; r < half; r++)
+        ss[r] = (upper ? ss[r + half] : ss[r]) + __shfl_xor_sync(0xffffffffu, upper ? ss[r] : ss[r + half], half * 4);
+    }
+    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 2);
+    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+    float inv = 1.0f / sqrtf(ss[0] + 1e-6f);
+    if (unit == 2) inv *= 1.0f / sqrtf((float)a.dim);
+#pragma unroll
+    for (int r = 0; r < RUN; r++) {
+      const float by = __shfl_sync(0xffffffffu, inv, r * 4);
+#pragma unroll
+      for (int i = 0; i < CH; i++) x[r][i] *= by;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < RUN; r++)
+    if (r < n) dp_put(a.qkv_out + (long long)(t0 + r) * a.C + c, x[r]);
 }
 
 template <typename TL, int TAPS, int RUN>
 __global__ void __launch_bounds__(256, RUN == 1 ? 4 : 3)
 delta_prepare_heads_kernel(const DeltaPrepare a, TL* __restrict__ low, int n_low) {
-  const int job = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, t0 = blockIdx.x * RUN;
+  const int job = ((int)blockIdx.y - 1) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, t0 = blockIdx.x * RUN;
   const int qk = 2 * a.n_kv;
   pdl_launch();
   pdl_wait();
-  if (blockIdx.y == gridDim.y - 1) {       // the last row of blocks: beta and the low-rank columns
+  if (blockIdx.y == 0) {      // the first row of blocks: beta and the low-rank columns, the run's tokens asked for together
     const int cols = a.n_heads + n_low;
-    for (int i = threadIdx.x; i < RUN * cols; i += 256) {
-      const int t = t0 + i / cols, j = i % cols;
-      if (t >= a.T) break;
-      const float x = a.proj[(long long)t * a.ld + a.C + j];
-      if (j < a.n_heads) a.beta_out[(long long)t * a.n_heads + j] = dr_sigmoid(x);
-      else low[(long long)t * n_low + j - a.n_heads] = from_f32<TL>(x);
+    for (int j = threadIdx.x; j < cols; j += 256) {
+      float x[RUN];
+#pragma unroll
+      for (int r = 0; r < RUN; r++) x[r] = t0 + r < a.T ? a.proj[(long long)(t0 + r) * a.ld + a.C + j] : 0.f;
+#pragma unroll
+      for (int r = 0; r < RUN; r++) {
+        const int t = t0 + r;
+        if (t >= a.T) break;
+        if (j < a.n_heads) a.beta_out[(long long)t * a.n_heads + j] = dr_sigmoid(x[r]);
+        else low[(long long)t * n_low + j - a.n_heads] = from_f32<TL>(x[r]);
+      }
     }
     return;
   }
   if (job < qk + a.n_heads) {
     const int unit = job < a.n_kv ? 2 : job < qk ? 1 : 0;
     const int d = unit ? a.dim : a.vdim, c0 = unit ? job * a.dim : qk * a.dim + (job - qk) * a.vdim;
-    if (d == 128) delta_prepare_head<4, TAPS, RUN>(a, c0 + lane * 4, unit, t0);
-    else delta_prepare_head<2, TAPS, RUN>(a, c0 + lane * 2, unit, t0);
+    if constexpr (RUN == 8) {
+      if (d == 128) delta_prepare_eight<4, TAPS>(a, c0 + lane * 4, unit, t0);
+      else delta_prepare_eight<2, TAPS>(a, c0 + lane * 2, unit, t0);
+    } else {
+      if (d == 128) delta_prepare_head<4, TAPS>(a, c0 + lane * 4, unit, t0);
+      else delta_prepare_head<2, TAPS>(a, c0 + lane * 2, unit, t0);
+    }
   }
 }
 
 template <typename TL, int TAPS>
 static int delta_prepare_heads(const DeltaPrepare& a, void* low, int n_low, cudaStream_t stream) {
   const unsigned rows = (unsigned)((2 * a.n_kv + a.n_heads + 7) / 8 + 1);
-  // runs of eight from 256 tokens on (36 us at 2,048; runs of four 39); one token a warp below, where blocks are few
+  // runs of eight from 256 tokens on (27 us at 2,048; sixteen and thirty-two 30: fewer blocks); one token a warp below, where blocks are few
   if (a.T >= 256)
     delta_prepare_heads_kernel<TL, TAPS, 8><<<dim3((a.T + 7) / 8, rows), 256, 0, stream>>>(a, (TL*)low, n_low);
   else

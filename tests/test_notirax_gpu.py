@@ -683,6 +683,40 @@ def test_delta_prepare_by_heads(lens, heads, n_kv, dim, vdim, taps):
     assert np.array_equal(low.cpu().numpy(), proj[:, C + heads:C + heads + n_low])
 
 
+@pytest.mark.parametrize("dim,vdim,taps", [(128, 128, 4), (64, 128, 3), (128, 64, 2), (64, 64, 1)])
+def test_delta_prepare_in_runs_keeps_the_bits_of_single_tokens(dim, vdim, taps):
+    """A step long enough for runs of eight tokens, its sequences' borders at every place of a run, against the same
+    sequences a step each, short enough for one token at a time: the same sums in the same order, so the same bits."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    lens, heads, n_kv, n_low = [1, 2, 3, 4, 5, 6, 7, 9, 10, 220, 1, 200], 3, 1, 300
+    gen = torch.Generator(device="cuda").manual_seed(dim + taps)
+    T, C = sum(lens), 2 * n_kv * dim + heads * vdim
+    ld = C + heads + n_low + (-(C + heads + n_low) % 4)
+    proj, w = torch.randn((T, ld), generator=gen, device="cuda"), torch.randn((C, taps), generator=gen, device="cuda")
+    state = torch.randn((len(lens), 8 + (taps - 1) * C), generator=gen, device="cuda")
+    i32 = lambda a: dev(np.asarray(a, np.int32))
+
+    def prepare(rows, own, st):
+        n = sum(own)
+        batch = SimpleNamespace(q_len=own, n_seqs=len(own), positions=i32(np.zeros(n)), slots=i32(np.arange(len(own))),
+                                seq_of_token=i32(np.repeat(np.arange(len(own)), own)), seq_q_start=i32(np.cumsum([0] + own[:-1])),
+                                seq_q_len=i32(own))
+        out = [torch.full((n, m), float("nan"), device="cuda", dtype=t)
+               for m, t in ((C, torch.float32), (heads, torch.float32), (n_low, torch.bfloat16))]
+        ops.delta_prepare(rows, w, taps, st, 8, batch, *out, heads, n_kv, dim, vdim)
+        return out
+
+    st = state.clone()
+    whole, at = prepare(proj, lens, st), 0
+    for i, n in enumerate(lens):
+        own = state[i:i + 1].clone()
+        for a, b in zip(whole, prepare(proj[at:at + n], [n], own)):
+            assert torch.equal(a[at:at + n], b)
+        assert torch.equal(st[i:i + 1], own)
+        at += n
+
+
 @pytest.mark.parametrize("heads,kv,dim,vdim,chunk,window,cap,seqs", [
     (16, 4, 128, 128, 2048, 0, 30.0, [(17, 1100), (1, 700), (2, 18)]),       # key ranges cut at 512, a tile of one query
     (12, 3, 64, 96, 0, 600, 0.0, [(40, 900), (16, 16)]),                     # a window cut at 512; heads that are no power of two
