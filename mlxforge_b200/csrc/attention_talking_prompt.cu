@@ -26,7 +26,7 @@
 //
 // What bounds it: the instructions of the softmax warps, 1,700 a warp, tile and four queries, and their supply: the loop over tiles is larger
 // than the SM's instruction cache.  16 heads, one prompt of 2,048 tokens in one chunk, with its merge: 215
-// (mma.sync, tiles of 32 keys) -> 113 us.  Measured on the way: the loop over a product's stages unrolled 122; so, and 1,024 single multiply-adds
+// (mma.sync, tiles of 32 keys) -> 111 us.  Measured on the way, at 113 us: the loop over a product's stages unrolled 122; so, and 1,024 single multiply-adds
 // instead of 512 of pairs 133, with the matrix in the constant bank 130; four groups, a reference that moves only by 2^8 and no scores kept
 // 125, but results 3 % further from 64 bits; cuts of 512 keys 153; products sent inside `if (lane == 0)` left the tile waiting for them
 // (1,000 cycles a stage beside warps that are busy with multiply-adds, 400 as they are sent now).
@@ -174,10 +174,10 @@ talking_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == 1) tmem_alloc(tmem_slot, COLS);
-  // No stage ever holds bits that could be no number: granules that are not fetched leave what was there, lines of fetched ones that no
-  // query sees are cleared behind the copy, and the start is zero.
-  for (int i = tid; i < RING * STAGE / 16; i += THREADS) *reinterpret_cast<uint4*>(smem + (ring_u - q_u) + i * 16) = make_uint4(0, 0, 0, 0);
-  fence_proxy();
+  // Lines of a stage that no query sees can hold anything: the page's bits behind a sequence's end, or, where a granule was not fetched,
+  // keys or values of any key head that stood there before.  Of keys they are scores that the mask takes away.  Of values, whose weight of
+  // zero would not take away what is not finite, granules that were not fetched are no part of the product and the lines of fetched ones
+  // are cleared behind the copy.
   __syncthreads();
 
   // a part of the launch's 168 registers a thread goes to the softmax warps: 128 x 56 + 256 x 224 = 384 x 168
@@ -250,32 +250,42 @@ talking_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
       constexpr bool values = decltype(what)::value;
       constexpr uint32_t desc = bf16_idesc(128, 64, values, values), step = (values ? 2048 : 32) >> 4;
       const int key0 = (kt0 + n) * KT;
-      const bool ragged = key0 < lo0 || key0 + KT - 1 > pos_last;
+      const bool ragged = values && (key0 < lo0 || key0 + KT - 1 > pos_last);
+      auto operands = [&](int part, int kv, unsigned long long& da, unsigned long long& db) {
+        da = ring_d + (uint32_t)(st * (STAGE >> 4)), db = (values ? p_d : q_d) + (uint32_t)(kv * (STAGE >> 4) + part * (8192 >> 4));
+        return tmem + (values ? O_COL : 0) + kv * 64;
+      };
       auto stage = [&](int part, int kv) {
         fence_after();
-        const unsigned long long da = ring_d + (uint32_t)(st * (STAGE >> 4)), db = (values ? p_d : q_d) + (uint32_t)(kv * (STAGE >> 4) + part * (8192 >> 4));
-        const uint32_t d = tmem + (values ? O_COL : 0) + kv * 64;
+        unsigned long long da, db;
+        const uint32_t d = operands(part, kv, da, db);
         umma(d, da, db, desc, part > 0 ? 1u : (values && n > 0 ? 1u : 0u));
 #pragma unroll
         for (uint32_t k = 1; k < 4; k++) umma(d, da + k * step, db + k * step, desc, 1u);
         umma_commit(empty0 + 8 * st);
       };
-      if (ragged) {                   // lines of fetched granules that no query sees are cleared
+      if (ragged) {                   // the granules that were fetched, without their lines that no query sees
+        const int first = max(0, (lo0 - key0) >> 4), last = min(7, (pos_last - key0) >> 4);
 #pragma unroll 1
         for (int i = 0; i < 2 * G; i++) {
-          wait(full0 + 8 * st, phase, values ? 98 : 95);
+          wait(full0 + 8 * st, phase, 98);
+          const int part = i / G;
 #pragma unroll 1
           for (int at = lane; at < 32 * 8; at += 32) {
-            const int r = at >> 3, key = r < 16 ? (lo0 & ~15) + r : (pos_last & ~15) + r - 16;
-            const int line = key - key0 - (values ? i / G * 64 : 0);
-            if ((r < 16 ? key >= lo0 : key <= pos_last) || line < 0 || line >= (values ? 64 : 128)) continue;
+            const int r = at >> 3, key = r < 16 ? (lo0 & ~15) + r : (pos_last & ~15) + r - 16, line = key - key0 - part * 64;
+            if ((r < 16 ? key >= lo0 : key <= pos_last) || line < 0 || line >= 64) continue;
             uint4* const to = reinterpret_cast<uint4*>(smem + (ring_u - q_u) + st * STAGE + line * 128 + (at & 7) * 16);
-            to[0] = make_uint4(0, 0, 0, 0);
-            if (values) to[8192 / 16] = make_uint4(0, 0, 0, 0);
+            to[0] = to[8192 / 16] = make_uint4(0, 0, 0, 0);
           }
           fence_proxy();
           __syncwarp();
-          stage(i / G, i % G);
+          fence_after();
+          unsigned long long da, db;
+          const uint32_t d = operands(part, i % G, da, db);
+#pragma unroll 1
+          for (int k = max(0, first - part * 4); k <= min(3, last - part * 4); k++)
+            umma(d, da + k * step, db + k * step, desc, n > 0 || part * 4 + k > first ? 1u : 0u);
+          umma_commit(empty0 + 8 * st);
           if (++st == RING) st = 0, phase ^= 1;
         }
       } else {                        // the next stage's barrier is looked at before this one's products are sent: its answer takes as long as two

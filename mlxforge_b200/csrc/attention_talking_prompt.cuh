@@ -9,7 +9,7 @@ __host__ __device__ inline int talking_prompt_keys(int ctx, int window, int chun
 }
 // From how many of them the kernel is the faster one (layer's attention, us, one portion, this kernel / the one of attention_talking_tc.cu):
 // 16 heads, 128 keys 26.8 / 28.8 where they fill its one tile of keys, 150 keys 37.0 / 33.6, 200 keys 37.0 / 39.1, 300 keys 47 / 56, 2,048 keys
-// 113 / 215; 8 heads, 64 keys 16.1 / 15.6, 100 keys 16.5 / 19.9, 300 keys 25 / 45.
+// 111 / 215; 8 heads, 64 keys 16.1 / 15.6, 100 keys 16.5 / 19.9, 300 keys 25 / 45.
 inline int talking_prompt_from(int n_heads) { return n_heads == 16 ? 192 : 80; }
 
 // Whether it takes these sizes (what else mf_attention_talking_tc takes has been checked).

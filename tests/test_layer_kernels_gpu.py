@@ -599,6 +599,75 @@ def test_talking_heads_prompt_kernel(H, page, lens, held, window, chunk, cap, ta
         at += n
 
 
+@pytest.mark.parametrize("H,lens,held,window,chunk,cap,talking", [
+    (16, 300, 0, 0, 0, 30.0, True), (16, 300, 0, 0, 0, 0.0, False), (8, 300, 0, 0, 0, 30.0, False), (8, 331, 5, 0, 0, 0.0, True),
+    (16, 90, 1000, 250, 0, 20.0, True), (8, 90, 1000, 250, 0, 0.0, False), (16, 60, 1490, 0, 2048, 0.0, False), (8, 200, 420, 0, 512, 30.0, True)])
+def test_talking_heads_prompt_kernel_keeps_what_is_not_finite_apart(H, lens, held, window, chunk, cap, talking):
+    """One number of a key or a value of one key head NaN or infinite, at places over all of a tile of 128 and at the ends of the range: the rows
+    that do not see it keep their bits (of a value up to the own 16 positions and its own channel, as the weights of a tile are one product),
+    values never pass to another key head's query heads, keys only through a matrix; an infinite key under a cap is what 64 bits say."""
+    import torch
+    from mlxforge_b200.csrc import binding, ops
+    g = torch.Generator(device="cuda").manual_seed(H + lens)
+    G, D, bf, ctx, page = H // 4, 128, torch.bfloat16, lens + held, 16
+    n = -(-ctx // page)
+    q = torch.randn((lens, H * D), generator=g, device="cuda").to(bf)
+    talk = torch.eye(H, device="cuda") + 0.1 * torch.randn((H, H), generator=g, device="cuda") if talking else None
+    pools = [torch.randn((n, G, page, D), generator=g, device="cuda").to(bf) for _ in range(2)]
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    table = torch.arange(n, dtype=torch.int32, device="cuda")[None]
+    splits = ops.attention_talking_prefill_splits(min(ctx, chunk or ctx, window or ctx), window, chunk)
+
+    def run(kp, vp):
+        f = lambda m: torch.full((max(m, 1),), float("nan"), device="cuda")
+        out, before = torch.full((lens, H * D), 7.0, device="cuda", dtype=bf), binding.kernel_launches()
+        ops.attention_talking_tc(q, kp, vp, out, i32([0]), i32([lens]), i32([ctx]), 0, lens, table, page, H, G, D, D, D ** -0.5, cap, talk, window, chunk,
+                                 splits, f(lens * splits * H * D), f(lens * splits * H * 2), 0, ctx, ctx)
+        ops.check_kernel_status()
+        assert _ran(before)["attn_talking_prompt"] == 1
+        return out.view(lens, H, D)
+
+    pos = torch.arange(held, ctx, device="cuda")
+    first = max(0, held - window + 1) if window else held // chunk * chunk if chunk else 0
+    at = {first, first + 1, first + 17, held, ctx - 1, ctx - 2, ctx - 17} | {t for t in range(first, ctx, 37)} | {t for t in range(held // 128 * 128, ctx, 64)}
+    bits = lambda x: x.view(torch.int16)
+    clean, same = run(*pools), lambda a, b: torch.equal(bits(a), bits(b))
+    assert bool(clean.isfinite().all())
+    for i, t in enumerate(sorted(t for t in at if first <= t < ctx)):
+        kv = i % G
+        own = slice(4 * kv, 4 * kv + 4)
+        other = [h for h in range(H) if h // 4 != kv]
+        sees = (pos >= t) & ((pos - t < window) if window else True) & ((pos // chunk == t // chunk) if chunk else True)
+        # rows of a tile that holds a row which sees it
+        near = torch.isin(pos // 16, pos[sees].unique() // 16) & ~sees
+        for bad in (float("nan"), float("inf"), float("-inf")):
+            kp, vp = (x.clone() for x in pools)
+            vp[t // page, kv, t % page, 5] = bad
+            out = run(pools[0], vp)
+            assert same(out[:, other], clean[:, other]), (t, bad)
+            assert same(out[..., [c for c in range(D) if c != 5]], clean[..., [c for c in range(D) if c != 5]]), (t, bad)
+            assert same(out[~(sees | near)], clean[~(sees | near)]), (t, bad)
+            assert not bool(out[sees][:, own, 5].isfinite().any()), (t, bad)
+            kp[t // page, kv, t % page, 9] = bad
+            out = run(kp, pools[1])
+            assert same(out[~sees], clean[~sees]), (t, bad)
+            if not talking:
+                assert same(out[:, other], clean[:, other]), (t, bad)
+            if bad != bad:
+                assert not bool(out[sees][:, own].isfinite().any()), t
+            elif cap:
+                k = kp.transpose(1, 2).reshape(n * page, G, D)[:ctx].double().repeat_interleave(4, 1)
+                v = pools[1].transpose(1, 2).reshape(n * page, G, D)[:ctx].double().repeat_interleave(4, 1)
+                key = torch.arange(ctx, device="cuda")[None]
+                ok = (key <= pos[:, None]) & ((pos[:, None] - key < window) if window else True) & ((pos[:, None] // chunk == key // chunk) if chunk else True)
+                s = cap * torch.tanh(torch.einsum("ihd,jhd->hij", q.double().view(lens, H, D), k) * D ** -0.5 / cap)
+                s = torch.einsum("hg,gij->hij", talk.double(), s) if talking else s
+                p = torch.softmax(s.masked_fill(~ok, -np.inf), 2)
+                want, mag = torch.einsum("hij,jhd->ihd", p, v), torch.einsum("hij,jhd->ihd", p, v.abs())
+                # a probability is rounded to 8 bits once, the result once more
+                assert bool(((out.double() - want).abs() <= 2 ** -8 * mag + 2 ** -8 * want.abs() + 1e-6).all()), (t, bad)
+
+
 # ----------------------------------------------------------------------------- latents: rotated query parts
 
 @pytest.mark.parametrize("T,heads,dim,rot,rank,rot_dims,pairs,extra", [
