@@ -279,7 +279,9 @@ retention_chunk_out_kernel(const float* __restrict__ qk, const float* __restrict
 }
 
 // ---------------------------------------------------------------------------- the same on the tensor cores
-// two 32-bit numbers as three pairs of bfloat16 whose sums they are
+// two 32-bit numbers as three pairs of bfloat16 whose sums they are.  Of what is infinite, or larger than bfloat16's largest, the first is an
+// infinity and the others are no numbers; a bfloat16 infinity meets pieces of either sign, or zeros.  Every product such a number is in
+// comes out as something that is not finite, so the kernels below work out those results again in IEEE 32-bit, and no others.
 __device__ __forceinline__ void pieces(float x, float y, uint32_t (&p)[3]) {
 #pragma unroll
   for (int i = 0; i < 3; i++) {
@@ -330,6 +332,7 @@ __device__ __forceinline__ void value_operands(uint32_t (&b)[4], const __nv_bflo
   const uint32_t at = (uint32_t)__cvta_generic_to_shared(row + (lane & 15) * ld + (lane >> 4) * 8);
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(at));
 }
+__device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) <= 3.402823466e38f); }
 template <int V, int THREADS>
 __device__ __forceinline__ void copy_values(__nv_bfloat16* vs, const __nv_bfloat16* v, long long v_ld, int n) {
 #pragma unroll 4
@@ -343,6 +346,20 @@ __device__ __forceinline__ void copy_values(__nv_bfloat16* vs, const __nv_bfloat
 // 20 us on the CUDA cores (half of their rate).
 template <int D, int V>
 constexpr size_t local_mma_smem() { return (size_t)L * (D + 4) * 4 + (size_t)L * (V + 8) * 2; }
+
+// a thread's results that are not finite: of a step of eight columns two neighbours, and those eight rows further
+template <int D, int V>
+__device__ __noinline__ void local_again(float* out, const float* ks, const __nv_bfloat16* vs, int n) {
+#pragma unroll 1
+  for (int i = 0; i < V / 2; i++) {
+    const int row = (i & 2) * 4, col = i / 4 * 8 + (i & 1);
+    if (!not_finite(out[row * V + col])) continue;
+    float x = 0.f;
+#pragma unroll 1
+    for (int s = 0; s < n; s++) x = fmaf(ks[s * (D + 4) + row], __bfloat162float(vs[s * (V + 8) + col]), x);
+    out[row * V + col] = x;
+  }
+}
 
 template <int D, int V>
 __global__ void __launch_bounds__(2 * D, 2)
@@ -390,11 +407,15 @@ retention_local_mma_kernel(const float* __restrict__ qk, const __nv_bfloat16* __
     }
   }
   float* out = states + ((long long)blockIdx.x * n_heads + h) * D * V + (warp * 16 + r0) * V + c2;
+  bool again = false;
 #pragma unroll
   for (int j = 0; j < V / 8; j++) {
     *reinterpret_cast<float2*>(out + j * 8) = make_float2(acc[j][0], acc[j][1]);
     *reinterpret_cast<float2*>(out + 8 * V + j * 8) = make_float2(acc[j][2], acc[j][3]);
+#pragma unroll
+    for (int e = 0; e < 4; e++) again |= not_finite(acc[j][e]);
   }
+  if (again) local_again<D, V>(out, ks + warp * 16 + r0, vs + c2, n);
 }
 
 // A block of 2 V threads per (chunk, head): P = q k^T under the decays, then q S_0 and P v; a warp has 16 tokens and 64 columns.  q, k, the
@@ -404,6 +425,34 @@ template <int D, int V>
 constexpr size_t out_mma_smem() {
   const int b = D + 8 > V + 4 ? D + 8 : V + 4;
   return (size_t)L * (D + 8 + b + L + 8) * 4 + (size_t)L * (V + 8) * 2;
+}
+
+// A chunk's weights and results that are not finite, by the whole block; behind the kernel's end, where nothing of it is held in registers
+// (a look at the weights where they are made took 2 us of 50).  `qk`, `state`, `out`: the chunk's and head's first.
+template <int D, int V>
+__device__ __noinline__ void read_again(const float* qk, long long qk_ld, int k_off, const float* state, float* out, long long out_ld, const float* qs,
+                                        float* ps, const float* pw, const __nv_bfloat16* vs, int n) {
+  for (int i = threadIdx.x; i < n * L; i += 2 * V) {
+    const int t = i / L, key = i % L;
+    if (key > t || !not_finite(ps[t * (L + 8) + key])) continue;
+    float x = 0.f;
+#pragma unroll 1
+    for (int d = 0; d < D; d++) x = fmaf(qs[t * (D + 8) + d], qk[key * qk_ld + k_off + d], x);
+    ps[t * (L + 8) + key] = x * pw[t - key];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n * V; i += 2 * V) {
+    const int t = i / V, c = i % V;
+    float* const to = out + t * out_ld + c;
+    if (!not_finite(*to)) continue;
+    float x = 0.f;
+#pragma unroll 1
+    for (int d = 0; d < D; d++) x = fmaf(qs[t * (D + 8) + d], state[d * V + c], x);
+    x *= pw[t + 1];
+#pragma unroll 1
+    for (int s = 0; s <= t; s++) x = fmaf(ps[t * (L + 8) + s], __bfloat162float(vs[s * (V + 8) + c]), x);
+    *to = x;
+  }
 }
 
 template <int D, int V>
@@ -537,14 +586,21 @@ retention_out_mma_kernel(const float* __restrict__ qk, const __nv_bfloat16* __re
 #pragma unroll
       for (int e = 0; e < 4; e++) acc[j][e] += part[j][e];
   }
+  bool again = false;
 #pragma unroll
   for (int e = 0; e < 4; e += 2) {
     const int t = row + e * 4;
     if (t >= n) continue;
     float* to = o_out + (t0 + t) * n_heads * V + (long long)h * V + half * 64 + c2;
 #pragma unroll
-    for (int j = 0; j < 8; j++) *reinterpret_cast<float2*>(to + j * 8) = make_float2(acc[j][e], acc[j][e + 1]);
+    for (int j = 0; j < 8; j++) {
+      *reinterpret_cast<float2*>(to + j * 8) = make_float2(acc[j][e], acc[j][e + 1]);
+      again |= not_finite(acc[j][e]) | not_finite(acc[j][e + 1]);
+    }
   }
+  if (__syncthreads_or(again))
+    read_again<D, V>(qk + t0 * 2 * n_heads * D + (long long)h * D, 2ll * n_heads * D, n_heads * D, from, o_out + t0 * n_heads * V + (long long)h * V,
+                     (long long)n_heads * V, qs, ps, pw, vs, n);
 }
 
 template <typename T, int D, int V>

@@ -656,6 +656,49 @@ def test_retention_chunks_keep_what_is_not_finite_from_earlier_tokens(t, what, d
         assert torch.equal(o[:, vdim:], res[0][:, vdim:])
 
 
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (128, 64), (64, 128), (64, 64)])
+@pytest.mark.parametrize("what,t", [("v", 17), ("v", 150), ("k", 63), ("k", 64), ("q", 299), ("state", 0)])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 3.4e38])
+def test_retention_chunks_of_both_value_types_agree_on_what_is_not_finite(what, t, bad, dim, vdim):
+    """Values that bfloat16 holds, as bfloat16 (products of pieces on the tensor cores) and in 32 bits (IEEE products): with an infinity, a NaN or a
+    number larger than bfloat16's largest in a value, key, query or the first state, the same results are infinite, of the same sign, and the
+    same are no numbers; the rest lie within the two orders' rounding."""
+    import torch
+    from types import SimpleNamespace
+    from mlxforge_b200.csrc import ops
+    rng = np.random.default_rng(dim + vdim + t)
+    T, heads = 300, 2
+    qk = rng.standard_normal((T, 2, heads, dim)).astype(np.float32) * np.float32(dim ** -0.25)
+    qk[:, :, 0] = np.abs(qk[:, :, 0])          # a head whose infinities keep their sign through sums
+    v = torch.from_numpy(rng.standard_normal((T, heads * vdim)).astype(np.float32)).cuda()
+    state = rng.standard_normal((1, heads, dim, vdim)).astype(np.float32)
+    if bad == 3.4e38:              # beside it numbers so small that no order of the sums overflows
+        qk, v, state = (x * 2.0 ** -20 for x in (qk, v, state))
+    for h in range(heads):
+        if what == "v":
+            v[t, h * vdim + 3] = bad if bad != 3.4e38 else 3.38e38          # finite in bfloat16
+        elif what == "state":
+            state[0, h, 5, 3] = bad
+        else:
+            qk[t, int(what == "k"), h, 5] = bad
+    v, i32 = v.bfloat16().float(), lambda a: dev(np.asarray(a, np.int32))
+    batch = SimpleNamespace(q_len=[T], n_seqs=1, seq_q_start=i32([0]), seq_q_len=i32([T]), slots=i32([0]))
+    res = []
+    for dtype in (torch.float32, torch.bfloat16):
+        st, o, vd = dev(state.reshape(1, -1)), torch.full((1, T, heads * vdim), float("nan"), device="cuda"), v.to(dtype)
+        chunks = ops.retention_chunks(batch, heads, dim, vdim, vd, heads * vdim, st)
+        ops.retention_chunked(dev(qk.reshape(T, -1)), vd, heads * vdim, dev(np.array([0.97, 0.5], np.float32)), st, batch, o, heads, dim, vdim,
+                              chunks, torch.empty(chunks * heads * dim * vdim, device="cuda"))
+        res.append((o[0], st.view(heads * dim, vdim)))
+    for a, b in zip(*res):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isposinf(), b.isposinf()) and torch.equal(a.isneginf(), b.isneginf())
+        a, b = (torch.where(x.isfinite(), x, 0).double() for x in (a, b))
+        # either is 2e-6 of a row's norm from 64 bits at most where its terms are of one size; the second number: sums that cancel
+        assert bool(((a - b).norm(dim=1) <= 4e-6 * a.norm(dim=1) + 1e-5).all())
+    if bad == np.inf and what != "q":          # a state of both signs beside it: no numbers
+        assert bool(res[1][0].isposinf().any())
+
+
 def retention_128(rt, rng, hidden=64):
     """Two heads of 128 x 128."""
     return build("MIXERS", "retention", {"hidden_size": hidden, "n_heads": 2, "head_dim": 128, "v_head_dim": 128, "rotary_dim": 128,
