@@ -604,7 +604,7 @@ def test_talking_heads_prompt_kernel(H, page, lens, held, window, chunk, cap, ta
     (16, 90, 1000, 250, 0, 20.0, True), (8, 90, 1000, 250, 0, 0.0, False), (16, 60, 1490, 0, 2048, 0.0, False), (8, 200, 420, 0, 512, 30.0, True)])
 def test_talking_heads_prompt_kernel_keeps_what_is_not_finite_apart(H, lens, held, window, chunk, cap, talking):
     """One number of a key or a value of one key head NaN or infinite, at places over all of a tile of 128 and at the ends of the range: the rows
-    that do not see it keep their bits (of a value up to the own 16 positions and its own channel, as the weights of a tile are one product),
+    that do not see it keep their bits (of a value up to the own 16 rows and its own channel, as the weights of a tile are one product),
     values never pass to another key head's query heads, keys only through a matrix; an infinite key under a cap is what 64 bits say."""
     import torch
     from mlxforge_b200.csrc import binding, ops
@@ -629,6 +629,7 @@ def test_talking_heads_prompt_kernel_keeps_what_is_not_finite_apart(H, lens, hel
 
     pos = torch.arange(held, ctx, device="cuda")
     first = max(0, held - window + 1) if window else held // chunk * chunk if chunk else 0
+    tile = (pos if chunk and held // chunk != (ctx - 1) // chunk else pos - held) // 16          # of 16 positions where chunks meet, else of 16 rows
     at = {first, first + 1, first + 17, held, ctx - 1, ctx - 2, ctx - 17} | {t for t in range(first, ctx, 37)} | {t for t in range(held // 128 * 128, ctx, 64)}
     bits = lambda x: x.view(torch.int16)
     clean, same = run(*pools), lambda a, b: torch.equal(bits(a), bits(b))
@@ -639,7 +640,7 @@ def test_talking_heads_prompt_kernel_keeps_what_is_not_finite_apart(H, lens, hel
         other = [h for h in range(H) if h // 4 != kv]
         sees = (pos >= t) & ((pos - t < window) if window else True) & ((pos // chunk == t // chunk) if chunk else True)
         # rows of a tile that holds a row which sees it
-        near = torch.isin(pos // 16, pos[sees].unique() // 16) & ~sees
+        near = torch.isin(tile, tile[sees]) & ~sees
         for bad in (float("nan"), float("inf"), float("-inf")):
             kp, vp = (x.clone() for x in pools)
             vp[t // page, kv, t % page, 5] = bad
@@ -666,6 +667,34 @@ def test_talking_heads_prompt_kernel_keeps_what_is_not_finite_apart(H, lens, hel
                 want, mag = torch.einsum("hij,jhd->ihd", p, v), torch.einsum("hij,jhd->ihd", p, v.abs())
                 # a probability is rounded to 8 bits once, the result once more
                 assert bool(((out.double() - want).abs() <= 2 ** -8 * mag + 2 ** -8 * want.abs() + 1e-6).all()), (t, bad)
+
+
+@pytest.mark.parametrize("H,window,chunk", [(16, 0, 0), (8, 250, 0), (16, 0, 2048), (8, 0, 512), (16, 0, 500)])
+def test_talking_heads_prompt_kernel_portions_give_the_bits_of_the_whole_prompt(H, window, chunk):
+    """A prompt at once and its tokens from any place on as a portion of their own: tiles of queries then begin elsewhere, reach over a chunk's
+    start or over a cut of the keys, and a row's numbers are the same."""
+    import torch
+    from mlxforge_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(H + window)
+    G, D, bf, T, page = H // 4, 128, torch.bfloat16, 1200, 16
+    q = torch.randn((T, H * D), generator=g, device="cuda").to(bf)
+    talk = torch.eye(H, device="cuda") + 0.1 * torch.randn((H, H), generator=g, device="cuda")
+    kp, vp = (torch.randn((T // page, G, page, D), generator=g, device="cuda").to(bf) for _ in range(2))
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    splits = ops.attention_talking_prefill_splits(min(T, chunk or T, window or T), window, chunk)
+    f = lambda n: torch.full((max(n, 1),), float("nan"), device="cuda")
+
+    def portion(start, end):
+        n = end - start
+        out = torch.full((n, H * D), float("nan"), device="cuda", dtype=bf)
+        ops.attention_talking_tc(q[start:end].contiguous(), kp, vp, out, i32([0]), i32([n]), i32([end]), 0, n, torch.arange(T // page, dtype=torch.int32, device="cuda")[None],
+                                 page, H, G, D, D, D ** -0.5, 30.0, talk, window, chunk, splits, f(n * splits * H * D), f(n * splits * H * 2), 0, end, end)
+        ops.check_kernel_status()
+        return out
+
+    whole = portion(0, T)
+    for start, end in ((1009, 1100), (1023, 1025), (491, 520), (300, 1200), (517, 560), (1, 700), (1003, 1031)):
+        assert torch.equal(portion(start, end), whole[start:end]), (start, end)
 
 
 # ----------------------------------------------------------------------------- latents: rotated query parts
