@@ -295,6 +295,7 @@ enum MfKernel {
   MF_K_RETENTION_STEP,        // retention_recurrence: one token of every sequence
   MF_K_MOE_GROUPED_TC,        // moe_grouped: the tcgen05 products
   MF_K_ATTN_TALKING_PROMPT,   // attn_talking_tc: portions of prompts on tcgen05
+  MF_K_ATTN_TALKING_MMA,      // attn_talking_tc: portions of prompts on mma.sync
   MF_K_MOE_ROWS_MMA,          // moe_rows: a chosen expert's matrices read once for all its tokens
   MF_K_COUNT
 };

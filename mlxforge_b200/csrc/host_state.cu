@@ -20,7 +20,7 @@ const char* const kNames[MF_K_COUNT] = {
     "selective_scan",   "scan_local",       "low_rank",         "post_norm",      "qkv_conv",
     "soft_cap",
     "attn_f32",         "attn_prefill_latent", "attn_talking_decode", "delta_runs",  "delta_step",       "retention_step",
-    "moe_grouped_tc",   "attn_talking_prompt", "moe_rows_mma",
+    "moe_grouped_tc",   "attn_talking_prompt", "attn_talking_mma", "moe_rows_mma",
 };
 int g_sm_count[MF_MAX_DEVICES] = {};
 }  // namespace

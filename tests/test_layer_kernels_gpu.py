@@ -697,6 +697,30 @@ def test_talking_heads_prompt_kernel_portions_give_the_bits_of_the_whole_prompt(
         assert torch.equal(portion(start, end), whole[start:end]), (start, end)
 
 
+@pytest.mark.parametrize("H,dim,ctx,chunk,bounds,prompt,mma,merge", [
+    (16, 128, [300, 90], 0, True, 1, 1, 0), (16, 128, [300, 90], 0, False, 1, 1, 0), (16, 128, [90, 70], 0, True, 0, 1, 0), (8, 128, [90, 300], 0, True, 1, 0, 0),
+    (16, 128, [2048, 90], 2048, True, 1, 1, 1), (16, 128, [2048], 2048, True, 1, 0, 1), (8, 128, [1024], 1024, True, 1, 0, 0), (4, 64, [1100], 1100, True, 0, 1, 1),
+    (4, 64, [90], 0, False, 0, 1, 0)])
+def test_talking_heads_launches_are_counted(H, dim, ctx, chunk, bounds, prompt, mma, merge):
+    """The library's count of launches and of each kernel, whichever of the two the portions go to and whether keys are cut."""
+    import torch
+    from mlxforge_b200.csrc import binding, ops
+    G, bf, page, i32 = H // 4, torch.bfloat16, 16, lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    lens, T = [20] * len(ctx), 20 * len(ctx)
+    q, out = (torch.zeros((T, H * dim), device="cuda", dtype=bf) for _ in range(2))
+    kp = torch.zeros((128, G, page, dim), device="cuda", dtype=bf)
+    table = torch.arange(128, dtype=torch.int32, device="cuda").repeat(len(ctx), 1)
+    splits = ops.attention_talking_prefill_splits(min(max(ctx), chunk or max(ctx)), 0, chunk)
+    part = [torch.empty((max(T * splits * H * n, 1),), device="cuda") for n in (dim, 2)]
+    launches, before = binding.launch_count(), binding.kernel_launches()
+    ops.attention_talking_tc(q, kp, kp, out, i32([20 * i for i in range(len(ctx))]), i32(lens), i32(ctx), 0, 20, table, page, H, G, dim, dim, 1.0, 0.0, None, 0, chunk,
+                             splits, *part, 0, *((min(ctx), max(ctx)) if bounds else (0, 0)))
+    ops.check_kernel_status()
+    ran = _ran(before)
+    assert [ran.get("attn_talking_" + k, 0) for k in ("prompt", "mma", "merge")] == [prompt, mma, merge] and ran["attn_talking_tc"] == 1
+    assert binding.launch_count() - launches == prompt + mma + merge
+
+
 # ----------------------------------------------------------------------------- latents: rotated query parts
 
 @pytest.mark.parametrize("T,heads,dim,rot,rank,rot_dims,pairs,extra", [
