@@ -42,6 +42,8 @@ namespace {
 using namespace tc5;
 
 constexpr int QT = 16, KT = 128, DIM = 128, CUT = 1024, STAGE = 16384, BOX = 16 * 128, SOFT = 8, THREADS = 32 * (SOFT + 4);
+// of 168 registers a thread at launch: 128 x 56 + 256 x 224 = 384 x 168
+constexpr int REGS_LESS = 56, REGS_MORE = 224, REGS_ALL = 128 * REGS_LESS + 32 * SOFT * REGS_MORE;
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct Args {
@@ -184,8 +186,8 @@ talking_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   // are cleared behind the copy.
   __syncthreads();
 
-  // a part of the launch's 168 registers a thread goes to the softmax warps: 128 x 56 + 256 x 224 = 384 x 168
-  if (warp < 4) regs_less<56>();
+  // a part of the launch's registers goes to the softmax warps
+  if (warp < 4) regs_less<REGS_LESS>();
   if (warp == 0 || warp == 2 || warp == 3) {
     // ------------------------------------------------------------ producers: K of tile 0, then K of tile n + 1 and V of tile n, a stage in three each
     int turn = warp == 0 ? 0 : warp - 1;          // stages until this warp's next one
@@ -318,7 +320,7 @@ talking_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     }
     __syncwarp();
   } else if (warp >= 4) {
-    regs_more<224>();
+    regs_more<REGS_MORE>();
     const int st_id = tid - 128;           // among the softmax threads
     for (int i = st_id; i < QT * NH; i += 32 * SOFT) reinterpret_cast<int*>(smem + (m_u - q_u))[i] = ordered(-INFINITY);
     if (MIXED)                        // every number twice
@@ -636,7 +638,10 @@ int launch(const void* k_pool, const void* v_pool, long long pool_rows, const Ar
   if (d < 0) return MF_ERR_BAD_ARG;
   if (!once.done[d]) {
     cudaError_t e = cudaFuncSetAttribute(talking_prompt_kernel<NH, MIXED, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncAttributes built;
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&built, talking_prompt_kernel<NH, MIXED, CAP>);
     if (e != cudaSuccess) return (int)e;
+    if (built.numRegs * THREADS < REGS_ALL) return MF_ERR_BAD_ARG;        // built with fewer, the softmax warps would wait for theirs for good
     once.done[d] = true;
   }
   const dim3 grid((max_q_len + QT - 1 + (a.chunk > 0 ? QT - 1 : 0)) / QT * a.cuts, n_seqs);
