@@ -1,5 +1,6 @@
-// What the kernels on the 5th-generation tensor cores share: bounded waits on barriers in shared memory, tensor copies, descriptors of
-// operands in shared memory, the product itself and the way its results come back.
+// What attention_talking_prompt.cu and gemm_tcgen05.cu share of the 5th-generation tensor cores: barriers in shared memory, tensor copies,
+// descriptors of operands in shared memory, products sent by an elected lane; and how the former waits (with a limit) and reads results
+// back.  The other kernels on these units keep helpers of their own: they send from one lane, where an elected one gained nothing or cost time.
 #pragma once
 #include <cuda.h>
 
@@ -43,10 +44,6 @@ __device__ __forceinline__ bool mbar_peek(uint32_t bar, uint32_t parity) {
       "selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done;
-}
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
-               ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
