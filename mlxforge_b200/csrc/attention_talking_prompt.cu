@@ -24,12 +24,15 @@
 // Keys are cut at multiples of 1024 where a query sees more; a block whose range is one cut writes its result itself, the others their
 // sums for the merge of attention_talking_tc.cu.  Blocks with the most keys first.
 //
-// What bounds it: the instructions of the softmax warps, 1,700 a warp, tile and four queries, and their supply: the loop over tiles is larger
-// than the SM's instruction cache.  16 heads, one prompt of 2,048 tokens in one chunk, with its merge: 215
+// What bounds it: the softmax warps' own chain, two of them a scheduler.  Counters: no pipe is full (issue slots 38 %, special functions 23, FMA 18,
+// integer 19, tensor 9); they wait for fixed latencies, tensor memory and barriers, a tenth of the time for instructions, as a loop over
+// tiles is larger than the SM's instruction cache.  16 heads, one prompt of 2,048 tokens in one chunk, with its merge: 215
 // (mma.sync, tiles of 32 keys) -> 111 us.  Measured on the way, at 113 us: the loop over a product's stages unrolled 122; so, and 1,024 single multiply-adds
 // instead of 512 of pairs 133, with the matrix in the constant bank 130; four groups, a reference that moves only by 2^8 and no scores kept
 // 125, but results 3 % further from 64 bits; cuts of 512 keys 153; products sent inside `if (lane == 0)` left the tile waiting for them
-// (1,000 cycles a stage beside warps that are busy with multiply-adds, 400 as they are sent now).
+// (1,000 cycles a stage beside warps that are busy with multiply-adds, 400 as they are sent now).  Results are 1.4 % further from 64 bits than
+// the other kernel's there (2.004e-3 of their norm, 1.976e-3): nothing is held in fewer bits, but a row's maximum, whose weight of 1 is not
+// rounded, is taken anew every 128 keys instead of 32 and in every cut of 1,024 instead of 512.
 #include <type_traits>
 
 #include "attention_talking_prompt.cuh"
@@ -651,6 +654,8 @@ int launch(const void* k_pool, const void* v_pool, long long pool_rows, const Ar
 
 }  // namespace
 
+// The groupings that configurations use.  Heads of 64 would be half a stage wide and other groupings no 64 columns a key head: they need stages and
+// products of another shape, which are not built.
 bool talking_prompt_takes(int n_heads, int n_kv, int dim, int vdim, const void* q, const void* k_pool, const void* v_pool,
                           long long pool_rows) {
   return (n_heads == 16 || n_heads == 8) && n_heads == 4 * n_kv && dim == DIM && vdim == DIM && pool_rows > 0 &&

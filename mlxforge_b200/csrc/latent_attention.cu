@@ -198,7 +198,7 @@ __global__ void latent_query_kernel(const T* q, long long q_ld, int n_heads, int
 
 // The same in pieces of eight channels, eight tokens a block: an angle is worked out once for all heads of its token (the kernel above works
 // it out in every head, two bytes a load).  2,048 tokens, 16 heads of 64 + 32: 5.6 -> 3.2 us, 8 tokens 2.5 -> 1.4.
-constexpr int LQ_TOKENS = 8, LQ_PAIRS = 128;         // of 16 tokens' worth of shared memory: rotated parts of up to 256 channels
+constexpr int LQ_TOKENS = 8, LQ_PAIRS = 128;         // 8 KB of shared memory: rotated parts of up to 256 channels
 __global__ void __launch_bounds__(256)
 latent_query_vec_kernel(const __nv_bfloat16* q, long long q_ld, int T, int n_heads, int dim, int rot, int rank, const int* positions,
                         const float* __restrict__ inv_f, const double* __restrict__ inv_d, __nv_bfloat16* __restrict__ q_full, int layout,

@@ -15,12 +15,13 @@
 //
 // Why: the recurrence token after token is serial (0.13 us a token), and its blocks, started early beside the tail of
 // the kernel before them, stacked up on the few SMs that had room first.  1,777 tokens of 8 heads of 128 x 128, bfloat16 values: 244 ->
-// 64 us on the CUDA cores (19 + 7 + 35; 850 us before when launches were queued back to back) -> 50 on the tensor cores (12 + 7 + 29), 2,048
-// of 16 heads 485 -> 120 -> 93, 300 tokens 37 -> 33; and a read-out is nearer to 64 bits (1.66e-7 of its norm, 1.81e-7 before, a
+// 64 us on the CUDA cores (19 + 7 + 35; 850 us before when launches were queued back to back) -> 50 on the tensor cores (12 + 7 + 29 and the
+// gaps between them), 2,048 of 16 heads 485 -> 120 -> 95, 300 tokens 37 -> 34; and a read-out is nearer to 64 bits (1.66e-7 of its norm, 1.81e-7 before, a
 // state 1.78e-7, 1.85e-7).  On the CUDA cores the products hold about half of the FMA pipe's rate (counters: the FMA pipe 46 % busy,
 // shared memory's 55 %), in one wave of blocks.  They run 8 x 8 results a thread (4 x 8 where the tile is smaller), because a lane
-// gets four bytes a cycle from shared memory at most.  On the tensor cores the read-outs are bound by 650 mma.sync a warp (13 cycles each and
-// scheduler) where two blocks share an SM.
+// gets four bytes a cycle from shared memory at most.  On the tensor cores 650 mma.sync a warp of the read-outs, 13 cycles each and
+// scheduler in a loop of nothing else, are 60 % of the time of an SM that has two blocks; the rest is what cuts operands into pieces and waits for them
+// (counters: tensor pipe 27 % busy, 36 where two blocks share an SM, issue slots 42 %).
 #include "common.cuh"
 
 namespace {
