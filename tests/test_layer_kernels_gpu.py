@@ -601,7 +601,8 @@ def test_talking_heads_prompt_kernel(H, page, lens, held, window, chunk, cap, ta
 
 @pytest.mark.parametrize("H,lens,held,window,chunk,cap,talking", [
     (16, 300, 0, 0, 0, 30.0, True), (16, 300, 0, 0, 0, 0.0, False), (8, 300, 0, 0, 0, 30.0, False), (8, 331, 5, 0, 0, 0.0, True),
-    (16, 90, 1000, 250, 0, 20.0, True), (8, 90, 1000, 250, 0, 0.0, False), (16, 60, 1490, 0, 2048, 0.0, False), (8, 200, 420, 0, 512, 30.0, True)])
+    (16, 90, 1000, 250, 0, 20.0, True), (8, 90, 1000, 250, 0, 0.0, False), (16, 60, 1490, 0, 2048, 0.0, False), (8, 200, 420, 0, 512, 30.0, True),
+    (16, 31, 1000, 0, 0, 0.0, False)])
 def test_talking_heads_prompt_kernel_keeps_what_is_not_finite_apart(H, lens, held, window, chunk, cap, talking):
     """One number of a key or a value of one key head NaN or infinite, at places over all of a tile of 128 and at the ends of the range: the rows
     that do not see it keep their bits (of a value up to the own 16 rows and its own channel, as the weights of a tile are one product),
