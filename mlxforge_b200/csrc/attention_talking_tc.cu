@@ -869,10 +869,6 @@ static int tt_launch(const TtArgs& a, int n_seqs, int max_q_len, cudaStream_t st
   return tt_launch_as<VDIM, MAXH, 0>(mk, mv, a, n_seqs, max_q_len, stream);
 }
 
-// Kernels that the calling thread's last mf_attention_talking_tc launched: one or both of the portions' kernels, the merge where keys were cut.
-static thread_local int g_last_talking_launches = 0;
-MF_API int mf_attention_talking_tc_launches() { return g_last_talking_launches; }
-
 // The sequences described by the three per-sequence arrays start at row `table_row0` of the
 // block table; q and out are the whole step's [T, n_heads * dim] and [T, n_heads * vdim].
 MF_API int mf_attention_talking_tc(const void* q, const void* k_pool, const void* v_pool, void* out,
@@ -882,7 +878,6 @@ MF_API int mf_attention_talking_tc(const void* q, const void* k_pool, const void
                                    const float* talk, int window, int chunk, int splits, float* part_o, float* part_ml,
                                    int first_row, int n_rows, int min_ctx, int max_ctx, int* status,
                                    cudaStream_t stream) {
-  g_last_talking_launches = 0;
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
   if (!mf_attention_talking_tc_ok(n_heads, n_kv, dim, vdim, page_size) || n_seqs > 65535 || splits < 0 || splits > 65535)
     return MF_ERR_BAD_ARG;
@@ -902,7 +897,7 @@ MF_API int mf_attention_talking_tc(const void* q, const void* k_pool, const void
     rc = talking_prompt_launch(q, k_pool, v_pool, out, seq_q_start, seq_q_len, seq_ctx_len, table_row0, n_seqs, max_q_len, n_heads,
                                block_table, bt_stride, page_size, pool_rows, scale, softcap, talk, window, chunk, cuts,
                                from, part_o, part_ml, status, stream);
-    g_last_talking_launches = cuts > 1 ? 2 : 1;
+    mf_count_own(cuts > 1 ? 2 : 1);
     if (rc == 0 && cuts > 1) rc = tt_merge(part_o, part_ml, out, cuts, n_heads, vdim, first_row, n_rows, stream);
     if (rc != 0 || least >= from) return rc;
     a.below_keys = from, a.splits = splits = 0;          // of the short ones a block walks all keys
@@ -915,7 +910,7 @@ MF_API int mf_attention_talking_tc(const void* q, const void* k_pool, const void
   TT_CASE(96)
   TT_CASE(128)
 #undef TT_CASE
-  g_last_talking_launches += splits > 0 ? 2 : 1;
+  mf_count_own(splits > 0 ? 2 : 1);
   if (rc != 0 || splits == 0) return rc;
   // the rows of the portions are rows first_row .. first_row + n_rows of the step
   return tt_merge(part_o, part_ml, out, splits, n_heads, vdim, first_row, n_rows, stream);

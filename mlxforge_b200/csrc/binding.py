@@ -88,7 +88,6 @@ _SIGNATURES = {
     "mf_attention_talking_tc_ok": [c_int, c_int, c_int, c_int, c_int],
     "mf_attention_talking_tc": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int,
                                 c_int, c_longlong, c_float, c_float, _P, c_int, c_int, c_int, _P, _P, c_int, c_int, c_int, c_int, _P, _P],
-    "mf_attention_talking_tc_launches": [],
     "mf_attention_talking_prefill_splits": [c_int, c_int, c_int],
     "mf_attention_talking_splits": [c_int],
     "mf_attention_talking_decode": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, c_int, c_int,
@@ -180,6 +179,7 @@ def library() -> ctypes.CDLL:
         lib.mf_kernel_name.restype = ctypes.c_char_p
         lib.mf_kernel_launches.argtypes = [c_int]
         lib.mf_kernel_launches.restype = c_longlong
+        lib.mf_own_launches.restype = c_longlong
         lib.mf_mid_rows_scratch.argtypes = [c_int]
         lib.mf_mid_rows_scratch.restype = c_longlong
         lib.mf_delta_runs_scratch.restype = c_longlong
@@ -203,7 +203,8 @@ _LAUNCHES = 0
 def launch_count() -> int:
     """Kernel launches of this library so far in this process (every entry point
     reports how many kernels it launched; graph replays add their kernel nodes)."""
-    return _LAUNCHES
+    own = int(_LIB.mf_own_launches()) if _LIB is not None else 0          # entries that count in the library, so that a call costs nothing
+    return _LAUNCHES + own
 
 
 def count_launches(n: int) -> None:

@@ -301,6 +301,9 @@ enum MfKernel {
 };
 extern unsigned long long g_mf_kernel_launches[MF_K_COUNT];
 inline void mf_count(MfKernel k) { g_mf_kernel_launches[k]++; }
+// Launches of the entries that count them themselves, because the number depends on what they choose (mf_own_launches).
+extern unsigned long long g_mf_own_launches;
+inline void mf_count_own(int n) { __atomic_fetch_add(&g_mf_own_launches, n, __ATOMIC_RELAXED); }
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

@@ -2,7 +2,7 @@
 // count and the table that says which kernels have been launched.
 #include "common.cuh"
 
-unsigned long long g_mf_kernel_launches[MF_K_COUNT] = {};
+unsigned long long g_mf_kernel_launches[MF_K_COUNT] = {}, g_mf_own_launches = 0;
 
 namespace {
 const char* const kNames[MF_K_COUNT] = {
@@ -40,6 +40,7 @@ int mf_sm_count() {
 // in this process (launches recorded into a CUDA graph count once, replays do not).
 MF_API int mf_kernel_kinds() { return MF_K_COUNT; }
 MF_API const char* mf_kernel_name(int id) { return id >= 0 && id < MF_K_COUNT ? kNames[id] : ""; }
+MF_API long long mf_own_launches() { return (long long)__atomic_load_n(&g_mf_own_launches, __ATOMIC_RELAXED); }
 MF_API long long mf_kernel_launches(int id) {
   return id >= 0 && id < MF_K_COUNT ? (long long)g_mf_kernel_launches[id] : -1;
 }

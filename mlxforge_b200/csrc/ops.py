@@ -1350,8 +1350,7 @@ def attention_talking_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Te
                                             block_table.data_ptr(), block_table.shape[1], page_size, k_pool.numel() // dim, scale,
                                             softcap, _ptr(talk), window, chunk, splits, _ptr(part_o), _ptr(part_ml), first_row,
                                             T - first_row, min_ctx, max_ctx, kernel_status(q.device).data_ptr(), _stream()), "attention_talking_tc",
-          launches=0)
-    count_launches(int(library().mf_attention_talking_tc_launches()))
+          launches=0)          # the library counts them: one or both of the portions' kernels, the merge where keys are cut
 
 
 def attention_talking_prefill_splits(max_keys: int, window: int = 0, chunk: int = 0) -> int:
