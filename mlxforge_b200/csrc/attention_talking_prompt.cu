@@ -119,13 +119,14 @@ talking_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   constexpr int G = NH / 4, RING = ring(NH), COLS = 2 * NH * QT;
   constexpr uint32_t O_COL = NH * QT;
   extern __shared__ __align__(1024) unsigned char smem[];
-  // A tile is 16 queries from the portion's first on; of a portion that goes on over the start of a chunk, 16 positions from a multiple of 16 on, so
-  // that none of its tiles has keys of two chunks (where the chunks' size is one too; keys are cut by that).  Always the latter, portions that
-  // begin in between have a tile more: 60 of 30 tokens over 300 others 180 blocks on 148 SMs, 70 us instead of 42, with chunks of 256 42
-  // instead of 24.  Always the former, the straddling tiles walk over both chunks: 2,048 tokens behind 3 others in chunks of 256 41 us instead of 33.
-  // The heaviest blocks first: of the last queries all cuts, then of the queries before them.
-  const int seq = blockIdx.y, q_len = a.seq_q_len[seq], ctx = a.seq_ctx_len[seq];
-  const int lead = a.chunk > 0 && (ctx - 1) / a.chunk * a.chunk > ctx - q_len ? (ctx - q_len) & (QT - 1) : 0;
+  // A tile is 16 positions from a multiple of 16 on: none has one key more than a tile of keys, or keys of two chunks (where the chunks' size is a
+  // multiple too; keys are cut by that).  Short portions that so have a tile more, and stay in their chunk, have their first tile begin with
+  // them: 60 of 30 tokens over 300 others are 120 blocks then and not 180 on 148 SMs, 43 us instead of 70, with chunks of 256 25 instead of 42.  Of
+  // longer ones it is a smaller part and keys that straddle cost as much: 300 tokens over 1,001 others 92 us as it is, 95 from their first on.  The
+  // heaviest blocks first: of the last queries all cuts, then of the queries before them.
+  const int seq = blockIdx.y, q_len = a.seq_q_len[seq], ctx = a.seq_ctx_len[seq], begin = ctx - q_len;
+  int lead = begin & (QT - 1);
+  if (q_len <= 4 * QT && (lead + q_len + QT - 1) / QT > (q_len + QT - 1) / QT && (a.chunk == 0 || begin / a.chunk == (ctx - 1) / a.chunk)) lead = 0;
   const int tile = (lead + q_len + QT - 1) / QT - 1 - (int)blockIdx.x / a.cuts, cut = (int)blockIdx.x % a.cuts;
   if (tile < 0 || q_len == 0) return;
   const int row0 = max(0, tile * QT - lead), rows = min(q_len, tile * QT + QT - lead) - row0;
@@ -647,7 +648,7 @@ int launch(const void* k_pool, const void* v_pool, long long pool_rows, const Ar
     if (built.numRegs * THREADS < REGS_ALL) return MF_ERR_BAD_ARG;        // built with fewer, the softmax warps would wait for theirs for good
     once.done[d] = true;
   }
-  const dim3 grid((max_q_len + QT - 1 + (a.chunk > 0 ? QT - 1 : 0)) / QT * a.cuts, n_seqs);
+  const dim3 grid((max_q_len + 2 * QT - 2) / QT * a.cuts, n_seqs);
   talking_prompt_kernel<NH, MIXED, CAP><<<grid, THREADS, bytes, stream>>>(k, v, k4, v4, a);
   return (int)cudaGetLastError();
 }

@@ -602,7 +602,7 @@ def test_talking_heads_prompt_kernel(H, page, lens, held, window, chunk, cap, ta
 @pytest.mark.parametrize("H,lens,held,window,chunk,cap,talking", [
     (16, 300, 0, 0, 0, 30.0, True), (16, 300, 0, 0, 0, 0.0, False), (8, 300, 0, 0, 0, 30.0, False), (8, 331, 5, 0, 0, 0.0, True),
     (16, 90, 1000, 250, 0, 20.0, True), (8, 90, 1000, 250, 0, 0.0, False), (16, 60, 1490, 0, 2048, 0.0, False), (8, 200, 420, 0, 512, 30.0, True),
-    (16, 31, 1000, 0, 0, 0.0, False)])
+    (16, 31, 1000, 0, 0, 0.0, False), (8, 30, 299, 0, 256, 30.0, True)])
 def test_talking_heads_prompt_kernel_keeps_what_is_not_finite_apart(H, lens, held, window, chunk, cap, talking):
     """One number of a key or a value of one key head NaN or infinite, at places over all of a tile of 128 and at the ends of the range: the rows
     that do not see it keep their bits (of a value up to the own 16 rows and its own channel, as the weights of a tile are one product),
@@ -630,7 +630,8 @@ def test_talking_heads_prompt_kernel_keeps_what_is_not_finite_apart(H, lens, hel
 
     pos = torch.arange(held, ctx, device="cuda")
     first = max(0, held - window + 1) if window else held // chunk * chunk if chunk else 0
-    tile = (pos if chunk and held // chunk != (ctx - 1) // chunk else pos - held) // 16          # of 16 positions where chunks meet, else of 16 rows
+    whole = lens > 64 or -(-(held % 16 + lens) // 16) == -(-lens // 16) or chunk and held // chunk != (ctx - 1) // chunk
+    tile = pos // 16 if whole else (pos - held) // 16          # of positions; of rows where a short portion has fewer so
     at = {first, first + 1, first + 17, held, ctx - 1, ctx - 2, ctx - 17} | {t for t in range(first, ctx, 37)} | {t for t in range(held // 128 * 128, ctx, 64)}
     bits = lambda x: x.view(torch.int16)
     clean, same = run(*pools), lambda a, b: torch.equal(bits(a), bits(b))
@@ -694,7 +695,7 @@ def test_talking_heads_prompt_kernel_portions_give_the_bits_of_the_whole_prompt(
         return out
 
     whole = portion(0, T)
-    for start, end in ((1009, 1100), (1023, 1025), (491, 520), (300, 1200), (517, 560), (1, 700), (1003, 1031)):
+    for start, end in ((1009, 1100), (1023, 1025), (491, 520), (300, 1200), (517, 560), (1, 700), (1003, 1031), (1009, 1025)):
         assert torch.equal(portion(start, end), whole[start:end]), (start, end)
 
 
