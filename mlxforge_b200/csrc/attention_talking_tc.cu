@@ -561,12 +561,10 @@ talking_attention_merge_kernel(const float* __restrict__ part_o, const float* __
   for (int i = 0; i < N; i++) acc[i] = 0.f;
   for (int z = 0; z < splits; z++) {
     const float2 x = ml[(long long)z * H];
-    if (x.x == -INFINITY) {           // no key, a sum of 0; or no key whose score is a number, and then it is none
-      l += x.y;
-      continue;
-    }
-    const float w = tt_exp2(x.x - m);
-    l += x.y * w;
+    const bool none = x.x == -INFINITY;           // no key, a sum of 0; or no key whose score is a number, and then it is none
+    const float w = none ? 1.f : tt_exp2(x.x - m);
+    l = fmaf(x.y, w, l);
+    if (none) continue;
 #pragma unroll
     for (int i = 0; i < N; i++) acc[i] += po[(long long)z * H * VDIM + i] * w;
   }
